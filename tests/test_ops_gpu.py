@@ -711,6 +711,48 @@ def test_sample_topk_topp_with_given_noise(kge, L):
     assert agree >= total - 2, f"{agree}/{total}"
 
 
+@pytest.mark.parametrize("B,V,ld", [(1, 1, 8), (3, 7, 7), (5, 4097, 4101), (2, 50272, 50304), (40, 16385, 16392), (3, 131073, 131073), (150, 2049, 2056),
+                                    (2, 786440, 786440)])
+def test_sample_row_split_over_a_cluster(kge, L, B, V, ld):
+    """Rows shorter than a piece, ragged ends, rows that are not 16-byte aligned, 1 to 8 CTAs per row, and rows too long to be
+    staged in shared memory: the draw with supplied noise is the oracle's rule in float64, where equal logits at the edge of the
+    top-p mass are kept together (a sort keeps some of them), and columns beyond V never win.  fp32 sums of V numbers in any
+    order are within 2^-24 V of each other: rows whose edge is closer to 1 - p than that may go either way."""
+    g = torch.Generator().manual_seed(B * 1000 + V)
+    lg = torch.full((B, ld), 30.0).to(BF)
+    lg[:, :V] = (torch.randn(B, V, generator=g) * 2.5).to(BF)
+    lg[0, V // 2] = -float("inf")
+    if V > 1:
+        lg[B - 1, :V // 2] = lg[B - 1, 0]                          # many equal keys
+    want = [(0.0, 0, 1.0), (0.7, 20, 0.8), (1.0, 0, 0.95), (0.6, 50, 1.0), (1.5, 0, 1.0), (1.0, 3, 0.4)]
+    temp = torch.tensor([want[b % 6][0] for b in range(B)])
+    k = torch.tensor([min(want[b % 6][1], V) for b in range(B)], dtype=torch.int32)
+    pp = torch.tensor([want[b % 6][2] for b in range(B)])
+    q = torch.empty(B, V).exponential_(generator=g)
+    lgd, td, kd, ppd, qd, out = dev(lg), dev(temp), dev(k), dev(pp), dev(q), torch.empty(B, dtype=torch.int32, device="cuda")
+    check_ok(kge, L.kge_sample(p(out), p(lgd), B, V, ld, p(td), p(kd), p(ppd), p(qd), None, 0, None, 0, None), "sample")
+    sync()
+    got = out.cpu().long()
+    assert ((got >= 0) & (got < V)).all()
+    for b in range(B):
+        x = lg[b, :V].double() / (temp[b].double() if temp[b] >= 1e-5 else 1.0)
+        if not torch.isfinite(x).any():
+            continue
+        keep, sure = torch.ones(V, dtype=torch.bool), True
+        if temp[b] >= 1e-5 and 0 < k[b] < V:
+            keep &= x >= x.topk(int(k[b])).values[-1]
+        if temp[b] >= 1e-5 and pp[b] < 1:
+            vals, inv = x.unique(return_inverse=True)
+            share = torch.zeros(len(vals), dtype=torch.float64).index_add_(0, inv[keep], torch.exp(x[keep] - x.max()))
+            cum = share.cumsum(0) / share.sum()
+            over = cum > 1 - pp[b].double()
+            sure = bool(((cum - (1 - pp[b].double())).abs() > 2.0 ** -24 * max(V, 16)).all())
+            keep &= x >= vals[int(over.nonzero()[0])]
+        score = torch.where(keep, torch.exp(x - x.max()) / (1.0 if temp[b] < 1e-5 else q[b].double()), torch.tensor(-1.0, dtype=torch.float64))
+        if sure:       # 1e-5: the fp32 exponential and quotient of the winning score
+            assert keep[got[b]] and score[got[b]] >= score.max() * (1 - 1e-5), (b, got[b], int(score.argmax()))
+
+
 def test_sample_philox_is_deterministic_and_in_support(kge, L):
     g = torch.Generator().manual_seed(2)
     B, V = 4, 2048
