@@ -49,6 +49,7 @@ int kge_device_sm_count(void);
  *   "gemm_wide" 1/0           GEMMs of up to 64 tokens: 1 = where it keeps as many CTAs streaming as the 128-row plan, tiles of
  *                             256 weight rows with the tokens as the MMA's M side and the weights as its N side (a tcgen05.mma
  *                             fed from shared memory costs ~165 cycles whatever its shape, so twice the weight bytes per MMA);
+ *                             (and up to 16 tokens, by size, weights streamed without staging tiles: csrc/gemm_rows.cuh);
  *                             0 = always 128-row tiles with the tokens as N.  C3 decode step 6.54-6.58 vs 6.64-6.71 ms
  *   "attn_persistent" 1/0     decode attention with 64-token KV blocks or larger: 1 = 2 x 148 resident CTAs each take an equal,
  *                             contiguous share of all key tiles of the launch (a (request, kv head) group is cut where shares

@@ -1207,6 +1207,8 @@ static bool plan_wide(int T, int n_out, int K, bool gated, GemmPlan& g) {
   return g.m_tiles * g.splits >= narrow_ctas;
 }
 
+#include "gemm_rows.cuh"
+
 // prefill-sized problems run as CTA pairs (cta_group::2, 256 x 256 MMA tiles)
 static bool gemm_uses_pair(const GemmPlan& g) { return g.tokn == 256 && g.splits == 1 && g.m_tiles >= 2; }
 
@@ -1292,6 +1294,11 @@ extern "C" int KGE_GEMM_NAME(void* y, const void* x, const void* w, const void* 
     use_ws = gq.ws && workspace_bytes >= ws_bytes_of(gq) && ((uintptr_t)workspace & 15) == 0;
   }
   if (!use_ws) {
+    if (use_rows(T, N, K)) {
+      GemmParams p;
+      p.y = (bf16*)y; p.bias = (const bf16*)bias; p.T = T; p.N = N; p.K = K; p.act = act;
+      return launch_rows<false>((const bf16*)x, (const bf16*)w, p, (cudaStream_t)stream);
+    }
     GemmPlan gw;
     if (plan_wide(T, N, K, false, gw)) {
       GemmParams p;
@@ -1336,6 +1343,11 @@ static int gemm_gated(void* y, const void* x, const void* w_gate_up, int T, int 
     use_ws = gq.ws && workspace_bytes >= ws_bytes_of(gq) && ((uintptr_t)workspace & 15) == 0;
   }
   if (!use_ws) {
+    if (use_rows(T, 2 * f, K)) {
+      GemmParams p;
+      p.y = (bf16*)y; p.bias = (const bf16*)bias_gate_up; p.T = T; p.N = f; p.K = K; p.act = 2; p.glu = glu; p.glu_alpha = glu_alpha; p.glu_limit = glu_limit;
+      return launch_rows<true>((const bf16*)x, (const bf16*)w_gate_up, p, (cudaStream_t)stream);
+    }
     GemmPlan gw;
     if (plan_wide(T, f, K, true, gw)) {
       GemmParams p;

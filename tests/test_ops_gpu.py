@@ -300,6 +300,40 @@ def test_gemm_bf16(kge, L, T, N, K, bias, act):
         assert (err / (ref.abs() + 1e-2 * scale)).mean().item() < 3e-3
 
 
+ROWS_CASES = [(1, 5, 8, True, 0), (2, 8, 64, False, 1), (3, 17, 72, True, 3), (7, 768, 3072, True, 0), (8, 1184, 2056, False, 4), (8, 1185, 2048, True, 0),
+              (9, 24, 520, True, 1), (15, 2368, 1032, False, 0), (16, 2369, 4096, True, 0), (16, 768, 2048, False, 0), (1, 32768, 136, True, 0), (5, 4096, 14336, False, 0)]
+
+
+@pytest.mark.parametrize("T,N,K,bias,act", ROWS_CASES)
+@pytest.mark.parametrize("dtype", ["bf16", "f16"])
+def test_gemm_few_rows(kge, L, T, N, K, bias, act, dtype):
+    """Up to 16 tokens without staging tiles: one token half or both, ragged last weight tiles, K that ends inside a piece, fewer
+    chunks of K than warps, 8 and 16 warps per CTA.  One rounding of an fp32 sum: half a unit in the last place of the result plus
+    K roundings of 2^-24 of the largest partial sum."""
+    dt = BF if dtype == "bf16" else torch.float16
+    g = torch.Generator().manual_seed(T * 7 + N * 3 + K)
+    x, w = torch.randn(T, K, generator=g).to(dt), (torch.randn(N, K, generator=g) * 0.05).to(dt)
+    b = torch.randn(N, generator=g).to(dt) if bias else None
+    xd, wd, bd = dev(x), dev(w), dev(b) if bias else None
+    y = torch.full((T + 1, N), float("nan"), dtype=dt, device="cuda")
+    fn = L.kge_gemm_bf16 if dtype == "bf16" else L.kge_gemm_f16
+    check_ok(kge, fn(p(y), p(xd), p(wd), p(bd), T, N, K, act, None, 0, None), "gemm")
+    sync()
+    ref = x.double() @ w.double().T + (b.double() if bias else 0)
+    size = x.double().abs() @ w.double().abs().T
+    ref = {0: ref, 1: ref.relu(), 3: torch.nn.functional.gelu(ref), 4: ref.relu() ** 2}[act]
+    slope = 1.2 if act != 4 else 2 * ref.sqrt() + 1e-3
+    ulp = 2.0 ** -8 if dtype == "bf16" else 2.0 ** -11
+    err = (y[:T].cpu().double() - ref).abs()
+    assert (err <= ulp * ref.abs() + slope * K * 2.0 ** -24 * size + 1e-7).all(), err.max().item()
+    assert torch.isnan(y[T]).all()
+
+
+@pytest.mark.parametrize("T,f,K", [(1, 64, 8), (4, 192, 1096), (8, 14336, 4096), (9, 128, 2048), (16, 2048, 4096)])
+def test_gemm_silu_gate_few_rows(kge, L, T, f, K):
+    test_gemm_silu_gate_fused(kge, L, T, f, K)
+
+
 @pytest.mark.parametrize("T,N,K,bias,act", [c for c in GEMM_CASES if c[0] <= 64])
 def test_gemm_128_row_tiles_for_small_batches(kge, L, T, N, K, bias, act):
     """Knob gemm_wide=0: batches of up to 64 tokens through the 128-row weight tiles (tokens as MMA N) instead of the
