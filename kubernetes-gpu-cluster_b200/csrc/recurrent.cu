@@ -514,6 +514,383 @@ __global__ void __launch_bounds__(MC_COLS * ML_NSL) mlstm_chunk_kernel(MlstmArgs
   }
 }
 
+// The same chunkwise form for bfloat16 operands on mma.sync tensor cores, 64 tokens at a time.  Block = one (request, head) and
+// 32 value columns; the columns of C stay in fp32 accumulators of the eight warps (16 key dimensions each) from the first chunk
+// to the last.  q, k and v are bfloat16 already; what is fp32 (C, the weighted scores, the weighted values) enters a product as
+// three bfloat16 terms that add up to its 24 bits, so every product is exact to fp32 and sums are fp32; a chunk's update is
+// summed by itself and then joined to C by one fma.  A chunk costs four barriers and ~250 MMAs per warp; the next chunk's
+// rows arrive by cp.async meanwhile.
+// What bounds it: the chain of chunks (2 requests x 4 heads x 8 column blocks = 64 blocks), not throughput: 7 us a chunk.
+// Prompts of 1150 and 1162 tokens, 4 heads of 128 x 256: 151 us (the fp32 kernel above 1101), error against 64 bits 1.0e-6 of
+// the read-out and 2.5e-7 of the state (1.5e-6 and 5.0e-7); one prompt of 1300 with a state before it: 159 us (1223), 6.6e-7
+// and 1.1e-7 (7.5e-7 and 2.3e-7).
+// A request with one row of the step takes a plain path on the same block (fp32, one pass over its columns).
+constexpr int MM_CH = 64, MM_COLS = 32, MM_THREADS = 256, MM_LDQ = 128 + 8, MM_LDV = MM_COLS + 8;
+struct MlstmTile {
+  __nv_bfloat16 q[2][MM_CH][MM_LDQ], k[2][MM_CH][MM_LDQ], v[2][MM_CH][MM_LDV];
+  __nv_bfloat16 x[3][MM_CH][MM_LDV];            // u_s v_s in three terms
+  __nv_bfloat16 c[3][128][MM_LDV];              // C before the chunk in three terms
+  float out[MM_CH][MM_COLS + 2], rows[MM_CH];   // the second key half's part of the read-out and of the weights' sum
+  float nv[128], nsum[2][128], nq[MM_CH];
+  float2 e[MM_CH], M[MM_CH];                    // i_s - b_s and m_t - b_t, each as a sum of two
+  float floor_[MM_CH], us[MM_CH], gt[MM_CH];    // e^(-m_t); weights of the tokens and of C in the new state
+  float G;
+};
+
+__device__ __forceinline__ void ml_mma(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ void ml_ldsm(uint32_t (&r)[4], const void* p) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"((uint32_t)__cvta_generic_to_shared(p)) : "memory");
+}
+__device__ __forceinline__ void ml_ldsm_t(uint32_t (&r)[4], const void* p) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"((uint32_t)__cvta_generic_to_shared(p)) : "memory");
+}
+// (lo, hi) as three packed pairs of bfloat16 whose sums are the fp32 values
+__device__ __forceinline__ void ml_split(float lo, float hi, uint32_t (&t)[3]) {
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    t[i] = pack_bf2(lo, hi);
+    lo -= bf_lo(t[i]); hi -= bf_hi(t[i]);
+  }
+}
+
+__global__ void __launch_bounds__(MM_THREADS) mlstm_mma_kernel(MlstmArgs a) {
+  pdl_launch_dependents();
+  pdl_wait();
+  typedef __nv_bfloat16 E;
+  extern __shared__ __align__(16) unsigned char mm_raw[];
+  MlstmTile& sm = *reinterpret_cast<MlstmTile*>(mm_raw);
+  const int b = blockIdx.x, h = blockIdx.y, c0 = blockIdx.z * MM_COLS, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t4 = lane & 3;
+  const int dim = a.dim, vdim = a.vdim, H = a.H;
+  const int rs = a.qsl[b], re = a.qsl[b + 1];
+  if (re <= rs) return;
+  const int p0 = a.positions[rs];
+  float* slot = a.state + (int64_t)a.slots[b] * a.slot_stride + (int64_t)h * ((int64_t)dim * vdim + dim + 1);
+  const bool fresh = p0 == 0;
+  const E *qp = (const E*)a.q + h * dim, *kp = (const E*)a.k + h * dim, *vp = (const E*)a.v + h * vdim + c0;
+  const int ncol = min(MM_COLS, vdim - c0);
+  const float m0 = fresh ? 0.f : slot[(int64_t)dim * vdim + dim];
+  for (int d = tid; d < 128; d += MM_THREADS) sm.nv[d] = d < dim && !fresh ? slot[(int64_t)dim * vdim + d] : 0.f;
+  // the blocks of a head form a cluster: the one that writes n and m back waits until all have read them
+  __syncthreads();
+  asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+
+  if (re - rs == 1) {
+    // one token: thread = (column, eighth of the key dimensions)
+    const int col = lane, per = (dim + 7) / 8, d0 = warp * per, d1 = min(dim, d0 + per);
+    const float it = a.gates[(int64_t)rs * 2 * H + h], ft = a.gates[(int64_t)rs * 2 * H + H + h];
+    const float mn = fmaxf(ft + m0, it), fa = expf(ft + m0 - mn), ia = expf(it - mn);
+    float* qs = &sm.out[0][0]; float* ks = qs + 128;
+    for (int d = tid; d < dim; d += MM_THREADS) { qs[d] = ldf(qp + (int64_t)rs * a.ld + d) * a.q_scale; ks[d] = ldf(kp + (int64_t)rs * a.ld + d); }
+    const float vv = col < ncol ? ia * ldf(vp + (int64_t)rs * a.ld + col) : 0.f;
+    __syncthreads();
+    float num = 0.f;
+    if (col < ncol)
+#pragma unroll 8
+      for (int d = d0; d < d1; ++d) {
+        float* s = slot + (int64_t)d * vdim + c0 + col;
+        const float n = fmaf(fa, fresh ? 0.f : *s, ks[d] * vv);
+        *s = n;
+        num = fmaf(n, qs[d], num);
+      }
+    float* part = &sm.out[16][0];                              // [8][32]
+    part[warp * 32 + col] = num;
+    float np = 0.f;
+    for (int d = tid; d < dim; d += MM_THREADS) {
+      const float n = fmaf(fa, sm.nv[d], ia * ks[d]);
+      sm.nv[d] = n;
+      np = fmaf(n, qs[d], np);
+    }
+    np = warp_sum(np);
+    if (lane == 0) sm.nq[warp] = np;
+    __syncthreads();
+    if (warp == 0 && col < ncol) {
+      float o = 0.f, nq = 0.f;
+#pragma unroll
+      for (int w = 0; w < 8; ++w) { o += part[w * 32 + col]; nq += sm.nq[w]; }
+      a.o_scratch[(int64_t)rs * H * vdim + h * vdim + c0 + col] = o / (fmaxf(fabsf(nq), expf(-mn)) + a.den_eps);
+    }
+    asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+    if (blockIdx.z == 0) {
+      for (int d = tid; d < dim; d += MM_THREADS) slot[(int64_t)dim * vdim + d] = sm.nv[d];
+      if (tid == 0) slot[(int64_t)dim * vdim + dim] = mn;
+    }
+    return;
+  }
+
+  const int mt0 = warp * 16;                                   // this warp's key dimensions of C
+  const bool has_c = mt0 < dim;
+  float C[MM_COLS / 8][4];
+  auto write_terms = [&]() {
+#pragma unroll
+    for (int n = 0; n < MM_COLS / 8; ++n)
+#pragma unroll
+      for (int r = 0; r < 2; ++r) {
+        uint32_t t[3];
+        ml_split(C[n][2 * r], C[n][2 * r + 1], t);
+#pragma unroll
+        for (int i = 0; i < 3; ++i) *reinterpret_cast<uint32_t*>(&sm.c[i][mt0 + g + 8 * r][n * 8 + t4 * 2]) = t[i];
+      }
+  };
+#pragma unroll
+  for (int n = 0; n < MM_COLS / 8; ++n)
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int d = mt0 + g + 8 * (q >> 1), col = n * 8 + t4 * 2 + (q & 1);
+      C[n][q] = d < dim && col < ncol && !fresh ? slot[(int64_t)d * vdim + c0 + col] : 0.f;
+    }
+  write_terms();
+
+  // rows of 64 tokens: q and k in 16-byte pieces (dim / 8 per row), v likewise (the host checked the alignment)
+  const int pieces = dim / 8;
+  auto copy16 = [&](void* dst, const E* src, bool in) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(in ? src : qp), "r"(in ? 16u : 0u) : "memory");
+  };
+  auto fetch = [&](int t0, int st) {
+    for (int i = tid; i < MM_CH * pieces; i += MM_THREADS) {
+      const int r = i / pieces, c = (i - r * pieces) * 8;
+      const bool in = t0 + r < re;
+      copy16(&sm.q[st][r][c], qp + (int64_t)(t0 + r) * a.ld + c, in);
+      copy16(&sm.k[st][r][c], kp + (int64_t)(t0 + r) * a.ld + c, in);
+    }
+    const int r = tid >> 2, c = (tid & 3) * 8;
+    copy16(&sm.v[st][r][c], vp + (int64_t)(t0 + r) * a.ld + c, t0 + r < re && c < ncol);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  const int rg = (warp & 3) * 16, half = warp >> 2;            // this warp's 16 tokens; its half of the keys / key dimensions
+  const int ksteps = dim / 16, kh = (ksteps + 1) / 2, k_begin = half ? kh : 0, k_end = half ? ksteps : kh;
+  double m = m0;                                               // (warp 0) the running maximum before the chunk
+  fetch(rs, 0);
+  int st = 0;
+  for (int t0 = rs; t0 < re; t0 += MM_CH, st ^= 1) {
+    // the gate scalars of the chunk, two tokens per lane of the first warp: with e_s = i_s - b_s and M_t = max(m, max_{s<=t} e_s),
+    // m_t = b_t + M_t, and the weights above are e^(m - M_t) and e^(e_s - M_t)
+    float it[2], ft[2];
+    if (warp == 0) {
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        const int t = t0 + 2 * lane + j;
+        it[j] = t < re ? a.gates[(int64_t)t * 2 * H + h] : -INFINITY;
+        ft[j] = t < re ? a.gates[(int64_t)t * 2 * H + H + h] : 0.f;
+      }
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();                                           // the chunk's rows and C's terms are there; the other stage is free
+    if (t0 + MM_CH < re) fetch(t0 + MM_CH, st ^ 1);
+    if (warp == 0) {
+      // running sums in 64 bits: b_t grows with the chunk, and what the weights need are differences
+      const double pair = (double)ft[0] + (double)ft[1];
+      double run = pair;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) { const double v = __shfl_up_sync(0xffffffffu, run, o); if (lane >= o) run += v; }
+      const double b1 = run, b0 = run - pair + (double)ft[0];
+      const double e0 = (double)it[0] - b0, e1 = (double)it[1] - b1;
+      double mx = fmax(e0, e1);
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) { const double v = __shfl_up_sync(0xffffffffu, mx, o); if (lane >= o) mx = fmax(mx, v); }
+      double before = __shfl_up_sync(0xffffffffu, mx, 1);
+      before = lane == 0 ? m : fmax(before, m);
+      const double M0 = fmax(before, e0), M1 = fmax(M0, e1);
+      const double bL = __shfl_sync(0xffffffffu, b1, 31), ML = __shfl_sync(0xffffffffu, M1, 31);
+      const int i0 = 2 * lane, i1 = i0 + 1;
+      auto two = [](double v) { const float hi = (float)v; return make_float2(hi, hi == -INFINITY ? 0.f : (float)(v - (double)hi)); };
+      sm.e[i0] = two(e0); sm.e[i1] = two(e1); sm.M[i0] = two(M0); sm.M[i1] = two(M1);
+      sm.floor_[i0] = expf(-(float)(b0 + M0)); sm.floor_[i1] = expf(-(float)(b1 + M1));
+      sm.us[i0] = expf((float)(e0 - ML)); sm.us[i1] = expf((float)(e1 - ML));
+      sm.gt[i0] = expf((float)(m - M0)); sm.gt[i1] = expf((float)(m - M1));
+      if (lane == 0) sm.G = expf((float)(m - ML));
+      m = bL + ML;
+    }
+    // q_t . k_s for this warp's tokens and its half of the keys (none where all keys lie behind the tokens)
+    const bool keys = half * 32 <= rg + 15;
+    float sc[4][4];
+#pragma unroll
+    for (int n = 0; n < 4; ++n) sc[n][0] = sc[n][1] = sc[n][2] = sc[n][3] = 0.f;
+    float in[MM_COLS / 8][4], ia[MM_COLS / 8][4];              // state part and chunk part of the read-out
+#pragma unroll
+    for (int n = 0; n < MM_COLS / 8; ++n)
+#pragma unroll
+      for (int q = 0; q < 4; ++q) in[n][q] = ia[n][q] = 0.f;
+    for (int k = 0; k < ksteps; ++k) {
+      uint32_t af[4];
+      const bool mine = k >= k_begin && k < k_end;
+      if (!keys && !mine) continue;
+      ml_ldsm(af, &sm.q[st][rg + (lane & 15)][k * 16 + (lane >> 4) * 8]);
+      if (keys)
+#pragma unroll
+        for (int n2 = 0; n2 < 2; ++n2) {
+          uint32_t bf[4];
+          ml_ldsm(bf, &sm.k[st][half * 32 + n2 * 16 + (lane & 7) + ((lane >> 4) & 1) * 8][k * 16 + ((lane >> 3) & 1) * 8]);
+          // each step's sums start from zero and join by a rounded addition: the tensor core's own accumulation truncates, and a
+          // token whose normaliser cancels shows it
+          float s0[4] = {0.f, 0.f, 0.f, 0.f}, s1[4] = {0.f, 0.f, 0.f, 0.f};
+          ml_mma(s0, af, bf[0], bf[1]);
+          ml_mma(s1, af, bf[2], bf[3]);
+#pragma unroll
+          for (int q = 0; q < 4; ++q) { sc[2 * n2][q] += s0[q]; sc[2 * n2 + 1][q] += s1[q]; }
+        }
+      if (mine)                                                // C^T q_t over this warp's half of the key dimensions
+#pragma unroll
+        for (int i = 0; i < 3; ++i)
+#pragma unroll
+          for (int n2 = 0; n2 < MM_COLS / 16; ++n2) {
+            uint32_t bf[4];
+            ml_ldsm_t(bf, &sm.c[i][k * 16 + (lane & 7) + ((lane >> 3) & 1) * 8][n2 * 16 + (lane >> 4) * 8]);
+            ml_mma(in[2 * n2], af, bf[0], bf[1]);
+            ml_mma(in[2 * n2 + 1], af, bf[2], bf[3]);
+          }
+    }
+    {
+      // n . q_t, four threads per token
+      const int tok = tid >> 2;
+      float acc = 0.f;
+      for (int d = (tid & 3) * 2; d < dim; d += 8) {
+        const uint32_t u = *reinterpret_cast<const uint32_t*>(&sm.q[st][tok][d]);
+        acc = fmaf(sm.nv[d], bf_lo(u), acc); acc = fmaf(sm.nv[d + 1], bf_hi(u), acc);
+      }
+      acc += __shfl_xor_sync(0xffffffffu, acc, 1);
+      acc += __shfl_xor_sync(0xffffffffu, acc, 2);
+      if ((tid & 3) == 0) sm.nq[tok] = acc * a.q_scale;
+    }
+    __syncthreads();                                           // the gate scalars are there
+    {
+      // the tokens' weighted values, in three terms, and their keys' weighted sum
+      const int r = tid >> 2, c = (tid & 3) * 8;
+      const float u = sm.us[r];
+      const uint4 v = *reinterpret_cast<const uint4*>(&sm.v[st][r][c]);
+      const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+      uint32_t o[3][4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        uint32_t t[3];
+        ml_split(u * bf_lo(w[j]), u * bf_hi(w[j]), t);
+        o[0][j] = t[0]; o[1][j] = t[1]; o[2][j] = t[2];
+      }
+#pragma unroll
+      for (int i = 0; i < 3; ++i) *reinterpret_cast<uint4*>(&sm.x[i][r][c]) = make_uint4(o[i][0], o[i][1], o[i][2], o[i][3]);
+      const int d = tid & 127, s0 = (tid >> 7) * 32;
+      float acc = 0.f;
+      if (d < dim)
+#pragma unroll 8
+        for (int s2 = s0; s2 < s0 + 32; ++s2) acc = fmaf(sm.us[s2], __bfloat162float(sm.k[st][s2][d]), acc);
+      sm.nsum[tid >> 7][d] = acc;
+    }
+    float rowsum[2] = {0.f, 0.f};
+    if (keys) {
+      uint32_t wt[2][3][4];                                    // weights as A fragments, [16 keys][term]
+#pragma unroll
+      for (int n = 0; n < 4; ++n)
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+          const int tok = rg + g + 8 * r, key = half * 32 + n * 8 + t4 * 2;
+          const float2 M = sm.M[tok];
+          float w[2];
+#pragma unroll
+          for (int j = 0; j < 2; ++j) {
+            const float2 e = sm.e[key + j];
+            w[j] = key + j <= tok ? expf((e.x - M.x) + (e.y - M.y)) * (sc[n][2 * r + j] * a.q_scale) : 0.f;
+            rowsum[r] += w[j];
+          }
+          uint32_t t[3];
+          ml_split(w[0], w[1], t);
+#pragma unroll
+          for (int i = 0; i < 3; ++i) wt[n >> 1][i][(n & 1) * 2 + r] = t[i];
+        }
+#pragma unroll
+      for (int k = 0; k < 2; ++k)
+#pragma unroll
+        for (int n2 = 0; n2 < MM_COLS / 16; ++n2) {
+          uint32_t bf[4];
+          ml_ldsm_t(bf, &sm.v[st][half * 32 + k * 16 + (lane & 7) + ((lane >> 3) & 1) * 8][n2 * 16 + (lane >> 4) * 8]);
+#pragma unroll
+          for (int i = 0; i < 3; ++i) {
+            ml_mma(ia[2 * n2], wt[k][i], bf[0], bf[1]);
+            ml_mma(ia[2 * n2 + 1], wt[k][i], bf[2], bf[3]);
+          }
+        }
+    }
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+      rowsum[r] += __shfl_xor_sync(0xffffffffu, rowsum[r], 1);
+      rowsum[r] += __shfl_xor_sync(0xffffffffu, rowsum[r], 2);
+    }
+    float num[MM_COLS / 8][4];
+#pragma unroll
+    for (int n = 0; n < MM_COLS / 8; ++n)
+#pragma unroll
+      for (int q = 0; q < 4; ++q) num[n][q] = fmaf(sm.gt[rg + g + 8 * (q >> 1)], in[n][q] * a.q_scale, ia[n][q]);
+    if (half) {
+#pragma unroll
+      for (int n = 0; n < MM_COLS / 8; ++n)
+#pragma unroll
+        for (int r = 0; r < 2; ++r)
+          *reinterpret_cast<float2*>(&sm.out[rg + g + 8 * r][n * 8 + t4 * 2]) = make_float2(num[n][2 * r], num[n][2 * r + 1]);
+      if (t4 == 0) { sm.rows[rg + g] = rowsum[0]; sm.rows[rg + g + 8] = rowsum[1]; }
+    }
+    __syncthreads();                                           // all have read C's terms; x, the sums and the halves are there
+    if (!half) {
+#pragma unroll
+      for (int r = 0; r < 2; ++r) {
+        const int tok = rg + g + 8 * r, t = t0 + tok;
+        if (t < re) {
+          const float den = fmaxf(fabsf(fmaf(sm.gt[tok], sm.nq[tok], rowsum[r] + sm.rows[tok])), sm.floor_[tok]) + a.den_eps;
+          float* o = a.o_scratch + (int64_t)t * H * vdim + h * vdim + c0;
+#pragma unroll
+          for (int n = 0; n < MM_COLS / 8; ++n) {
+            const float2 o2 = *reinterpret_cast<const float2*>(&sm.out[tok][n * 8 + t4 * 2]);
+            const int col = n * 8 + t4 * 2;
+            if (col < ncol) o[col] = (num[n][2 * r] + o2.x) / den;
+            if (col + 1 < ncol) o[col + 1] = (num[n][2 * r + 1] + o2.y) / den;
+          }
+        }
+      }
+    }
+    // C' = G C + k^T x
+    const float G = sm.G;
+    if (has_c) {
+      float D[MM_COLS / 8][4];
+#pragma unroll
+      for (int n = 0; n < MM_COLS / 8; ++n) D[n][0] = D[n][1] = D[n][2] = D[n][3] = 0.f;
+#pragma unroll
+      for (int k = 0; k < MM_CH / 16; ++k) {
+        uint32_t af[4];
+        ml_ldsm_t(af, &sm.k[st][k * 16 + (lane & 7) + (lane >> 4) * 8][mt0 + ((lane >> 3) & 1) * 8]);
+#pragma unroll
+        for (int i = 0; i < 3; ++i)
+#pragma unroll
+          for (int n2 = 0; n2 < MM_COLS / 16; ++n2) {
+            uint32_t bf[4];
+            ml_ldsm_t(bf, &sm.x[i][k * 16 + (lane & 7) + ((lane >> 3) & 1) * 8][n2 * 16 + (lane >> 4) * 8]);
+            ml_mma(D[2 * n2], af, bf[0], bf[1]);
+            ml_mma(D[2 * n2 + 1], af, bf[2], bf[3]);
+          }
+      }
+#pragma unroll
+      for (int n = 0; n < MM_COLS / 8; ++n)
+#pragma unroll
+        for (int q = 0; q < 4; ++q) C[n][q] = fmaf(G, C[n][q], D[n][q]);
+      write_terms();
+    }
+    if (tid < 128) sm.nv[tid] = fmaf(G, sm.nv[tid], sm.nsum[0][tid] + sm.nsum[1][tid]);
+  }
+  if (has_c) {
+#pragma unroll
+    for (int n = 0; n < MM_COLS / 8; ++n)
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const int d = mt0 + g + 8 * (q >> 1), col = n * 8 + t4 * 2 + (q & 1);
+        if (col < ncol) slot[(int64_t)d * vdim + c0 + col] = C[n][q];
+      }
+  }
+  asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+  if (blockIdx.z == 0) {
+    if (tid < dim) slot[(int64_t)dim * vdim + tid] = sm.nv[tid];           // its own entry of the last update
+    if (tid == 0) slot[(int64_t)dim * vdim + dim] = (float)m;
+  }
+}
+
 template <typename E>
 __global__ void mlstm_norm_gate_kernel(MlstmArgs a) {
   pdl_launch_dependents();
@@ -539,6 +916,24 @@ int mlstm_step(const MlstmArgs& a, cudaStream_t st) {
     KGE_CUDA_OK(launch_pdl(mlstm_log_gates_kernel, dim3((a.T * 2 * a.H + 255) / 256), dim3(256), 0, st, const_cast<float*>(a.gates), a.T, a.H, a.cap));
     const size_t csm_bytes = ((size_t)2 * ML_CH * a.dim + ML_CH * ML_CH + ML_MAXD + 5 * ML_CH + (1 + ML_NSL) * ML_CH * MC_COLS) * 4;
     const dim3 cgrid(a.B, a.H, (a.vdim + MC_COLS - 1) / MC_COLS);
+    // tensor-core chunks: bfloat16 rows in 16-byte pieces, key dimensions in steps of 16, a head's column blocks in one cluster
+    const bool mma_ok = a.elt == KGE_ELT_BF16 && a.dim % 16 == 0 && a.vdim % 8 == 0 && a.vdim <= 8 * MM_COLS && a.ld % 8 == 0 &&
+                        ((reinterpret_cast<uintptr_t>(a.q) | reinterpret_cast<uintptr_t>(a.k) | reinterpret_cast<uintptr_t>(a.v)) & 15) == 0;
+    if (a.T > a.B && mma_ok) {
+      KGE_CUDA_OK(cudaFuncSetAttribute(mlstm_mma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(MlstmTile)));
+      prefer_max_shared(mlstm_mma_kernel);
+      cudaLaunchConfig_t cfg = {};
+      cfg.gridDim = dim3(a.B, a.H, (a.vdim + MM_COLS - 1) / MM_COLS); cfg.blockDim = dim3(MM_THREADS); cfg.dynamicSmemBytes = sizeof(MlstmTile); cfg.stream = st;
+      cudaLaunchAttribute attr[2];
+      attr[0].id = cudaLaunchAttributeClusterDimension;
+      attr[0].val.clusterDim.x = 1; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = cfg.gridDim.z;
+      attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+      attr[1].val.programmaticStreamSerializationAllowed = 1;
+      cfg.attrs = attr; cfg.numAttrs = pdl_for_this_launch() ? 2 : 1;
+      KGE_CUDA_OK(cudaLaunchKernelEx(&cfg, mlstm_mma_kernel, a));
+      KGE_CUDA_OK(launch_pdl(mlstm_norm_gate_kernel<__nv_bfloat16>, g2, dim3(nt), 0, st, a));
+      return 0;
+    }
     if (a.T > a.B) {
       // some request brings several rows: 32 tokens at a time (single-token requests of the same step are chunks of one)
       static bool smem_set = false;

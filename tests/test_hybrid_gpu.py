@@ -66,6 +66,43 @@ def test_mechanism_alone(kge, tmp_path, mech, dtype):
     check(got, oh.forward(cfg, W, toks), dtype, mech)
 
 
+@pytest.mark.parametrize("m_dim,m_vdim", [(16, 8), (64, 40), (128, 256)])
+def test_matrix_memory_in_chunks_of_64(kge, tmp_path, m_dim, m_vdim):
+    """bfloat16 head sizes that take the tensor-core chunks: pieces that end before, at and behind a chunk's edge, single tokens
+    among them, with and without a state from before; then many single-token requests beside a prompt, whose column blocks start
+    at different times and must all read the normaliser as it was.  A row whose normaliser cancels amplifies the rounding of the
+    bfloat16 projections; it does so alike when the same tokens come one by one (fp32 recurrence), so a row may be off by three
+    times what it is there, beside the bound of rows that do not cancel."""
+    cfg = oh.make_config(layers=("parallel",), mlps=(None,), left_scale=0.0, m_dim=m_dim, m_vdim=m_vdim)
+    W = oh.make_weights(cfg, seed=13)
+    toks = prompt(cfg, 150)
+    want = oh.forward(cfg, W, toks).numpy()
+    llm = make_engine(kge, tmp_path, cfg, W, "bfloat16", tokens=2048, seqs=48)
+    size = np.sqrt((want ** 2).mean())
+
+    def off(got, rows):
+        return np.sqrt(((got - want[rows]) ** 2).mean(-1)) / size
+    singly = off(run_pieces(llm, 99, toks, [1] * 150), slice(None))
+    llm.trace_end(99)
+    assert np.median(singly) < 1e-2
+
+    def close(got, rows, what):
+        assert (off(got, rows) <= 3 * singly[rows] + 2e-2).all(), (what, off(got, rows).max())
+    for rid, pieces in enumerate([[150], [63, 64, 23], [64, 65, 1, 20], [1, 2, 127, 20]]):
+        close(run_pieces(llm, rid, toks, pieces), slice(None), pieces)
+        llm.trace_end(rid)
+    n = 40
+    for rid in range(n):
+        llm.trace_add(rid, toks[:3 + rid % 5])
+        llm.trace_step([(rid, 3 + rid % 5, [])])
+    for rid in range(n):
+        llm.trace_add(rid, [toks[3 + rid % 5]])
+    llm.trace_add(n, toks[:70])
+    got = llm.trace_step([(rid, 1, [0]) for rid in range(n)] + [(n, 70, [69])])
+    close(got, [3 + rid % 5 for rid in range(n)] + [69], "mixed step")
+    llm.close()
+
+
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 def test_prefill_decode_and_pieces_agree_with_the_oracle(kge, tmp_path, dtype):
     cfg = oh.make_config(**FULL, chunk=24)
