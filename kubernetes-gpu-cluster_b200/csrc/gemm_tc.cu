@@ -97,6 +97,25 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
+// 16 TMEM lanes x 8 G columns as MMA accumulator fragments: register 4 k + i holds lane (l / 4) + 8 (i / 2), column 8 k + 2 (l % 4) + i % 2.
+// The caller waits (tmem_wait_ld).
+template <int G>
+__device__ __forceinline__ void tmem_ld_frag(uint32_t taddr, uint32_t (&r)[4 * G]) {
+  static_assert(G == 2 || G == 4, "");
+  if constexpr (G == 4)
+    asm volatile("tcgen05.ld.sync.aligned.16x256b.x4.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+                   "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+                 : "r"(taddr));
+  else
+    asm volatile("tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]) : "r"(taddr));
+}
+__device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+__device__ __forceinline__ void stsm_trans(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+  asm volatile("stmatrix.sync.aligned.m8n8.x4.trans.shared.b16 [%0], {%1,%2,%3,%4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
+}
+
 // K-major, 128B-swizzled operand tile (rows of 128 B, 8-row atoms 1024 B apart).
 __device__ __forceinline__ uint64_t umma_desc_sw128(uint32_t saddr) {
   uint64_t d = (uint64_t)((saddr & 0x3FFFFu) >> 4);
@@ -165,13 +184,8 @@ __device__ __forceinline__ float4 lds_f4(uint32_t addr) {
 // exchange buffer of the split variant: [src rank][local column][128 rows] fp32
 __host__ __device__ constexpr int xbuf_bytes(int tokn) { return (tokn + 8) * BLK_M * 4; }
 
-// GATED: the 128 MMA rows of a tile are 64 gate rows (TMEM lanes 0-63) and the matching 64 up rows
-// (lanes 64-127) of a stacked [2f, K] weight; the epilogue emits silu(gate) * up for the 64
-// outputs with vLLM's cast points (vllm:model_executor/layers/activation.py:137-141).
-// n: the output column; with a bias ([gate | up] halves of p.N numbers each) it joins the accumulators before the rounding.
-__device__ __forceinline__ float silu_gate_bf16(const GemmParams& p, float g_acc, float u_acc, int n) {
-  if (p.bias && n < p.N) { g_acc += bf2f(p.bias[n]); u_acc += bf2f(p.bias[p.N + n]); }
-  float g = rbf(g_acc), u = rbf(u_acc);                  // the gate_up GEMM output is bf16
+// the gated pair of pre-activations that are rounded already
+__device__ __forceinline__ float silu_gate_rounded(const GemmParams& p, float g, float u) {
   if (p.glu == 1) {                                      // clamped pair with a sigmoid gate: fp32 from the rounded pre-activations
     g = fminf(g, p.glu_limit);
     u = fminf(fmaxf(u, -p.glu_limit), p.glu_limit);
@@ -179,6 +193,15 @@ __device__ __forceinline__ float silu_gate_bf16(const GemmParams& p, float g_acc
   }
   const float sg = rbf(__fdividef(g, 1.0f + __expf(-g))); // F.silu rounds to bf16 (fast exp/div: <= 2 ulp in fp32)
   return sg * u;                                          // caller rounds the product once
+}
+
+// GATED: the 128 MMA rows of a tile are 64 gate rows (TMEM lanes 0-63) and the matching 64 up rows
+// (lanes 64-127) of a stacked [2f, K] weight; the epilogue emits silu(gate) * up for the 64
+// outputs with vLLM's cast points (vllm:model_executor/layers/activation.py:137-141).
+// n: the output column; with a bias ([gate | up] halves of p.N numbers each) it joins the accumulators before the rounding.
+__device__ __forceinline__ float silu_gate_bf16(const GemmParams& p, float g_acc, float u_acc, int n) {
+  if (p.bias && n < p.N) { g_acc += bf2f(p.bias[n]); u_acc += bf2f(p.bias[p.N + n]); }
+  return silu_gate_rounded(p, rbf(g_acc), rbf(u_acc));   // the gate_up GEMM output is bf16
 }
 
 __device__ __forceinline__ void tma_load_2d_cg2_hint(uint32_t dst, const CUtensorMap* map, uint32_t bar_cluster, int c0, int c1, uint64_t pol) {
@@ -224,7 +247,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant
   // bars: full[STAGES], empty[STAGES], tmem_full[2], tmem_empty[2]
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * STAGES + 4);
   float* xbuf = reinterpret_cast<float*>(smem + STAGES * STAGE_BYTES + 2048);   // SPLIT: exchange buffer;
-                                                                                // GATED && !SPLIT: up->gate hand-off [2][16][64]
+                                                                                // GATED && !SPLIT: gate / up hand-off, 8 KB
   constexpr int ROWS_OUT = GATED ? 64 : BLK_M;           // output columns produced per tile
   const uint32_t smem_base = smem_addr(smem);
   const uint32_t bar_base = smem_addr(bars);
@@ -435,12 +458,13 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant
     const int q = warp - 4;                      // TMEM lane quarter == warp % 4
     const int et = threadIdx.x - 128;            // 0..127 == weight row within the tile
     int acc = 0; uint32_t acc_phase = 0;
+    [[maybe_unused]] int hand = 0;               // GATED: which hand-off buffer is next
     SegIter it = segments();
     int w, kb0, kb1;
     while (it.next(w, kb0, kb1)) {
       const int n_tile = w % p.n_tiles, m_tile = m_tile_of(w);
       if (no_rows(w)) continue;
-      const int n = m_tile * ROWS_OUT + (GATED ? (et & 63) : et);   // output column of this thread's row
+      [[maybe_unused]] const int n = m_tile * ROWS_OUT + (GATED ? (et & 63) : et);   // output column of this thread's row
       const int t0 = n_tile * TOKN;
       mbar_wait(tfull_bar(acc), acc_phase);
       tc_fence_after();
@@ -530,56 +554,98 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant
           }
           if (et == 0) p.ws_count[w] = 0;                  // ready for the next launch
         }
-      } else if (!SPLIT && !GATED) {
-#pragma unroll 1
-        for (int c = 0; c < TOKN; c += 16) {
-          uint32_t r[16];
-          tmem_ld16(taddr + c, r);
-          if (n < p.N) {
+      } else if (!SPLIT) {
+        // 32 tokens (columns) at a time: both 16-lane halves of this warp's rows come as MMA fragments, are finished and rounded
+        // in registers, and stmatrix turns them into rows of 32 outputs per token in a staging tile of this warp's own, from where
+        // a lane stores 16 bytes of an output row.  (One 2-byte store per output and a wait per 16 columns made the epilogue 10 us
+        // of a single-wave launch: 1339 x 2048 x 2048 took 23 us, 10 of them in the main loop.)
+        // GATED: gate rows live in warps q = 0, 1 and their up rows in q = 2, 3; each hands the other half of its tokens, rounded to
+        // the element type as the product is, through shared memory.
+        constexpr int G = TOKN >= 32 ? 4 : 2, CH = 8 * G;
+        const uint32_t stage_buf = smem_addr(smem) + STAGES * STAGE_BYTES + 2048 + (GATED ? 8192 : 0) + q * 2048;
+        uint32_t* swap = reinterpret_cast<uint32_t*>(xbuf);
+        const int nq = m_tile * ROWS_OUT + (GATED ? (q & 1) : q) * 32;        // first output of this warp
+        const bool vec = (p.N & 7) == 0 && (reinterpret_cast<uintptr_t>(p.y) & 15) == 0 && nq + 32 <= p.N;
+        float bq[4];                                                          // bias of rows l / 4 + 8 i
 #pragma unroll
-            for (int j = 0; j < 16; ++j) {
-              const int t = t0 + c + j;
-              if (t < p.T) {
-                float v = __uint_as_float(r[j]) + bv;
-                v = apply_act(v, p.act);
-                p.y[(int64_t)t * p.N + n] = f2bf(v);
+        for (int i = 0; i < 4; ++i) {
+          const int nb = nq + 8 * i + (lane >> 2);
+          bq[i] = p.bias && nb < p.N ? bf2f(p.bias[(GATED && q >= 2 ? p.N : 0) + nb]) : 0.f;
+        }
+#pragma unroll 1
+        for (int c = 0; c < TOKN; c += CH) {
+          if (t0 + c >= p.T) break;                                           // the same for all epilogue warps
+          uint32_t r[2][4 * G];
+          tmem_ld_frag<G>(taddr + c, r[0]);
+          tmem_ld_frag<G>(taddr + c + (16u << 16), r[1]);
+          tmem_wait_ld();
+          uint32_t o[G][4];                                                   // [8 tokens][8 rows]: two tokens of a row per register
+          if (!GATED) {
+            float v[2][4 * G];
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+#pragma unroll
+              for (int i = 0; i < 4 * G; ++i) v[h][i] = __uint_as_float(r[h][i]) + bq[2 * h + ((i >> 1) & 1)];
+            if (p.act != 0) {
+#pragma unroll
+              for (int h = 0; h < 2; ++h)
+#pragma unroll
+                for (int i = 0; i < 4 * G; ++i) v[h][i] = apply_act(v[h][i], p.act);
+            }
+#pragma unroll
+            for (int k = 0; k < G; ++k)
+#pragma unroll
+              for (int i = 0; i < 4; ++i) o[k][i] = pack_bf2(v[i >> 1][4 * k + 2 * (i & 1)], v[i >> 1][4 * k + 2 * (i & 1) + 1]);
+          } else {
+            constexpr int HG = G / 2;
+            const bool is_up = q >= 2;
+            uint32_t mine[G][4];
+#pragma unroll
+            for (int k = 0; k < G; ++k)
+#pragma unroll
+              for (int i = 0; i < 4; ++i)
+                mine[k][i] = pack_bf2(__uint_as_float(r[i >> 1][4 * k + 2 * (i & 1)]) + bq[i], __uint_as_float(r[i >> 1][4 * k + 2 * (i & 1) + 1]) + bq[i]);
+            // [parity][pair][gate -> up, up -> gate][register][lane]
+            uint32_t* hb = swap + (hand * 4 + (q & 1) * 2) * (8 * 32) + lane;
+            hand ^= 1;                                                        // two buffers in turn, across tiles too
+#pragma unroll
+            for (int k = 0; k < HG; ++k)
+#pragma unroll
+              for (int i = 0; i < 4; ++i) hb[(is_up ? 256 : 0) + (k * 4 + i) * 32] = is_up ? mine[k][i] : mine[k + HG][i];
+            asm volatile("bar.sync %0, 64;" ::"r"(2 + (q & 1)) : "memory");
+#pragma unroll
+            for (int k = 0; k < HG; ++k)
+#pragma unroll
+              for (int i = 0; i < 4; ++i) {
+                const uint32_t other = hb[(is_up ? 0 : 256) + (k * 4 + i) * 32], own = is_up ? mine[k + HG][i] : mine[k][i];
+                const uint32_t gv = is_up ? other : own, uv = is_up ? own : other;
+                o[k][i] = pack_bf2(silu_gate_rounded(p, bf_lo(gv), bf_lo(uv)), silu_gate_rounded(p, bf_hi(gv), bf_hi(uv)));
+              }
+          }
+          constexpr int OG = GATED ? G / 2 : G;                               // groups of 8 tokens that this warp stores
+#pragma unroll
+          for (int k = 0; k < OG; ++k) {
+            const int tok = k * 8 + (lane & 7), piece = lane >> 3;
+            stsm_trans(stage_buf + tok * 64 + ((piece ^ ((tok >> 1) & 3)) << 4), o[k][0], o[k][1], o[k][2], o[k][3]);
+          }
+          __syncwarp();
+          const int tb = t0 + c + (GATED && q >= 2 ? CH / 2 : 0);
+#pragma unroll
+          for (int k = 0; k < OG; ++k) {
+            const int tok = k * 8 + (lane >> 2), piece = lane & 3, t = tb + tok, n0 = nq + piece * 8;
+            const float4 f = lds_f4(stage_buf + tok * 64 + ((piece ^ ((tok >> 1) & 3)) << 4));
+            if (t < p.T) {
+              bf16* dst = p.y + (int64_t)t * p.N + n0;
+              if (vec) {
+                *reinterpret_cast<float4*>(dst) = f;
+              } else {
+                const bf16* e = reinterpret_cast<const bf16*>(&f);
+#pragma unroll
+                for (int j = 0; j < 8; ++j) if (n0 + j < p.N) dst[j] = e[j];
               }
             }
           }
-        }
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) { if (PAIR) mbar_arrive_cluster(mapa_u32(tempty_bar(acc), 0u)); else mbar_arrive(tempty_bar(acc)); }
-      } else if (!SPLIT) {
-        // Gate rows live in warps q=0,1 and their up rows in warps q=2,3 (TMEM lane quarters), so each
-        // pair swaps half of every 16-column chunk through shared memory: the gate warp finishes
-        // columns 0-7, the up warp columns 8-15.  Double-buffered, one 64-thread named barrier per chunk.
-        const int pair = q & 1, r64 = et & 63;
-        const int bar_id = 2 + pair;
-        const bool is_up = q >= 2;
-#pragma unroll 1
-        for (int c = 0; c < TOKN; c += 16) {
-          uint32_t r[16];
-          tmem_ld16(taddr + c, r);
-          float* hb = xbuf + ((c >> 4) & 1) * (2 * 8 * 64);     // [0]: up cols 0-7, [1]: gate cols 8-15
-          if (is_up) {
-#pragma unroll
-            for (int j = 0; j < 8; ++j) hb[j * 64 + r64] = __uint_as_float(r[j]);
-          } else {
-#pragma unroll
-            for (int j = 0; j < 8; ++j) hb[(8 + j) * 64 + r64] = __uint_as_float(r[8 + j]);
-          }
-          asm volatile("bar.sync %0, 64;" ::"r"(bar_id) : "memory");
-          if (n < p.N) {
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-              const int col = is_up ? 8 + j : j;
-              const int t = t0 + c + col;
-              const float gacc = is_up ? hb[(8 + j) * 64 + r64] : __uint_as_float(r[j]);
-              const float uacc = is_up ? __uint_as_float(r[8 + j]) : hb[j * 64 + r64];
-              if (t < p.T) p.y[(int64_t)t * p.N + n] = f2bf(silu_gate_bf16(p, gacc, uacc, n));
-            }
-          }
+          __syncwarp();
         }
         tc_fence_before();
         __syncwarp();
@@ -1000,8 +1066,8 @@ constexpr int kGemmSmemBudget = 224 * 1024;
 template <int TOKN, bool SPLIT, bool GATED, bool PAIR = false, bool WS = false>
 static int launch_gemm(const CUtensorMap& tw, const CUtensorMap& tx, const GemmParams& p, cudaStream_t st) {
   constexpr int stage_bytes = BLK_M * BLK_K * 2 + (PAIR ? 128 : TOKN) * BLK_K * 2;
-  // barriers + column map, then the cluster exchange buffer (SPLIT) or the up->gate hand-off (GATED)
-  constexpr int extra = 2048 + (SPLIT ? xbuf_bytes(TOKN) : (GATED ? 2 * 16 * 64 * 4 : 0));
+  // barriers, then the cluster exchange buffer (SPLIT), or the gate / up hand-off (GATED) and the epilogue's staging tiles
+  constexpr int extra = 2048 + (SPLIT ? xbuf_bytes(TOKN) : (GATED ? 8192 : 0) + 8192);
   constexpr int budget = kGemmSmemBudget - 1024 - extra;
   constexpr int STAGES = (budget / stage_bytes) > 8 ? 8 : (budget / stage_bytes);
   static_assert(STAGES >= 3, "pipeline too shallow");
