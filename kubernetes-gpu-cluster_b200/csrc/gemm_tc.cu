@@ -29,6 +29,8 @@
 #include <cuda.h>
 #include <stdlib.h>
 
+#include <algorithm>
+#include <atomic>
 #include <mutex>
 #include <unordered_map>
 
@@ -42,6 +44,7 @@ constexpr int BLK_M = 128;   // weight rows per tile (UMMA M)
 constexpr int BLK_K = 64;    // 64 bf16 = 128 B = one swizzle row
 constexpr int UMMA_K = 16;
 constexpr int kGemmThreads = 256;
+constexpr int kPairSub = 2;     // k-blocks per stage of the pair kernel: half the barriers (64-token tiles 0.30 -> 0.25 us a k-block)
 constexpr uint32_t kSpinLimit = 1u << 24;   // seconds at most: a lost arrival traps instead of hanging the GPU
 
 __device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -135,6 +138,7 @@ struct GemmParams {
   int l2_hints;              // 1: weights evict_first, activations evict_last, output stored streaming
   int m_tiles, n_tiles, splits, kb_total, kb_per_split;
   int rows;                  // gemm_wide_kernel: outputs per tile
+  int tokn = 0;              // PAIR: tokens per tile, a multiple of 32 up to 256
   unsigned long long* trace; // phase timestamps, 16 per CTA (tools/gemm_trace.py); null outside that tool
   int glu = 0;               // gated pair: 0 silu(gate) * up; 1 clamped: g = min(gate, limit), u = clamp(up, +-limit), g * sigmoid(alpha g) * (u + 1)
   float glu_alpha = 0.f, glu_limit = 0.f;
@@ -174,6 +178,9 @@ __device__ __forceinline__ uint32_t mapa_u32(uint32_t local, uint32_t rank) {
 }
 __device__ __forceinline__ void st_cluster_f32(uint32_t addr, float v) {
   asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory");
+}
+__device__ __forceinline__ void st_cluster_f4(uint32_t addr, float a, float b, float c, float d) {
+  asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
 }
 __device__ __forceinline__ float4 lds_f4(uint32_t addr) {
   float4 v;
@@ -229,17 +236,25 @@ __device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar_cluster) {
 // leader CTA issues tcgen05.mma.cta_group::2 for both, accumulators land in each CTA's own TMEM.
 // All TMA loads of a stage complete on the LEADER's full barrier; tcgen05.commit multicasts the
 // "stage free" and "accumulator ready" arrivals to both CTAs; both epilogues release the accumulator
-// on the leader's tmem_empty barrier.
+// on the leader's tmem_empty barrier.  The width of the token tile is a launch parameter (p.tokn): the host picks what leaves
+// the last round of tiles fullest.
+// PAIR && SPLIT: a cluster of S pairs shares one tile, each pair takes 1/S of K.  Once all of them are past their main loops the
+// pipeline stages hold the exchange: pair o finishes the o-th share of the tile's 32-token groups, and every other pair sends it
+// its fp32 accumulators of those, in the fragment order in which the epilogue reads TMEM (512-byte warp stores); the owner adds
+// them in rank order.
 template <int TOKN, int STAGES, bool SPLIT, bool GATED, bool PAIR = false, bool WS = false>
 __global__ void __launch_bounds__(kGemmThreads, 1)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x,
                const GemmParams p) {
-  static_assert(!(PAIR && SPLIT) && !(WS && (SPLIT || PAIR)), "one split scheme at a time");
+  static_assert(!(WS && (SPLIT || PAIR)), "one split scheme at a time");
+  constexpr bool XSPLIT = SPLIT && !PAIR;               // K split over single CTAs, exchanged through a buffer of its own
   constexpr uint32_t A_BYTES = BLK_M * BLK_K * 2, B_BYTES = (PAIR ? 128 : TOKN) * BLK_K * 2;
-  constexpr uint32_t STAGE_BYTES = A_BYTES + B_BYTES;
+  constexpr int SUB = PAIR ? kPairSub : 1;               // k-blocks per stage
+  constexpr uint32_t STAGE_BYTES = SUB * (A_BYTES + B_BYTES);
   constexpr uint32_t TMEM_COLS = (2 * TOKN < 32) ? 32 : 2 * TOKN;
-  constexpr uint32_t IDESC = (1u << 4) | KGE_IDESC_AB | ((uint32_t)(TOKN >> 3) << 17) |
-                             ((uint32_t)((PAIR ? 2 * BLK_M : BLK_M) >> 4) << 24);
+  const int tokn = PAIR ? p.tokn : TOKN;
+  const uint32_t IDESC = (1u << 4) | KGE_IDESC_AB | ((uint32_t)(tokn >> 3) << 17) |
+                         ((uint32_t)((PAIR ? 2 * BLK_M : BLK_M) >> 4) << 24);
 
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -291,18 +306,19 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant
 
   // work decomposition: persistent round-robin over tiles, or (SPLIT) one tile per cluster with
   // the cluster rank selecting the K range
-  const int S = SPLIT ? (int)cluster_nctarank() : 1;
-  const int crank = SPLIT ? (int)cluster_ctarank() : 0;
+  const int S = SPLIT ? (int)cluster_nctarank() / (PAIR ? 2 : 1) : 1;
+  const int crank = SPLIT ? (int)cluster_ctarank() / (PAIR ? 2 : 1) : 0;      // which share of K
   constexpr bool TWO = PAIR;
-  const int mrank = TWO ? (int)cluster_ctarank() : 0;            // which tile of the weight-row pair
+  const int mrank = TWO ? (int)cluster_ctarank() & 1 : 0;        // which tile of the weight-row pair
+  const uint32_t leader = TWO ? cluster_ctarank() & ~1u : 0u;    // the pair's CTA that issues the MMAs
   const int total = (TWO ? (p.m_tiles + 1) / 2 : p.m_tiles) * p.n_tiles;
-  const int w_first = SPLIT ? (int)blockIdx.x / S : TWO ? (int)blockIdx.x / 2 : (int)blockIdx.x;
+  const int w_first = SPLIT ? (int)blockIdx.x / (PAIR ? 2 * S : S) : TWO ? (int)blockIdx.x / 2 : (int)blockIdx.x;
   const int w_step = SPLIT ? (1 << 30) : TWO ? (int)gridDim.x / 2 : (int)gridDim.x;
   auto m_tile_of = [&](int w) { return TWO ? 2 * (w / p.n_tiles) + mrank : w / p.n_tiles; };
   // grouped rows: a tile beyond the last group has no work (every role reads the table after pdl_wait and skips alike)
-  auto no_rows = [&](int w) { return p.tile_group != nullptr && p.tile_group[((w % p.n_tiles) * TOKN) >> 8] < 0; };
-  // PAIR: every TMA of a stage completes on the leader's (rank 0) full barrier
-  auto lead_full = [&](int s) { return PAIR ? mapa_u32(full_bar(s), 0u) : full_bar(s); };
+  auto no_rows = [&](int w) { return p.tile_group != nullptr && p.tile_group[((w % p.n_tiles) * tokn) >> 8] < 0; };
+  // PAIR: every TMA of a stage completes on the leader's full barrier
+  auto lead_full = [&](int s) { return PAIR ? mapa_u32(full_bar(s), leader) : full_bar(s); };
   const int kb0f = crank * p.kb_per_split, kb1f = min(p.kb_total, kb0f + p.kb_per_split);
   const int cols_per = (TOKN + S - 1) / S;               // columns finished by each cluster rank
   // A CTA's work as a sequence of segments (tile w, k-blocks [kb0, kb1)).  Persistent / split variants: its tiles, each
@@ -328,15 +344,16 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant
     }
   };
   auto segments = [&]() { return WS ? SegIter{u_begin, u_end, 0, KB, 0, 0} : SegIter{(int64_t)w_first, (int64_t)total, w_step, KB, kb0f, kb1f}; };
-  if (SPLIT) cluster_arrive_relaxed();                   // phase A: every CTA of the cluster has started (nothing to publish: no release)
+  if (XSPLIT) cluster_arrive_relaxed();                  // phase A: every CTA of the cluster has started (nothing to publish: no release)
 
   if (warp == 0) {
     if (lane == 0) {
       int stage = 0; uint32_t phase = 0;
       const bool hint = p.l2_hints != 0;
       const uint64_t pol_w = l2_policy(false), pol_x = l2_policy(true);
-      auto load_a = [&](int st, int kb, int m_tile, int woff) {
-        const uint32_t a_dst = smem_base + st * STAGE_BYTES;
+      auto load_a = [&](int st, int kb, int m_tile, int woff, int sub) {
+        const uint32_t a_dst = smem_base + st * STAGE_BYTES + sub * (A_BYTES + B_BYTES);
+        kb += sub;
         if (PAIR && hint) {
           if (GATED) {
             tma_load_2d_cg2_hint(a_dst, &tmap_w, lead_full(st), kb * BLK_K, woff + m_tile * 64, pol_w);
@@ -366,17 +383,18 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant
         }
       };
       // the barrier that counts a stage's bytes: own (48 KB) or, PAIR, the leader's for both CTAs (2 x 32 KB)
-      auto expect = [&](int st) {
+      auto expect = [&](int st, int subs) {
         if (!PAIR) mbar_expect_tx(full_bar(st), STAGE_BYTES);
-        else if (mrank == 0) mbar_expect_tx(full_bar(st), 2 * STAGE_BYTES);
+        else if (mrank == 0) mbar_expect_tx(full_bar(st), subs * (2 * A_BYTES + (uint32_t)tokn * BLK_K * 2));
       };
       // Weights do not depend on the previous kernel: stream the first stages of W while it is
       // still running, then wait for its output (the activations) and add the X tiles.
       int pre = 0;
-      auto load_b = [&](int st, int kb, int n_tile) {
-        const uint32_t b_dst = smem_base + st * STAGE_BYTES + A_BYTES;
-        if (PAIR && hint) tma_load_2d_cg2_hint(b_dst, &tmap_x, lead_full(st), kb * BLK_K, n_tile * TOKN + mrank * 128, pol_x);
-        else if (PAIR) tma_load_2d_cg2(b_dst, &tmap_x, lead_full(st), kb * BLK_K, n_tile * TOKN + mrank * 128);
+      auto load_b = [&](int st, int kb, int n_tile, int sub) {
+        const uint32_t b_dst = smem_base + st * STAGE_BYTES + sub * (A_BYTES + B_BYTES) + A_BYTES;
+        kb += sub;
+        if (PAIR && hint) tma_load_2d_cg2_hint(b_dst, &tmap_x, lead_full(st), kb * BLK_K, n_tile * tokn + mrank * (tokn / 2), pol_x);
+        else if (PAIR) tma_load_2d_cg2(b_dst, &tmap_x, lead_full(st), kb * BLK_K, n_tile * tokn + mrank * (tokn / 2));
         else if (hint) tma_load_2d_hint(b_dst, &tmap_x, full_bar(st), kb * BLK_K, n_tile * TOKN, pol_x);
         else tma_load_2d(b_dst, &tmap_x, full_bar(st), kb * BLK_K, n_tile * TOKN);
       };
@@ -386,10 +404,11 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant
         SegIter peek = segments();
         if (peek.next(w, kb0, kb1)) {            // the first segment's first stages (a later segment's are loaded in the loop)
           const int m_tile = m_tile_of(w);
-          pre = p.tile_group ? 0 : min(STAGES, kb1 - kb0);      // which weights a tile needs is the previous kernel's output
-          for (int i = 0; i < pre; ++i) {
-            expect(i);
-            load_a(i, kb0 + i, m_tile, 0);
+          pre = p.tile_group ? 0 : min(STAGES * SUB, kb1 - kb0);      // which weights a tile needs is the previous kernel's output
+          for (int i = 0; i * SUB < pre; ++i) {
+            const int subs = min(SUB, kb1 - kb0 - i * SUB);
+            expect(i, subs);
+            for (int u = 0; u < subs; ++u) load_a(i, kb0 + i * SUB, m_tile, 0, u);
             if (i == 0) trace_stamp(p, 13);
           }
         }
@@ -402,15 +421,15 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant
       while (it.next(w, kb0, kb1)) {
         const int n_tile = w % p.n_tiles, m_tile = m_tile_of(w);
         if (no_rows(w)) continue;
-        const int woff = p.tile_group ? p.tile_group[(n_tile * TOKN) >> 8] * p.group_rows : 0;
-        for (int kb = kb0; kb < kb1; ++kb) {
+        const int woff = p.tile_group ? p.tile_group[(n_tile * tokn) >> 8] * p.group_rows : 0;
+        for (int kb = kb0; kb < kb1; kb += SUB) {
+          const int subs = min(SUB, kb1 - kb);
           if (first_seg && kb - kb0 < pre) {
-            load_b(stage, kb, n_tile);
+            for (int u = 0; u < subs; ++u) load_b(stage, kb, n_tile, u);
           } else {
             mbar_wait(empty_bar(stage), phase ^ 1);
-            expect(stage);
-            load_a(stage, kb, m_tile, woff);
-            load_b(stage, kb, n_tile);
+            expect(stage, subs);
+            for (int u = 0; u < subs; ++u) { load_a(stage, kb, m_tile, woff, u); load_b(stage, kb, n_tile, u); }
           }
           if (++stage == STAGES) { stage = 0; phase ^= 1; }
         }
@@ -434,21 +453,26 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant
         mbar_wait(tempty_bar(acc), acc_phase ^ 1);
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + acc * TOKN;
-        for (int kb = kb0; kb < kb1; ++kb) {
+        for (int kb = kb0; kb < kb1; kb += SUB) {
           mbar_wait(full_bar(stage), phase);
           tc_fence_after();
 #pragma unroll
-          for (int k = 0; k < BLK_K / UMMA_K; ++k) {
-            // +32 B per 16-element k step inside the 128 B swizzle row (start address field is >>4)
-            if (PAIR) tc_mma_bf16_cg2(d_tmem, adesc + (uint64_t)(k * 2), bdesc + (uint64_t)(k * 2), IDESC, (kb > kb0 || k > 0) ? 1u : 0u);
-            else tc_mma_bf16(d_tmem, adesc + (uint64_t)(k * 2), bdesc + (uint64_t)(k * 2), IDESC, (kb > kb0 || k > 0) ? 1u : 0u);
+          for (int u = 0; u < SUB; ++u) {
+            if (u > 0 && kb + u >= kb1) break;
+#pragma unroll
+            for (int k = 0; k < BLK_K / UMMA_K; ++k) {
+              // +32 B per 16-element k step inside the 128 B swizzle row (start address field is >>4)
+              const uint64_t off = (uint64_t)(u * ((A_BYTES + B_BYTES) >> 4) + k * 2);
+              if (PAIR) tc_mma_bf16_cg2(d_tmem, adesc + off, bdesc + off, IDESC, (kb > kb0 || u + k > 0) ? 1u : 0u);
+              else tc_mma_bf16(d_tmem, adesc + off, bdesc + off, IDESC, (kb > kb0 || u + k > 0) ? 1u : 0u);
+            }
           }
-          if (PAIR) tc_commit_cg2(empty_bar(stage), (uint16_t)3); // frees the stage in both CTAs
+          if (PAIR) tc_commit_cg2(empty_bar(stage), (uint16_t)(3u << leader)); // frees the stage in both CTAs
           else tc_commit(empty_bar(stage));     // frees the smem slot when these MMAs retire
           adesc += STAGE_BYTES >> 4; bdesc += STAGE_BYTES >> 4;
           if (++stage == STAGES) { stage = 0; phase ^= 1; adesc = adesc0; bdesc = bdesc0; }
         }
-        if (PAIR) tc_commit_cg2(tfull_bar(acc), (uint16_t)3);   // both CTAs' epilogues
+        if (PAIR) tc_commit_cg2(tfull_bar(acc), (uint16_t)(3u << leader));   // both CTAs' epilogues
         else tc_commit(tfull_bar(acc));         // accumulator complete
         if (++acc == 2) { acc = 0; acc_phase ^= 1; }
       }
@@ -465,7 +489,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant
       const int n_tile = w % p.n_tiles, m_tile = m_tile_of(w);
       if (no_rows(w)) continue;
       [[maybe_unused]] const int n = m_tile * ROWS_OUT + (GATED ? (et & 63) : et);   // output column of this thread's row
-      const int t0 = n_tile * TOKN;
+      const int t0 = n_tile * tokn;
       mbar_wait(tfull_bar(acc), acc_phase);
       tc_fence_after();
       if (et == 0) trace_stamp(p, 7);              // (of the CTA's last segment: later segments overwrite the stamp)
@@ -554,7 +578,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant
           }
           if (et == 0) p.ws_count[w] = 0;                  // ready for the next launch
         }
-      } else if (!SPLIT) {
+      } else if (!XSPLIT) {
         // 32 tokens (columns) at a time: both 16-lane halves of this warp's rows come as MMA fragments, are finished and rounded
         // in registers, and stmatrix turns them into rows of 32 outputs per token in a staging tile of this warp's own, from where
         // a lane stores 16 bytes of an output row.  (One 2-byte store per output and a wait per 16 columns made the epilogue 10 us
@@ -572,13 +596,59 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant
           const int nb = nq + 8 * i + (lane >> 2);
           bq[i] = p.bias && nb < p.N ? bf2f(p.bias[(GATED && q >= 2 ? p.N : 0) + nb]) : 0.f;
         }
+        int c_begin = 0, c_end = tokn;
+        const int share = SPLIT ? (tokn / 32 + S - 1) / S : 0;                // SPLIT: 32-token groups per pair of the cluster
+        // [source][group of the owner's share][register quad][thread] of 16 bytes, over the pipeline stages
+        auto xslot = [&](int src, int grp, int quad) { return smem_base + (uint32_t)((((src * share + grp) * 8 + quad) * 128 + et) * 16); };
+        if constexpr (SPLIT) {
+          cluster_arrive(); cluster_wait();                                   // no CTA of the cluster reads its stages any more
 #pragma unroll 1
-        for (int c = 0; c < TOKN; c += CH) {
+          for (int c = 0; c < tokn; c += CH) {
+            const int grp = c / 32, owner = grp / share;
+            if (owner == crank || t0 + c >= p.T) continue;
+            uint32_t r[2][4 * G];
+            tmem_ld_frag<G>(taddr + c, r[0]);
+            tmem_ld_frag<G>(taddr + c + (16u << 16), r[1]);
+            tmem_wait_ld();
+#pragma unroll
+            for (int quad = 0; quad < 8; ++quad) {
+              const uint32_t* v = &r[quad >> 2][(quad & 3) * 4];
+              st_cluster_f4(mapa_u32(xslot(crank, grp - owner * share, quad), (uint32_t)(2 * owner + mrank)), __uint_as_float(v[0]), __uint_as_float(v[1]),
+                            __uint_as_float(v[2]), __uint_as_float(v[3]));
+            }
+          }
+          cluster_arrive(); cluster_wait();                                   // the owners have everything
+          c_begin = crank * share * 32; c_end = min(tokn, c_begin + share * 32);
+        }
+#pragma unroll 1
+        for (int c = c_begin; c < c_end; c += CH) {
           if (t0 + c >= p.T) break;                                           // the same for all epilogue warps
           uint32_t r[2][4 * G];
           tmem_ld_frag<G>(taddr + c, r[0]);
           tmem_ld_frag<G>(taddr + c + (16u << 16), r[1]);
           tmem_wait_ld();
+          if constexpr (SPLIT) {
+            float sum[2][4 * G];
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+#pragma unroll
+              for (int i = 0; i < 4 * G; ++i) sum[h][i] = 0.f;
+#pragma unroll 1
+            for (int src = 0; src < S; ++src) {
+#pragma unroll
+              for (int quad = 0; quad < 8; ++quad) {
+                float* d = &sum[quad >> 2][(quad & 3) * 4];
+                const uint32_t* o = &r[quad >> 2][(quad & 3) * 4];
+                const float4 f = src == crank ? make_float4(__uint_as_float(o[0]), __uint_as_float(o[1]), __uint_as_float(o[2]), __uint_as_float(o[3]))
+                                              : lds_f4(xslot(src, (c - c_begin) / 32, quad));
+                d[0] += f.x; d[1] += f.y; d[2] += f.z; d[3] += f.w;
+              }
+            }
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+#pragma unroll
+              for (int i = 0; i < 4 * G; ++i) r[h][i] = __float_as_uint(sum[h][i]);
+          }
           uint32_t o[G][4];                                                   // [8 tokens][8 rows]: two tokens of a row per register
           if (!GATED) {
             float v[2][4 * G];
@@ -649,7 +719,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant
         }
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) { if (PAIR) mbar_arrive_cluster(mapa_u32(tempty_bar(acc), 0u)); else mbar_arrive(tempty_bar(acc)); }
+        if (lane == 0) { if (PAIR) mbar_arrive_cluster(mapa_u32(tempty_bar(acc), leader)); else mbar_arrive(tempty_bar(acc)); }
       } else {
         cluster_wait();                          // phase A done: peers' shared memory is live
         // Phase 1: my 128 x TOKN fp32 partial goes to the owners' exchange buffers, [src rank][local column][128 rows]:
@@ -724,6 +794,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant
     if (et == 0) trace_stamp(p, 10);
   }
   if (SPLIT && warp < 4) {                       // non-epilogue warps take part in both cluster phases
+    if (PAIR) cluster_arrive();
     cluster_wait();
     cluster_arrive();
     cluster_wait();
@@ -755,10 +826,6 @@ constexpr uint32_t WIDE_A_BYTES = WIDE_M * BLK_K * 2, WIDE_B_BYTES = WIDE_N * BL
 constexpr uint32_t WIDE_STAGE = WIDE_A_BYTES + WIDE_B_BYTES;
 constexpr int kWideStages = 5;
 constexpr int kWideThreads = 384;           // warps 0-3 as in gemm_tc_kernel, two epilogue warpgroups
-
-__device__ __forceinline__ void st_cluster_f4(uint32_t addr, float a, float b, float c, float d) {
-  asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
-}
 
 template <bool SPLIT, bool GATED>
 __global__ void __launch_bounds__(kWideThreads, 1)
@@ -1065,9 +1132,9 @@ constexpr int kGemmSmemBudget = 224 * 1024;
 
 template <int TOKN, bool SPLIT, bool GATED, bool PAIR = false, bool WS = false>
 static int launch_gemm(const CUtensorMap& tw, const CUtensorMap& tx, const GemmParams& p, cudaStream_t st) {
-  constexpr int stage_bytes = BLK_M * BLK_K * 2 + (PAIR ? 128 : TOKN) * BLK_K * 2;
+  constexpr int stage_bytes = (BLK_M * BLK_K * 2 + (PAIR ? 128 : TOKN) * BLK_K * 2) * (PAIR ? kPairSub : 1);
   // barriers, then the cluster exchange buffer (SPLIT), or the gate / up hand-off (GATED) and the epilogue's staging tiles
-  constexpr int extra = 2048 + (SPLIT ? xbuf_bytes(TOKN) : (GATED ? 8192 : 0) + 8192);
+  constexpr int extra = 2048 + (SPLIT && !PAIR ? xbuf_bytes(TOKN) : (GATED ? 8192 : 0) + 8192);
   constexpr int budget = kGemmSmemBudget - 1024 - extra;
   constexpr int STAGES = (budget / stage_bytes) > 8 ? 8 : (budget / stage_bytes);
   static_assert(STAGES >= 3, "pipeline too shallow");
@@ -1087,9 +1154,10 @@ static int launch_gemm(const CUtensorMap& tw, const CUtensorMap& tx, const GemmP
   if (WS) {
     cfg.gridDim = dim3(p.splits);                // stream-K: `splits` CTAs (one per SM), each a contiguous share of all k-blocks
   } else if (SPLIT) {
-    cfg.gridDim = dim3(tiles * p.splits);
+    const int ctas = PAIR ? 2 * p.splits : p.splits;
+    cfg.gridDim = dim3((PAIR ? (p.m_tiles + 1) / 2 * p.n_tiles : tiles) * ctas);
     attr[1].id = cudaLaunchAttributeClusterDimension;
-    attr[1].val.clusterDim.x = p.splits; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = 1;
+    attr[1].val.clusterDim.x = ctas; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = 1;
     cfg.numAttrs = 2;
   } else if (PAIR) {
     const int pairs = ((p.m_tiles + 1) / 2) * p.n_tiles;
@@ -1146,7 +1214,7 @@ static int max_clusters(int tokn, int S) {
   return cache[ti][S];
 }
 
-struct GemmPlan { int tokn, m_tiles, n_tiles, splits, kb_total, kb_per_split; bool ws; int rows; };
+struct GemmPlan { int tokn, m_tiles, n_tiles, splits, kb_total, kb_per_split; bool ws; int rows; bool pair = false; };
 
 constexpr int64_t kWsCounterBytes = 1024;        // per-tile arrival counters at the head of the workspace (<= 256 tiles)
 
@@ -1275,11 +1343,68 @@ static bool plan_wide(int T, int n_out, int K, bool gated, GemmPlan& g) {
 
 #include "gemm_rows.cuh"
 
-// prefill-sized problems run as CTA pairs (cta_group::2, 256 x 256 MMA tiles)
-static bool gemm_uses_pair(const GemmPlan& g) { return g.tokn == 256 && g.splits == 1 && g.m_tiles >= 2; }
+// How many clusters of `size` CTAs of the pair kernel can be co-resident.
+static int max_clusters_pair(int size) {
+  static std::atomic<int> cache[9];
+  int n = cache[size].load(std::memory_order_relaxed);
+  if (n == 0) {
+    constexpr int stage_bytes = 2 * BLK_M * BLK_K * 2 * kPairSub, extra = 2048 + 8192, STAGES = (kGemmSmemBudget - 1024 - extra) / stage_bytes;
+    constexpr int smem = STAGES * stage_bytes + 1024 + extra;
+    auto kern = gemm_tc_kernel<256, STAGES, true, false, true>;
+    int got = 0;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) == cudaSuccess) {
+      cudaLaunchConfig_t cfg = {};
+      cfg.gridDim = dim3(size * 64); cfg.blockDim = dim3(kGemmThreads); cfg.dynamicSmemBytes = smem;
+      cudaLaunchAttribute attr[1];
+      attr[0].id = cudaLaunchAttributeClusterDimension;
+      attr[0].val.clusterDim.x = size; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+      cfg.attrs = attr; cfg.numAttrs = 1;
+      if (cudaOccupancyMaxActiveClusters(&got, kern, &cfg) != cudaSuccess) { (void)cudaGetLastError(); got = 0; }
+    }
+    n = got + 1;
+    cache[size].store(n, std::memory_order_relaxed);
+  }
+  return n - 1;
+}
+
+// More than 64 tokens run as CTA pairs (cta_group::2, 256 weight rows x up to 256 tokens).  The width of the token tile and the
+// split of K are those with the least estimated time, fitted to measurements: a k-block takes 0.235 us and 0.055 more for a full
+// 256 tokens (data and MMAs; narrow tiles are hardly faster, so what a narrow tile saves is an empty last round), a launch 3.9 us
+// and up to 3.3 for the epilogue of the last tile, an exchange 1.2 per further share and up to 2.  us with tiles of 256 and K
+// whole, and now: 200 x 4096 x 4096 23.5 / 14.9, 256 x 4096 x 14336 71.7 / 37.7, 700 x 2048 x 8192 49 / 24.5, 1339 x 2048 x 2048
+// 15.8 / 13.7, 2312 x 2048 x 8192 82.5 / 70.5, 333 x 6144 x 4096 24.7 / 22.1.
+// Up to 128 tokens the single-CTA kernel keeps what it splits into four shares of K or more (128 x 2048 x 8192: 14.3 us, 16.1 here).
+// fixed: the token tile has to be 256 wide and K whole (grouped rows).
+static bool plan_pairs(int T, int n_out, int K, int rows_out, bool fixed, GemmPlan& g) {
+  if (T <= 128 && g.splits >= 4) return false;
+  const int m_tiles = (n_out + rows_out - 1) / rows_out, kb_total = (K + BLK_K - 1) / BLK_K;
+  if (T <= WIDE_M || m_tiles < 2) return false;
+  const int pairs = (m_tiles + 1) / 2;
+  double best = 1e30;
+  for (int S = 1; S <= (fixed ? 1 : 4); ++S) {
+    if (S > 1 && kb_total / S < 4) break;
+    const int kb = (kb_total + S - 1) / S;
+    for (int tokn = 256; tokn >= (fixed ? 256 : 32); tokn -= 32) {
+      const int64_t tiles = (int64_t)pairs * ((T + tokn - 1) / tokn);
+      if (S > 1 && tiles > max_clusters_pair(2 * S)) break;              // narrower tiles are more tiles
+      const int64_t rounds = S > 1 ? 1 : (tiles + 73) / 74;
+      const double us = rounds * (kb * (0.235 + 0.055 * tokn / 256) + 0.3) + 3.9 + 3.3 * tokn / 256 + (S > 1 ? 1.2 * (S - 1) + 2.0 * tokn / 256 : 0.0);
+      if (us < best) {
+        best = us;
+        g.tokn = tokn; g.splits = S;
+      }
+    }
+  }
+  g.ws = false; g.pair = true;
+  g.m_tiles = m_tiles; g.n_tiles = (T + g.tokn - 1) / g.tokn;
+  g.kb_total = kb_total; g.kb_per_split = (kb_total + g.splits - 1) / g.splits;
+  g.splits = (kb_total + g.kb_per_split - 1) / g.kb_per_split;           // drop empty splits
+  return true;
+}
 
 template <bool GATED>
 static int dispatch_gemm(const GemmPlan& g, const CUtensorMap& tw, const CUtensorMap& tx, const GemmParams& p, cudaStream_t st) {
+  if (g.pair) return g.splits > 1 ? launch_gemm<256, true, GATED, true>(tw, tx, p, st) : launch_gemm<256, false, GATED, true>(tw, tx, p, st);
   if (g.ws) {
     switch (g.tokn) {
       case 16: return launch_gemm<16, false, GATED, false, true>(tw, tx, p, st);
@@ -1302,7 +1427,6 @@ static int dispatch_gemm(const GemmPlan& g, const CUtensorMap& tw, const CUtenso
     case 64: return launch_gemm<64, false, GATED>(tw, tx, p, st);
     case 128: return launch_gemm<128, false, GATED>(tw, tx, p, st);
     default:
-      if (gemm_uses_pair(g)) return launch_gemm<256, false, GATED, true>(tw, tx, p, st);
       return launch_gemm<256, false, GATED>(tw, tx, p, st);
   }
 }
@@ -1381,6 +1505,7 @@ extern "C" int KGE_GEMM_NAME(void* y, const void* x, const void* w, const void* 
   GemmPlan g = plan_gemm(T, N, K, BLK_M, workspace != nullptr);
   if (g.ws && (workspace_bytes < ws_bytes_of(g) || ((uintptr_t)workspace & 15) != 0))
     g = plan_gemm(T, N, K);                        // scratch too small for this shape: split K inside a cluster instead
+  if (!g.ws) (void)plan_pairs(T, N, K, BLK_M, false, g);
   GemmParams p;
   p.y = (bf16*)y; p.bias = (const bf16*)bias; p.T = T; p.N = N; p.K = K; p.act = act;
   p.l2_hints = tunable(TUN_GEMM_L2_HINTS);
@@ -1388,10 +1513,10 @@ extern "C" int KGE_GEMM_NAME(void* y, const void* x, const void* w, const void* 
   p.ws_count = g.ws ? (unsigned int*)workspace : nullptr;
   p.ws_part = g.ws ? (float*)((uint8_t*)workspace + kWsCounterBytes) : nullptr;
   p.m_tiles = g.m_tiles; p.n_tiles = g.n_tiles; p.splits = g.splits;
-  p.kb_total = g.kb_total; p.kb_per_split = g.kb_per_split;
+  p.kb_total = g.kb_total; p.kb_per_split = g.kb_per_split; p.tokn = g.tokn;
   CUtensorMap tw, tx;
   if (int rc = make_tmap(&tw, w, N, K, BLK_M)) return rc;
-  if (int rc = make_tmap(&tx, x, T, K, gemm_uses_pair(g) ? 128 : g.tokn)) return rc;
+  if (int rc = make_tmap(&tx, x, T, K, g.pair ? g.tokn / 2 : g.tokn)) return rc;
   cudaStream_t st = (cudaStream_t)stream;
   return dispatch_gemm<false>(g, tw, tx, p, st);
 }
@@ -1429,6 +1554,7 @@ static int gemm_gated(void* y, const void* x, const void* w_gate_up, int T, int 
   }
   GemmPlan g = plan_gemm(T, f, K, 64, workspace != nullptr);
   if (g.ws && (workspace_bytes < ws_bytes_of(g) || ((uintptr_t)workspace & 15) != 0)) g = plan_gemm(T, f, K, 64);
+  if (!g.ws) (void)plan_pairs(T, f, K, 64, false, g);
   GemmParams p;
   p.y = (bf16*)y; p.bias = (const bf16*)bias_gate_up; p.T = T; p.N = f; p.K = K; p.act = 2; p.glu = glu; p.glu_alpha = glu_alpha; p.glu_limit = glu_limit;
   p.l2_hints = tunable(TUN_GEMM_L2_HINTS);
@@ -1436,10 +1562,10 @@ static int gemm_gated(void* y, const void* x, const void* w_gate_up, int T, int 
   p.ws_count = g.ws ? (unsigned int*)workspace : nullptr;
   p.ws_part = g.ws ? (float*)((uint8_t*)workspace + kWsCounterBytes) : nullptr;
   p.m_tiles = g.m_tiles; p.n_tiles = g.n_tiles; p.splits = g.splits;
-  p.kb_total = g.kb_total; p.kb_per_split = g.kb_per_split;
+  p.kb_total = g.kb_total; p.kb_per_split = g.kb_per_split; p.tokn = g.tokn;
   CUtensorMap tw, tx;
   if (int rc = make_tmap(&tw, w_gate_up, 2 * (int64_t)f, K, 64)) return rc;     // 64-row boxes: gate half, up half
-  if (int rc = make_tmap(&tx, x, T, K, gemm_uses_pair(g) ? 128 : g.tokn)) return rc;
+  if (int rc = make_tmap(&tx, x, T, K, g.pair ? g.tokn / 2 : g.tokn)) return rc;
   return dispatch_gemm<true>(g, tw, tx, p, (cudaStream_t)stream);
 }
 
@@ -1469,17 +1595,18 @@ int gemm_grouped(void* y, const void* x, const void* w, int T, int N, int K, int
   KGE_REQUIRE(y && x && w && tile_group && groups > 0, "gemm_grouped: null pointer");
   KGE_REQUIRE(T > 256 && T % 256 == 0 && N > 0 && K > 0 && K % 8 == 0 && (!gated || N % 64 == 0), "gemm_grouped: T=%d N=%d K=%d", T, N, K);
   KGE_REQUIRE(((uintptr_t)x & 15) == 0 && ((uintptr_t)w & 15) == 0, "gemm_grouped: x and w must be 16-byte aligned");
-  const GemmPlan g = plan_gemm(T, N, K, gated ? 64 : BLK_M);
+  GemmPlan g = plan_gemm(T, N, K, gated ? 64 : BLK_M);
+  (void)plan_pairs(T, N, K, gated ? 64 : BLK_M, true, g);
   KGE_REQUIRE(!g.ws && g.splits == 1 && 256 % g.tokn == 0, "gemm_grouped: internal: unexpected plan");
   GemmParams p;
   p.y = (bf16*)y; p.bias = nullptr; p.T = T; p.N = N; p.K = K; p.act = gated ? 2 : (glu == -2 ? 4 : 0);
   p.glu = gated ? glu : 0; p.glu_alpha = glu_alpha; p.glu_limit = glu_limit;
   p.l2_hints = tunable(TUN_GEMM_L2_HINTS); p.trace = g_gemm_trace; p.ws_count = nullptr; p.ws_part = nullptr;
-  p.m_tiles = g.m_tiles; p.n_tiles = g.n_tiles; p.splits = g.splits; p.kb_total = g.kb_total; p.kb_per_split = g.kb_per_split;
+  p.m_tiles = g.m_tiles; p.n_tiles = g.n_tiles; p.splits = g.splits; p.kb_total = g.kb_total; p.kb_per_split = g.kb_per_split; p.tokn = g.tokn;
   p.tile_group = tile_group; p.group_rows = gated ? 2 * N : N;
   CUtensorMap tw, tx;
   if (int rc = make_tmap(&tw, w, (int64_t)groups * p.group_rows, K, gated ? 64 : BLK_M)) return rc;
-  if (int rc = make_tmap(&tx, x, T, K, gemm_uses_pair(g) ? 128 : g.tokn)) return rc;
+  if (int rc = make_tmap(&tx, x, T, K, g.pair ? g.tokn / 2 : g.tokn)) return rc;
   return gated ? dispatch_gemm<true>(g, tw, tx, p, st) : dispatch_gemm<false>(g, tw, tx, p, st);
 }
 }  // namespace KGE_ELT_NS

@@ -334,6 +334,23 @@ def test_gemm_silu_gate_few_rows(kge, L, T, f, K):
     test_gemm_silu_gate_fused(kge, L, T, f, K)
 
 
+PAIR_CASES = [(65, 264, 64, True, 0), (129, 1000, 1096, True, 3), (200, 4096, 4096, False, 1), (255, 513, 2056, True, 0), (256, 4096, 14336, False, 0),
+              (257, 129, 520, False, 4), (333, 6144, 4096, True, 0), (512, 3072, 2048, False, 0), (700, 2048, 8192, True, 1), (1339, 2048, 2048, False, 0),
+              (2312, 2047, 1032, True, 0)]
+
+
+@pytest.mark.parametrize("T,N,K,bias,act", PAIR_CASES)
+def test_gemm_pairs(kge, L, T, N, K, bias, act):
+    """CTA pairs with token tiles of 32 to 256, an odd number of k-blocks, K split over two to four pairs of a cluster, a last weight
+    tile that is missing or ragged, outputs that cannot be stored 16 bytes at a time; the bound of the few-row projections."""
+    test_gemm_few_rows(kge, L, T, N, K, bias, act, "bf16")
+
+
+@pytest.mark.parametrize("T,f,K", [(65, 64, 520), (129, 192, 4096), (300, 1984, 2056), (777, 8192, 2048)])
+def test_gemm_silu_gate_pairs(kge, L, T, f, K):
+    test_gemm_silu_gate_fused(kge, L, T, f, K)
+
+
 @pytest.mark.parametrize("T,N,K,bias,act", [c for c in GEMM_CASES if c[0] <= 64])
 def test_gemm_128_row_tiles_for_small_batches(kge, L, T, N, K, bias, act):
     """Knob gemm_wide=0: batches of up to 64 tokens through the 128-row weight tiles (tokens as MMA N) instead of the
