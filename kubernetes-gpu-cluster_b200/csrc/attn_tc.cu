@@ -197,7 +197,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
   const uint32_t p_full = bar0 + 48, o_full = bar0 + 56, q_full = bar0 + 64;
   auto v_empty = [&](int s) { return bar0 + 72u + 8u * s; };
 
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = uniform_warp(), lane = tid & 31;
   if (warp == 4) {
     if (lane == 0) {
       // TMA: the producer's expect_tx is the one arrival of a K/V barrier; cp.async: every loading thread arrives
@@ -227,17 +227,17 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
 
   if (warp == 4) {
     // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
+    if (elect_one()) {
       auto issue_s = [&](int j) {
         const int st = j & 1;
         mbar_wait(k_full(st), (uint32_t)((j >> 1) & 1));
         tc_after();
-        const uint32_t kt = sK + st * TILE_BYTES;
+        const uint64_t qd = desc_kmajor(sQ), kd = desc_kmajor(sK + st * TILE_BYTES);
 #pragma unroll
         for (int k = 0; k < HD / 16; ++k) {
           const uint32_t qoff = (uint32_t)((k >> 2) * (128 * 128) + (k & 3) * 32);
           const uint32_t koff = (uint32_t)((k >> 2) * (BNK * 128) + (k & 3) * 32);
-          tc_mma(tmem + st * BNK, desc_kmajor(sQ + qoff), desc_kmajor(kt + koff), IDESC_S, k > 0 ? 1u : 0u);
+          tc_mma(tmem + st * BNK, qd + (qoff >> 4), kd + (koff >> 4), IDESC_S, k > 0 ? 1u : 0u);
         }
         tc_commit(s_full(st));
       };
@@ -250,12 +250,12 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
         mbar_wait(p_full, (uint32_t)(j & 1));
         mbar_wait(v_full(j & 1), (uint32_t)((j >> 1) & 1));
         tc_after();
-        const uint32_t vt = sV + (j & 1) * TILE_BYTES;
+        const uint64_t pd = desc_kmajor(sP), vd = desc_mnmajor(sV + (j & 1) * TILE_BYTES);
 #pragma unroll
         for (int k = 0; k < BNK / 16; ++k) {
           const uint32_t aoff = (uint32_t)((k >> 2) * (128 * 128) + (k & 3) * 32);   // P: keys are the K dimension (one 64-key half)
           const uint32_t boff = (uint32_t)(k * 16 * 128);                             // V: 16 keys = 16 rows of 128 B
-          tc_mma(tmem + O_COL, desc_kmajor(sP + aoff), desc_mnmajor(vt + boff), IDESC_O, (j > 0 || k > 0) ? 1u : 0u);
+          tc_mma(tmem + O_COL, pd + (aoff >> 4), vd + (boff >> 4), IDESC_O, (j > 0 || k > 0) ? 1u : 0u);
         }
         tc_commit(o_full);
         if (TMA) tc_commit(v_empty(j & 1));      // PV_j has read V stage j&1: the producer may refill it
@@ -266,7 +266,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
     // One thread: per tile it reads the tile's block ids and issues one box per (block, 64-column half).  (Spreading the
     // issue over several lanes with the block ids handed out by shuffle measured SLOWER here: 364 vs 471 TFLOP/s at
     // 4 x 2048, profiles/r02_vs_libs_*.json; a prefill tile lasts long enough for one thread to stay ahead.)
-    if (lane == 0) {
+    if (elect_one()) {
       const int bs = 1 << bs_shift;
       const int box_rows = bs < BNK ? bs : BNK;
       const int boxes = BNK / box_rows;

@@ -131,6 +131,18 @@ inline cudaError_t launch_pdl(void (*kern)(KArgs...), dim3 grid, dim3 block, siz
   return cudaLaunchKernelEx(&cfg, kern, KArgs(args)...);
 }
 
+// One lane of a converged warp, for the instructions that one thread issues (TMA copies, tcgen05.mma, commits).  Behind this
+// branch the compiler knows that a single lane runs and keeps descriptors and addresses in uniform registers, where those
+// instructions want them; behind `lane == 0` it moves them there before each one, which paced the MMA loops: 88 cycles to issue
+// a tcgen05.mma whatever its shape, against 35 to 48 here (128 x 64 x 16 then runs in 48 cycles, 128 x 128 in 65, 128 x 256 in 128).
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n.reg .pred q;\nelect.sync _|q, 0xffffffff;\nselp.u32 %0, 1, 0, q;\n}" : "=r"(p));
+  return p != 0;
+}
+// the warp's index as a value that is the same in all its lanes
+__device__ __forceinline__ int uniform_warp() { return __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0); }
+
 __device__ __forceinline__ uint4 ld_nc_v4(const void* p) {
   uint4 r;
   asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];"

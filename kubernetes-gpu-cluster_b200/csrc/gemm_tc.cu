@@ -271,7 +271,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant
   auto tfull_bar = [&](int s) { return bar_base + 8u * (2 * STAGES + s); };
   auto tempty_bar = [&](int s) { return bar_base + 8u * (2 * STAGES + 2 + s); };
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = uniform_warp(), lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     trace_stamp(p, 0);
     if (p.trace) { uint32_t sm; asm volatile("mov.u32 %0, %%smid;" : "=r"(sm)); p.trace[(size_t)blockIdx.x * 16 + 15] = sm; }
@@ -347,7 +347,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant
   if (XSPLIT) cluster_arrive_relaxed();                  // phase A: every CTA of the cluster has started (nothing to publish: no release)
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       int stage = 0; uint32_t phase = 0;
       const bool hint = p.l2_hints != 0;
       const uint64_t pol_w = l2_policy(false), pol_x = l2_policy(true);
@@ -438,7 +438,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant
       trace_stamp(p, 4);
     }
   } else if (warp == 1) {
-    if (lane == 0 && (!PAIR || mrank == 0)) {          // PAIR: the leader issues for both CTAs
+    if ((!PAIR || mrank == 0) && elect_one()) {        // PAIR: the leader issues for both CTAs
       int stage = 0; uint32_t phase = 0;
       int acc = 0; uint32_t acc_phase = 0;
       SegIter it = segments();
@@ -851,7 +851,7 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
   auto empty_bar = [&](int s) { return bar_base + 8u * (STAGES + s); };
   const uint32_t tfull_bar = bar_base + 8u * (2 * STAGES);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = uniform_warp(), lane = threadIdx.x & 31;
   if (threadIdx.x == 0) trace_stamp(p, 0);
   if (warp == 0 && lane == 0) {
     asm volatile("prefetch.tensormap [%0];" ::"l"(&tmap_w) : "memory");
@@ -881,7 +881,7 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
   const int n0 = m_tile * OUT_PER_TILE;                                         // first output column of the tile
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       auto load_w = [&](int st, int kb) {
         const uint32_t dst = smem_base + st * WIDE_STAGE + WIDE_A_BYTES;
         if (GATED) {
@@ -914,7 +914,7 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
       trace_stamp(p, 4);
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (elect_one()) {
       if (p.trace) { mbar_wait(full_bar(0), 0); trace_stamp(p, 5); }
       int stage = 0; uint32_t phase = 0;
       const uint64_t adesc0 = umma_desc_sw128(smem_base), bdesc0 = umma_desc_sw128(smem_base + WIDE_A_BYTES);
