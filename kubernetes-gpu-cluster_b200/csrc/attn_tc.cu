@@ -4,9 +4,8 @@
 // causal prefix of that request, walked in 64-key tiles (two CTAs per SM):
 //   S  = Q K^T      tcgen05.mma, A = Q tile, B = K tile (both K-major, 128B swizzle), D in TMEM (2 buffers)
 //   P  = softmax    4 warps, ONE THREAD PER ROW: tcgen05.ld its S row, scale + causal mask + running
-//                   max/sum in fp32 (no shuffles), bf16 P written straight into the swizzled A-operand
-//                   layout in shared memory
-//   O_t = P V       tcgen05.mma, A = P, B = V tile as stored ([key][hd] = MN-major), D in TMEM [128,128+hd)
+//                   max/sum in fp32 (no shuffles), bf16 P written over the row's scores in TMEM (tcgen05.st)
+//   O_t = P V       tcgen05.mma, A = P from TMEM, B = V tile as stored ([key][hd] = MN-major), D in TMEM [128,128+hd)
 //   O accumulates in TMEM across tiles; it is rescaled (tcgen05.ld / st) only when a row's running maximum has grown
 //   by more than 2^8 since its reference maximum was fixed (lazy rescale, see kRescaleThreshold below)
 // K/V tiles (TMA = true, the default): a producer thread fetches every tile from the paged cache with
@@ -68,6 +67,11 @@ __device__ __forceinline__ void tc_commit(uint32_t bar) {
 __device__ __forceinline__ void tc_mma(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t acc) {
   asm volatile("{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\ntcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}"
                ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(acc) : "memory");
+}
+// A from TMEM (rows = lanes, two 16-bit numbers per column)
+__device__ __forceinline__ void tc_mma_ts(uint32_t d, uint32_t a, uint64_t b, uint32_t idesc, uint32_t acc) {
+  asm volatile("{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\ntcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}"
+               ::"r"(d), "r"(a), "l"(b), "r"(idesc), "r"(acc) : "memory");
 }
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
   asm volatile(
@@ -151,8 +155,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
   constexpr int CH = HD / 8;                       // 16-byte chunks per row
   constexpr uint32_t Q_BYTES = 128 * HD * 2;
   constexpr uint32_t TILE_BYTES = BNK * HD * 2;    // K or V tile
-  constexpr uint32_t P_BYTES = 128 * BNK * 2;
-  constexpr uint32_t TMEM_COLS = 256;              // S0 [0,64), S1 [64,128), O [128,128+HD)
+  constexpr uint32_t TMEM_COLS = 256;              // S0 [0,64), S1 [64,128), O [128,128+HD); P_j over the first half of S_j
   constexpr uint32_t O_COL = 128;
   // S: M=128, N=128, both K-major.  PV: M=128, N=HD, A K-major, B MN-major (bit 16).
   constexpr uint32_t IDESC_S = (1u << 4) | KGE_IDESC_AB | ((uint32_t)(BNK >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
@@ -186,15 +189,15 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
   const uint32_t sQ = s_addr(smem);
   const uint32_t sK = sQ + Q_BYTES;                // 2 stages
   const uint32_t sV = sK + 2 * TILE_BYTES;         // 2 stages
-  const uint32_t sP = sV + 2 * TILE_BYTES;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + Q_BYTES + 4 * TILE_BYTES + P_BYTES);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + Q_BYTES + 4 * TILE_BYTES);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 12);
   const uint32_t bar0 = s_addr(bars);
-  // k_full[2], v_full[2], s_full[2], p_full, o_full, q_full, v_empty[2]
+  // k_full[2], v_full[2], s_full[2], p_full[0], o_full, q_full, v_empty[2], p_full[1]
   auto k_full = [&](int s) { return bar0 + 8u * s; };
   auto v_full = [&](int s) { return bar0 + 16u + 8u * s; };
   auto s_full = [&](int s) { return bar0 + 32u + 8u * s; };
-  const uint32_t p_full = bar0 + 48, o_full = bar0 + 56, q_full = bar0 + 64;
+  const uint32_t o_full = bar0 + 56, q_full = bar0 + 64;
+  auto p_full = [&](int s) { return bar0 + 48u + 40u * s; };      // two in turn: a warp may be a tile ahead of another
   auto v_empty = [&](int s) { return bar0 + 72u + 8u * s; };
 
   const int tid = threadIdx.x, warp = uniform_warp(), lane = tid & 31;
@@ -204,7 +207,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
       mbar_init(k_full(0), TMA ? 1 : 128); mbar_init(k_full(1), TMA ? 1 : 128);
       mbar_init(v_full(0), TMA ? 1 : 128); mbar_init(v_full(1), TMA ? 1 : 128);
       mbar_init(s_full(0), 1); mbar_init(s_full(1), 1);
-      mbar_init(p_full, 128); mbar_init(o_full, 1);
+      mbar_init(p_full(0), 128); mbar_init(p_full(1), 128); mbar_init(o_full, 1);
       mbar_init(q_full, 128); mbar_init(v_empty(0), 1); mbar_init(v_empty(1), 1);
       asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
       if (TMA) {
@@ -244,18 +247,21 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
       if (TMA) { mbar_wait(q_full, 0u); tc_after(); }      // the Q tile (cp.async by the softmax threads) has landed
       issue_s(0);
       for (int j = 0; j < ntiles; ++j) {
-        // S_{j+1} may overwrite S buffer (j+1)&1 = the buffer of S_{j-1}: the softmax warps finished
-        // reading it before they arrived on p_full(j-1), which this thread has already waited for
-        if (j + 1 < ntiles) issue_s(j + 1);
-        mbar_wait(p_full, (uint32_t)(j & 1));
+        // S_{j+1} overwrites S buffer (j+1)&1 = the buffer of S_{j-1} and P_{j-1}: the softmax warps finished reading the scores
+        // before they arrived on p_full(j-1), which this thread has waited for; PV_{j-1} must have read P_{j-1} (MMAs of different
+        // shapes are not ordered among themselves) - it runs while the softmax warps are busy with tile j
+        if (j + 1 < ntiles) {
+          if (j > 0) { mbar_wait(o_full, (uint32_t)((j - 1) & 1)); tc_after(); }
+          issue_s(j + 1);
+        }
+        mbar_wait(p_full(j & 1), (uint32_t)((j >> 1) & 1));
         mbar_wait(v_full(j & 1), (uint32_t)((j >> 1) & 1));
         tc_after();
-        const uint64_t pd = desc_kmajor(sP), vd = desc_mnmajor(sV + (j & 1) * TILE_BYTES);
+        const uint64_t vd = desc_mnmajor(sV + (j & 1) * TILE_BYTES);
 #pragma unroll
         for (int k = 0; k < BNK / 16; ++k) {
-          const uint32_t aoff = (uint32_t)((k >> 2) * (128 * 128) + (k & 3) * 32);   // P: keys are the K dimension (one 64-key half)
           const uint32_t boff = (uint32_t)(k * 16 * 128);                             // V: 16 keys = 16 rows of 128 B
-          tc_mma(tmem + O_COL, pd + (aoff >> 4), vd + (boff >> 4), IDESC_O, (j > 0 || k > 0) ? 1u : 0u);
+          tc_mma_ts(tmem + O_COL, tmem + (j & 1) * BNK + k * 8, vd + (boff >> 4), IDESC_O, (j > 0 || k > 0) ? 1u : 0u);
         }
         tc_commit(o_full);
         if (TMA) tc_commit(v_empty(j & 1));      // PV_j has read V stage j&1: the producer may refill it
@@ -405,9 +411,12 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
       }
       const float mx_raw = fmaxf(fmaxf(mxa[0], mxa[1]), fmaxf(mxa[2], mxa[3]));
       const float mx = mx_raw * scale_log2;                     // -inf stays -inf
-      // PV_{j-1} must be done before O is rescaled, sP is overwritten or V stage (j+1)&1 is refilled
-      if (j > 0) { mbar_wait(o_full, (uint32_t)((j - 1) & 1)); tc_after(); }
-      if (!TMA) load_tile(j + 1, false);
+      // PV_{j-1} must be done before O is rescaled (or, cp.async path, V stage (j+1)&1 refilled); otherwise the softmax runs ahead
+      // of it (PV_{j-2} was done before S_j was issued, so the parity is unambiguous)
+      if (!TMA) {
+        if (j > 0) { mbar_wait(o_full, (uint32_t)((j - 1) & 1)); tc_after(); }
+        load_tile(j + 1, false);
+      }
       const bool grow = mx > m_ref + kRescaleThreshold;        // includes the first finite maximum
       if (__any_sync(0xffffffffu, grow)) {
         float alpha = 1.f;
@@ -417,6 +426,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
           l *= alpha;
         }
         if (j > 0) {
+          if (TMA) { mbar_wait(o_full, (uint32_t)((j - 1) & 1)); tc_after(); }
 #pragma unroll 1
           for (int c = 0; c < HD; c += 32) {
             uint32_t v[32];
@@ -429,27 +439,25 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
       }
       const float base = (m_ref == -INFINITY) ? 0.f : m_ref;
       float rsa[4] = {0.f, 0.f, 0.f, 0.f};
+      uint32_t pk[BNK / 2];
 #pragma unroll
-      for (int c8 = 0; c8 < BNK / 8; ++c8) {
-        uint32_t pk[4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const float p0 = ex2_ftz(fmaf(__uint_as_float(sv[c8 * 8 + i * 2]), scale_log2, -base));       // masked: -inf -> 0
-          const float p1 = ex2_ftz(fmaf(__uint_as_float(sv[c8 * 8 + i * 2 + 1]), scale_log2, -base));
-          rsa[i] += p0 + p1;
-          pk[i] = pack_bf2(p0, p1);
-        }
-        const uint32_t dst = sP + tile_off<128>(r, c8);
-        asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(dst), "r"(pk[0]), "r"(pk[1]), "r"(pk[2]), "r"(pk[3]) : "memory");
+      for (int i = 0; i < BNK / 2; ++i) {
+        const float p0 = ex2_ftz(fmaf(__uint_as_float(sv[2 * i]), scale_log2, -base));       // masked: -inf -> 0
+        const float p1 = ex2_ftz(fmaf(__uint_as_float(sv[2 * i + 1]), scale_log2, -base));
+        rsa[i & 3] += p0 + p1;
+        pk[i] = pack_bf2(p0, p1);
       }
+      tmem_st32(t_row + (j & 1) * BNK, pk);
       l += (rsa[0] + rsa[1]) + (rsa[2] + rsa[3]);
       if (!TMA) cp_wait<2>();             // V_j (committed one tile ago) has landed
-      fence_async_smem();                 // P (and, cp.async path, V_j) bytes -> tensor-core proxy
+      if (!TMA) fence_async_smem();       // V_j bytes -> tensor-core proxy
       tc_before();                        // my TMEM reads/writes are ordered before the MMAs that follow
       if (!TMA) mbar_arrive(v_full(j & 1));
-      mbar_arrive(p_full);
+      mbar_arrive(p_full(j & 1));
     }
     if (!TMA) cp_wait<0>();
+    // the last scores say that PV_{ntiles-3} is done: the next two phases in turn, so that neither parity is taken for an older one
+    if (ntiles > 1) mbar_wait(o_full, (uint32_t)((ntiles - 2) & 1));
     mbar_wait(o_full, (uint32_t)((ntiles - 1) & 1));
     tc_after();
     {
@@ -483,7 +491,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
   }
 }
 
-template <int HD> constexpr int tc_smem() { return 128 * HD * 2 + 4 * BNK * HD * 2 + 128 * BNK * 2 + 256; }
+template <int HD> constexpr int tc_smem() { return 128 * HD * 2 + 4 * BNK * HD * 2 + 256; }
 
 }  // namespace atc
 
