@@ -37,9 +37,72 @@ __global__ void rglru_conv_kernel(RglruArgs a) {
   }
 }
 
+// The same for bfloat16 rows in 16-byte pieces: a thread takes eight channels of four tokens, so that all its loads (taps x tokens,
+// and the taps' weights once) are in flight together.  Same order of summation.  2312 tokens x 2560: 28 us (43 with a
+// channel per thread and pass), 2 tokens: 10 us (27).
+constexpr int RC_TOK = 4;
+__global__ void __launch_bounds__(128) rglru_conv_vec_kernel(RglruArgs a) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const int c = (blockIdx.y * 128 + threadIdx.x) * 8, t0 = blockIdx.x * RC_TOK;
+  if (c >= a.width) return;
+  const __nv_bfloat16* yx = (const __nv_bfloat16*)a.yx + a.width + c;
+  float acc[RC_TOK][8], bias[8];
+  int back_rows[RC_TOK], back_pos[RC_TOK], p0s[RC_TOK];
+  const float* tails[RC_TOK];
+  {
+    const uint4 v = *reinterpret_cast<const uint4*>((const __nv_bfloat16*)a.conv_b + c);
+    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+    for (int i = 0; i < 8; ++i) bias[i] = (i & 1) ? bf_hi(w[i / 2]) : bf_lo(w[i / 2]);
+  }
+#pragma unroll
+  for (int k = 0; k < RC_TOK; ++k) {
+    const int t = min(t0 + k, a.T - 1), b = a.token_req[t], rs = a.qsl[b];
+    p0s[k] = a.positions[rs];
+    back_pos[k] = a.positions[t];
+    back_rows[k] = t;
+    tails[k] = a.state + (int64_t)a.slots[b] * a.slot_stride + a.width + c;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) acc[k][i] = bias[i];
+  }
+#pragma unroll 4
+  for (int j = 0; j < a.taps; ++j) {
+    const int back = a.taps - 1 - j;
+    float w[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) w[i] = ldf((const __nv_bfloat16*)a.conv_w + (int64_t)(c + i) * a.taps + j);
+#pragma unroll
+    for (int k = 0; k < RC_TOK; ++k) {
+      const int sp = back_pos[k] - back;
+      float x[8];
+      if (sp >= p0s[k]) {
+        const uint4 v = *reinterpret_cast<const uint4*>(yx + (int64_t)(back_rows[k] - back) * 2 * a.width);
+        const uint32_t u[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int i = 0; i < 8; ++i) x[i] = (i & 1) ? bf_hi(u[i / 2]) : bf_lo(u[i / 2]);
+      } else {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) x[i] = sp >= 0 ? tails[k][(int64_t)(sp - p0s[k] + a.taps - 1) * a.width + i] : 0.f;
+      }
+#pragma unroll
+      for (int i = 0; i < 8; ++i) acc[k][i] = fmaf(w[i], x[i], acc[k][i]);
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < RC_TOK; ++k)
+    if (t0 + k < a.T)
+      *reinterpret_cast<uint4*>((__nv_bfloat16*)a.u + (int64_t)(t0 + k) * a.width + c) =
+          make_uint4(pack_bf2(acc[k][0], acc[k][1]), pack_bf2(acc[k][2], acc[k][3]), pack_bf2(acc[k][4], acc[k][5]), pack_bf2(acc[k][6], acc[k][7]));
+}
+
 int rglru_conv(const RglruArgs& a, cudaStream_t st) {
   if (a.T <= 0) return 0;
   KGE_REQUIRE(a.taps >= 1 && a.taps <= MAX_TAPS, "rglru_conv: %d taps (1..%d)", a.taps, MAX_TAPS);
+  if (a.elt == KGE_ELT_BF16 && a.width % 8 == 0 && ((reinterpret_cast<uintptr_t>(a.yx) | reinterpret_cast<uintptr_t>(a.u) | reinterpret_cast<uintptr_t>(a.conv_b)) & 15) == 0) {
+    KGE_CUDA_OK(launch_pdl(rglru_conv_vec_kernel, dim3((a.T + RC_TOK - 1) / RC_TOK, (a.width / 8 + 127) / 128), dim3(128), 0, st, a));
+    return 0;
+  }
   cudaError_t ce = a.elt == KGE_ELT_F32 ? launch_pdl(rglru_conv_kernel<float>, dim3(a.T), dim3(256), 0, st, a)
                                         : launch_pdl(rglru_conv_kernel<__nv_bfloat16>, dim3(a.T), dim3(256), 0, st, a);
   KGE_CUDA_OK(ce);
@@ -111,50 +174,86 @@ __global__ void __launch_bounds__(128) rglru_scan_kernel(RglruArgs a) {
 // Prompt steps: everything of the recurrence that does not depend on the previous token is done for all tokens at once.
 // rglru_ab_kernel turns the gate pre-activations, in place, into the recurrence's coefficients (a_t, b_t = sqrt(1 - a_t^2)
 // i_t u_t); rglru_chain_kernel is then one fma per token and channel (S_t written over a_t) plus the state hand-over; and
-// rglru_out_kernel multiplies by gelu(y).  Same arithmetic per element as the fused kernel.
+// rglru_out_kernel multiplies by gelu(y).  Same arithmetic per element as the fused kernel.  A thread keeps its channel and walks
+// over tokens (no divisions by the width).  2312 tokens x 2560, us
+// (before): coefficients 41 (50), chain 57 (145), products 17 (23).  All three in one kernel, with seven warps of a block feeding the
+// chain, took 422: too few warps for the exponentials' latency.
 template <typename E>
-__global__ void rglru_ab_kernel(RglruArgs a, float* gates) {
+__global__ void __launch_bounds__(256) rglru_ab_kernel(RglruArgs a, float* gates) {
   pdl_launch_dependents();
   pdl_wait();
-  const int64_t n = (int64_t)a.T * a.width;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t t = i / a.width; const int c = (int)(i % a.width);
-    const float sp = a.decay_c * softplusf_(ldf((const E*)a.lam + c));
-    const float r = sigmoidf_(gates[t * 2 * a.width + c]), ig = sigmoidf_(gates[t * 2 * a.width + a.width + c]);
+  const int c = blockIdx.y * 256 + threadIdx.x;
+  if (c >= a.width) return;
+  const float sp = a.decay_c * softplusf_(ldf((const E*)a.lam + c));
+  for (int t = blockIdx.x; t < a.T; t += gridDim.x) {
+    float* gt = gates + (int64_t)t * 2 * a.width + c;
+    const float r = sigmoidf_(gt[0]), ig = sigmoidf_(gt[a.width]);
     const float log_a = -sp * r;
-    gates[t * 2 * a.width + c] = expf(log_a);
-    gates[t * 2 * a.width + a.width + c] = sqrtf(-expm1f(2.f * log_a)) * ig * ldf((const E*)a.u + t * a.width + c);
+    gt[0] = expf(log_a);
+    gt[a.width] = sqrtf(-expm1f(2.f * log_a)) * ig * ldf((const E*)a.u + (int64_t)t * a.width + c);
   }
 }
 
+// One warp per 32 channels of a request: the coefficients of 64 tokens at a time arrive by cp.async, three stages ahead, so that the
+// chain waits for its fma's and not for memory (with eight tokens' loads in flight it took 145 us).
+constexpr int RS_TOK = 64, RS_STAGES = 4, RS_SMEM = RS_STAGES * 2 * RS_TOK * 32 * 4;
 template <typename E>
-__global__ void __launch_bounds__(128) rglru_chain_kernel(RglruArgs a, float* gates) {
+__global__ void __launch_bounds__(32) rglru_chain_kernel(RglruArgs a, float* gates) {
   pdl_launch_dependents();
   pdl_wait();
-  const int b = blockIdx.x, c = blockIdx.y * blockDim.x + threadIdx.x;
-  if (c >= a.width) return;
-  const int rs = a.qsl[b], re = a.qsl[b + 1], p0 = a.positions[rs], n = re - rs;
+  extern __shared__ __align__(16) float rs_sm[];          // [stage][a | b][token][channel]
+  const int b = blockIdx.x, lane = threadIdx.x, c0 = blockIdx.y * 32, c = c0 + lane;
+  const bool in = c < a.width;
+  const int rs = a.qsl[b], re = a.qsl[b + 1], n = re - rs;
+  if (n <= 0) return;
+  const int p0 = a.positions[rs], tiles = (n + RS_TOK - 1) / RS_TOK;
   float* slot = a.state + (int64_t)a.slots[b] * a.slot_stride;
   const E* yx = (const E*)a.yx;
-  float S = p0 > 0 ? slot[c] : 0.f;
-  constexpr int G = 8;
-  for (int t0 = rs; t0 < re; t0 += G) {
-    float av[G], bv[G];
+  auto fetch = [&](int tile) {
+    if (tile < tiles) {
+      float* dst = rs_sm + (tile % RS_STAGES) * (2 * RS_TOK * 32);
+      const int len = min(RS_TOK, n - tile * RS_TOK), piece = (lane & 7) * 4, left = a.width - c0 - piece;
+      const int bytes = left >= 4 ? 16 : left > 0 ? left * 4 : 0;
+      for (int k = lane >> 3; k < len; k += 4) {
+        const float* src = gates + (int64_t)(rs + tile * RS_TOK + k) * 2 * a.width + (bytes > 0 ? c0 + piece : 0);
 #pragma unroll
-    for (int k = 0; k < G; ++k) {
-      const int t = min(t0 + k, re - 1);
-      av[k] = gates[(int64_t)t * 2 * a.width + c];
-      bv[k] = gates[(int64_t)t * 2 * a.width + a.width + c];
-    }
-#pragma unroll
-    for (int k = 0; k < G; ++k) {
-      if (t0 + k < re) {
-        S = fmaf(av[k], S, bv[k]);
-        gates[(int64_t)(t0 + k) * 2 * a.width + c] = S;
+        for (int w = 0; w < 2; ++w)
+          asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst + (w * RS_TOK + k) * 32 + piece)), "l"(src + w * a.width), "r"(bytes) : "memory");
       }
     }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  float S = in && p0 > 0 ? slot[c] : 0.f;
+#pragma unroll
+  for (int i = 0; i < RS_STAGES - 1; ++i) fetch(i);
+  for (int tile = 0; tile < tiles; ++tile) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(RS_STAGES - 2) : "memory");
+    __syncwarp();
+    fetch(tile + RS_STAGES - 1);                           // the stage that the previous turn has read
+    const float* av = rs_sm + (tile % RS_STAGES) * (2 * RS_TOK * 32) + lane;
+    const float* bv = av + RS_TOK * 32;
+    const int len = min(RS_TOK, n - tile * RS_TOK);
+    float* out = gates + (int64_t)(rs + tile * RS_TOK) * 2 * a.width + c;
+    int k = 0;
+    for (; k + 16 <= len; k += 16) {
+      float x[16], y[16];
+#pragma unroll
+      for (int i = 0; i < 16; ++i) { x[i] = av[(k + i) * 32]; y[i] = bv[(k + i) * 32]; }
+#pragma unroll
+      for (int i = 0; i < 16; ++i) {
+        S = fmaf(x[i], S, y[i]);
+        if (in) out[(int64_t)(k + i) * 2 * a.width] = S;
+      }
+    }
+    for (; k < len; ++k) {
+      S = fmaf(av[k * 32], S, bv[k * 32]);
+      if (in) out[(int64_t)k * 2 * a.width] = S;
+    }
+    __syncwarp();
   }
+  if (!in) return;
   slot[c] = S;
+  // the convolution's next inputs: the last taps - 1 rows of this step, or of the old tail
   float nt[MAX_TAPS];
   float* tail = slot + a.width;
 #pragma unroll
@@ -174,14 +273,26 @@ __global__ void __launch_bounds__(128) rglru_chain_kernel(RglruArgs a, float* ga
 }
 
 template <typename E>
-__global__ void rglru_out_kernel(RglruArgs a, const float* gates) {
+__global__ void __launch_bounds__(256) rglru_out_kernel(RglruArgs a, const float* gates) {
   pdl_launch_dependents();
   pdl_wait();
-  const int64_t n = (int64_t)a.T * a.width;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t t = i / a.width; const int c = (int)(i % a.width);
-    stf((E*)a.out + i, gates[t * 2 * a.width + c] * gelu_tanhf_(ldf((const E*)a.yx + t * 2 * a.width + c)));
-  }
+  const int c = blockIdx.y * 256 + threadIdx.x;
+  if (c >= a.width) return;
+  for (int t = blockIdx.x; t < a.T; t += gridDim.x)
+    stf((E*)a.out + (int64_t)t * a.width + c, gates[(int64_t)t * 2 * a.width + c] * gelu_tanhf_(ldf((const E*)a.yx + (int64_t)t * 2 * a.width + c)));
+}
+
+template <typename E>
+static int rglru_prompt(const RglruArgs& a, cudaStream_t st) {
+  float* gates = const_cast<float*>(a.gates);
+  const int slices = (a.width + 255) / 256;
+  const dim3 eg(std::min(a.T, std::max(1, 148 * 8 / slices)), slices), cg(a.B, (a.width + 31) / 32);
+  KGE_REQUIRE(cg.y <= 65535, "rglru_scan: width %d", a.width);
+  KGE_CUDA_OK(cudaFuncSetAttribute(rglru_chain_kernel<E>, cudaFuncAttributeMaxDynamicSharedMemorySize, RS_SMEM));
+  KGE_CUDA_OK(launch_pdl(rglru_ab_kernel<E>, eg, dim3(256), 0, st, a, gates));
+  KGE_CUDA_OK(launch_pdl(rglru_chain_kernel<E>, cg, dim3(32), RS_SMEM, st, a, gates));
+  KGE_CUDA_OK(launch_pdl(rglru_out_kernel<E>, eg, dim3(256), 0, st, a, (const float*)gates));
+  return 0;
 }
 
 int rglru_scan(const RglruArgs& a, cudaStream_t st) {
@@ -189,18 +300,8 @@ int rglru_scan(const RglruArgs& a, cudaStream_t st) {
   KGE_REQUIRE(a.taps >= 1 && a.taps <= MAX_TAPS, "rglru_scan: %d taps (1..%d)", a.taps, MAX_TAPS);
   const dim3 grid(a.B, (a.width + 127) / 128), block(128);
   if (a.T > a.B) {                       // some request brings several rows
-    float* gates = const_cast<float*>(a.gates);
-    const int eg = (int)std::min<int64_t>(((int64_t)a.T * a.width + 255) / 256, 148 * 16);
-    if (a.elt == KGE_ELT_F32) {
-      KGE_CUDA_OK(launch_pdl(rglru_ab_kernel<float>, dim3(eg), dim3(256), 0, st, a, gates));
-      KGE_CUDA_OK(launch_pdl(rglru_chain_kernel<float>, grid, block, 0, st, a, gates));
-      KGE_CUDA_OK(launch_pdl(rglru_out_kernel<float>, dim3(eg), dim3(256), 0, st, a, (const float*)gates));
-    } else {
-      KGE_CUDA_OK(launch_pdl(rglru_ab_kernel<__nv_bfloat16>, dim3(eg), dim3(256), 0, st, a, gates));
-      KGE_CUDA_OK(launch_pdl(rglru_chain_kernel<__nv_bfloat16>, grid, block, 0, st, a, gates));
-      KGE_CUDA_OK(launch_pdl(rglru_out_kernel<__nv_bfloat16>, dim3(eg), dim3(256), 0, st, a, (const float*)gates));
-    }
-    return 0;
+    // the chain copies 16-byte pieces of rows
+    if (a.width % 4 == 0 && (reinterpret_cast<uintptr_t>(a.gates) & 15) == 0) return a.elt == KGE_ELT_F32 ? rglru_prompt<float>(a, st) : rglru_prompt<__nv_bfloat16>(a, st);
   }
   cudaError_t ce = a.elt == KGE_ELT_F32 ? launch_pdl(rglru_scan_kernel<float>, grid, block, 0, st, a)
                                         : launch_pdl(rglru_scan_kernel<__nv_bfloat16>, grid, block, 0, st, a);
