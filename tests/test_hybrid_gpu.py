@@ -66,6 +66,21 @@ def test_mechanism_alone(kge, tmp_path, mech, dtype):
     check(got, oh.forward(cfg, W, toks), dtype, mech)
 
 
+@pytest.mark.parametrize("experts,m_heads", [(5, 3), (17, 4), (32, 9)])
+def test_narrow_projections(kge, tmp_path, experts, m_heads):
+    """Gates and routers of up to 8, 16 and 32 columns over rows long enough (width 264) for the kernel that splits K over warps,
+    with a K that ends inside a piece; one row, a ragged last row tile, several tiles."""
+    cfg = oh.make_config(width=264, layers=("parallel", "rglru"), mlps=("moe", "moe"), experts=experts, m_heads=m_heads, top=experts)
+    W = oh.make_weights(cfg, seed=17)
+    toks = prompt(cfg, 75)
+    want = oh.forward(cfg, W, toks)
+    llm = make_engine(kge, tmp_path, cfg, W, "bfloat16")
+    for rid, pieces in enumerate([[75], [16, 1, 17, 41]]):
+        check(run_pieces(llm, rid, toks, pieces), want, "bfloat16", f"pieces {pieces}")
+        llm.trace_end(rid)
+    llm.close()
+
+
 @pytest.mark.parametrize("m_dim,m_vdim", [(16, 8), (64, 40), (128, 256)])
 def test_matrix_memory_in_chunks_of_64(kge, tmp_path, m_dim, m_vdim):
     """bfloat16 head sizes that take the tensor-core chunks: pieces that end before, at and behind a chunk's edge, single tokens
