@@ -129,8 +129,12 @@ __device__ __forceinline__ uint32_t pack2(float lo, float hi) {
   __nv_bfloat162 p = __floats2bfloat162_rn(lo, hi);
   return *reinterpret_cast<uint32_t*>(&p);
 }
-__device__ __forceinline__ uint32_t pack2raw(__nv_bfloat16 lo, __nv_bfloat16 hi) {
-  return (uint32_t)__bfloat16_as_ushort(lo) | ((uint32_t)__bfloat16_as_ushort(hi) << 16);
+
+__device__ __forceinline__ void ab_ldsm(uint32_t (&r)[4], const void* p) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"((uint32_t)__cvta_generic_to_shared(p)) : "memory");
+}
+__device__ __forceinline__ void ab_ldsm_t(uint32_t (&r)[4], const void* p) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"((uint32_t)__cvta_generic_to_shared(p)) : "memory");
 }
 
 // ROWS = false: a CTA owns 16 rows and its warps split the key tiles (decoding, short pieces).  ROWS = true: a CTA owns
@@ -251,9 +255,11 @@ __global__ void __launch_bounds__(AM_WARPS * 32) attn_bias_mma_kernel(AttnBiasAr
     for (int ks = 0; ks < AM_MAXD / 16; ++ks) {
       if (ks < ksteps) {
 #pragma unroll
-        for (int nt = 0; nt < 4; ++nt) {
-          const E* kp = Ks + (nt * 8 + qr) * kst + ks * 16 + qc;
-          mma_16816(sacc[nt], qf[ks], *reinterpret_cast<const uint32_t*>(kp), *reinterpret_cast<const uint32_t*>(kp + 8));
+        for (int nt = 0; nt < 4; nt += 2) {
+          uint32_t kf[4];                                    // keys nt * 8 .. + 15, both halves of the 16 dimensions
+          ab_ldsm(kf, Ks + (nt * 8 + (lane & 7) + ((lane >> 4) & 1) * 8) * kst + ks * 16 + ((lane >> 3) & 1) * 8);
+          mma_16816(sacc[nt], qf[ks], kf[0], kf[1]);
+          mma_16816(sacc[nt + 1], qf[ks], kf[2], kf[3]);
         }
       }
     }
@@ -301,12 +307,14 @@ __global__ void __launch_bounds__(AM_WARPS * 32) attn_bias_mma_kernel(AttnBiasAr
       pf[kk][3] = pack2(sacc[2 * kk + 1][2], sacc[2 * kk + 1][3]);
     }
 #pragma unroll
-    for (int v = 0; v < AM_MAXD / 8; ++v) {
+    for (int v = 0; v < AM_MAXD / 8; v += 2) {
       if (v < vtiles) {
 #pragma unroll
         for (int kk = 0; kk < 2; ++kk) {
-          const E* vp = Vs + (kk * 16 + qc) * vst + v * 8 + qr;
-          mma_16816(o[v], pf[kk], pack2raw(vp[0], vp[vst]), pack2raw(vp[8 * vst], vp[9 * vst]));
+          uint32_t vf[4];                                    // 16 keys x 16 columns (an odd last tile reads the row's padding)
+          ab_ldsm_t(vf, Vs + (kk * 16 + (lane & 7) + ((lane >> 3) & 1) * 8) * vst + v * 8 + (lane >> 4) * 8);
+          mma_16816(o[v], pf[kk], vf[0], vf[1]);
+          if (v + 1 < vtiles) mma_16816(o[v + 1], pf[kk], vf[2], vf[3]);
         }
       }
     }
