@@ -147,7 +147,7 @@ __global__ void __launch_bounds__(TMA ? 192 : 160, 2)
 attn_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
                bf16* __restrict__ out, const bf16* __restrict__ q, int q_stride, const bf16* __restrict__ k_cache,
                const bf16* __restrict__ v_cache, const int32_t* __restrict__ block_table, int max_blocks,
-               const int32_t* __restrict__ seq_lens, const int32_t* __restrict__ qsl, int H, int KV, int bs_shift,
+               const int32_t* __restrict__ seq_lens, const int32_t* __restrict__ qsl, int num_reqs, int by_request, int H, int KV, int bs_shift,
                float scale_log2_in, float cap_in2, float cap_log2, const float* __restrict__ sinks,
                const __grid_constant__ CUtensorMap tm_pk, const __grid_constant__ CUtensorMap tm_pv, WinArgs win) {
   static_assert(!WIN || TMA, "window kernels fetch their tiles by TMA");
@@ -161,13 +161,28 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
   constexpr uint32_t IDESC_S = (1u << 4) | KGE_IDESC_AB | ((uint32_t)(BNK >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
   constexpr uint32_t IDESC_O = (1u << 4) | KGE_IDESC_AB | (1u << 16) | ((uint32_t)(HD >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
 
-  const int b = blockIdx.z, kvh = blockIdx.y;
+  // The order of the CTAs (one per query tile, request and kv head).  Requests of like lengths: by distance of the query tile from
+  // its request's last one, then request and kv head, so that the tiles that walk the longest causal prefixes come first and the
+  // launch ends on short ones (request after request left SMs idle at the end: 2 x 1011 tokens behind 2777 keys 150 -> 137 us,
+  // 4 x 2048 with 12 heads of 64 80 -> 56).  by_request (most of the grid is empty: decode rows beside long pieces): request after
+  // request, so that the pieces' tiles are not strung out between empty CTAs (37 decode rows with up to 3000 keys and two such
+  // pieces: 185 us against 240; 253 with the decode rows last, whose serial walk over their keys then is the tail).
   const int G = H / KV;
   const int TT = BM / G;
+  const int tiles_max = (int)gridDim.x / (KV * num_reqs);
+  int b, kvh, rank;
+  if (by_request) {
+    rank = (int)blockIdx.x % tiles_max;
+    const int rem = (int)blockIdx.x / tiles_max;
+    kvh = rem % KV; b = rem / KV;
+  } else {
+    const int per_rank = KV * num_reqs, rem = (int)blockIdx.x % per_rank;
+    rank = (int)blockIdx.x / per_rank;
+    b = rem / KV; kvh = rem % KV;
+  }
   const int q0 = qsl[b], q_len = qsl[b + 1] - q0;
-  // heaviest (latest) query tiles first: their CTAs walk the longest causal prefix
-  const int tok0 = ((int)gridDim.x - 1 - (int)blockIdx.x) * TT;
-  if (tok0 >= q_len) return;
+  const int tok0 = ((q_len + TT - 1) / TT - 1 - rank) * TT;
+  if (tok0 < 0) return;
   const int seq_len = seq_lens[b];
   const int ctx0 = seq_len - q_len;
   const int ntok = min(TT, q_len - tok0);
@@ -497,9 +512,16 @@ template <int HD> constexpr int tc_smem() { return 128 * HD * 2 + 4 * BNK * HD *
 
 int make_tmap(CUtensorMap* m, const void* ptr, int64_t rows, int64_t cols, int box_rows);   // gemm_tc.cu (cached)
 
+// CTAs of a launch: one per (query tile, request, kv head); most of them are empty when a few requests are much longer than T / B
+static int64_t tc_grid(int B, int T, int max_q_len, int TT, int KV, int& by_request) {
+  const int64_t even = (int64_t)((max_q_len + TT - 1) / TT) * B;
+  by_request = 2 * ((int64_t)T / TT + B) < even;
+  return even * KV;
+}
+
 template <int HD>
 static int launch_tc(bf16* out, const bf16* q, int q_stride, const bf16* kc, const bf16* vc, const int32_t* bt,
-                     int max_blocks, const int32_t* sl, const int32_t* qsl, int B, int max_q_len, int H, int KV, int bs,
+                     int max_blocks, const int32_t* sl, const int32_t* qsl, int B, int T, int max_q_len, int H, int KV, int bs,
                      float scale, float softcap, const float* sinks, cudaStream_t st) {
   const bool cap = softcap > 0.f;
   const float cap_in2 = cap ? 2.f * atc::kLog2e * scale / softcap : 0.f, cap_log2 = softcap * atc::kLog2e;
@@ -507,6 +529,9 @@ static int launch_tc(bf16* out, const bf16* q, int q_stride, const bf16* kc, con
   while ((1 << bs_shift) < bs) ++bs_shift;
   const int G = H / KV;
   const int TT = atc::BM / G;
+  int by_request = 0;
+  const int64_t ctas = tc_grid(B, T, max_q_len, TT, KV, by_request);
+  KGE_REQUIRE(ctas <= INT32_MAX, "kge_paged_attn: too many query tiles");
   CUtensorMap tk, tv;
   const bool tma = tunable(TUN_ATTN_TMA) != 0 && bs >= 8;
   if (tma) {
@@ -516,25 +541,28 @@ static int launch_tc(bf16* out, const bf16* q, int q_stride, const bf16* kc, con
     if (int rc = make_tmap(&tv, vc, rows, HD, box_rows)) return rc;
     auto kern = cap ? atc::attn_tc_kernel<HD, true, true> : atc::attn_tc_kernel<HD, true, false>;
     KGE_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, atc::tc_smem<HD>()));
-    KGE_CUDA_OK(launch_pdl(kern, dim3((max_q_len + TT - 1) / TT, KV, B), dim3(192), atc::tc_smem<HD>(), st, tk, tv, out, q, q_stride,
-                           kc, vc, bt, max_blocks, sl, qsl, H, KV, bs_shift, scale * atc::kLog2e, cap_in2, cap_log2, sinks, tk, tv, atc::WinArgs()));
+    KGE_CUDA_OK(launch_pdl(kern, dim3((unsigned)ctas), dim3(192), atc::tc_smem<HD>(), st, tk, tv, out, q, q_stride,
+                           kc, vc, bt, max_blocks, sl, qsl, B, by_request, H, KV, bs_shift, scale * atc::kLog2e, cap_in2, cap_log2, sinks, tk, tv, atc::WinArgs()));
     return 0;
   }
   memset(&tk, 0, sizeof tk); memset(&tv, 0, sizeof tv);
   auto kern = cap ? atc::attn_tc_kernel<HD, false, true> : atc::attn_tc_kernel<HD, false, false>;
   KGE_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, atc::tc_smem<HD>()));
-  KGE_CUDA_OK(launch_pdl(kern, dim3((max_q_len + TT - 1) / TT, KV, B), dim3(160), atc::tc_smem<HD>(), st, tk, tv, out, q, q_stride, kc,
-                         vc, bt, max_blocks, sl, qsl, H, KV, bs_shift, scale * atc::kLog2e, cap_in2, cap_log2, sinks, tk, tv, atc::WinArgs()));
+  KGE_CUDA_OK(launch_pdl(kern, dim3((unsigned)ctas), dim3(160), atc::tc_smem<HD>(), st, tk, tv, out, q, q_stride, kc,
+                         vc, bt, max_blocks, sl, qsl, B, by_request, H, KV, bs_shift, scale * atc::kLog2e, cap_in2, cap_log2, sinks, tk, tv, atc::WinArgs()));
   return 0;
 }
 
 template <int HD>
 static int launch_tc_window(bf16* out, const bf16* q, int q_stride, const bf16* kc, const bf16* vc, const bf16* pkc, const bf16* pvc, const int32_t* bt,
-                            int max_blocks, const int32_t* sl, const int32_t* qsl, int B, int max_q_len, int H, int KV, int bs, float scale,
+                            int max_blocks, const int32_t* sl, const int32_t* qsl, int B, int T, int max_q_len, int H, int KV, int bs, float scale,
                             const atc::WinArgs& win, const float* sinks, cudaStream_t st) {
   int bs_shift = 0;
   while ((1 << bs_shift) < bs) ++bs_shift;
   const int TT = atc::BM / (H / KV);
+  int by_request = 0;
+  const int64_t ctas = tc_grid(B, T, max_q_len, TT, KV, by_request);
+  KGE_REQUIRE(ctas <= INT32_MAX, "paged_attn_window_tc: too many query tiles");
   CUtensorMap tk, tv, tpk, tpv;
   const int box_rows = bs < atc::BNK ? bs : atc::BNK;
   const int64_t rows = (int64_t)1 << 30;
@@ -548,8 +576,8 @@ static int launch_tc_window(bf16* out, const bf16* q, int q_stride, const bf16* 
   }
   auto kern = atc::attn_tc_kernel<HD, true, false, true>;
   KGE_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, atc::tc_smem<HD>()));
-  KGE_CUDA_OK(launch_pdl(kern, dim3((max_q_len + TT - 1) / TT, KV, B), dim3(192), atc::tc_smem<HD>(), st, tk, tv, out, q, q_stride, kc, vc, bt,
-                         max_blocks, sl, qsl, H, KV, bs_shift, scale * atc::kLog2e, 0.f, 0.f, sinks, tpk, tpv, win));
+  KGE_CUDA_OK(launch_pdl(kern, dim3((unsigned)ctas), dim3(192), atc::tc_smem<HD>(), st, tk, tv, out, q, q_stride, kc, vc, bt,
+                         max_blocks, sl, qsl, B, by_request, H, KV, bs_shift, scale * atc::kLog2e, 0.f, 0.f, sinks, tpk, tpv, win));
   return 0;
 }
 
@@ -564,24 +592,24 @@ bool paged_attn_window_tc_ok(int H, int KV, int hd, int vd, int bs, int pool, in
 // Steps with prompt pieces, a sliding window with kept first tokens (keep_first > 0) or pooled blocks (pool > 0): the
 // tcgen05 kernel above with the window's tile range and masks, optional sinks.  Sizes: paged_attn_window_tc_ok.
 int paged_attn_window_tc(void* out, const void* q, int q_stride, const void* kc, const void* vc, const void* pkc, const void* pvc, const int32_t* bt,
-                         int max_blocks, const int32_t* sl, const int32_t* qsl, int B, int max_q_len, int H, int KV, int hd, int bs, float scale,
+                         int max_blocks, const int32_t* sl, const int32_t* qsl, int B, int T, int max_q_len, int H, int KV, int hd, int bs, float scale,
                          int window, int keep_first, int pool, int pool_slots, const float* sinks, cudaStream_t st) {
   KGE_REQUIRE(window > 0 && paged_attn_window_tc_ok(H, KV, hd, hd, bs, pool, pool_slots), "paged_attn_window_tc: unsupported sizes");
   atc::WinArgs win;
   win.window = window; win.keep_first = keep_first; win.pool = pool; win.pool_slots = pool_slots;
-  if (hd == 128) return launch_tc_window<128>((bf16*)out, (const bf16*)q, q_stride, (const bf16*)kc, (const bf16*)vc, (const bf16*)pkc, (const bf16*)pvc, bt, max_blocks, sl, qsl, B,
+  if (hd == 128) return launch_tc_window<128>((bf16*)out, (const bf16*)q, q_stride, (const bf16*)kc, (const bf16*)vc, (const bf16*)pkc, (const bf16*)pvc, bt, max_blocks, sl, qsl, B, T,
                                                max_q_len, H, KV, bs, scale, win, sinks, st);
-  return launch_tc_window<64>((bf16*)out, (const bf16*)q, q_stride, (const bf16*)kc, (const bf16*)vc, (const bf16*)pkc, (const bf16*)pvc, bt, max_blocks, sl, qsl, B, max_q_len,
+  return launch_tc_window<64>((bf16*)out, (const bf16*)q, q_stride, (const bf16*)kc, (const bf16*)vc, (const bf16*)pkc, (const bf16*)pvc, bt, max_blocks, sl, qsl, B, T, max_q_len,
                               H, KV, bs, scale, win, sinks, st);
 }
 
 // Called by kge_paged_attn (attn.cu) for batches with query chunks longer than one token.
 int paged_attn_prefill_tc(bf16* out, const bf16* q, int q_stride, const bf16* kc, const bf16* vc, const int32_t* bt,
-                          int max_blocks, const int32_t* sl, const int32_t* qsl, int B, int max_q_len, int H, int KV,
+                          int max_blocks, const int32_t* sl, const int32_t* qsl, int B, int T, int max_q_len, int H, int KV,
                           int hd, int bs, float scale, float softcap, const float* sinks, cudaStream_t st) {
   KGE_REQUIRE(H / KV <= 128, "kge_paged_attn: GQA group %d > 128 unsupported", H / KV);
-  if (hd == 128) return launch_tc<128>(out, q, q_stride, kc, vc, bt, max_blocks, sl, qsl, B, max_q_len, H, KV, bs, scale, softcap, sinks, st);
-  return launch_tc<64>(out, q, q_stride, kc, vc, bt, max_blocks, sl, qsl, B, max_q_len, H, KV, bs, scale, softcap, sinks, st);
+  if (hd == 128) return launch_tc<128>(out, q, q_stride, kc, vc, bt, max_blocks, sl, qsl, B, T, max_q_len, H, KV, bs, scale, softcap, sinks, st);
+  return launch_tc<64>(out, q, q_stride, kc, vc, bt, max_blocks, sl, qsl, B, T, max_q_len, H, KV, bs, scale, softcap, sinks, st);
 }
 
 }  // namespace KGE_ELT_NS

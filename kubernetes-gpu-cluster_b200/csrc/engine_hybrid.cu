@@ -32,7 +32,7 @@ bool paged_attn_extras_decode_ok(int B, int H, int KV, int hd, int block_size);
 // attn_tc.cu: the tcgen05 prompt kernel with a sliding window and kept first tokens or pooled blocks (64- / 128-wide heads)
 bool paged_attn_window_tc_ok(int H, int KV, int hd, int vd, int bs, int pool, int pool_slots);
 int paged_attn_window_tc(void* out, const void* q, int q_stride, const void* kc, const void* vc, const void* pkc, const void* pvc, const int32_t* bt,
-                         int max_blocks, const int32_t* sl, const int32_t* qsl, int B, int max_q_len, int H, int KV, int hd, int bs, float scale,
+                         int max_blocks, const int32_t* sl, const int32_t* qsl, int B, int T, int max_q_len, int H, int KV, int hd, int bs, float scale,
                          int window, int keep_first, int pool, int pool_slots, const float* sinks, cudaStream_t st);
 // attn_decode_tma.cu: one token per request under a sliding window, keys and values staged by TMA (sizes: paged_attn_extras_decode_ok)
 int paged_attn_window_decode(void* out, const void* q, int q_stride, const void* kc, const void* vc, const int32_t* bt, int max_blocks, const int32_t* sl, const int32_t* qsl,
@@ -1007,7 +1007,7 @@ int hybrid_forward(kge_engine* e, int T, int B, int R, int max_blocks, const Ste
                       paged_attn_window_tc_ok(h.heads, h.kv_heads, h.dim, h.vdim, bs, h.pool, ps);
       HFWD(decode_only ? C_ATT_DEC : C_ATT_GEN, (decode_only ? keys : (double)T) * h.kv_heads * (h.dim + h.vdim) * es + (double)T * h.heads * (h.dim + h.vdim) * es,
            2.0 * keys * h.heads * (h.dim + h.vdim),
-           tc ? paged_attn_window_tc(e->mixbuf, qkv, ldq, L.kc, L.vc, L.pkc, L.pvc, m.btab, max_blocks, m.seq_lens, m.qsl, B, aa.max_q, h.heads, h.kv_heads, h.dim, bs,
+           tc ? paged_attn_window_tc(e->mixbuf, qkv, ldq, L.kc, L.vc, L.pkc, L.pvc, m.btab, max_blocks, m.seq_lens, m.qsl, B, T, aa.max_q, h.heads, h.kv_heads, h.dim, bs,
                                      h.scale, h.window, h.keep_first, h.pool, ps, nullptr, st)
               : attn_bias_chunk(aa, st));
       if (h.v_rot) HFWD(C_ACT, (double)T * ka * 2 * es, 0, rotate_heads_halves(e->mixbuf, ka, m.pos, L.v_freq, T, h.heads, h.vdim, -1.f, elt, st));
@@ -1141,7 +1141,7 @@ int hybrid_forward(kge_engine* e, int T, int B, int R, int max_blocks, const Ste
           HFWD(C_KVW, er * (L.lat_ukv.N + H * (h.dim + h.vdim) + h.rot_part) * es, 0,
                latent_expand_write(e->exp_k, e->exp_v, e->exp_kv, cache, e->exp_src, pages, bs, H, h.dim, h.vdim, rank, h.rot_part, elt, st));
           HFWD(C_ATT_GEN, er * H * (h.dim + h.vdim) * es + (double)(hm.qsl[r0 + n] - hm.qsl[r0]) * H * (h.dim + h.vdim) * es, 2.0 * gkeys * H * (h.dim + h.vdim),
-               paged_attn_window_tc(e->mixbuf, e->pbuf, ldp, e->exp_k, e->exp_v, nullptr, nullptr, e->exp_table, max_blocks, m.seq_lens + r0, m.qsl + r0, n, mq, H, H, h.dim, bs, h.scale,
+               paged_attn_window_tc(e->mixbuf, e->pbuf, ldp, e->exp_k, e->exp_v, nullptr, nullptr, e->exp_table, max_blocks, m.seq_lens + r0, m.qsl + r0, n, T, mq, H, H, h.dim, bs, h.scale,
                                     win, 0, 0, 0, L.sinks, st));
           r0 += n;
         }
@@ -1220,7 +1220,7 @@ int hybrid_forward(kge_engine* e, int T, int B, int R, int max_blocks, const Ste
            2.0 * keys * h.heads * (h.dim + h.vdim),
            dec_tc ? paged_attn_window_decode(e->mixbuf, e->pbuf, ldp, L.kc, L.vc, m.btab, max_blocks, m.seq_lens, m.qsl, B, h.heads, h.kv_heads, h.dim, bs, h.scale, h.window,
                                              max_blocks * bs, e->ws_attn, e->ws_attn_bytes, st)
-           : tc ? paged_attn_window_tc(e->mixbuf, e->pbuf, ldp, L.kc, L.vc, nullptr, nullptr, m.btab, max_blocks, m.seq_lens, m.qsl, B, aa.max_q, h.heads, h.kv_heads, h.dim, bs,
+           : tc ? paged_attn_window_tc(e->mixbuf, e->pbuf, ldp, L.kc, L.vc, nullptr, nullptr, m.btab, max_blocks, m.seq_lens, m.qsl, B, T, aa.max_q, h.heads, h.kv_heads, h.dim, bs,
                                      h.scale, h.window, 0, 0, 0, nullptr, st)
               : attn_bias_chunk(aa, st));
       HFWD(C_ACT, (double)T * ka * 3 * es, 0, sigmoid_gate_mul(e->mixbuf, ka, at(e->pbuf, L.off_mg), ldp, T, ka, elt, st));
