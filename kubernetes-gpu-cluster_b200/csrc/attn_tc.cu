@@ -205,15 +205,29 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
   const uint32_t sK = sQ + Q_BYTES;                // 2 stages
   const uint32_t sV = sK + 2 * TILE_BYTES;         // 2 stages
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + Q_BYTES + 4 * TILE_BYTES);
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 12);
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 13);
   const uint32_t bar0 = s_addr(bars);
-  // k_full[2], v_full[2], s_full[2], p_full[0], o_full, q_full, v_empty[2], p_full[1]
+  // k_full[2], v_full[2], s_full[2], p_full[2], o_full[2], v_empty[2], q_full.  A pair's barrier j & 1 completes its phase j >> 1
+  // with tile j.  A parity wait holds only while no later phase of the same barrier can complete, so each wait for tile j must come
+  // before something of its own that tile j + 2 needs, and after the phase of tile j - 2 is known to be over:
+  //   k_full(j)   issuer, before S_j: K_{j+2} is copied into this stage only after S_j
+  //   v_full(j)   issuer, before PV_j: V_{j+2} likewise only after PV_j
+  //   s_full(j)   softmax, before its arrival on p_full(j), without which the issuer does not get to S_{j+2}; producer, before it
+  //               fetches the K_{j+2} that S_{j+2} reads
+  //   p_full(j)   issuer, before it issues S_{j+2}, without whose scores no thread arrives for tile j + 2
+  //   o_full(j)   issuer, before S_{j+2}; softmax in tile j + 1, before its arrival on p_full(j + 1), and after the last tile: PV_{j+2}
+  //               needs the one and does not exist after the other.  PV_{j-2} was over before S_j was issued.  (One barrier for all
+  //               tiles is not enough: after the last tile a thread holds back neither PV_{n-2} nor PV_{n-1}, and one that sampled
+  //               the barrier after both had completed would wait for PV_{n-2}'s parity for ever.)
+  //   v_empty(j)  producer, before it fetches the V_{j+2} that PV_{j+2} reads
   auto k_full = [&](int s) { return bar0 + 8u * s; };
   auto v_full = [&](int s) { return bar0 + 16u + 8u * s; };
   auto s_full = [&](int s) { return bar0 + 32u + 8u * s; };
-  const uint32_t o_full = bar0 + 56, q_full = bar0 + 64;
-  auto p_full = [&](int s) { return bar0 + 48u + 40u * s; };      // two in turn: a warp may be a tile ahead of another
-  auto v_empty = [&](int s) { return bar0 + 72u + 8u * s; };
+  auto p_full = [&](int s) { return bar0 + 48u + 8u * s; };
+  auto o_full = [&](int s) { return bar0 + 64u + 8u * s; };
+  auto v_empty = [&](int s) { return bar0 + 80u + 8u * s; };
+  auto wait_o = [&](int j) { mbar_wait(o_full(j & 1), (uint32_t)((j >> 1) & 1)); };      // PV_j is done
+  const uint32_t q_full = bar0 + 96;
 
   const int tid = threadIdx.x, warp = uniform_warp(), lane = tid & 31;
   if (warp == 4) {
@@ -222,7 +236,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
       mbar_init(k_full(0), TMA ? 1 : 128); mbar_init(k_full(1), TMA ? 1 : 128);
       mbar_init(v_full(0), TMA ? 1 : 128); mbar_init(v_full(1), TMA ? 1 : 128);
       mbar_init(s_full(0), 1); mbar_init(s_full(1), 1);
-      mbar_init(p_full(0), 128); mbar_init(p_full(1), 128); mbar_init(o_full, 1);
+      mbar_init(p_full(0), 128); mbar_init(p_full(1), 128); mbar_init(o_full(0), 1); mbar_init(o_full(1), 1);
       mbar_init(q_full, 128); mbar_init(v_empty(0), 1); mbar_init(v_empty(1), 1);
       asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
       if (TMA) {
@@ -266,7 +280,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
         // before they arrived on p_full(j-1), which this thread has waited for; PV_{j-1} must have read P_{j-1} (MMAs of different
         // shapes are not ordered among themselves) - it runs while the softmax warps are busy with tile j
         if (j + 1 < ntiles) {
-          if (j > 0) { mbar_wait(o_full, (uint32_t)((j - 1) & 1)); tc_after(); }
+          if (j > 0) { wait_o(j - 1); tc_after(); }
           issue_s(j + 1);
         }
         mbar_wait(p_full(j & 1), (uint32_t)((j >> 1) & 1));
@@ -278,7 +292,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
           const uint32_t boff = (uint32_t)(k * 16 * 128);                             // V: 16 keys = 16 rows of 128 B
           tc_mma_ts(tmem + O_COL, tmem + (j & 1) * BNK + k * 8, vd + (boff >> 4), IDESC_O, (j > 0 || k > 0) ? 1u : 0u);
         }
-        tc_commit(o_full);
+        tc_commit(o_full(j & 1));
         if (TMA) tc_commit(v_empty(j & 1));      // PV_j has read V stage j&1: the producer may refill it
       }
     }
@@ -427,9 +441,9 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
       const float mx_raw = fmaxf(fmaxf(mxa[0], mxa[1]), fmaxf(mxa[2], mxa[3]));
       const float mx = mx_raw * scale_log2;                     // -inf stays -inf
       // PV_{j-1} must be done before O is rescaled (or, cp.async path, V stage (j+1)&1 refilled); otherwise the softmax runs ahead
-      // of it (PV_{j-2} was done before S_j was issued, so the parity is unambiguous)
+      // of it
       if (!TMA) {
-        if (j > 0) { mbar_wait(o_full, (uint32_t)((j - 1) & 1)); tc_after(); }
+        if (j > 0) { wait_o(j - 1); tc_after(); }
         load_tile(j + 1, false);
       }
       const bool grow = mx > m_ref + kRescaleThreshold;        // includes the first finite maximum
@@ -441,7 +455,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
           l *= alpha;
         }
         if (j > 0) {
-          if (TMA) { mbar_wait(o_full, (uint32_t)((j - 1) & 1)); tc_after(); }
+          if (TMA) { wait_o(j - 1); tc_after(); }
 #pragma unroll 1
           for (int c = 0; c < HD; c += 32) {
             uint32_t v[32];
@@ -471,9 +485,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
       mbar_arrive(p_full(j & 1));
     }
     if (!TMA) cp_wait<0>();
-    // the last scores say that PV_{ntiles-3} is done: the next two phases in turn, so that neither parity is taken for an older one
-    if (ntiles > 1) mbar_wait(o_full, (uint32_t)((ntiles - 2) & 1));
-    mbar_wait(o_full, (uint32_t)((ntiles - 1) & 1));
+    wait_o(ntiles - 1);                   // commits cover all MMAs before them: the earlier products are in O too
     tc_after();
     {
       // tcgen05.ld is warp-collective (.sync.aligned): every lane loads, only rows with a token store

@@ -687,6 +687,23 @@ def test_prefill_attention_tma_and_cp_async_agree(kge, L, H, KV, hd, bs, q_lens,
     assert torch.equal(a.view(torch.int16), b.view(torch.int16))
 
 
+@pytest.mark.parametrize("hd", [64, 128])
+@pytest.mark.parametrize("length", [64, 65, 129, 193, 1000])
+def test_prefill_attention_by_key_tiles(kge, L, hd, length):
+    """1, 2, 3, 4 and many 64-key tiles per query tile, both ways of staging K and V: the end of the kernel's pipeline comes before
+    its barriers have turned, at each of their phases, and late.  Many CTAs, two per SM; same bits both ways and in a second run."""
+    args = (kge, L, 16, 8, hd, 16, [length] * 24, [length] * 24, length + hd)
+    try:
+        a = run_attn_case(*args)
+        a2 = run_attn_case(*args)
+        check_ok(kge, L.kge_set_tunable(b"attn_tma", 0), "tunable")
+        b = run_attn_case(*args)
+    finally:
+        L.kge_set_tunable(b"attn_tma", 1)
+    assert torch.equal(a.view(torch.int16), b.view(torch.int16))
+    assert torch.equal(a.view(torch.int16), a2.view(torch.int16))
+
+
 def test_attention_block_sizes(kge, L):
     """Block sizes from 8 (one TMA box per block, eight boxes per tile) to 128 (two tiles per block) and 4 (below the TMA
     box granularity: cp.async path), decode and prefill."""
