@@ -43,16 +43,10 @@ __device__ __forceinline__ void mma_bf16(float (&c)[4], const uint32_t (&a)[4], 
                : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
-// thread-block cluster helpers (split-KV partials are merged through distributed shared memory)
-__device__ __forceinline__ void cluster_sync_all() {
-  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
+// split-KV partials are merged through distributed shared memory
 __device__ __forceinline__ float ld_dsmem_f32(uint32_t local_addr, uint32_t rank) {
-  uint32_t remote;
   float v;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(local_addr), "r"(rank));
-  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(remote) : "memory");
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(mapa_u32(local_addr, rank)) : "memory");
   return v;
 }
 
@@ -272,7 +266,7 @@ attn_decode_kernel(bf16* __restrict__ out, float* __restrict__ part_o, float* __
     }
   }
   if (CLUSTER && nsplit > 1) {
-    cluster_sync_all();                                   // every rank's partial is in its shared memory
+    cluster_arrive(); cluster_wait();                     // every rank's partial is in its shared memory
     const uint32_t sp = smem_u32(sPart);
     const int total = G * HD, per = (total + nsplit - 1) / nsplit;
     const int e_end = min(total, (split + 1) * per);
@@ -289,7 +283,7 @@ attn_decode_kernel(bf16* __restrict__ out, float* __restrict__ part_o, float* __
       }
       out[(int64_t)qrow * H * HD + (kvh * G + r) * HD + c] = f2bf(ll > 0.f ? acc / ll : 0.f);
     }
-    cluster_sync_all();                                   // nobody exits while a peer still reads its partial
+    cluster_arrive(); cluster_wait();                     // nobody exits while a peer still reads its partial
   }
 }
 

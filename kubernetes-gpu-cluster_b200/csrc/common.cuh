@@ -110,6 +110,19 @@ namespace kge {
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
+// Thread-block clusters.  A block's shared memory may be touched by its peers only once it is known to run: a kernel arrives
+// (relaxed: there is nothing to publish) at its start and waits before its first remote access, which its own work hides.
+__device__ __forceinline__ uint32_t cluster_ctarank() { uint32_t r; asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r)); return r; }
+__device__ __forceinline__ uint32_t cluster_nctarank() { uint32_t r; asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r)); return r; }
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
+__device__ __forceinline__ void cluster_arrive_relaxed() { asm volatile("barrier.cluster.arrive.relaxed;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
+__device__ __forceinline__ uint32_t mapa_u32(uint32_t local, uint32_t rank) {      // the address of `local` in block `rank`
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(local), "r"(rank));
+  return r;
+}
+
 // Every kernel of a step asks for the same L1 / shared-memory split (all shared memory): the GEMM and attention kernels
 // need ~200 KB per SM anyway, and an SM that has to change its split between two kernels must drain first, which
 // serialises exactly the kernel boundaries that programmatic dependent launch is there to overlap.  (Knob

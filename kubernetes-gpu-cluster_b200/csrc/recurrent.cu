@@ -676,7 +676,7 @@ __global__ void __launch_bounds__(MM_THREADS) mlstm_mma_kernel(MlstmArgs a) {
   for (int d = tid; d < 128; d += MM_THREADS) sm.nv[d] = d < dim && !fresh ? slot[(int64_t)dim * vdim + d] : 0.f;
   // the blocks of a head form a cluster: the one that writes n and m back waits until all have read them
   __syncthreads();
-  asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+  cluster_arrive();
 
   if (re - rs == 1) {
     // one token: thread = (column, eighth of the key dimensions)
@@ -713,7 +713,7 @@ __global__ void __launch_bounds__(MM_THREADS) mlstm_mma_kernel(MlstmArgs a) {
       for (int w = 0; w < 8; ++w) { o += part[w * 32 + col]; nq += sm.nq[w]; }
       a.o_scratch[(int64_t)rs * H * vdim + h * vdim + c0 + col] = o / (fmaxf(fabsf(nq), expf(-mn)) + a.den_eps);
     }
-    asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+    cluster_wait();
     if (blockIdx.z == 0) {
       for (int d = tid; d < dim; d += MM_THREADS) slot[(int64_t)dim * vdim + d] = sm.nv[d];
       if (tid == 0) slot[(int64_t)dim * vdim + dim] = mn;
@@ -985,7 +985,7 @@ __global__ void __launch_bounds__(MM_THREADS) mlstm_mma_kernel(MlstmArgs a) {
         if (col < ncol) slot[(int64_t)d * vdim + c0 + col] = C[n][q];
       }
   }
-  asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+  cluster_wait();
   if (blockIdx.z == 0) {
     if (tid < dim) slot[(int64_t)dim * vdim + tid] = sm.nv[tid];           // its own entry of the last update
     if (tid == 0) slot[(int64_t)dim * vdim + dim] = (float)m;

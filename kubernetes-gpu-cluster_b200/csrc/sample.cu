@@ -62,15 +62,8 @@ __device__ __forceinline__ uint32_t value_key(float v) {      // the key of v ro
   return pack_keys(*reinterpret_cast<const unsigned short*>(&h)) & 0xffffu;
 }
 
-__device__ __forceinline__ uint32_t cluster_rank() { uint32_t r; asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r)); return r; }
-__device__ __forceinline__ uint32_t cluster_size() { uint32_t r; asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r)); return r; }
-__device__ __forceinline__ void cluster_sync_all() {
-  asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
-}
 __device__ __forceinline__ void st_cluster(const void* local, uint32_t rank, uint32_t v) {
-  uint32_t a;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"((uint32_t)__cvta_generic_to_shared(local)), "r"(rank));
-  asm volatile("st.shared::cluster.u32 [%0], %1;" :: "r"(a), "r"(v) : "memory");
+  asm volatile("st.shared::cluster.u32 [%0], %1;" :: "r"(mapa_u32((uint32_t)__cvta_generic_to_shared(local), rank)), "r"(v) : "memory");
 }
 
 constexpr int kSampleWarps = kSampleThreads / 32;
@@ -88,7 +81,7 @@ struct MaxOp { template <typename T> __device__ __forceinline__ T operator()(T a
 template <int N, typename T, typename OP>
 __device__ __forceinline__ void cluster_reduce(T (&v)[N], SampleShared& sh, int& phase, OP op) {
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const uint32_t nc = cluster_size();
+  const uint32_t nc = cluster_nctarank();
 #pragma unroll
   for (int k = 0; k < N; ++k) {
     if constexpr (std::is_same<T, int>::value && std::is_same<OP, AddOp>::value) {
@@ -107,9 +100,9 @@ __device__ __forceinline__ void cluster_reduce(T (&v)[N], SampleShared& sh, int&
     T t = *reinterpret_cast<T*>(&raw);
 #pragma unroll
     for (int o = kSampleWarps / 2; o > 0; o >>= 1) t = op(t, __shfl_xor_sync(0xffffffffu, t, o));
-    if (lane < (int)nc) st_cluster(&sh.all[phase & 1][cluster_rank()][wid], lane, *reinterpret_cast<uint32_t*>(&t));
+    if (lane < (int)nc) st_cluster(&sh.all[phase & 1][cluster_ctarank()][wid], lane, *reinterpret_cast<uint32_t*>(&t));
   }
-  cluster_sync_all();
+  cluster_arrive(); cluster_wait();
   // lane (r, k) takes value k of ranks r and r + 4 (zero is neutral for the sums and for the maxima taken here)
   const int kk = lane & 7, r = lane >> 3;
   uint32_t raw = r < (int)nc && kk < N ? sh.all[phase & 1][r][kk] : 0u, raw4 = r + 4 < (int)nc && kk < N ? sh.all[phase & 1][r + 4][kk] : 0u;
@@ -148,15 +141,16 @@ sample_kernel(int32_t* __restrict__ out, const bf16* __restrict__ logits, int V,
               const uint64_t* __restrict__ seeds, uint64_t step) {
   __shared__ SampleShared sh;
   extern __shared__ uint4 held[];
+  cluster_arrive_relaxed();                                  // see the wait below
   pdl_launch_dependents();
   pdl_wait();
-  const int nc = (int)cluster_size(), b = blockIdx.x / nc, tid = threadIdx.x;
+  const int nc = (int)cluster_nctarank(), b = blockIdx.x / nc, tid = threadIdx.x;
   const bf16* row = logits + (int64_t)b * ld;
   const bool aligned = (reinterpret_cast<uintptr_t>(row) & 15) == 0;
   const float temp = temperature ? temperature[b] : 0.f;
   const bool greedy = temp < 1e-5f;
   const float inv_t = greedy ? 1.f : 1.f / temp;
-  const int pieces = (V + 7) / 8, stride = nc * kSampleThreads, first = (int)cluster_rank() * kSampleThreads + tid;
+  const int pieces = (V + 7) / 8, stride = nc * kSampleThreads, first = (int)cluster_ctarank() * kSampleThreads + tid;
   int phase = 0;
 
   if constexpr (STAGED) {
@@ -223,6 +217,7 @@ sample_kernel(int32_t* __restrict__ out, const bf16* __restrict__ logits, int V,
       }
     }
   }
+  cluster_wait();                                              // the peers run: their shared memory may be written
   if (greedy) {
     if (top[0]) offer(key_value(top[0]), at);                  // the first of equal keys
   } else {
@@ -343,12 +338,12 @@ sample_kernel(int32_t* __restrict__ out, const bf16* __restrict__ logits, int V,
     bi = (int)sh.warp[1][lane % kSampleWarps];
     warp_best();
     if (lane == 0) {
-      st_cluster(&sh.all[phase & 1][cluster_rank()][0], 0, __float_as_uint(best));
-      st_cluster(&sh.all[phase & 1][cluster_rank()][1], 0, (uint32_t)bi);
+      st_cluster(&sh.all[phase & 1][cluster_ctarank()][0], 0, __float_as_uint(best));
+      st_cluster(&sh.all[phase & 1][cluster_ctarank()][1], 0, (uint32_t)bi);
     }
   }
-  cluster_sync_all();
-  if (cluster_rank() == 0 && tid == 0) {
+  cluster_arrive(); cluster_wait();
+  if (cluster_ctarank() == 0 && tid == 0) {
     best = -INFINITY; bi = 0x7fffffff;
     for (int r = 0; r < nc; ++r) {
       const float ov = __uint_as_float(sh.all[phase & 1][r][0]);

@@ -1,0 +1,38 @@
+"""Distributed shared memory is touched only behind a cluster barrier: a block's peers may not have started before it.  Read from
+the kernels' sources, since a store that comes too early need not show in a result."""
+import glob
+import os
+import re
+
+import pytest
+
+CSRC = os.path.join(os.path.dirname(__file__), "..", "kubernetes-gpu-cluster_b200", "csrc")
+# what reaches into a peer's shared memory, or signals a barrier there, from a kernel's body
+REMOTE = re.compile(r"\b(st_cluster\w*|ld_dsmem_\w+|cluster_reduce|mapa_u32|mbar_arrive_cluster)\(|shared::cluster\.(?!b64)")
+BARRIER = re.compile(r"\bcluster_wait\(\)")
+
+
+def kernels():
+    for path in sorted(glob.glob(os.path.join(CSRC, "*.cu*"))):
+        src = re.sub(r"//[^\n]*", "", open(path).read())
+        for m in re.finditer(r"__global__[^;{]*?(\w+_kernel)\(", src):
+            body = src[src.index("{", m.end()):]
+            end = re.search(r"\n}\n", body)
+            yield os.path.basename(path), m.group(1), body[:end.start() if end else len(body)]
+
+
+USERS = [(f, k, b) for f, k, b in kernels() if REMOTE.search(b)]
+
+
+def test_the_kernels_are_found():
+    assert {k for _, k, _ in USERS} >= {"sample_kernel", "gemm_tc_kernel", "gemm_wide_kernel", "attn_decode_kernel"}
+
+
+@pytest.mark.parametrize("file,kernel,body", USERS, ids=[k for _, k, _ in USERS])
+def test_a_cluster_barrier_comes_before_the_first_remote_access(file, kernel, body):
+    # a lambda that only forms an address is not an access: calls count from where the first one is made
+    code = re.sub(r"auto \w+ = \[&\]\([^)]*\) \{[^\n]*\};", "", body)
+    first = REMOTE.search(code)
+    assert first, (file, kernel)
+    wait = BARRIER.search(code)
+    assert wait and wait.start() < first.start(), (file, kernel, code[first.start():first.start() + 80])
