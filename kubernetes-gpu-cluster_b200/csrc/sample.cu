@@ -385,7 +385,8 @@ extern "C" int KGE_API(kge_sample)(int32_t* out_ids, const void* logits, int B, 
   const bool staged = trips * kSampleThreads * 16 <= 192 * 1024;
   const size_t smem = staged ? (size_t)(trips * kSampleThreads * 16) : 0;
   auto kern = staged ? sample_kernel<true> : sample_kernel<false>;
-  if (smem > 48 * 1024) KGE_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 192 * 1024));
+  // 48 KB of static and dynamic shared memory together go without the attribute (rows of 163841 to 196608 have 48 KB dynamic)
+  if (smem + sizeof(SampleShared) > 48 * 1024) KGE_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 192 * 1024));
   prefer_max_shared(kern);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)B * nc); cfg.blockDim = dim3(kSampleThreads); cfg.dynamicSmemBytes = smem; cfg.stream = (cudaStream_t)stream;

@@ -821,6 +821,14 @@ def test_sample_row_split_over_a_cluster(kge, L, B, V, ld):
             assert keep[got[b]] and score[got[b]] >= score.max() * (1 - 1e-5), (b, got[b], int(score.argmax()))
 
 
+@pytest.mark.parametrize("V", [196608, 163841, 163840, 196609, 262144, 786432])
+def test_sample_vocabularies_by_shared_memory(kge, L, V):
+    """5, 6, 7 and more 8 KB pieces of a row per CTA: below, at and above the 48 KB that a launch gets without asking (with the
+    kernel's own static arrays), and the most that is staged.  The size at the edge comes first, before a larger one has asked."""
+    for B in (1, 40):
+        test_sample_row_split_over_a_cluster(kge, L, B, V, V)
+
+
 def test_sample_philox_is_deterministic_and_in_support(kge, L):
     g = torch.Generator().manual_seed(2)
     B, V = 4, 2048
