@@ -779,46 +779,73 @@ def test_sample_topk_topp_with_given_noise(kge, L):
     assert agree >= total - 2, f"{agree}/{total}"
 
 
-@pytest.mark.parametrize("B,V,ld", [(1, 1, 8), (3, 7, 7), (5, 4097, 4101), (2, 50272, 50304), (40, 16385, 16392), (3, 131073, 131073), (150, 2049, 2056),
+def check_draws(got, lg, V, temp, k, pp, q):
+    """Draws with supplied noise against the oracle's rule in float64, where equal logits at the edge of the top-p mass are kept
+    together (a sort keeps some of them).  The kernel's masses are fp32: an exponential of |x| <= 32 is off by 2^-17 (the roundings of
+    x and of the maximum), and a sum of n terms along its longest chain, a thread's V / 512 of them and the tree above, by n 2^-24.
+    Any edge whose mass is within that of 1 - p is admissible, so is the draw of each, and nothing below the lowest one is."""
+    checked = 0
+    for b in range(lg.shape[0]):
+        greedy = temp[b] < 1e-5
+        x = lg[b, :V].double() / (1.0 if greedy else temp[b].double())
+        if not torch.isfinite(x).any():
+            continue
+        keep = torch.ones(V, dtype=torch.bool)
+        if not greedy and 0 < k[b] < V:
+            keep &= x >= x.topk(int(k[b])).values[-1]
+        edges = [-float("inf")]
+        if not greedy and pp[b] < 1:
+            vals, inv = x.unique(return_inverse=True)
+            share = torch.zeros(len(vals), dtype=torch.float64).index_add_(0, inv[keep], torch.exp(x[keep] - x.max()))
+            cum, low, tol = share.cumsum(0) / share.sum(), 1 - pp[b].double(), (V / 512 + 64) * 2.0 ** -24 + 2.0 ** -17
+            before = torch.cat([torch.zeros(1, dtype=torch.float64), cum[:-1]])
+            edges = vals[(cum > low - tol) & (before <= low + tol) & (share > 0)].tolist()
+            checked += 1
+        score = torch.exp(x - x.max()) / (1.0 if greedy else q[b].double())
+        assert keep[got[b]] and x[got[b]] >= min(edges), (b, got[b])
+        # 1e-5: the fp32 exponentials and quotients of two scores
+        best = [score[keep & (x >= e)].max() for e in edges]
+        assert any(x[got[b]] >= e and score[got[b]] >= s * (1 - 1e-5) for e, s in zip(edges, best)), (b, got[b], len(edges))
+    return checked
+
+
+def edge_noise(lg, temp):
+    """q = e^(2 (x - max)): a score e^(x - max) / q is the larger the smaller the logit is."""
+    x = lg.double() / torch.where(temp < 1e-5, torch.ones_like(temp), temp).double()[:, None]
+    q = torch.exp(2 * (x - x.max(1, keepdim=True).values).clamp(min=-42.0))
+    return torch.where(torch.isfinite(x), q, torch.ones_like(q)).float()
+
+
+@pytest.mark.parametrize("B,V,ld", [(1, 1, 8), (3, 7, 7), (5, 4097, 4101), (2, 50272, 50304), (64, 50272, 50272), (40, 16385, 16392), (3, 131073, 131073), (150, 2049, 2056),
                                     (2, 786440, 786440)])
 def test_sample_row_split_over_a_cluster(kge, L, B, V, ld):
     """Rows shorter than a piece, ragged ends, rows that are not 16-byte aligned, 1 to 8 CTAs per row, and rows too long to be
-    staged in shared memory: the draw with supplied noise is the oracle's rule in float64, where equal logits at the edge of the
-    top-p mass are kept together (a sort keeps some of them), and columns beyond V never win.  fp32 sums of V numbers in any
-    order are within 2^-24 V of each other: rows whose edge is closer to 1 - p than that may go either way."""
+    staged in shared memory, each with every setting; columns beyond V never win.  Drawn noise, and noise under which the smallest
+    kept logit wins, so that the draw tells where the row was cut."""
     g = torch.Generator().manual_seed(B * 1000 + V)
     lg = torch.full((B, ld), 30.0).to(BF)
     lg[:, :V] = (torch.randn(B, V, generator=g) * 2.5).to(BF)
     lg[0, V // 2] = -float("inf")
     if V > 1:
         lg[B - 1, :V // 2] = lg[B - 1, 0]                          # many equal keys
-    want = [(0.0, 0, 1.0), (0.7, 20, 0.8), (1.0, 0, 0.95), (0.6, 50, 1.0), (1.5, 0, 1.0), (1.0, 3, 0.4)]
-    temp = torch.tensor([want[b % 6][0] for b in range(B)])
-    k = torch.tensor([min(want[b % 6][1], V) for b in range(B)], dtype=torch.int32)
-    pp = torch.tensor([want[b % 6][2] for b in range(B)])
     q = torch.empty(B, V).exponential_(generator=g)
-    lgd, td, kd, ppd, qd, out = dev(lg), dev(temp), dev(k), dev(pp), dev(q), torch.empty(B, dtype=torch.int32, device="cuda")
-    check_ok(kge, L.kge_sample(p(out), p(lgd), B, V, ld, p(td), p(kd), p(ppd), p(qd), None, 0, None, 0, None), "sample")
-    sync()
-    got = out.cpu().long()
-    assert ((got >= 0) & (got < V)).all()
-    for b in range(B):
-        x = lg[b, :V].double() / (temp[b].double() if temp[b] >= 1e-5 else 1.0)
-        if not torch.isfinite(x).any():
-            continue
-        keep, sure = torch.ones(V, dtype=torch.bool), True
-        if temp[b] >= 1e-5 and 0 < k[b] < V:
-            keep &= x >= x.topk(int(k[b])).values[-1]
-        if temp[b] >= 1e-5 and pp[b] < 1:
-            vals, inv = x.unique(return_inverse=True)
-            share = torch.zeros(len(vals), dtype=torch.float64).index_add_(0, inv[keep], torch.exp(x[keep] - x.max()))
-            cum = share.cumsum(0) / share.sum()
-            over = cum > 1 - pp[b].double()
-            sure = bool(((cum - (1 - pp[b].double())).abs() > 2.0 ** -24 * max(V, 16)).all())
-            keep &= x >= vals[int(over.nonzero()[0])]
-        score = torch.where(keep, torch.exp(x - x.max()) / (1.0 if temp[b] < 1e-5 else q[b].double()), torch.tensor(-1.0, dtype=torch.float64))
-        if sure:       # 1e-5: the fp32 exponential and quotient of the winning score
-            assert keep[got[b]] and score[got[b]] >= score.max() * (1 - 1e-5), (b, got[b], int(score.argmax()))
+    lgd, out = dev(lg), torch.empty(B, dtype=torch.int32, device="cuda")
+    want = [(0.0, 0, 1.0), (0.7, 20, 0.8), (1.0, 0, 0.95), (0.6, 50, 1.0), (1.5, 0, 1.0), (1.0, 3, 0.4), (1.0, 0, 0.1), (0.8, 0, 0.5)]
+    checked = 0
+    for first in range(0, len(want), B):
+        row = [want[(first + b) % len(want)] for b in range(B)]
+        temp = torch.tensor([r[0] for r in row])
+        k = torch.tensor([min(r[1], V) for r in row], dtype=torch.int32)
+        pp = torch.tensor([r[2] for r in row])
+        td, kd, ppd = dev(temp), dev(k), dev(pp)
+        for noise in (q, edge_noise(lg[:, :V], temp)):
+            qd = dev(noise)
+            check_ok(kge, L.kge_sample(p(out), p(lgd), B, V, ld, p(td), p(kd), p(ppd), p(qd), None, 0, None, 0, None), "sample")
+            sync()
+            got = out.cpu().long()
+            assert ((got >= 0) & (got < V)).all()
+            checked += check_draws(got, lg, V, temp, k, pp, noise)
+    assert checked > 0 or V == 1
 
 
 @pytest.mark.parametrize("V", [196608, 163841, 163840, 196609, 262144, 786432])
