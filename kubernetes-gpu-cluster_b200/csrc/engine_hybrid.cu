@@ -196,7 +196,7 @@ int hybrid_engine_build(kge_engine* e, const ModelDir& md, int64_t dummy_seed, s
   int max_abs = 0, max_olat = 0, max_exp_row = 0, max_exp_k = 0, max_exp_v = 0, max_win = 0, max_qkv32 = 0;
   int64_t lat_ws = 0;
   bool lat_tc = true;                                         // every cached-latent layer takes the expanded tcgen05 path in prompt steps
-  int max_mo = 1;
+  int max_mo = 1, max_nm = 0;
   int max_proj = 1, max_mix = 1, max_ff = 1, max_gate = 1, max_u = 1, max_top = 0, max_eff = 1, max_E = 1;
   int max_hd = 0, max_qr = 0, max_kvr = 0, max_lkv = 0, max_lq = 0;      // WKV heads * dim; latent ranks, [k | v] and query widths
   int max_mix2 = 0, max_bc = 0, max_dt = 0;
@@ -516,7 +516,7 @@ int hybrid_engine_build(kge_engine* e, const ModelDir& md, int64_t dummy_seed, s
         HB_OK(L.o2.w = b.upload(cat));
       }
       state_floats += mlstm_state_floats(h.m_heads, h.m_dim, h.m_vdim);
-      max_mo = std::max(max_mo, mv);
+      max_mo = std::max(max_mo, mv); max_nm = std::max(max_nm, h.m_heads * (h.m_dim + 1));
       max_proj = std::max(max_proj, L.proj.N); max_mix = std::max(max_mix, ko); max_gate = std::max(max_gate, 2 * h.m_heads);
     }
     if (s.streams > 0) {
@@ -647,7 +647,7 @@ int hybrid_engine_build(kge_engine* e, const ModelDir& md, int64_t dummy_seed, s
   e->obuf2 = aalloc((int64_t)Tm * d, es);
   e->ffbuf = aalloc((int64_t)Tm * max_ff, es);
   e->gates32 = (float*)aalloc((int64_t)Tm * max_gate, 4);
-  e->mo32 = (float*)aalloc((int64_t)Tm * max_mo, 4);
+  e->mo32 = (float*)aalloc((int64_t)Tm * max_mo + (int64_t)Rm * max_nm, 4);      // read-outs of a step's tokens, and behind them new normalisers of its requests
   e->hsel = aalloc((int64_t)std::max(Rm, Tm) * d, es);
   // logits rows: the sampled rows of a step, or every row a trace asks for
   e->logits32 = (float*)aalloc((int64_t)std::max(Rm, Tm) * s.vocab, 4);
@@ -1304,7 +1304,7 @@ int hybrid_forward(kge_engine* e, int T, int B, int R, int max_blocks, const Ste
            2.0 * keys * h.heads * (h.dim + h.vdim), attn_bias_chunk(aa, st));
       MlstmArgs ma;
       ma.q = at(e->pbuf, L.off_mq); ma.k = at(e->pbuf, L.off_mk); ma.v = at(e->pbuf, L.off_mv); ma.g = at(e->pbuf, L.off_mg); ma.ld = ldp;
-      ma.gates = e->gates32; ma.o_scratch = e->mo32; ma.norm_w = L.m_norm; ma.out = at(e->mixbuf, ka); ma.ldo = ko;
+      ma.gates = e->gates32; ma.o_scratch = e->mo32; ma.nm_scratch = e->mo32 + (int64_t)T * h.m_heads * h.m_vdim; ma.norm_w = L.m_norm; ma.out = at(e->mixbuf, ka); ma.ldo = ko;
       ma.state = e->state + L.state_off; ma.slot_stride = e->slot_stride; ma.slots = m.sslot; ma.qsl = m.qsl; ma.positions = m.pos;
       ma.B = B; ma.T = T; ma.H = h.m_heads; ma.dim = h.m_dim; ma.vdim = h.m_vdim;
       ma.cap = h.gate_cap; ma.q_scale = 1.f / sqrtf((float)h.m_dim); ma.eps = s.eps; ma.den_eps = 1e-6f; ma.out_scale = h.right_scale; ma.elt = elt;

@@ -277,6 +277,7 @@ struct MlstmArgs {
   const void* norm_w = nullptr; void* out = nullptr; int ldo = 0;
   float* o_scratch = nullptr;              // fp32 [T, H * vdim]: with it (and dim <= 128) the value columns of a head are split
                                            // over several blocks with the state in registers, and a second kernel normalises
+  float* nm_scratch = nullptr;             // fp32 [B, H * (dim + 1)], goes with o_scratch: a head's new n and m until all its blocks have read the old ones
   float* state = nullptr; int64_t slot_stride = 0;
   const int32_t* slots = nullptr; const int32_t* qsl = nullptr; const int32_t* positions = nullptr;
   int B = 0, T = 0, H = 0, dim = 0, vdim = 0;

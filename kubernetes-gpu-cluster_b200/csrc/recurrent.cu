@@ -376,6 +376,8 @@ __global__ void mlstm_step_kernel(MlstmArgs a) {
 // The same recurrence with a head's value columns split over blocks of 64 threads: a thread keeps its column of the
 // state in registers (dim <= 128), the first warp keeps the normaliser n, and the un-normalised read-out goes to an fp32
 // scratch; mlstm_norm_gate_kernel then divides each head by its root mean square and applies weight and output gate.
+// All blocks of a head read n and m at their start, and not all blocks of a launch start together: the block that has the new
+// ones leaves them in scratch, and the second kernel, which runs when all blocks are done, puts them into the state.
 // More blocks than (request, head) pairs fill the machine when few requests prefill, and the state never sits in shared memory.
 constexpr int ML_MAXD = 128, ML_COLS = 64, ML_THREADS = ML_COLS + 32;      // two warps of value columns, one for the normaliser
 
@@ -466,8 +468,9 @@ __global__ void __launch_bounds__(ML_THREADS) mlstm_cols_kernel(MlstmArgs a) {
   }
   if (blockIdx.z == 0) {
     __syncthreads();
-    for (int d = tid; d < dim; d += ML_THREADS) slot[(int64_t)dim * vdim + d] = nv[d];
-    if (tid == 0) slot[(int64_t)dim * vdim + dim] = m;
+    float* nm = a.nm_scratch + ((int64_t)b * a.H + h) * (dim + 1);
+    for (int d = tid; d < dim; d += ML_THREADS) nm[d] = nv[d];
+    if (tid == 0) nm[dim] = m;
   }
 }
 
@@ -609,9 +612,10 @@ __global__ void __launch_bounds__(MC_COLS * ML_NSL) mlstm_chunk_kernel(MlstmArgs
 #pragma unroll
     for (int d = 0; d < ML_DS; ++d) if (d0 + d < dim) slot[(int64_t)(d0 + d) * vdim + c] = C[d];
   }
-  if (blockIdx.z == 0) {
-    for (int d = tid; d < dim; d += NT) slot[(int64_t)dim * vdim + d] = nv[d];
-    if (tid == 0) slot[(int64_t)dim * vdim + dim] = m;
+  if (blockIdx.z == 0) {                                       // see mlstm_cols_kernel
+    float* nm = a.nm_scratch + ((int64_t)b * a.H + h) * (dim + 1);
+    for (int d = tid; d < dim; d += NT) nm[d] = nv[d];
+    if (tid == 0) nm[dim] = m;
   }
 }
 
@@ -998,6 +1002,13 @@ __global__ void mlstm_norm_gate_kernel(MlstmArgs a) {
   pdl_wait();
   __shared__ float red[33];
   const int t = blockIdx.x, h = blockIdx.y;
+  if (t >= a.T) {                                              // blocks beyond the tokens: a request's new n and m
+    const int b = t - a.T;
+    const float* nm = a.nm_scratch + ((int64_t)b * a.H + h) * (a.dim + 1);
+    float* slot = a.state + (int64_t)a.slots[b] * a.slot_stride + ((int64_t)h + 1) * ((int64_t)a.dim * a.vdim + a.dim + 1) - (a.dim + 1);
+    for (int d = threadIdx.x; d <= a.dim; d += blockDim.x) slot[d] = nm[d];
+    return;
+  }
   const float* o = a.o_scratch + (int64_t)t * a.H * a.vdim + h * a.vdim;
   float ss = 0.f;
   for (int c = threadIdx.x; c < a.vdim; c += blockDim.x) ss = fmaf(o[c], o[c], ss);
@@ -1011,8 +1022,8 @@ __global__ void mlstm_norm_gate_kernel(MlstmArgs a) {
 
 int mlstm_step(const MlstmArgs& a, cudaStream_t st) {
   if (a.T <= 0 || a.B <= 0) return 0;
-  if (a.o_scratch && a.dim <= ML_MAXD && a.dim % 4 == 0 && a.H <= 65535) {
-    const dim3 grid(a.B, a.H, (a.vdim + ML_COLS - 1) / ML_COLS), g2(a.T, a.H);
+  if (a.o_scratch && a.nm_scratch && a.dim <= ML_MAXD && a.dim % 4 == 0 && a.H <= 65535) {
+    const dim3 grid(a.B, a.H, (a.vdim + ML_COLS - 1) / ML_COLS), g2(a.T + a.B, a.H);
     const int nt = std::min(256, (a.vdim + 31) / 32 * 32);
     KGE_CUDA_OK(launch_pdl(mlstm_log_gates_kernel, dim3((a.T * 2 * a.H + 255) / 256), dim3(256), 0, st, const_cast<float*>(a.gates), a.T, a.H, a.cap));
     const size_t csm_bytes = ((size_t)2 * ML_CH * a.dim + ML_CH * ML_CH + ML_MAXD + 5 * ML_CH + (1 + ML_NSL) * ML_CH * MC_COLS) * 4;
@@ -1032,7 +1043,7 @@ int mlstm_step(const MlstmArgs& a, cudaStream_t st) {
       attr[1].val.programmaticStreamSerializationAllowed = 1;
       cfg.attrs = attr; cfg.numAttrs = pdl_for_this_launch() ? 2 : 1;
       KGE_CUDA_OK(cudaLaunchKernelEx(&cfg, mlstm_mma_kernel, a));
-      KGE_CUDA_OK(launch_pdl(mlstm_norm_gate_kernel<__nv_bfloat16>, g2, dim3(nt), 0, st, a));
+      KGE_CUDA_OK(launch_pdl(mlstm_norm_gate_kernel<__nv_bfloat16>, dim3(a.T, a.H), dim3(nt), 0, st, a));
       return 0;
     }
     if (a.T > a.B) {
