@@ -1141,7 +1141,7 @@ int hybrid_forward(kge_engine* e, int T, int B, int R, int max_blocks, const Ste
           HFWD(C_KVW, er * (L.lat_ukv.N + H * (h.dim + h.vdim) + h.rot_part) * es, 0,
                latent_expand_write(e->exp_k, e->exp_v, e->exp_kv, cache, e->exp_src, pages, bs, H, h.dim, h.vdim, rank, h.rot_part, elt, st));
           HFWD(C_ATT_GEN, er * H * (h.dim + h.vdim) * es + (double)(hm.qsl[r0 + n] - hm.qsl[r0]) * H * (h.dim + h.vdim) * es, 2.0 * gkeys * H * (h.dim + h.vdim),
-               paged_attn_window_tc(e->mixbuf, e->pbuf, ldp, e->exp_k, e->exp_v, nullptr, nullptr, e->exp_table, max_blocks, m.seq_lens + r0, m.qsl + r0, n, T, mq, H, H, h.dim, bs, h.scale,
+               paged_attn_window_tc(e->mixbuf, e->pbuf, ldp, e->exp_k, e->exp_v, nullptr, nullptr, e->exp_table, max_blocks, m.seq_lens + r0, m.qsl + r0, n, hm.qsl[r0 + n] - hm.qsl[r0], mq, H, H, h.dim, bs, h.scale,
                                     win, 0, 0, 0, L.sinks, st));
           r0 += n;
         }
