@@ -195,9 +195,10 @@ __global__ void __launch_bounds__(256) rglru_ab_kernel(RglruArgs a, float* gates
 }
 
 // One warp per 32 channels of a request: the coefficients of 64 tokens at a time arrive by cp.async, three stages ahead, so that the
-// chain waits for its fma's and not for memory (with eight tokens' loads in flight it took 145 us).
+// chain waits for its fma's and not for memory (with eight tokens' loads in flight it took 145 us).  N: numbers per copy, four
+// where the rows are aligned for it, one elsewhere (widths that are no multiple of four).
 constexpr int RS_TOK = 64, RS_STAGES = 4, RS_SMEM = RS_STAGES * 2 * RS_TOK * 32 * 4;
-template <typename E>
+template <typename E, int N>
 __global__ void __launch_bounds__(32) rglru_chain_kernel(RglruArgs a, float* gates) {
   pdl_launch_dependents();
   pdl_wait();
@@ -212,13 +213,17 @@ __global__ void __launch_bounds__(32) rglru_chain_kernel(RglruArgs a, float* gat
   auto fetch = [&](int tile) {
     if (tile < tiles) {
       float* dst = rs_sm + (tile % RS_STAGES) * (2 * RS_TOK * 32);
-      const int len = min(RS_TOK, n - tile * RS_TOK), piece = (lane & 7) * 4, left = a.width - c0 - piece;
-      const int bytes = left >= 4 ? 16 : left > 0 ? left * 4 : 0;
-      for (int k = lane >> 3; k < len; k += 4) {
+      constexpr int LANES = 32 / N;                        // lanes that copy a token's 32 channels
+      const int len = min(RS_TOK, n - tile * RS_TOK), piece = (lane % LANES) * N;
+      const int bytes = c0 + piece < a.width ? N * 4 : 0;
+      for (int k = lane / LANES; k < len; k += N) {
         const float* src = gates + (int64_t)(rs + tile * RS_TOK + k) * 2 * a.width + (bytes > 0 ? c0 + piece : 0);
 #pragma unroll
-        for (int w = 0; w < 2; ++w)
-          asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst + (w * RS_TOK + k) * 32 + piece)), "l"(src + w * a.width), "r"(bytes) : "memory");
+        for (int w = 0; w < 2; ++w) {
+          const uint32_t to = (uint32_t)__cvta_generic_to_shared(dst + (w * RS_TOK + k) * 32 + piece);
+          if constexpr (N == 4) asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(to), "l"(src + w * a.width), "r"(bytes) : "memory");
+          else asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(to), "l"(src + w * a.width), "r"(bytes) : "memory");
+        }
       }
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
@@ -282,15 +287,15 @@ __global__ void __launch_bounds__(256) rglru_out_kernel(RglruArgs a, const float
     stf((E*)a.out + (int64_t)t * a.width + c, gates[(int64_t)t * 2 * a.width + c] * gelu_tanhf_(ldf((const E*)a.yx + (int64_t)t * 2 * a.width + c)));
 }
 
-template <typename E>
+template <typename E, int N>
 static int rglru_prompt(const RglruArgs& a, cudaStream_t st) {
   float* gates = const_cast<float*>(a.gates);
   const int slices = (a.width + 255) / 256;
   const dim3 eg(std::min(a.T, std::max(1, 148 * 8 / slices)), slices), cg(a.B, (a.width + 31) / 32);
   KGE_REQUIRE(cg.y <= 65535, "rglru_scan: width %d", a.width);
-  KGE_CUDA_OK(cudaFuncSetAttribute(rglru_chain_kernel<E>, cudaFuncAttributeMaxDynamicSharedMemorySize, RS_SMEM));
+  KGE_CUDA_OK(cudaFuncSetAttribute(rglru_chain_kernel<E, N>, cudaFuncAttributeMaxDynamicSharedMemorySize, RS_SMEM));
   KGE_CUDA_OK(launch_pdl(rglru_ab_kernel<E>, eg, dim3(256), 0, st, a, gates));
-  KGE_CUDA_OK(launch_pdl(rglru_chain_kernel<E>, cg, dim3(32), RS_SMEM, st, a, gates));
+  KGE_CUDA_OK(launch_pdl(rglru_chain_kernel<E, N>, cg, dim3(32), RS_SMEM, st, a, gates));
   KGE_CUDA_OK(launch_pdl(rglru_out_kernel<E>, eg, dim3(256), 0, st, a, (const float*)gates));
   return 0;
 }
@@ -300,8 +305,8 @@ int rglru_scan(const RglruArgs& a, cudaStream_t st) {
   KGE_REQUIRE(a.taps >= 1 && a.taps <= MAX_TAPS, "rglru_scan: %d taps (1..%d)", a.taps, MAX_TAPS);
   const dim3 grid(a.B, (a.width + 127) / 128), block(128);
   if (a.T > a.B) {                       // some request brings several rows
-    // the chain copies 16-byte pieces of rows
-    if (a.width % 4 == 0 && (reinterpret_cast<uintptr_t>(a.gates) & 15) == 0) return a.elt == KGE_ELT_F32 ? rglru_prompt<float>(a, st) : rglru_prompt<__nv_bfloat16>(a, st);
+    if (a.width % 4 == 0 && (reinterpret_cast<uintptr_t>(a.gates) & 15) == 0) return a.elt == KGE_ELT_F32 ? rglru_prompt<float, 4>(a, st) : rglru_prompt<__nv_bfloat16, 4>(a, st);
+    return a.elt == KGE_ELT_F32 ? rglru_prompt<float, 1>(a, st) : rglru_prompt<__nv_bfloat16, 1>(a, st);
   }
   cudaError_t ce = a.elt == KGE_ELT_F32 ? launch_pdl(rglru_scan_kernel<float>, grid, block, 0, st, a)
                                         : launch_pdl(rglru_scan_kernel<__nv_bfloat16>, grid, block, 0, st, a);

@@ -81,6 +81,22 @@ def test_narrow_projections(kge, tmp_path, experts, m_heads):
     llm.close()
 
 
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+@pytest.mark.parametrize("width", [33, 36, 66, 128])
+def test_gated_recurrence_by_width(kge, tmp_path, width, dtype):
+    """The recurrence of prompt steps in 64-token stages: widths that are copied number by number and in fours, a last block of 32
+    channels with one of them and with all, pieces around a stage's edge, more stages than the ring has, one token."""
+    cfg = oh.make_config(layers=("rglru",), mlps=(None,), r_width=width, r_blocks=3 if width % 3 == 0 else 2)
+    W = oh.make_weights(cfg, seed=23)
+    toks = prompt(cfg, 340)
+    want = oh.forward(cfg, W, toks)
+    llm = make_engine(kge, tmp_path, cfg, W, dtype)
+    for rid, pieces in enumerate([[340], [63, 64, 65, 1, 2, 145]]):
+        check(run_pieces(llm, rid, toks, pieces), want, dtype, f"pieces {pieces}")
+        llm.trace_end(rid)
+    llm.close()
+
+
 @pytest.mark.parametrize("m_dim,m_vdim", [(16, 8), (64, 40), (128, 256)])
 def test_matrix_memory_in_chunks_of_64(kge, tmp_path, m_dim, m_vdim):
     """bfloat16 head sizes that take the tensor-core chunks: pieces that end before, at and behind a chunk's edge, single tokens
