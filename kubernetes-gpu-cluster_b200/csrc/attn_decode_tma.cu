@@ -34,7 +34,6 @@ namespace adt {
 
 constexpr int BN = 64;                       // keys per tile
 constexpr int kStages = 3;
-constexpr uint32_t kSpin = 1u << 26;
 constexpr int kMaxGroups = 1 << 16;          // (request, kv head) pairs one launch may have
 
 // arrival counters of the split-KV merge, one per (request, kv head); zero at load, reset by the CTA that merges
@@ -49,14 +48,6 @@ __device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
 }
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ void mbar_wait(uint32_t bar, uint32_t parity) {
-  uint32_t ok, spins = 0;
-  do {
-    asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}"
-                 : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
-    if (!ok && ++spins > kSpin) __trap();
-  } while (!ok);
 }
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int c0, int c1) {
   asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"

@@ -110,6 +110,22 @@ namespace kge {
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
+// Wait until the phase of a shared-memory barrier that `parity` names has completed; a lost arrival becomes an error within seconds
+// and not a hang.  Bounded by the clock and not by a count of tries: a try that fails lasts about 7800 cycles (4 us), so 2^26 of
+// them, once taken for seconds, are four and a half minutes.  No wait here spans the previous kernel: its callers are past pdl_wait.
+constexpr long long kBarrierCycles = 10000000000ll;      // 5 s at 1.97 GHz
+__device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}" : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+  return ok != 0;
+}
+__device__ __forceinline__ void mbar_wait(uint32_t bar, uint32_t parity) {
+  if (mbar_try(bar, parity)) return;
+  const long long t0 = clock64();
+  while (!mbar_try(bar, parity))
+    if (clock64() - t0 > kBarrierCycles) __trap();
+}
+
 // Thread-block clusters.  A block's shared memory may be touched by its peers only once it is known to run: a kernel arrives
 // (relaxed: there is nothing to publish) at its start and waits before its first remote access, which its own work hides.
 __device__ __forceinline__ uint32_t cluster_ctarank() { uint32_t r; asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r)); return r; }

@@ -1,5 +1,5 @@
-"""Distributed shared memory is touched only behind a cluster barrier: a block's peers may not have started before it.  Read from
-the kernels' sources, since a store that comes too early need not show in a result."""
+"""Rules of the kernels that no result shows, read from their sources: distributed shared memory is touched only behind a cluster
+barrier, since a block's peers may not have started before it; and barrier waits are bounded in time, in one place."""
 import glob
 import os
 import re
@@ -36,3 +36,11 @@ def test_a_cluster_barrier_comes_before_the_first_remote_access(file, kernel, bo
     assert first, (file, kernel)
     wait = BARRIER.search(code)
     assert wait and wait.start() < first.start(), (file, kernel, code[first.start():first.start() + 80])
+
+
+def test_barrier_waits_are_bounded_by_the_clock():
+    """A try on a shared-memory barrier that fails lasts microseconds: counting tries bounds a wait by minutes."""
+    users = {os.path.basename(p) for p in glob.glob(os.path.join(CSRC, "*.cu*")) if "try_wait" in re.sub(r"//[^\n]*", "", open(p).read())}
+    assert users == {"common.cuh"}
+    src = open(os.path.join(CSRC, "common.cuh")).read()
+    assert 1e9 <= int(re.search(r"kBarrierCycles = (\d+)ll", src).group(1)) <= 2e10
