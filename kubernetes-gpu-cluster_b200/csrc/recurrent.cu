@@ -197,8 +197,8 @@ __global__ void __launch_bounds__(256) rglru_ab_kernel(RglruArgs a, float* gates
 // One warp per 32 channels of a request: the coefficients of 64 tokens at a time arrive by cp.async, three stages ahead, so that the
 // chain waits for its fma's and not for memory (with eight tokens' loads in flight it took 145 us).  N: numbers per copy, four
 // where the rows are aligned for it, one elsewhere (widths that are no multiple of four).
-constexpr int RS_TOK = 64, RS_STAGES = 4, RS_SMEM = RS_STAGES * 2 * RS_TOK * 32 * 4;
-template <typename E, int N>
+constexpr int RS_STAGES = 3;
+template <typename E, int N, int TOK>
 __global__ void __launch_bounds__(32) rglru_chain_kernel(RglruArgs a, float* gates) {
   pdl_launch_dependents();
   pdl_wait();
@@ -207,20 +207,20 @@ __global__ void __launch_bounds__(32) rglru_chain_kernel(RglruArgs a, float* gat
   const bool in = c < a.width;
   const int rs = a.qsl[b], re = a.qsl[b + 1], n = re - rs;
   if (n <= 0) return;
-  const int p0 = a.positions[rs], tiles = (n + RS_TOK - 1) / RS_TOK;
+  const int p0 = a.positions[rs], tiles = (n + TOK - 1) / TOK;
   float* slot = a.state + (int64_t)a.slots[b] * a.slot_stride;
   const E* yx = (const E*)a.yx;
   auto fetch = [&](int tile) {
     if (tile < tiles) {
-      float* dst = rs_sm + (tile % RS_STAGES) * (2 * RS_TOK * 32);
+      float* dst = rs_sm + (tile % RS_STAGES) * (2 * TOK * 32);
       constexpr int LANES = 32 / N;                        // lanes that copy a token's 32 channels
-      const int len = min(RS_TOK, n - tile * RS_TOK), piece = (lane % LANES) * N;
+      const int len = min(TOK, n - tile * TOK), piece = (lane % LANES) * N;
       const int bytes = c0 + piece < a.width ? N * 4 : 0;
       for (int k = lane / LANES; k < len; k += N) {
-        const float* src = gates + (int64_t)(rs + tile * RS_TOK + k) * 2 * a.width + (bytes > 0 ? c0 + piece : 0);
+        const float* src = gates + (int64_t)(rs + tile * TOK + k) * 2 * a.width + (bytes > 0 ? c0 + piece : 0);
 #pragma unroll
         for (int w = 0; w < 2; ++w) {
-          const uint32_t to = (uint32_t)__cvta_generic_to_shared(dst + (w * RS_TOK + k) * 32 + piece);
+          const uint32_t to = (uint32_t)__cvta_generic_to_shared(dst + (w * TOK + k) * 32 + piece);
           if constexpr (N == 4) asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(to), "l"(src + w * a.width), "r"(bytes) : "memory");
           else asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(to), "l"(src + w * a.width), "r"(bytes) : "memory");
         }
@@ -235,24 +235,24 @@ __global__ void __launch_bounds__(32) rglru_chain_kernel(RglruArgs a, float* gat
     asm volatile("cp.async.wait_group %0;" ::"n"(RS_STAGES - 2) : "memory");
     __syncwarp();
     fetch(tile + RS_STAGES - 1);                           // the stage that the previous turn has read
-    const float* av = rs_sm + (tile % RS_STAGES) * (2 * RS_TOK * 32) + lane;
-    const float* bv = av + RS_TOK * 32;
-    const int len = min(RS_TOK, n - tile * RS_TOK);
-    float* out = gates + (int64_t)(rs + tile * RS_TOK) * 2 * a.width + c;
-    int k = 0;
-    for (; k + 16 <= len; k += 16) {
-      float x[16], y[16];
+    const float* av = rs_sm + (tile % RS_STAGES) * (2 * TOK * 32) + lane;
+    const float* bv = av + TOK * 32;
+    const int len = min(TOK, n - tile * TOK);
+    float* out = gates + (int64_t)(rs + tile * TOK) * 2 * a.width + c;
+    if (len == TOK) {
+      float x[TOK], y[TOK];
 #pragma unroll
-      for (int i = 0; i < 16; ++i) { x[i] = av[(k + i) * 32]; y[i] = bv[(k + i) * 32]; }
+      for (int i = 0; i < TOK; ++i) { x[i] = av[i * 32]; y[i] = bv[i * 32]; }
 #pragma unroll
-      for (int i = 0; i < 16; ++i) {
+      for (int i = 0; i < TOK; ++i) {
         S = fmaf(x[i], S, y[i]);
-        if (in) out[(int64_t)(k + i) * 2 * a.width] = S;
+        if (in) out[(int64_t)i * 2 * a.width] = S;
       }
-    }
-    for (; k < len; ++k) {
-      S = fmaf(av[k * 32], S, bv[k * 32]);
-      if (in) out[(int64_t)k * 2 * a.width] = S;
+    } else {
+      for (int k = 0; k < len; ++k) {
+        S = fmaf(av[k * 32], S, bv[k * 32]);
+        if (in) out[(int64_t)k * 2 * a.width] = S;
+      }
     }
     __syncwarp();
   }
@@ -287,17 +287,21 @@ __global__ void __launch_bounds__(256) rglru_out_kernel(RglruArgs a, const float
     stf((E*)a.out + (int64_t)t * a.width + c, gates[(int64_t)t * 2 * a.width + c] * gelu_tanhf_(ldf((const E*)a.yx + (int64_t)t * 2 * a.width + c)));
 }
 
-template <typename E, int N>
-static int rglru_prompt(const RglruArgs& a, cudaStream_t st) {
+template <typename E, int N, int TOK>
+static int rglru_prompt_as(const RglruArgs& a, cudaStream_t st) {
   float* gates = const_cast<float*>(a.gates);
   const int slices = (a.width + 255) / 256;
   const dim3 eg(std::min(a.T, std::max(1, 148 * 8 / slices)), slices), cg(a.B, (a.width + 31) / 32);
   KGE_REQUIRE(cg.y <= 65535, "rglru_scan: width %d", a.width);
-  KGE_CUDA_OK(cudaFuncSetAttribute(rglru_chain_kernel<E, N>, cudaFuncAttributeMaxDynamicSharedMemorySize, RS_SMEM));
   KGE_CUDA_OK(launch_pdl(rglru_ab_kernel<E>, eg, dim3(256), 0, st, a, gates));
-  KGE_CUDA_OK(launch_pdl(rglru_chain_kernel<E, N>, cg, dim3(32), RS_SMEM, st, a, gates));
+  KGE_CUDA_OK(launch_pdl(rglru_chain_kernel<E, N, TOK>, cg, dim3(32), RS_STAGES * 2 * TOK * 32 * 4, st, a, gates));
   KGE_CUDA_OK(launch_pdl(rglru_out_kernel<E>, eg, dim3(256), 0, st, a, (const float*)gates));
   return 0;
+}
+
+template <typename E, int N>
+static int rglru_prompt(const RglruArgs& a, cudaStream_t st) {
+  return a.T < 8 * a.B ? rglru_prompt_as<E, N, 8>(a, st) : rglru_prompt_as<E, N, 16>(a, st);
 }
 
 int rglru_scan(const RglruArgs& a, cudaStream_t st) {

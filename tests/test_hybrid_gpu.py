@@ -84,16 +84,27 @@ def test_narrow_projections(kge, tmp_path, experts, m_heads):
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 @pytest.mark.parametrize("width", [33, 36, 66, 128])
 def test_gated_recurrence_by_width(kge, tmp_path, width, dtype):
-    """The recurrence of prompt steps in 64-token stages: widths that are copied number by number and in fours, a last block of 32
-    channels with one of them and with all, pieces around a stage's edge, more stages than the ring has, one token."""
+    """The recurrence of prompt steps in stages of 16 tokens, of 8 where most requests bring one: widths that are copied number by
+    number and in fours, a last block of 32 channels with one of them and with all, pieces around a stage's edge, more stages than
+    the ring has, one token; then single tokens beside pieces."""
     cfg = oh.make_config(layers=("rglru",), mlps=(None,), r_width=width, r_blocks=3 if width % 3 == 0 else 2)
     W = oh.make_weights(cfg, seed=23)
     toks = prompt(cfg, 340)
     want = oh.forward(cfg, W, toks)
-    llm = make_engine(kge, tmp_path, cfg, W, dtype)
-    for rid, pieces in enumerate([[340], [63, 64, 65, 1, 2, 145]]):
+    llm = make_engine(kge, tmp_path, cfg, W, dtype, tokens=1024, seqs=16)
+    for rid, pieces in enumerate([[340], [15, 16, 17, 33, 1, 2, 64, 65, 127]]):
         check(run_pieces(llm, rid, toks, pieces), want, dtype, f"pieces {pieces}")
         llm.trace_end(rid)
+    n = 12
+    for rid in range(n):
+        llm.trace_add(rid, toks[:2 + rid])
+        llm.trace_step([(rid, 2 + rid, [])])
+    for turn, long in enumerate((7, 8, 9, 25)):
+        for rid in range(n):
+            llm.trace_add(rid, [toks[2 + rid + turn]])
+        llm.trace_add(n + turn, toks[:long])
+        got = llm.trace_step([(rid, 1, [0]) for rid in range(n)] + [(n + turn, long, list(range(long)))])
+        check(got, want[[2 + rid + turn for rid in range(n)] + list(range(long))], dtype, f"beside {long} rows")
     llm.close()
 
 
