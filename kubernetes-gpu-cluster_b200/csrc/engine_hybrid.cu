@@ -1306,7 +1306,7 @@ int hybrid_forward(kge_engine* e, int T, int B, int R, int max_blocks, const Ste
       ma.q = at(e->pbuf, L.off_mq); ma.k = at(e->pbuf, L.off_mk); ma.v = at(e->pbuf, L.off_mv); ma.g = at(e->pbuf, L.off_mg); ma.ld = ldp;
       ma.gates = e->gates32; ma.o_scratch = e->mo32; ma.nm_scratch = e->mo32 + (int64_t)T * h.m_heads * h.m_vdim; ma.norm_w = L.m_norm; ma.out = at(e->mixbuf, ka); ma.ldo = ko;
       ma.state = e->state + L.state_off; ma.slot_stride = e->slot_stride; ma.slots = m.sslot; ma.qsl = m.qsl; ma.positions = m.pos;
-      ma.B = B; ma.T = T; ma.H = h.m_heads; ma.dim = h.m_dim; ma.vdim = h.m_vdim;
+      ma.B = B; ma.T = T; ma.max_rows = aa.max_q; ma.H = h.m_heads; ma.dim = h.m_dim; ma.vdim = h.m_vdim;
       ma.cap = h.gate_cap; ma.q_scale = 1.f / sqrtf((float)h.m_dim); ma.eps = s.eps; ma.den_eps = 1e-6f; ma.out_scale = h.right_scale; ma.elt = elt;
       HFWD(C_MLSTM, 2.0 * B * mlstm_state_floats(h.m_heads, h.m_dim, h.m_vdim) * 4 + (double)T * h.m_heads * (2 * h.m_dim + 3 * h.m_vdim) * es,
            4.0 * T * h.m_heads * (double)h.m_dim * h.m_vdim, mlstm_step(ma, st));

@@ -281,6 +281,7 @@ struct MlstmArgs {
   float* state = nullptr; int64_t slot_stride = 0;
   const int32_t* slots = nullptr; const int32_t* qsl = nullptr; const int32_t* positions = nullptr;
   int B = 0, T = 0, H = 0, dim = 0, vdim = 0;
+  int max_rows = 0;                        // the most rows of the step that one request brings; 0: not known
   float cap = 1.f, q_scale = 1.f, eps = 1e-5f, den_eps = 1e-6f, out_scale = 1.f;
   int elt = KGE_ELT_BF16;
 };

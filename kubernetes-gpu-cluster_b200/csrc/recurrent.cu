@@ -1029,6 +1029,15 @@ __global__ void mlstm_norm_gate_kernel(MlstmArgs a) {
   }
 }
 
+// Tensor-core chunks or the fp32 ones, by estimates (us) from measurements at 8 x 32 x 32 to 4 x 128 x 256 and 1 to 256 requests: a
+// tensor-core block fills an SM and takes 9 us beside 7 per 64 tokens of the longest request, an fp32 one shares it with two others,
+// 8 us and 1.1 per token (0.6 to 1.1 by head size).  4 x 128 x 256, tensor cores and fp32: 2 x 1150 tokens 152 / 1278, 200 and 64
+// single ones 134 / 290, 8 x 40 36 / 65; 30 x 16 88 / 84, 64 x 8 178 / 73, 60 and 200 single ones 429 / 174, 100 x 2 263 / 60.
+static bool mlstm_use_mma(const MlstmArgs& a) {
+  const double rows = a.max_rows > 0 ? a.max_rows : a.T - a.B + 1, blocks = (double)a.B * a.H * ((a.vdim + 31) / 32);
+  return 9.0 * blocks / 148 + 7.0 * ((int)(rows + 63) / 64) < 8.0 * blocks / (3 * 148) + 1.1 * rows;
+}
+
 int mlstm_step(const MlstmArgs& a, cudaStream_t st) {
   if (a.T <= 0 || a.B <= 0) return 0;
   if (a.o_scratch && a.nm_scratch && a.dim <= ML_MAXD && a.dim % 4 == 0 && a.H <= 65535) {
@@ -1040,7 +1049,7 @@ int mlstm_step(const MlstmArgs& a, cudaStream_t st) {
     // tensor-core chunks: bfloat16 rows in 16-byte pieces, key dimensions in steps of 16, a head's column blocks in one cluster
     const bool mma_ok = a.elt == KGE_ELT_BF16 && a.dim % 16 == 0 && a.vdim % 8 == 0 && a.vdim <= 8 * MM_COLS && a.ld % 8 == 0 &&
                         ((reinterpret_cast<uintptr_t>(a.q) | reinterpret_cast<uintptr_t>(a.k) | reinterpret_cast<uintptr_t>(a.v)) & 15) == 0;
-    if (a.T > a.B && mma_ok) {
+    if (a.T > a.B && mma_ok && mlstm_use_mma(a)) {
       KGE_CUDA_OK(cudaFuncSetAttribute(mlstm_mma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(MlstmTile)));
       prefer_max_shared(mlstm_mma_kernel);
       cudaLaunchConfig_t cfg = {};

@@ -145,19 +145,19 @@ def test_matrix_memory_in_chunks_of_64(kge, tmp_path, m_dim, m_vdim):
     llm.close()
 
 
-@pytest.mark.parametrize("dtype,m_vdim", [("float32", 256), ("bfloat16", 256), ("bfloat16", 264)])
-def test_matrix_memory_of_more_requests_than_fit_at_once(kge, tmp_path, dtype, m_vdim):
+@pytest.mark.parametrize("dtype,m_vdim,long", [("float32", 256, 70), ("bfloat16", 256, 70), ("bfloat16", 256, 240), ("bfloat16", 264, 70)])
+def test_matrix_memory_of_more_requests_than_fit_at_once(kge, tmp_path, dtype, m_vdim, long):
     """A head's value columns are spread over blocks that all read its normaliser, and with 70 requests not all blocks of a launch
-    start together: a pure decode step, then a step of single tokens beside a prompt (float32 and 264 columns: 32 tokens at a time;
-    256: 64), then another decode step on the state that it left."""
+    start together: a pure decode step, then a step of single tokens beside a prompt (32 tokens at a time in fp32; 64 on
+    tensor cores where the prompt is long: 240), then another decode step on the state that it left."""
     cfg = oh.make_config(layers=("parallel",), mlps=(None,), left_scale=0.0, m_heads=4, m_dim=128, m_vdim=m_vdim)
     W = oh.make_weights(cfg, seed=19)
-    toks = prompt(cfg, 80)
+    toks = prompt(cfg, long + 10)
     want = oh.forward(cfg, W, toks).numpy()
     n = 70
     llm = make_engine(kge, tmp_path, cfg, W, dtype, tokens=2560, seqs=n + 1)
     size = np.sqrt((want ** 2).mean())
-    singly = np.sqrt(((run_pieces(llm, 999, toks, [1] * 80) - want) ** 2).mean(-1)) / size
+    singly = np.sqrt(((run_pieces(llm, 999, toks, [1] * len(toks)) - want) ** 2).mean(-1)) / size
     llm.trace_end(999)
 
     def close(got, rows, what):
@@ -173,9 +173,9 @@ def test_matrix_memory_of_more_requests_than_fit_at_once(kge, tmp_path, dtype, m
             llm.trace_add(rid, [toks[have[rid]]])
         rows = [(rid, 1, [0]) for rid in range(n)]
         if turn == "mixed":
-            llm.trace_add(n, toks[:70])
-            rows.append((n, 70, [69]))
-        close(llm.trace_step(rows), have + ([69] if turn == "mixed" else []), turn)
+            llm.trace_add(n, toks[:long])
+            rows.append((n, long, [long - 1]))
+        close(llm.trace_step(rows), have + ([long - 1] if turn == "mixed" else []), turn)
         have = [h + 1 for h in have]
     llm.close()
 
