@@ -467,7 +467,7 @@ __global__ void __launch_bounds__(256) linear_narrow_kernel(LinearArgs a) {
         const int k = (warp + i * 8) * 64 + h * 32;
         const bool in = k + t * 8 < a.K;
 #pragma unroll
-        for (int j = 0; j < NT; ++j) copy(dst + (2 * j + h) * 32, wrow[j] + k, in);
+        for (int j = 0; j < NT; ++j) copy(dst + (2 * j + h) * 32, wrow[j] + k, in && j * 8 + g < a.N);      // no reads of one row in the place of many
 #pragma unroll
         for (int j = 0; j < 2; ++j) copy(dst + (2 * (NT + j) + h) * 32, xrow[j] + k, in);
       }
@@ -515,7 +515,11 @@ __global__ void __launch_bounds__(256) linear_narrow_kernel(LinearArgs a) {
     linear_store(a, (float*)a.y + (int64_t)(m0 + r) * a.ldy + n, (const E*)a.bias, n, v, 0.f);
   }
 }
+// The general kernels keep short sums over many rows where three or four column tiles are in use: a CTA would set up 144 KB of ring
+// for six chunks of K (us here and there by 32 columns: 16384 x 256 13.9 and 8.3, 16384 x 264 16.6 and 13.9, 8192 x 264 10.0 and 9.4;
+// but 16384 x 384 14.5 and 16.2, 4096 x 264 5.9 and 8.1).
 static bool linear_narrow_ok(const LinearArgs& a) {
+  if (a.N > 16 && a.K < 384 && a.T > 4096) return false;
   return a.elt == KGE_ELT_BF16 && a.out_f32 && !a.w2 && !a.group_off && !a.xrows && !a.yrows && !a.row_scale && a.nz == 1 && a.N <= 32 && a.K >= 256 && a.K % 8 == 0 && a.ldx % 8 == 0 &&
          ((reinterpret_cast<uintptr_t>(a.x) | reinterpret_cast<uintptr_t>(a.w)) & 15) == 0;
 }

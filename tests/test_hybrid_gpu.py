@@ -81,6 +81,19 @@ def test_narrow_projections(kge, tmp_path, experts, m_heads):
     llm.close()
 
 
+@pytest.mark.parametrize("rows", [4096, 4097])
+def test_narrow_projections_of_long_steps(kge, tmp_path, rows):
+    """A router of 20 columns over a width of 264: the last row count of the kernel above and the first of the general ones."""
+    cfg = oh.make_config(width=264, layers=("rglru",), mlps=("moe",), experts=20, top=20)
+    W = oh.make_weights(cfg, seed=29)
+    toks = prompt(cfg, rows)
+    llm = make_engine(kge, tmp_path, cfg, W, "bfloat16", tokens=rows + 16)
+    at = [0, 17, 2048, rows - 2, rows - 1]
+    llm.trace_add(0, toks)
+    check(llm.trace_step([(0, rows, at)]), oh.forward(cfg, W, toks)[at], "bfloat16", f"{rows} rows")
+    llm.close()
+
+
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 @pytest.mark.parametrize("width", [33, 36, 66, 128])
 def test_gated_recurrence_by_width(kge, tmp_path, width, dtype):
