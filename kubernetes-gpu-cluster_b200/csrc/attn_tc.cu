@@ -138,7 +138,7 @@ __global__ void __launch_bounds__(TMA ? 192 : 160, 2)
 attn_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
                bf16* __restrict__ out, const bf16* __restrict__ q, int q_stride, const bf16* __restrict__ k_cache,
                const bf16* __restrict__ v_cache, const int32_t* __restrict__ block_table, int max_blocks,
-               const int32_t* __restrict__ seq_lens, const int32_t* __restrict__ qsl, int num_reqs, int by_request, int H, int KV, int bs_shift,
+               const int32_t* __restrict__ seq_lens, const int32_t* __restrict__ qsl, int by_request, int H, int KV, int bs_shift,
                float scale_log2_in, float cap_in2, float cap_log2, const float* __restrict__ sinks,
                const __grid_constant__ CUtensorMap tm_pk, const __grid_constant__ CUtensorMap tm_pv, WinArgs win) {
   static_assert(!WIN || TMA, "window kernels fetch their tiles by TMA");
@@ -160,17 +160,8 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
   // pieces: 185 us against 240; 253 with the decode rows last, whose serial walk over their keys then is the tail).
   const int G = H / KV;
   const int TT = BM / G;
-  const int tiles_max = (int)gridDim.x / (KV * num_reqs);
-  int b, kvh, rank;
-  if (by_request) {
-    rank = (int)blockIdx.x % tiles_max;
-    const int rem = (int)blockIdx.x / tiles_max;
-    kvh = rem % KV; b = rem / KV;
-  } else {
-    const int per_rank = KV * num_reqs, rem = (int)blockIdx.x % per_rank;
-    rank = (int)blockIdx.x / per_rank;
-    b = rem / KV; kvh = rem % KV;
-  }
+  // The grid's dimensions are what they are in either order, so that an empty CTA has nothing to divide.
+  const int rank = by_request ? blockIdx.x : blockIdx.z, kvh = by_request ? blockIdx.y : blockIdx.x, b = by_request ? blockIdx.z : blockIdx.y;
   const int q0 = qsl[b], q_len = qsl[b + 1] - q0;
   const int tok0 = ((q_len + TT - 1) / TT - 1 - rank) * TT;
   if (tok0 < 0) return;
@@ -516,10 +507,10 @@ template <int HD> constexpr int tc_smem() { return 128 * HD * 2 + 4 * BNK * HD *
 int make_tmap(CUtensorMap* m, const void* ptr, int64_t rows, int64_t cols, int box_rows);   // gemm_tc.cu (cached)
 
 // CTAs of a launch: one per (query tile, request, kv head); most of them are empty when a few requests are much longer than T / B
-static int64_t tc_grid(int B, int T, int max_q_len, int TT, int KV, int& by_request) {
-  const int64_t even = (int64_t)((max_q_len + TT - 1) / TT) * B;
-  by_request = 2 * ((int64_t)T / TT + B) < even;
-  return even * KV;
+static dim3 tc_grid(int B, int T, int max_q_len, int TT, int KV, int& by_request) {
+  const unsigned tiles = (max_q_len + TT - 1) / TT;
+  by_request = tiles > 65535 || 2 * ((int64_t)T / TT + B) < (int64_t)tiles * B;
+  return by_request ? dim3(tiles, KV, B) : dim3(KV, B, tiles);
 }
 
 template <int HD>
@@ -533,8 +524,7 @@ static int launch_tc(bf16* out, const bf16* q, int q_stride, const bf16* kc, con
   const int G = H / KV;
   const int TT = atc::BM / G;
   int by_request = 0;
-  const int64_t ctas = tc_grid(B, T, max_q_len, TT, KV, by_request);
-  KGE_REQUIRE(ctas <= INT32_MAX, "kge_paged_attn: too many query tiles");
+  const dim3 grid = tc_grid(B, T, max_q_len, TT, KV, by_request);
   CUtensorMap tk, tv;
   const bool tma = tunable(TUN_ATTN_TMA) != 0 && bs >= 8;
   if (tma) {
@@ -544,15 +534,15 @@ static int launch_tc(bf16* out, const bf16* q, int q_stride, const bf16* kc, con
     if (int rc = make_tmap(&tv, vc, rows, HD, box_rows)) return rc;
     auto kern = cap ? atc::attn_tc_kernel<HD, true, true> : atc::attn_tc_kernel<HD, true, false>;
     KGE_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, atc::tc_smem<HD>()));
-    KGE_CUDA_OK(launch_pdl(kern, dim3((unsigned)ctas), dim3(192), atc::tc_smem<HD>(), st, tk, tv, out, q, q_stride,
-                           kc, vc, bt, max_blocks, sl, qsl, B, by_request, H, KV, bs_shift, scale * atc::kLog2e, cap_in2, cap_log2, sinks, tk, tv, atc::WinArgs()));
+    KGE_CUDA_OK(launch_pdl(kern, grid, dim3(192), atc::tc_smem<HD>(), st, tk, tv, out, q, q_stride,
+                           kc, vc, bt, max_blocks, sl, qsl, by_request, H, KV, bs_shift, scale * atc::kLog2e, cap_in2, cap_log2, sinks, tk, tv, atc::WinArgs()));
     return 0;
   }
   memset(&tk, 0, sizeof tk); memset(&tv, 0, sizeof tv);
   auto kern = cap ? atc::attn_tc_kernel<HD, false, true> : atc::attn_tc_kernel<HD, false, false>;
   KGE_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, atc::tc_smem<HD>()));
-  KGE_CUDA_OK(launch_pdl(kern, dim3((unsigned)ctas), dim3(160), atc::tc_smem<HD>(), st, tk, tv, out, q, q_stride, kc,
-                         vc, bt, max_blocks, sl, qsl, B, by_request, H, KV, bs_shift, scale * atc::kLog2e, cap_in2, cap_log2, sinks, tk, tv, atc::WinArgs()));
+  KGE_CUDA_OK(launch_pdl(kern, grid, dim3(160), atc::tc_smem<HD>(), st, tk, tv, out, q, q_stride, kc,
+                         vc, bt, max_blocks, sl, qsl, by_request, H, KV, bs_shift, scale * atc::kLog2e, cap_in2, cap_log2, sinks, tk, tv, atc::WinArgs()));
   return 0;
 }
 
@@ -564,8 +554,7 @@ static int launch_tc_window(bf16* out, const bf16* q, int q_stride, const bf16* 
   while ((1 << bs_shift) < bs) ++bs_shift;
   const int TT = atc::BM / (H / KV);
   int by_request = 0;
-  const int64_t ctas = tc_grid(B, T, max_q_len, TT, KV, by_request);
-  KGE_REQUIRE(ctas <= INT32_MAX, "paged_attn_window_tc: too many query tiles");
+  const dim3 grid = tc_grid(B, T, max_q_len, TT, KV, by_request);
   CUtensorMap tk, tv, tpk, tpv;
   const int box_rows = bs < atc::BNK ? bs : atc::BNK;
   const int64_t rows = (int64_t)1 << 30;
@@ -579,8 +568,8 @@ static int launch_tc_window(bf16* out, const bf16* q, int q_stride, const bf16* 
   }
   auto kern = atc::attn_tc_kernel<HD, true, false, true>;
   KGE_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, atc::tc_smem<HD>()));
-  KGE_CUDA_OK(launch_pdl(kern, dim3((unsigned)ctas), dim3(192), atc::tc_smem<HD>(), st, tk, tv, out, q, q_stride, kc, vc, bt,
-                         max_blocks, sl, qsl, B, by_request, H, KV, bs_shift, scale * atc::kLog2e, 0.f, 0.f, sinks, tpk, tpv, win));
+  KGE_CUDA_OK(launch_pdl(kern, grid, dim3(192), atc::tc_smem<HD>(), st, tk, tv, out, q, q_stride, kc, vc, bt,
+                         max_blocks, sl, qsl, by_request, H, KV, bs_shift, scale * atc::kLog2e, 0.f, 0.f, sinks, tpk, tpv, win));
   return 0;
 }
 
