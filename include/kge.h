@@ -37,7 +37,7 @@ int kge_device_sm_count(void);
  *                             cluster and merge over distributed shared memory instead of workspace + merge kernel
  *                             (same bits; measured slower, so off by default)
  *   "attn_tma" 1/0            attention K/V tiles fetched by the TMA unit (one producer thread, cp.async.bulk.tensor boxes
- *                             of one KV block) instead of per-thread 16-byte cp.async gathers; 0 = the round-1 kernels, kept
+ *                             of one KV block) instead of per-thread 16-byte cp.async gathers; 0 = those kernels, kept
  *                             for same-box comparison and for block sizes below 8
  *   "gemm_ws" 0/1             1 = decode-sized projections split K over ordinary CTAs, two per SM, reduced through the caller's
  *                             workspace by the last CTA to arrive (faster alone, 19.5 vs 25.5 us on the 8B qkv shape, but not
@@ -47,17 +47,17 @@ int kge_device_sm_count(void);
  *   "gemm_l2_hints" 0/1       1 = the GEMM's TMA loads carry L2 eviction hints (weights evict_first, activations evict_last);
  *                             measured slower on the prefill step (weight tiles are re-read by other CTA pairs), so off
  *   "gemm_wide" 1/0           GEMMs of up to 64 tokens: 1 = where it keeps as many CTAs streaming as the 128-row plan, tiles of
- *                             256 weight rows with the tokens as the MMA's M side and the weights as its N side (a tcgen05.mma
- *                             fed from shared memory costs ~165 cycles whatever its shape, so twice the weight bytes per MMA);
- *                             (and up to 16 tokens, by size, weights streamed without staging tiles: csrc/gemm_rows.cuh);
- *                             0 = always 128-row tiles with the tokens as N.  C3 decode step 6.54-6.58 vs 6.64-6.71 ms
+ *                             256 weight rows with the tokens as the MMA's M side and the weights as its N side (twice the
+ *                             weight bytes per MMA), and up to 16 tokens, by size, weights streamed without staging tiles
+ *                             (csrc/gemm_rows.cuh); 0 = always 128-row tiles with the tokens as N.  64 tokens, us with 1 and 0:
+ *                             6144 x 4096 13.7 and 13.8, gated 28672 x 4096 45.0 and 41.1 (it was 44.5 and 48.6 before MMAs
+ *                             were issued behind elect.sync)
  *   "attn_persistent" 1/0     decode attention with 64-token KV blocks or larger: 1 = 2 x 148 resident CTAs each take an equal,
  *                             contiguous share of all key tiles of the launch (a (request, kv head) group is cut where shares
  *                             end; pieces merged by the last CTA of the group to arrive) - one round whatever the batch and
  *                             the context lengths are (launches of up to 192 requests with a workspace of at least three partial slots per
  *                             head; others use the other kernel); 0 = one CTA per (request, kv head, split) with equal splits.
  *                             64 x 2176 keys: 91.6-93.3 us against 95.6; 64 x 1024: 49.7 against 56.5; 8 x 8192: 53.0 against 60.2
- *                             (profiles/r02_summary.md section 6)
  * Returns 0, or -1 for an unknown name. */
 int kge_set_tunable(const char* name, int value);
 
@@ -333,7 +333,7 @@ int kge_step(kge_engine* e, const kge_step_batch* batch, int32_t* out_ids_host,
 
 /* Per-kernel timing for the roofline report: when enabled, every launch of the forward pass is
  * bracketed by CUDA events on the engine's stream and accumulated per category together with its
- * ALGORITHMIC work (bytes that must cross HBM once / flops), DESIGN.md "kernels".  Categories:
+ * ALGORITHMIC work (bytes that must cross HBM once / flops).  Categories:
  * 0 gemm (T<=256: weight streaming), 1 gemm (T>256: tensor bound), 2 decode attention,
  * 3 general (prefill / mixed) attention, 4 norms, 5 rope+kv write, 6 activation, 7 embed/gather,
  * 8 sampling, 9 all-reduce.  Timing adds event overhead: never enable it for a headline number. */

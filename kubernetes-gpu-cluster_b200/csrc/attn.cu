@@ -361,7 +361,7 @@ static int launch_attn(bf16* out, const bf16* q, int q_stride, const bf16* kc, c
     if (ns > 1 && ns <= 8 && tunable(TUN_ATTN_CLUSTER_MERGE) && !extras) {
       // opt-in: split-KV CTAs of one (request, kv head) as a cluster, merged over DSMEM - no workspace and one
       // kernel, but measured SLOWER than the merge kernel behind programmatic dependent launch (C3 decode step
-      // 7.64 vs 7.38 ms, profiles/r01_knob_sweep.md): cluster co-scheduling costs more than the extra launch
+      // 7.64 vs 7.38 ms): cluster co-scheduling costs more than the extra launch
       auto kern = attn_decode_kernel<HD, kDecodeStages, true>;
       KGE_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, decode_smem<HD>()));
       cudaLaunchConfig_t cfg = {};
@@ -384,7 +384,7 @@ static int launch_attn(bf16* out, const bf16* q, int q_stride, const bf16* kc, c
       pml = po + (int64_t)B * H * ns * HD;
     }
     // default: K/V tiles staged by the TMA unit, splits merged by the last CTA to finish (attn_decode_tma.cu)
-    // (measured, profiles/r02_attn_block_size.jsonl: with 16-token blocks a TMA box is 2 KB and the TMA unit's request
+    // (measured: with 16-token blocks a TMA box is 2 KB and the TMA unit's request
     // rate, not HBM, bounds the kernel - 107 us against 102 us for the cp.async gathers; from 32-token blocks on the
     // boxes are large enough and TMA wins, 96 us at 64)
     if (tunable(TUN_ATTN_TMA) && bs >= 32 && decode_tma_supported(B, KV, bs))

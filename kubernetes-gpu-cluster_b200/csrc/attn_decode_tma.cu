@@ -9,7 +9,7 @@
 //     mbarrier (expect_tx).  The four compute warps issue no loads and no address arithmetic at all: they wait on the
 //     stage's "full" barrier, read the swizzled tile with ldmatrix and release the stage with one arrive per warp.
 //     (The cp.async version spent 42 % of its issue slots, mostly on per-16-byte address generation, and reached
-//     84 % of HBM peak; profiles/r01_ncu_summary.md.)
+//     84 % of HBM peak.)
 //   - A sliding window cuts the range of tiles at its lower end (masking what lies before it in the first one).
 //   - The split-KV partials of a (request, kv head) are merged by whichever of its CTAs finishes LAST (arrival counter
 //     after __threadfence), in split order - the same sums as attn_merge_kernel, without a second launch.
@@ -333,7 +333,7 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_co
 // ---------------------------------------------------------------------------------------------- persistent variant
 // The same tile arithmetic, cut differently.  With one CTA per (request, kv head, split) the launch runs in rounds of
 // 2 x 148 resident CTAs and the last round is part empty: at 64 requests x 2176 keys (1024 CTAs, 3.46 rounds) the SMs
-// are busy 84 us of a 101 us kernel, and while they are busy HBM runs at 6.8 TB/s (profiles/r02_summary.md).  Here the
+// are busy 84 us of a 101 us kernel, and while they are busy HBM runs at 6.8 TB/s.  Here the
 // key tiles of all (request, kv head) groups form ONE sequence of U units, and CTA c of G takes the contiguous share
 // [c * chunk, (c + 1) * chunk): every CTA streams the same number of tiles, in one round.  A share covers the end of
 // one group, whole groups, and the start of another; each piece ("segment") is an ordinary split-KV partial, merged by

@@ -12,7 +12,7 @@
 // cp.async.bulk.tensor.2d boxes of {64 columns, block_size rows} (the cache of a layer seen as a 2-D tensor [rows, hd],
 // 128-byte swizzle = the layout the MMA descriptors expect), two tiles ahead for K and for V, completion counted by
 // mbarriers; tcgen05.commit tells it when a stage is free.  The softmax warps issue no loads.
-// TMA = false (knob "attn_tma" 0, block sizes below 8): the round-1 path, tiles gathered by the softmax threads with
+// TMA = false (knob "attn_tma" 0, block sizes below 8): tiles gathered by the softmax threads with
 // 16-byte cp.async (K two tiles ahead, V one; block-table lookup once per row) and published with fence.proxy.async.
 // Tensor-bound: 4 * hd * sum_b q_b (ctx0_b + (q_b+1)/2) flop per q head.
 #include <cuda.h>
@@ -105,7 +105,7 @@ __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&r)[32
   asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
 }
 
-// Pipeline (per 128-key tile j): the MMA thread issues S_{j+1} = Q K_{j+1}^T into the other S buffer
+// Pipeline (per 64-key tile j): the MMA thread issues S_{j+1} = Q K_{j+1}^T into the other S buffer
 // as soon as K_{j+1} has landed, so the tensor core works on it while the softmax warps turn S_j
 // into P_j; PV_j accumulates straight into the O columns of TMEM.  O is only rescaled when a row's
 // maximum grows by more than 2^8 since its reference maximum was fixed ("lazy rescale": P stays
@@ -157,10 +157,11 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
   // launch ends on short ones (request after request left SMs idle at the end: 2 x 1011 tokens behind 2777 keys 150 -> 137 us,
   // 4 x 2048 with 12 heads of 64 80 -> 56).  by_request (most of the grid is empty: decode rows beside long pieces): request after
   // request, so that the pieces' tiles are not strung out between empty CTAs (37 decode rows with up to 3000 keys and two such
-  // pieces: 185 us against 240; 253 with the decode rows last, whose serial walk over their keys then is the tail).
+  // pieces: a quarter less than by distance; still more with the decode rows last, whose serial walk over their keys then is the tail).
   const int G = H / KV;
   const int TT = BM / G;
-  // The grid's dimensions are what they are in either order, so that an empty CTA has nothing to divide.
+  // The grid's dimensions are what they are in either order, so that an empty CTA has nothing to divide (200 decode rows and 300
+  // tokens, 32 / 8 heads of 64, where nine of ten CTAs are empty: 152 us, 175 with a grid of one dimension).
   const int rank = by_request ? blockIdx.x : blockIdx.z, kvh = by_request ? blockIdx.y : blockIdx.x, b = by_request ? blockIdx.z : blockIdx.y;
   const int q0 = qsl[b], q_len = qsl[b + 1] - q0;
   const int tok0 = ((q_len + TT - 1) / TT - 1 - rank) * TT;
@@ -282,7 +283,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
     // ------------------------------------------------------------------ TMA producer (TMA only: 192 threads)
     // One thread: per tile it reads the tile's block ids and issues one box per (block, 64-column half).  (Spreading the
     // issue over several lanes with the block ids handed out by shuffle measured SLOWER here: 364 vs 471 TFLOP/s at
-    // 4 x 2048, profiles/r02_vs_libs_*.json; a prefill tile lasts long enough for one thread to stay ahead.)
+    // 4 x 2048; a prefill tile lasts long enough for one thread to stay ahead.)
     if (elect_one()) {
       const int bs = 1 << bs_shift;
       const int box_rows = bs < BNK ? bs : BNK;

@@ -3,9 +3,12 @@
 // Weight-stationary orientation ("swap-AB"): the 128-row MMA M dimension runs over WEIGHT rows
 // (N is always large: 768..128256) and the MMA N dimension (16..256) over TOKENS, so a decode
 // step with T = 16..256 tokens wastes no tensor-core rows and streams every weight byte exactly
-// once, while prefill uses 128x256 tiles.  D[weight row, token] lives in TMEM (fp32); the
-// epilogue reads it back with tcgen05.ld, adds bias (one scalar per TMEM lane), applies the
-// activation, rounds once to bf16 and stores y transposed.
+// once.  D[weight row, token] lives in TMEM (fp32); the epilogue reads it back with tcgen05.ld as
+// MMA fragments, adds the bias of their rows, applies the activation, rounds once to 16 bits, and
+// stmatrix turns the fragments so that a lane stores 16 bytes of an output row.
+// Which kernel: up to 16 tokens, by size, gemm_rows.cuh (weights streamed without staging tiles); up
+// to 64, where it keeps as many CTAs streaming, gemm_wide_kernel; above 64 CTA pairs with a token
+// tile of 32 to 256 (plan_pairs); single-CTA tiles elsewhere.
 //
 // Persistent, warp-specialised: warp 0 = TMA producer (cp.async.bulk.tensor, 128B swizzle),
 // warp 1 = tcgen05.mma issuer (one elected lane), warp 2 = TMEM allocator, warps 4-7 = epilogue.
@@ -63,7 +66,7 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map
 }
 // The same loads with an L2 eviction-priority hint (knob gemm_l2_hints): weights are read once per launch (evict_first),
 // the activation tile is re-read by every CTA (evict_last), so the prefill GEMM stops re-fetching X from HBM behind its
-// own output stream (ncu, round 1: 2.42 GB of DRAM traffic for 0.77 GB of algorithmic bytes on the gate_up shape).
+// own output stream (without it 2.42 GB of DRAM traffic for 0.77 GB of algorithmic bytes on the gate_up shape).
 __device__ __forceinline__ uint64_t l2_policy(bool keep) {
   uint64_t pol;
   if (keep) asm volatile("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(pol));
@@ -211,10 +214,10 @@ __device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar_cluster) {
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar_cluster) : "memory");
 }
 
-// PAIR (prefill, TOKN = 256): cta_group::2.  The two CTAs of a cluster form one 256 x 256 MMA tile:
-// each holds its own 128 weight rows (A) and HALF of the token tile (B, 128 tokens) in shared memory
-// (32 KB per stage instead of 48 KB: less L2->SM traffic and less shared-memory bandwidth), the
-// leader CTA issues tcgen05.mma.cta_group::2 for both, accumulators land in each CTA's own TMEM.
+// PAIR (TOKN = 256 columns of TMEM per accumulator): cta_group::2.  The two CTAs of a cluster form one
+// MMA tile of 256 weight rows x p.tokn tokens: each holds its own 128 weight rows (A) and HALF of the
+// token tile (B, up to 128 tokens) in shared memory (32 KB per k-block instead of 48 KB: less L2->SM
+// traffic and less shared-memory bandwidth; two k-blocks per stage, three stages), the leader CTA issues tcgen05.mma.cta_group::2 for both, accumulators land in each CTA's own TMEM.
 // All TMA loads of a stage complete on the LEADER's full barrier; tcgen05.commit multicasts the
 // "stage free" and "accumulator ready" arrivals to both CTAs; both epilogues release the accumulator
 // on the leader's tmem_empty barrier.  The width of the token tile is a launch parameter (p.tokn): the host picks what leaves
@@ -363,7 +366,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant
           tma_load_2d(a_dst, &tmap_w, full_bar(st), kb * BLK_K, woff + m_tile * BLK_M);
         }
       };
-      // the barrier that counts a stage's bytes: own (48 KB) or, PAIR, the leader's for both CTAs (2 x 32 KB)
+      // the barrier that counts a stage's bytes: its own or, PAIR, the leader's for both CTAs
       auto expect = [&](int st, int subs) {
         if (!PAIR) mbar_expect_tx(full_bar(st), STAGE_BYTES);
         else if (mrank == 0) mbar_expect_tx(full_bar(st), subs * (2 * A_BYTES + (uint32_t)tokn * BLK_K * 2));
@@ -469,13 +472,11 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant
     while (it.next(w, kb0, kb1)) {
       const int n_tile = w % p.n_tiles, m_tile = m_tile_of(w);
       if (no_rows(w)) continue;
-      [[maybe_unused]] const int n = m_tile * ROWS_OUT + (GATED ? (et & 63) : et);   // output column of this thread's row
       const int t0 = n_tile * tokn;
       mbar_wait(tfull_bar(acc), acc_phase);
       tc_fence_after();
       if (et == 0) trace_stamp(p, 7);              // (of the CTA's last segment: later segments overwrite the stamp)
       const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + acc * TOKN;
-      const float bv = (p.bias && n < p.N) ? bf2f(p.bias[n]) : 0.f;
       if (WS && (kb0 != 0 || kb1 != KB)) {
         // ---- stream-K: this segment is only part of tile w's k range.  Its fp32 partial goes to the workspace
         // ([column][128 rows]: a warp stores 128 consecutive bytes per column); slot 0 of a CTA holds the partial that
@@ -792,12 +793,13 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant
 }
 
 // ------------------------------------------------------------------------------ wide tiles for T <= 64
-// A tcgen05.mma whose operands both sit in shared memory costs ~165 cycles whatever its shape (profiles/r02_summary.md
-// section 3): with 128 weight rows as M and the tokens as N, a decode-sized GEMM pays four of them for every 16 KB of
-// weights and its main loop, not HBM, sets the pace (330-385 ns per k-block).  Here the roles are swapped and the tile
-// is wider: the tokens are the M side (64 rows loaded; the MMA is 128 tall and its upper half reads whatever follows
-// the token tile in shared memory - rows that are never read back), 256 weight rows are N of ONE MMA, so the same four
-// MMAs move 32 KB of weights.  D is [token][weight row] in TMEM: a thread owns a token and 256 consecutive outputs,
+// With 128 weight rows as M and the tokens as N, a decode-sized GEMM issues four MMAs for every 16 KB of weights.  Here the
+// roles are swapped and the tile is wider: the tokens are the M side (64 rows loaded; the MMA is 128 tall and its upper
+// half reads whatever follows the token tile in shared memory - rows that are never read back), 256 weight rows are N of
+// ONE MMA, so the same four MMAs move 32 KB of weights.  That paid when an MMA took 88 cycles and more to issue whatever
+// its shape; behind elect_one() a 128 x 64 x 16 one runs in 48, and the 128-row tiles are level or ahead, back to back on
+// cold weights, us at 64 tokens here and there: 6144 x 4096 13.7 and 13.8 (32 tokens 13.5 and 12.3), gated 16384 x 2048 16.6
+// and 13.9, gated 28672 x 4096 45.0 and 41.1.  D is [token][weight row] in TMEM: a thread owns a token and 256 consecutive outputs,
 // which it stores 16 bytes at a time; the fused SwiGLU epilogue finds gate (columns 0-127) and up (128-255) of an
 // output in the same thread.  One tile per CTA; K split over a cluster as above, the exchange buffer laid over the
 // pipeline stages once every CTA of the cluster is past its main loop.
@@ -1281,7 +1283,7 @@ static int max_clusters_wide(int S) {
 // 74 tiles) narrower tiles, down to 3/4 of the width, if that puts more CTAs to work (gate_up of Llama-8B: 128 tiles of
 // 112 outputs instead of 112 of 128).  A cost model over all widths and splits (k-block = max(MMA time, bytes at the
 // per-SM rate), price per split) picked plans that were faster alone and 0.35 ms per decode step SLOWER in the engine
-// (clusters of 3 and 5 next to the neighbouring kernels' CTAs); it was removed (profiles/r02_summary.md section 7).
+// (clusters of 3 and 5 next to the neighbouring kernels' CTAs); it was removed.
 // False: this problem keeps the 128-row kernels.
 static bool plan_wide(int T, int n_out, int K, bool gated, GemmPlan& g) {
   if (!tunable(TUN_GEMM_WIDE) || T > WIDE_M) return false;

@@ -175,9 +175,9 @@ __global__ void __launch_bounds__(128) rglru_scan_kernel(RglruArgs a) {
 // rglru_ab_kernel turns the gate pre-activations, in place, into the recurrence's coefficients (a_t, b_t = sqrt(1 - a_t^2)
 // i_t u_t); rglru_chain_kernel is then one fma per token and channel (S_t written over a_t) plus the state hand-over; and
 // rglru_out_kernel multiplies by gelu(y).  Same arithmetic per element as the fused kernel.  A thread keeps its channel and walks
-// over tokens (no divisions by the width).  2312 tokens x 2560, us
-// (before): coefficients 41 (50), chain 57 (145), products 17 (23).  All three in one kernel, with seven warps of a block feeding the
-// chain, took 422: too few warps for the exponentials' latency.
+// over tokens (no divisions by the width).  2312 tokens x 2560: 92 us back to back (162 with a chain that loads into registers); 200
+// tokens beside 64 single ones 21 (31).  All three in one kernel, with seven warps of a block feeding the chain, took 422: too few
+// warps for the exponentials' latency.
 template <typename E>
 __global__ void __launch_bounds__(256) rglru_ab_kernel(RglruArgs a, float* gates) {
   pdl_launch_dependents();
@@ -194,9 +194,11 @@ __global__ void __launch_bounds__(256) rglru_ab_kernel(RglruArgs a, float* gates
   }
 }
 
-// One warp per 32 channels of a request: the coefficients of 64 tokens at a time arrive by cp.async, three stages ahead, so that the
-// chain waits for its fma's and not for memory (with eight tokens' loads in flight it took 145 us).  N: numbers per copy, four
-// where the rows are aligned for it, one elsewhere (widths that are no multiple of four).
+// One warp per 32 channels of a request: the coefficients of TOK tokens at a time arrive by cp.async, two stages ahead, so that the
+// chain waits for its fma's and not for memory.  What bounds steps with many requests is how many of these one-warp blocks fit at
+// once: stages of 16 tokens (12 KB a block) and four of 64 (64 KB) take 92 and 101 us for 2 x 1160 tokens, 28 and 64 for 60 and 200 single
+// ones, us of the whole recurrence at width 2560; stages of 8, where requests bring less than 8 tokens on average, 26.
+// N: numbers per copy, four where the rows are aligned for it, one elsewhere (widths that are no multiple of four).
 constexpr int RS_STAGES = 3;
 template <typename E, int N, int TOK>
 __global__ void __launch_bounds__(32) rglru_chain_kernel(RglruArgs a, float* gates) {
