@@ -1,5 +1,5 @@
 #!/usr/bin/env python
-"""Headline benchmark: output tokens/s at fixed concurrency (BASELINE.json `metric`).
+"""Headline benchmark: output tokens/s at fixed concurrency of a named model and load.
 
   python bench.py --gpus N --steps K --warmup W [--workload c3|c2|c1] [--impl ours|reference]
   python bench.py --designs [safupel|girolorn|zezilix|balenex|kogonex|nosolix]   (a layer-list design beside the closest other model of equal size; one JSON line per size)
@@ -12,7 +12,7 @@ per engine step as the continuous-batching scheduler cuts them) and decoded gree
   e2e    the same job through the public API (LLM.generate -> C++ continuous-batching scheduler):
          host token lists in, host token lists out; every engine step copies its metadata from pinned
          host memory and reads the sampled ids back, both inside the timed region.
-At N > 1 every rank is an independent replica (request-level data parallelism, BASELINE config 5:
+At N > 1 every rank is an independent replica (request-level data parallelism:
 no data-path collective), timing is barrier-bracketed and the max over ranks; scaling is weak.
 """
 import argparse
@@ -32,14 +32,14 @@ WORKLOADS = {
     "c3": ("llama-3.1-8b", 64, 2048, 256, 4),
     "c2": ("llama-3.2-1b", 32, 128, 128, 32),
     "c1": ("opt-125m", 1, 128, 128, 1),
-    # tensor parallel over all --gpus ranks (BASELINE config 4): one model, NCCL all-reduce, strong scaling
+    # tensor parallel over all --gpus ranks: one model, NCCL all-reduce, strong scaling
     "c4": ("llama-3.1-70b", 64, 2048, 256, 4),
 }
 CPU_SAMPLE = {"c3": (4, 128, 8), "c2": (8, 128, 16), "c1": (1, 128, 128), "c4": (1, 64, 2)}   # (requests, in, out)
 
 
 def model_cfg(name):
-    """HF config.json of the named model (published hyper-parameters, SURVEY.md Appendix B)."""
+    """HF config.json of the named model (published hyper-parameters)."""
     l3 = lambda f: {"factor": f, "low_freq_factor": 1.0, "high_freq_factor": 4.0,
                     "original_max_position_embeddings": 8192, "rope_type": "llama3"}
     if name == "opt-125m":
@@ -264,12 +264,12 @@ def connect_tp(kge, llm, how, rank):
         llm.tp_connect_torch()
 
 
-# decode-only HBM ceilings of Llama-3.1-70B on the C3 load, output tok/s (BASELINE.md section 3)
+# decode-only HBM ceilings of Llama-3.1-70B on the C3 load, output tok/s
 C4_DECODE_CEILING = {2: 4540.0, 4: 9080.0, 8: 18160.0}
 
 
 def tp_subrecord(kge, args, world, rank, local, mx, barrier):
-    """BASELINE config 4 on the same ranks: ONE Llama-3.1-70B engine sharded over all `world` GPUs (tensor parallel,
+    """Tensor parallel on the same ranks: ONE Llama-3.1-70B engine sharded over all `world` GPUs (tensor parallel,
     strong scaling), same 64 x 2048-in/256-out load, device-resident replay like the headline `value`, plus one job
     through the public API and the per-category device times of an instrumented job."""
     import tempfile
@@ -424,7 +424,7 @@ def run_ours(args):
         {"requests": B, "first_divergences": 0, "not_near_tie": 0, "recorded_job_equal_to_timed_job": toks_rec == toks_e2e}
     log(f"legs: {same}/{B * pout} tokens equal; {divergence}")
 
-    # ---- latency (extra job through the public API; BASELINE.json's metric also names p50 TTFT and ITL)
+    # ---- latency (extra job through the public API: p50 TTFT and ITL)
     try:
         latency = latency_probe(llm, prompts, sp)
     except Exception as ex:      # never let the side measurement take the bench line down
@@ -482,7 +482,7 @@ def run_ours(args):
     }
     llm.close()
     if world > 1 and tp == 1 and not args.no_tp:
-        # BASELINE config 4 on the same ranks.  Guarded: whatever happens in this leg, the headline line is printed -
+        # Tensor parallel on the same ranks.  Guarded: whatever happens in this leg, the headline line is printed -
         # a watchdog prints it without the sub-record and ends the process if the leg does not finish in time.
         import threading
 

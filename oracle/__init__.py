@@ -1,7 +1,7 @@
 """CPU oracle for the serving-engine hot path.  TEST INFRASTRUCTURE ONLY.
 
-PARITY UNPINNED: the reference (/root/reference) holds no tests, golden vectors or
-compute code for this path (SURVEY.md section 8c).  The arithmetic lives in a third-party
+PARITY UNPINNED: the reference holds no tests, golden vectors or
+compute code for this path.  The arithmetic lives in a third-party
 dependency, vLLM, pinned by container tag v0.8.5 / v0.8.4
 (ref:values-01-minimal-example.yaml:5-6, ref:values-01-minimal-example2.yaml:6-7).
 This package restates vLLM's published op order and cast points in plain PyTorch on

@@ -86,7 +86,7 @@ def _llama3_scaling(factor: float) -> dict:
             "original_max_position_embeddings": 8192, "rope_type": "llama3"}
 
 
-# Published hyper-parameters (SURVEY.md Appendix B); the reference holds none of these.
+# Published hyper-parameters; the reference holds none of these.
 CONFIGS: dict[str, ModelConfig] = {
     "opt-125m": ModelConfig("opt", 50272, 768, 12, 12, 12, 64, 3072, 2048, 1e-5, True,
                             bos=2, eos=2, name="facebook/opt-125m"),
@@ -148,7 +148,7 @@ def make_weights(cfg: ModelConfig, seed: int = 0, dtype=torch.bfloat16,
                  std: float = 0.02) -> dict[str, torch.Tensor]:
     """Seeded HF-named weights.  Matrices N(0, std); norm weights 1 + N(0, 0.1);
     biases N(0, std).  (vLLM's dummy init U(+-1e-3) gives flat logits and meaningless
-    argmax parity - SURVEY.md section 7 'hard parts' - so it is not used.)
+    argmax parity - so it is not used.)
     One CPU generator, fixed order, so the same (cfg, seed) gives the same bytes on
     every machine with the same torch."""
     g = torch.Generator().manual_seed(seed)
@@ -291,7 +291,7 @@ def save_model_dir(path: str, cfg: ModelConfig, weights: dict[str, torch.Tensor]
 
 
 def make_prompts(cfg: ModelConfig, n: int, length: int, seed: int = 0) -> list[list[int]]:
-    """Token-id prompts ~ U[lo, hi) (no tokenizer offline; SURVEY.md section 8d)."""
+    """Token-id prompts ~ U[lo, hi) (no tokenizer offline)."""
     g = torch.Generator().manual_seed(seed)
     lo = 1000 if cfg.vocab_size > 4000 else 3
     hi = cfg.vocab_size - 1000 if cfg.vocab_size > 4000 else cfg.vocab_size

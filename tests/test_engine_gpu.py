@@ -1,7 +1,7 @@
 """End-to-end parity of the engine (C++ scheduler + paged KV + sm_100a kernels, through the C ABI)
 against the CPU oracle on identical seeded safetensors and token-id prompts.
 
-Bar (BASELINE.json north_star): greedy ids bit-exact for the first N tokens while the oracle's own
+Bar: greedy ids bit-exact for the first N tokens while the oracle's own
 top-1/top-2 margin exceeds bf16 noise; logits within bf16 tolerance (max-abs stated per test).
 A mismatch is only accepted at a step where the oracle's top-2 margin is below `MARGIN` (two fp32
 GEMM summation orders legitimately round differently there); after such a step the sequences
@@ -130,7 +130,7 @@ def test_real_width_models_logits_and_ids(kge, model_dirs, name):
     assert near <= 2, (equal, near)
 
 
-# ----------------------------------------------------------------- BASELINE.json configurations at full size
+# ----------------------------------------------------------------- the benchmark's configurations at full size
 # Row n1 of the scope table: parity on the models the bench is quoted on, not on toy shapes.
 #   C1  facebook/opt-125m, all 12 layers, 1 x 128-in/128-out    (ref:values-01-minimal-example.yaml:7)
 #   C2  Llama-3.2-1B, all 16 layers, 4 x 128-in/32-out

@@ -675,7 +675,7 @@ def test_decode_attention_persistent(kge, L, H, KV, hd, bs, seq_lens, splits):
 
 @pytest.mark.parametrize("H,KV,hd,bs,q_lens,seq_lens", [c for c in ATTN_CASES if max(c[4]) > 1][:5] + [ATTN_LONG_CASES[2][:3] + (16,) + ATTN_LONG_CASES[2][3:5]])
 def test_prefill_attention_tma_and_cp_async_agree(kge, L, H, KV, hd, bs, q_lens, seq_lens):
-    """The tcgen05 prefill kernel with TMA-staged K/V (default) and with the round-1 cp.async gathers computes the same
+    """The tcgen05 prefill kernel with TMA-staged K/V (default) and with cp.async gathers computes the same
     tiles in the same order: same bits."""
     seed = H * 13 + sum(seq_lens)
     try:

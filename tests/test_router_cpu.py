@@ -1,4 +1,4 @@
-"""kge-router (the request router in front of engine replicas, BASELINE config 5) against fake engine backends:
+"""kge-router (the request router in front of engine replicas) against fake engine backends:
 round-robin, session stickiness, model filtering, failover when a backend dies, verbatim relay of SSE streams,
 /v1/models aggregation, /health and /metrics.  CPU only."""
 import http.server

@@ -1,6 +1,6 @@
 """The `vllm serve` command line of the reference's values files, parsed by the drop-in binary
 (kge-serve --dry-run needs no GPU).  Flag sets are the ones the chart would pass for each values
-file (SURVEY.md Appendix A): vllmConfig keys become flags, extraArgs are appended verbatim."""
+file: vllmConfig keys become flags, extraArgs are appended verbatim."""
 import json
 import os
 import subprocess

@@ -517,7 +517,7 @@ def test_concurrent_clients_under_thread_sanitizer(mock_lib, tmp_path):
 
 
 def test_replicas_behind_the_router(mock_lib, tmp_path):
-    """BASELINE config 5 in miniature, without GPUs: two server processes (mock engines) behind kge-router - requests
+    """Replicas in miniature, without GPUs: two server processes (mock engines) behind kge-router - requests
     alternate between the replicas, SSE passes through, /v1/models is merged."""
     router = os.path.join(PKG, "bin", "kge-router")
     if not os.path.exists(router):

@@ -1,6 +1,6 @@
 """Third opinion: tokens and log-probabilities recorded from the installed vLLM (0.22.0) running its OWN CUDA
 kernels on a B200 (FlashInfer/TRTLLM attention, cuBLAS GEMMs) on the oracle's seeded tiny models
-(tests/golden/vllm_cuda.json, made by tests/golden/make_vllm_cuda_golden.py under gpurun).  Not the pinned
+(tests/golden/vllm_cuda.json, made by tests/golden/make_vllm_cuda_golden.py).  Not the pinned
 v0.8.x and not vLLM's CPU backend, but it is the dependency the reference deploys running the same graph.
 
   CPU:  the oracle, teacher-forced on vLLM's tokens, gives the same top-1 token at every step (unless vLLM's own
