@@ -99,7 +99,9 @@ __global__ void __launch_bounds__(128) rglru_conv_vec_kernel(RglruArgs a) {
 int rglru_conv(const RglruArgs& a, cudaStream_t st) {
   if (a.T <= 0) return 0;
   KGE_REQUIRE(a.taps >= 1 && a.taps <= MAX_TAPS, "rglru_conv: %d taps (1..%d)", a.taps, MAX_TAPS);
-  if (a.elt == KGE_ELT_BF16 && a.width % 8 == 0 && ((reinterpret_cast<uintptr_t>(a.yx) | reinterpret_cast<uintptr_t>(a.u) | reinterpret_cast<uintptr_t>(a.conv_b)) & 15) == 0) {
+  // few rows of few channels leave its threads a chain of loads each where the other kernel has a thread for every channel (64 rows of
+  // 64 channels 5.1 us here and 2.6 there, of 264 5.6 and 3.6; 64 of 1024 6.3 and 6.1, 256 of 1024 6.4 and 7.0, 2312 of 64 4.3 and 4.7)
+  if (a.elt == KGE_ELT_BF16 && (a.width >= 1024 || a.T > 1024) && a.width % 8 == 0 && ((reinterpret_cast<uintptr_t>(a.yx) | reinterpret_cast<uintptr_t>(a.u) | reinterpret_cast<uintptr_t>(a.conv_b)) & 15) == 0) {
     KGE_CUDA_OK(launch_pdl(rglru_conv_vec_kernel, dim3((a.T + RC_TOK - 1) / RC_TOK, (a.width / 8 + 127) / 128), dim3(128), 0, st, a));
     return 0;
   }

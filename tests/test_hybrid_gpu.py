@@ -94,6 +94,18 @@ def test_narrow_projections_of_long_steps(kge, tmp_path, rows):
     llm.close()
 
 
+@pytest.mark.parametrize("width,taps,pieces", [(1032, 4, [1, 2, 3, 4, 5, 60]), (1024, 2, [75]), (2048, 7, [33, 1, 41]), (72, 4, [1030, 1, 9]), (72, 4, [1024, 16])])
+def test_convolution_in_pieces_of_eight_channels(kge, tmp_path, width, taps, pieces):
+    """bfloat16 rows by eight channels of four tokens: widths with a last block of one thread, of all, of two blocks, tails carried over
+    pieces shorter than the taps; narrow rows with enough tokens for it, and one token too few."""
+    cfg = oh.make_config(layers=("rglru",), mlps=(None,), r_width=width, r_blocks=8, r_conv=taps)
+    W = oh.make_weights(cfg, seed=31)
+    toks = prompt(cfg, sum(pieces))
+    llm = make_engine(kge, tmp_path, cfg, W, "bfloat16", tokens=max(sum(pieces), 512) + 16)
+    check(run_pieces(llm, 0, toks, pieces), oh.forward(cfg, W, toks), "bfloat16", f"pieces {pieces}")
+    llm.close()
+
+
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 @pytest.mark.parametrize("width", [33, 36, 66, 128])
 def test_gated_recurrence_by_width(kge, tmp_path, width, dtype):
