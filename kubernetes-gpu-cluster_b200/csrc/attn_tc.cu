@@ -14,11 +14,14 @@
 // mbarriers; tcgen05.commit tells it when a stage is free.  The softmax warps issue no loads.
 // TMA = false (knob "attn_tma" 0, block sizes below 8): tiles gathered by the softmax threads with
 // 16-byte cp.async (K two tiles ahead, V one; block-table lookup once per row) and published with fence.proxy.async.
+// Which kernel takes what: attn_pair.cuh has the plain prompts (see launch_tc); this one short contexts in small launches, soft caps,
+// windows with prefix keys and block sizes below 8.
 // Tensor-bound: 4 * hd * sum_b q_b (ctx0_b + (q_b+1)/2) flop per q head.
 #include <cuda.h>
 #include <string.h>
 
 #include "common.cuh"
+#include "f32x2.cuh"
 #include "kge.h"
 
 namespace kge {
@@ -514,9 +517,11 @@ static dim3 tc_grid(int B, int T, int max_q_len, int TT, int KV, int& by_request
   return by_request ? dim3(tiles, KV, B) : dim3(KV, B, tiles);
 }
 
+#include "attn_pair.cuh"
+
 template <int HD>
 static int launch_tc(bf16* out, const bf16* q, int q_stride, const bf16* kc, const bf16* vc, const int32_t* bt,
-                     int max_blocks, const int32_t* sl, const int32_t* qsl, int B, int T, int max_q_len, int H, int KV, int bs,
+                     int max_blocks, const int32_t* sl, const int32_t* qsl, int B, int T, int max_q_len, int max_seq_len, int H, int KV, int bs,
                      float scale, float softcap, const float* sinks, cudaStream_t st) {
   const bool cap = softcap > 0.f;
   const float cap_in2 = cap ? 2.f * atc::kLog2e * scale / softcap : 0.f, cap_log2 = softcap * atc::kLog2e;
@@ -528,6 +533,11 @@ static int launch_tc(bf16* out, const bf16* q, int q_stride, const bf16* kc, con
   const dim3 grid = tc_grid(B, T, max_q_len, TT, KV, by_request);
   CUtensorMap tk, tv;
   const bool tma = tunable(TUN_ATTN_TMA) != 0 && bs >= 8;
+  // Two query tiles per CTA (attn_pair.cuh) but for launches of short contexts that do not fill the chip: there its 384 threads, all of
+  // TMEM and 226 KB start later than two of these CTAs per SM (us here / there: 8 x 128 tokens 10.3 / 11.4, 2 x 300 10.3 / 11.5, 64 tokens
+  // 5.6 / 7.0; but 8 x 300 26.5 / 23.3, one of 512 14.2 / 11.3; 32 / 8 heads of 128).
+  if (bs >= 8 && !cap && B <= 65535 && !(max_seq_len <= 320 && (int64_t)T * KV <= 256 * TT))
+    return launch_pair<HD>(out, q, q_stride, kc, vc, bt, max_blocks, sl, qsl, B, T, max_q_len, max_seq_len, H, KV, bs, bs_shift, scale, sinks, st);
   if (tma) {
     const int box_rows = bs < atc::BNK ? bs : atc::BNK;
     const int64_t rows = (int64_t)1 << 30;      // the pool's extent is not known here; it only bounds out-of-range handling, never relied on
@@ -598,11 +608,11 @@ int paged_attn_window_tc(void* out, const void* q, int q_stride, const void* kc,
 
 // Called by kge_paged_attn (attn.cu) for batches with query chunks longer than one token.
 int paged_attn_prefill_tc(bf16* out, const bf16* q, int q_stride, const bf16* kc, const bf16* vc, const int32_t* bt,
-                          int max_blocks, const int32_t* sl, const int32_t* qsl, int B, int T, int max_q_len, int H, int KV,
+                          int max_blocks, const int32_t* sl, const int32_t* qsl, int B, int T, int max_q_len, int max_seq_len, int H, int KV,
                           int hd, int bs, float scale, float softcap, const float* sinks, cudaStream_t st) {
   KGE_REQUIRE(H / KV <= 128, "kge_paged_attn: GQA group %d > 128 unsupported", H / KV);
-  if (hd == 128) return launch_tc<128>(out, q, q_stride, kc, vc, bt, max_blocks, sl, qsl, B, T, max_q_len, H, KV, bs, scale, softcap, sinks, st);
-  return launch_tc<64>(out, q, q_stride, kc, vc, bt, max_blocks, sl, qsl, B, T, max_q_len, H, KV, bs, scale, softcap, sinks, st);
+  if (hd == 128) return launch_tc<128>(out, q, q_stride, kc, vc, bt, max_blocks, sl, qsl, B, T, max_q_len, max_seq_len, H, KV, bs, scale, softcap, sinks, st);
+  return launch_tc<64>(out, q, q_stride, kc, vc, bt, max_blocks, sl, qsl, B, T, max_q_len, max_seq_len, H, KV, bs, scale, softcap, sinks, st);
 }
 
 }  // namespace KGE_ELT_NS

@@ -1111,6 +1111,26 @@ int make_tmap(CUtensorMap* m, const void* ptr, int64_t rows, int64_t cols, int b
   return 0;
 }
 
+// Queries of a packed projection, [tokens][heads][hd] with tokens `stride` numbers apart: boxes of 64 columns x box_heads x
+// box_tokens, 128B swizzle.  The number of tokens is not known to the callers: a box must lie within the rows they may read.
+int encode_tmap_q(CUtensorMap* m, const void* ptr, int64_t stride, int hd, int heads, int box_heads, int box_tokens) {
+  EncodeTiledFn enc = get_encode_fn();
+  KGE_REQUIRE(enc, "cuTensorMapEncodeTiled unavailable (no CUDA driver?)");
+  cuuint64_t dims[3] = {(cuuint64_t)hd, (cuuint64_t)heads, (cuuint64_t)1 << 30};
+  cuuint64_t strides[2] = {(cuuint64_t)hd * 2, (cuuint64_t)stride * 2};
+  cuuint32_t box[3] = {64, (cuuint32_t)box_heads, (cuuint32_t)box_tokens};
+  cuuint32_t estr[3] = {1, 1, 1};
+#ifdef KGE_HALF
+  const CUtensorMapDataType dt = CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
+#else
+  const CUtensorMapDataType dt = CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
+#endif
+  CUresult r = enc(m, dt, 3, const_cast<void*>(ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                   CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  KGE_REQUIRE(r == CUDA_SUCCESS, "cuTensorMapEncodeTiled failed (%d) stride=%lld heads=%d", (int)r, (long long)stride, heads);
+  return 0;
+}
+
 constexpr int kGemmSmemBudget = 224 * 1024;
 
 template <int TOKN, bool SPLIT, bool GATED, bool PAIR = false, bool WS = false>

@@ -1,0 +1,209 @@
+"""The barrier protocol of the prompt attention kernel with two query tiles per CTA (csrc/attn_pair.cuh), explored on the CPU over
+every order in which its roles can run: no wait may be left behind by its barrier (a parity wait that is sampled a phase late never
+ends), none may pass early, and no buffer may be overwritten before its readers are done."""
+import os
+import re
+
+import pytest
+
+SRC = os.path.join(os.path.dirname(__file__), "..", "kubernetes-gpu-cluster_b200", "csrc", "attn_pair.cuh")
+
+# every barrier operation of the kernel after the barriers' set-up, in the order of the source: what the programs below transcribe
+OPS = [
+    # producer
+    "arrive gathered", "wait item_empty(slot), ((ni >> 1) - 1) & 1", "arrive item_full(slot)",
+    "wait is_k ? k_empty(st) : v_empty(st), (nk / NST - 1) & 1",
+    "wait q_empty, (ni - 1) & 1", "wait clc_full, nclc & 1", "wait item_empty(slot), ((ni >> 1) - 1) & 1", "arrive item_full(slot)",
+    # issuers
+    "wait item_full(ni & 1), (ni >> 1) & 1", "arrive item_empty(ni & 1)", "wait q_full, ni & 1",
+    "wait k_full(st), ((nk + js) / NST) & 1", "wait s_read(a), (ns - 1) & 1", "commit s_full(a)", "commit k_empty(st)", "commit q_empty",
+    "wait v_full(st), ((nk + j) / NST) & 1", "wait p_full(a, np), (np >> 1) & 1", "commit o_full(a, np)", "commit v_empty(st)",
+    # softmax warps
+    "wait item_full(ni & 1), (ni >> 1) & 1", "arrive item_empty(ni & 1)", "wait s_full(a), ns & 1", "arrive s_read(a)",
+    "wait o_full(a, ns - 1), ((ns - 1) >> 1) & 1", "wait o_full(a, ns), ((ns - 2) >> 1) & 1", "arrive p_full(a, ns)",
+    "wait o_full(a, ns - 1), ((ns - 1) >> 1) & 1",
+]
+
+
+def barrier_ops():
+    src = open(SRC).read()
+    body = src[src.index("if (warp == 10) {\n"):src.index("}  // namespace atc2")]
+    body = re.sub(r"//[^\n]*", "", body)
+    out = []
+    for m in re.finditer(r"\b(mbar_wait|mbar_arrive|tc_commit)\(", body):
+        depth, i = 1, m.end()
+        while depth:
+            depth += {"(": 1, ")": -1}.get(body[i], 0)
+            i += 1
+        out.append(m.group(1).replace("mbar_", "").replace("tc_", "") + " " + body[m.end():i - 1])
+    return out
+
+
+def test_transcription_matches_the_kernel():
+    assert barrier_ops() == OPS
+
+
+def programs(items, nst):
+    """Instruction lists of the roles.  items: (key tiles of the first query tile, of the second[, whether they share the key tiles of one
+    query tile between them]).  BAR: a barrier of the two groups of softmax threads.  An MMA is ("mma", barriers that it
+    commits to, buffers it reads, buffers it writes); a copy ("load", barrier, buffer)."""
+    def wait(bar, k, optional=False):
+        return ("maybe" if optional else "wait", bar, k)
+    prod, nk, end = [], 0, len(items)
+    items = [(*i, 0)[:3] for i in items]
+    tiles = [i[0] + i[1] if i[2] else max(i) for i in items]
+    for ni in range(end + 1):
+        if ni >= 2:
+            prod.append(wait(("item_empty", ni & 1), (ni >> 1) - 1))
+        prod.append(("arrive", ("item_full", ni & 1)))
+        if ni == end:
+            break
+        if ni:
+            prod.append(wait(("q_empty",), ni - 1))
+        prod.append(("load", ("q_full",), ("q",)))
+        for _ in range(tiles[ni]):
+            for x in "kv":
+                if nk >= nst:
+                    prod.append(wait((x + "_empty", nk % nst), nk // nst - 1))
+                prod.append(("load", (x + "_full", nk % nst), (x, nk % nst)))
+            nk += 1
+    roles = [prod]
+    for a in range(2):
+        issue, ns, np, nk = [], 0, 0, 0
+        for ni, nn in enumerate(items):
+            n, ahead = tiles[ni], 1 + nn[2]
+            issue += [wait(("item_full", ni & 1), ni >> 1), ("arrive", ("item_empty", ni & 1)), wait(("q_full",), ni)]
+            for j in range(-ahead, n):
+                js = j + ahead
+                if js < n:
+                    st = (nk + js) % nst
+                    issue.append(wait(("k_full", st), (nk + js) // nst))
+                    if js % 2 == a if nn[2] else js < nn[a]:
+                        if ns:
+                            issue.append(wait(("s_read", a), ns - 1))
+                        issue.append(("mma", [("s_full", a)], [("q",), ("k", st)], [("s", a)]))
+                        ns += 1
+                    issue.append(("mma", [("k_empty", st)] + ([("q_empty",)] if js + 1 == n else []), [], []))
+                if j >= 0:
+                    st = (nk + j) % nst
+                    issue.append(wait(("v_full", st), (nk + j) // nst))
+                    if j % 2 == a if nn[2] else j < nn[a]:
+                        issue += [wait(("p_full", a, np & 1), np >> 1),
+                                  ("mma", [("o_full", a, np & 1)], [("p", a, np & 1), ("v", st)], [("o", a)])]
+                        np += 1
+                    issue.append(("mma", [("v_empty", st)], [], []))
+            nk += n
+        issue.append(wait(("item_full", end & 1), end >> 1))
+        roles.append(issue)
+    for a in range(2):
+        s, ns, nb, nt = [], 0, 0, 0
+        for ni, nn in enumerate(items):
+            s += [wait(("item_full", ni & 1), ni >> 1), ("arrive", ("item_empty", ni & 1))]
+            turns = nn[1] >= 3
+            for j in range(nn[a]):
+                s += [wait(("s_full", a), ns), ("read", ("s", a)), ("arrive", ("s_read", a))]
+                if j:
+                    s += [wait(("o_full", a, (ns - 1) & 1), (ns - 1) >> 1, True)]        # only where a row's maximum has grown
+                if ns >= 2:
+                    s.append(wait(("o_full", a, ns & 1), (ns - 2) >> 1))
+                if turns and j == 0:
+                    s += [("arrive", ("bar1",))] + ([wait(("bar1",), nt)] if a else [])
+                    nt += 1
+                s += [("write", ("p", a, ns & 1)), ("arrive", ("p_full", a, ns & 1))]
+                ns += 1
+            if nn[a]:
+                s += [wait(("o_full", a, (ns - 1) & 1), (ns - 1) >> 1), ("read", ("o", a))]
+            if nn[2]:
+                s += [("arrive", ("bar2",)), wait(("bar2",), nb)] + ([] if a else [("read", ("o", 1))]) + [("arrive", ("bar3",)), wait(("bar3",), nb)]
+                nb += 1
+        s.append(wait(("item_full", end & 1), end >> 1))
+        roles.append(s)
+    return roles
+
+
+def explore(items, nst, only=None, drop=None):
+    """True if some order leaves a role waiting for ever, or lets a buffer be written while an MMA in flight uses it.  An issuer's MMAs
+    complete in the order of issue, copies in any.  only: the query tile whose roles are run (the other's arrivals are taken out), which
+    keeps the number of states small; drop: a wait that is left out."""
+    roles = programs(items, nst)
+    need = {"item_empty": 4, "k_empty": 2, "v_empty": 2, "q_empty": 2, "bar1": 2, "bar2": 2, "bar3": 2}
+    if only is not None:
+        roles = [roles[0], roles[1 + only], roles[3 + only]]
+        need = {"item_empty": 2}
+        roles = [[op for op in r if op[0] == "mma" or op[1][0][:3] != "bar"] for r in roles]
+    if drop:
+        roles = [[op for op in r if not (op[0] == "wait" and op[1][0] == drop)] for r in roles]
+    bars = sorted({b for r in roles for op in r for b in (op[1] if op[0] == "mma" else [op[1]] if op[0] in ("wait", "maybe", "arrive", "load") else [])}, key=str)
+    index = {b: i for i, b in enumerate(bars)}
+    mmas = [[op for op in r if op[0] == "mma"] for r in roles]
+    before = [[sum(op[0] == "mma" for op in r[:i]) for i in range(len(r) + 1)] for r in roles]
+
+    def arrive(state, bar):
+        done, got = state[index[bar]]
+        got += 1
+        if got == need.get(bar[0], 1):
+            done, got = done + 1, 0
+        return state[:index[bar]] + ((done, got),) + state[index[bar] + 1:]
+
+    start = ((0,) * len(roles), ((0, 0),) * len(bars), (0,) * len(roles), ())            # positions, barriers, MMAs done, copies in flight
+    seen, todo = {start}, [start]
+    while todo:
+        pcs, state, done_mma, loads = todo.pop()
+        flight = [f for m, d, b, pc in zip(mmas, done_mma, before, pcs) for f in m[d:b[pc]]]
+        succ = []
+        for r, prog in enumerate(roles):
+            if pcs[r] == len(prog):
+                continue
+            op = prog[pcs[r]]
+            nxt = pcs[:r] + (pcs[r] + 1,) + pcs[r + 1:]
+            if op[0] in ("wait", "maybe"):
+                if op[0] == "maybe":
+                    succ.append((nxt, state, done_mma, loads))
+                done = state[index[op[1]]][0]
+                if (done & 1) != (op[2] & 1):                    # mbarrier.try_wait.parity
+                    if done != op[2] + 1:
+                        return True
+                    succ.append((nxt, state, done_mma, loads))
+            elif op[0] == "arrive":
+                succ.append((nxt, arrive(state, op[1]), done_mma, loads))
+            elif op[0] == "load":
+                if any(op[2] in f[2] for f in flight):           # a copy into what an MMA reads
+                    return True
+                succ.append((nxt, state, done_mma, tuple(sorted(loads + (op[1],), key=str))))
+            else:
+                # threads: what an MMA in flight writes may not be read, what it reads may not be written
+                if op[0] == "read" and any(op[1] in f[3] for f in flight) or op[0] == "write" and any(op[1] in f[2] for f in flight):
+                    return True
+                succ.append((nxt, state, done_mma, loads))
+        for r, m in enumerate(mmas):
+            if done_mma[r] < before[r][pcs[r]]:
+                s = state
+                for b in m[done_mma[r]][1]:
+                    s = arrive(s, b)
+                succ.append((pcs, s, done_mma[:r] + (done_mma[r] + 1,) + done_mma[r + 1:], loads))
+        for i, b in enumerate(loads):
+            succ.append((pcs, arrive(state, b), done_mma, loads[:i] + loads[i + 1:]))
+        if not succ and any(pcs[r] < len(prog) for r, prog in enumerate(roles)):
+            return True
+        for s in succ:
+            if s not in seen:
+                seen.add(s)
+                todo.append(s)
+    return False
+
+
+@pytest.mark.parametrize("items", [[(1, 0)], [(1, 1)], [(1, 2)], [(1, 0), (1, 1)], [(1, 1, 1), (1, 0)], [(2, 1, 1)], [(3, 3)]], ids=str)
+def test_every_wait_ends_in_every_order(items):
+    assert not explore(items, 2)
+
+
+@pytest.mark.parametrize("nst", [2, 4])
+@pytest.mark.parametrize("items", [[(5, 6)], [(2, 3), (1, 0), (3, 3)], [(1, 1)] * 4, [(4, 5), (2, 0)], [(3, 2, 1), (2, 2)], [(1, 1, 1)] * 3, [(3, 3, 1), (1, 2)]], ids=str)
+@pytest.mark.parametrize("only", [0, 1])
+def test_every_wait_of_one_query_tile_ends_in_every_order(items, nst, only):
+    assert not explore(items, nst, only)
+
+
+@pytest.mark.parametrize("drop", ["o_full", "p_full", "s_read", "k_empty", "q_empty"])
+def test_the_exploration_finds_a_missing_wait(drop):
+    assert explore([(3, 3), (2, 1)], 2, 0, drop)
