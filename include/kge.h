@@ -46,12 +46,10 @@ int kge_device_sm_count(void);
  *                             SM reconfigure (and drain) between them; 0 = small kernels keep the driver's default split
  *   "gemm_l2_hints" 0/1       1 = the GEMM's TMA loads carry L2 eviction hints (weights evict_first, activations evict_last);
  *                             measured slower on the prefill step (weight tiles are re-read by other CTA pairs), so off
- *   "gemm_wide" 1/0           GEMMs of up to 64 tokens: 1 = where it keeps as many CTAs streaming as the 128-row plan, tiles of
- *                             256 weight rows with the tokens as the MMA's M side and the weights as its N side (twice the
- *                             weight bytes per MMA), and up to 16 tokens, by size, weights streamed without staging tiles
- *                             (csrc/gemm_rows.cuh); 0 = always 128-row tiles with the tokens as N.  64 tokens, us with 1 and 0:
- *                             6144 x 4096 13.7 and 13.8, gated 28672 x 4096 45.0 and 41.1 (it was 44.5 and 48.6 before MMAs
- *                             were issued behind elect.sync)
+ *   "gemm_wide" 1/0           GEMMs of up to 64 tokens: 1 = from 33 tokens on, where the 128-row plan splits K in two, tiles of 256
+ *                             weight rows with the tokens as the MMA's M side (64 tokens, us with 1 and 0: 6144 x 4096 13.6 and
+ *                             13.8, 8192 x 8192 26.1 and 27.3), and up to 16 tokens, by size, weights streamed without staging
+ *                             tiles (csrc/gemm_rows.cuh); 0 = always 128-row tiles with the tokens as N
  *   "attn_persistent" 1/0     decode attention with 64-token KV blocks or larger: 1 = 2 x 148 resident CTAs each take an equal,
  *                             contiguous share of all key tiles of the launch (a (request, kv head) group is cut where shares
  *                             end; pieces merged by the last CTA of the group to arrive) - one round whatever the batch and

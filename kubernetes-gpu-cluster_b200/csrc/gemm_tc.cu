@@ -6,9 +6,9 @@
 // once.  D[weight row, token] lives in TMEM (fp32); the epilogue reads it back with tcgen05.ld as
 // MMA fragments, adds the bias of their rows, applies the activation, rounds once to 16 bits, and
 // stmatrix turns the fragments so that a lane stores 16 bytes of an output row.
-// Which kernel: up to 16 tokens, by size, gemm_rows.cuh (weights streamed without staging tiles); up
-// to 64, where it keeps as many CTAs streaming, gemm_wide_kernel; above 64 CTA pairs with a token
-// tile of 32 to 256 (plan_pairs); single-CTA tiles elsewhere.
+// Which kernel: up to 16 tokens, by size, gemm_rows.cuh (weights streamed without staging tiles); 33
+// to 64 tokens where 128-row tiles would be split in two, gemm_wide_kernel; above 64 CTA pairs with a
+// token tile of 32 to 256 (plan_pairs); single-CTA tiles elsewhere.
 //
 // Persistent, warp-specialised: warp 0 = TMA producer (cp.async.bulk.tensor, 128B swizzle),
 // warp 1 = tcgen05.mma issuer (one elected lane), warp 2 = TMEM allocator, warps 4-7 = epilogue.
@@ -131,7 +131,6 @@ struct GemmParams {
   int T, N, K, act;
   int l2_hints;              // 1: weights evict_first, activations evict_last, output stored streaming
   int m_tiles, n_tiles, splits, kb_total, kb_per_split;
-  int rows;                  // gemm_wide_kernel: outputs per tile
   int tokn = 0;              // PAIR: tokens per tile, a multiple of 32 up to 256
   unsigned long long* trace; // phase timestamps, 16 per CTA (tools/gemm_trace.py); null outside that tool
   int glu = 0;               // gated pair: 0 silu(gate) * up; 1 clamped: g = min(gate, limit), u = clamp(up, +-limit), g * sigmoid(alpha g) * (u + 1)
@@ -792,37 +791,26 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant
   }
 }
 
-// ------------------------------------------------------------------------------ wide tiles for T <= 64
-// With 128 weight rows as M and the tokens as N, a decode-sized GEMM issues four MMAs for every 16 KB of weights.  Here the
-// roles are swapped and the tile is wider: the tokens are the M side (64 rows loaded; the MMA is 128 tall and its upper
-// half reads whatever follows the token tile in shared memory - rows that are never read back), 256 weight rows are N of
-// ONE MMA, so the same four MMAs move 32 KB of weights.  That paid when an MMA took 88 cycles and more to issue whatever
-// its shape; behind elect_one() a 128 x 64 x 16 one runs in 48, and the 128-row tiles are level or ahead, back to back on
-// cold weights, us at 64 tokens here and there: 6144 x 4096 13.7 and 13.8 (32 tokens 13.5 and 12.3), gated 16384 x 2048 16.6
-// and 13.9, gated 28672 x 4096 45.0 and 41.1.  D is [token][weight row] in TMEM: a thread owns a token and 256 consecutive outputs,
-// which it stores 16 bytes at a time; the fused SwiGLU epilogue finds gate (columns 0-127) and up (128-255) of an
-// output in the same thread.  One tile per CTA; K split over a cluster as above, the exchange buffer laid over the
-// pipeline stages once every CTA of the cluster is past its main loop.
-constexpr int WIDE_N = 256;                 // weight rows per tile (GATED: 128 gate rows + their 128 up rows)
+// ------------------------------------------------------------------------------ wide tiles for 33 to 64 tokens
+// The operand roles swapped: the tokens are the M side (64 rows loaded; the MMA is 128 tall and its upper half reads whatever
+// follows the token tile in shared memory - rows that are never read back), 256 weight rows are N of ONE MMA.  A token tile then
+// goes with twice the weights, and a matrix of 43 to 74 tiles of 128 rows, which a split of K in two spreads over 86 to 148 CTAs,
+// has 22 to 37 of these and a finer split.  D is [token][weight row] in TMEM: a thread owns a token and 256 consecutive outputs,
+// which it stores 16 bytes at a time.  One tile per cluster, K split over its CTAs, the exchange buffer laid over the pipeline
+// stages once every CTA of the cluster is past its main loop.
+constexpr int WIDE_N = 256;                 // weight rows per tile
 constexpr int WIDE_M = 64;                  // token rows per tile
 constexpr uint32_t WIDE_A_BYTES = WIDE_M * BLK_K * 2, WIDE_B_BYTES = WIDE_N * BLK_K * 2;
 constexpr uint32_t WIDE_STAGE = WIDE_A_BYTES + WIDE_B_BYTES;
 constexpr int kWideStages = 5;
 constexpr int kWideThreads = 384;           // warps 0-3 as in gemm_tc_kernel, two epilogue warpgroups
 
-template <bool SPLIT, bool GATED>
 __global__ void __launch_bounds__(kWideThreads, 1)
 gemm_wide_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x, const GemmParams p) {
   constexpr int STAGES = kWideStages;
   constexpr uint32_t TMEM_COLS = WIDE_N;
-  // p.rows outputs per tile (a multiple of 16, up to 256; GATED: up to 128 gate rows + their up rows): the MMA's N
-  const int OUT_PER_TILE = p.rows;
-  const int N_MMA = GATED ? 2 * OUT_PER_TILE : OUT_PER_TILE;
-  const uint32_t IDESC = (1u << 4) | KGE_IDESC_AB | ((uint32_t)(N_MMA >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
-  constexpr int UNIT = 16;                                     // outputs per exchange unit (GATED: 16 gate + 16 up columns)
-  const int N_UNITS = OUT_PER_TILE / UNIT;
-  constexpr int UNIT_F = GATED ? 2 * UNIT : UNIT;              // fp32 values of a unit
-  const uint32_t tx_bytes = WIDE_A_BYTES + (uint32_t)N_MMA * BLK_K * 2;
+  constexpr uint32_t IDESC = (1u << 4) | KGE_IDESC_AB | ((uint32_t)(WIDE_N >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
+  constexpr int UNIT = 16, N_UNITS = WIDE_N / UNIT;            // outputs per exchange unit
 
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -857,27 +845,17 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
   pdl_launch_dependents();
   if (warp != 0) pdl_wait();          // warp 0 (TMA producer) prefetches weights first, then waits
 
-  const int S = SPLIT ? (int)cluster_nctarank() : 1;
-  const int crank = SPLIT ? (int)cluster_ctarank() : 0;
-  const int m_tile = SPLIT ? (int)blockIdx.x / S : (int)blockIdx.x;            // one tile per CTA (cluster)
+  const int S = (int)cluster_nctarank(), crank = (int)cluster_ctarank(), m_tile = (int)blockIdx.x / S;
   const int kb0 = crank * p.kb_per_split, kb1 = min(p.kb_total, kb0 + p.kb_per_split);
-  const int n0 = m_tile * OUT_PER_TILE;                                         // first output column of the tile
+  const int n0 = m_tile * WIDE_N;                                               // first output column of the tile
 
   if (warp == 0) {
     if (elect_one()) {
-      auto load_w = [&](int st, int kb) {
-        const uint32_t dst = smem_base + st * WIDE_STAGE + WIDE_A_BYTES;
-        if (GATED) {
-          tma_load_2d(dst, &tmap_w, full_bar(st), kb * BLK_K, n0);                              // the gate rows
-          tma_load_2d(dst + OUT_PER_TILE * BLK_K * 2, &tmap_w, full_bar(st), kb * BLK_K, p.N + n0);   // their up rows
-        } else {
-          tma_load_2d(dst, &tmap_w, full_bar(st), kb * BLK_K, n0);
-        }
-      };
+      auto load_w = [&](int st, int kb) { tma_load_2d(smem_base + st * WIDE_STAGE + WIDE_A_BYTES, &tmap_w, full_bar(st), kb * BLK_K, n0); };
       trace_stamp(p, 12);
       const int pre = min(STAGES, kb1 - kb0);
       for (int i = 0; i < pre; ++i) {
-        mbar_expect_tx(full_bar(i), tx_bytes);
+        mbar_expect_tx(full_bar(i), WIDE_STAGE);
         load_w(i, kb0 + i);
         if (i == 0) trace_stamp(p, 13);
       }
@@ -888,7 +866,7 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
       for (int kb = kb0; kb < kb1; ++kb) {
         if (kb - kb0 >= pre) {
           mbar_wait(empty_bar(stage), phase ^ 1);
-          mbar_expect_tx(full_bar(stage), tx_bytes);
+          mbar_expect_tx(full_bar(stage), WIDE_STAGE);
           load_w(stage, kb);
         }
         tma_load_2d(smem_base + stage * WIDE_STAGE, &tmap_x, full_bar(stage), kb * BLK_K, 0);
@@ -929,18 +907,12 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
     if (et == 0) trace_stamp(p, 7);
     const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16);
     const bool vec_ok = (p.N & 7) == 0;
-    // the 16 outputs of unit u for my token from raw accumulators: bias / ReLU, or silu(gate) * up
-    auto finish = [&](int u, const float (&a)[16], const float (&up)[16], float (&o)[16]) {
+    // the 16 outputs of unit u from raw accumulators: bias, activation
+    auto finish = [&](int u, const float (&a)[16], float (&o)[16]) {
 #pragma unroll
       for (int j = 0; j < 16; ++j) {
-        if (GATED) {
-          o[j] = silu_gate_bf16(p, a[j], up[j], n0 + u * UNIT + j);
-        } else {
-          const int n = n0 + u * UNIT + j;
-          float v = a[j] + ((p.bias && n < p.N) ? bf2f(p.bias[n]) : 0.f);
-          v = apply_act(v, p.act);
-          o[j] = v;
-        }
+        const int n = n0 + u * UNIT + j;
+        o[j] = apply_act(a[j] + ((p.bias && n < p.N) ? bf2f(p.bias[n]) : 0.f), p.act);
       }
     };
     auto store16 = [&](int t, int u, const float (&o)[16]) {
@@ -958,81 +930,52 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
         for (int j = 0; j < 16; ++j) if (n + j < p.N) dst[j] = f2bf(o[j]);
       }
     };
-    if (!SPLIT) {
-      if (q < 2) {
+    const int units_per = (N_UNITS + S - 1) / S;
+    constexpr int NJ = UNIT / 4;                            // 16-byte pieces of a unit
+    // exchange buffer of a CTA: [source rank][local unit][piece][token][4 fp32] - a warp stores (and later loads) 512
+    // contiguous bytes
+    const uint32_t xb = smem_base;                          // over the pipeline stages: dead once phase A completes
+    cluster_arrive();                                       // phase A: my MMAs have read their last stage
+    cluster_wait();
+    if (q < 2) {
 #pragma unroll 1
-        for (int u = u_lo; u < u_hi; ++u) {
-          uint32_t r[16], r2[16];
-          float a[16], up[16], o[16];
-          tmem_ld16(taddr + u * UNIT, r);
-          if (GATED) tmem_ld16(taddr + OUT_PER_TILE + u * UNIT, r2);
+      for (int u = u_lo; u < u_hi; ++u) {
+        uint32_t r[16];
+        tmem_ld16(taddr + u * UNIT, r);
+        const int owner = u / units_per, lu = u - owner * units_per;
+        const uint32_t dst = mapa_u32(xb + (uint32_t)(((((crank * units_per + lu) * NJ) * WIDE_M) + tok) * 16), (uint32_t)owner);
 #pragma unroll
-          for (int j = 0; j < 16; ++j) { a[j] = __uint_as_float(r[j]); up[j] = GATED ? __uint_as_float(r2[j]) : 0.f; }
-          finish(u, a, up, o);
-          store16(tok, u, o);
+        for (int j = 0; j < NJ; ++j)
+          st_cluster_f4(dst + j * (WIDE_M * 16), __uint_as_float(r[4 * j]), __uint_as_float(r[4 * j + 1]), __uint_as_float(r[4 * j + 2]), __uint_as_float(r[4 * j + 3]));
+      }
+    }
+    tc_fence_before();
+    if (et == 0) trace_stamp(p, 8);
+    cluster_arrive();                                       // phase B: my partials are in the owners' buffers
+    cluster_wait();
+    if (et == 0) trace_stamp(p, 9);
+    // my units, summed over the ranks in rank order; one item = one token's 16 outputs of one unit
+    const int u_begin = crank * units_per;
+    const int my_units = min(N_UNITS, u_begin + units_per) - u_begin;
+    for (int item = et; item < my_units * WIDE_M; item += 256) {
+      const int t = item & (WIDE_M - 1), lu = item / WIDE_M;
+      float a[16], o[16];
+#pragma unroll
+      for (int j = 0; j < 16; ++j) a[j] = 0.f;
+      for (int s2 = 0; s2 < S; ++s2) {
+        const uint32_t src = xb + (uint32_t)(((((s2 * units_per + lu) * NJ) * WIDE_M) + t) * 16);
+#pragma unroll
+        for (int j = 0; j < NJ; ++j) {
+          const float4 v = lds_f4(src + j * (WIDE_M * 16));
+          a[4 * j] += v.x; a[4 * j + 1] += v.y; a[4 * j + 2] += v.z; a[4 * j + 3] += v.w;
         }
       }
-    } else {
-      const int units_per = (N_UNITS + S - 1) / S;
-      constexpr int NJ = UNIT_F / 4;                        // 16-byte pieces of a unit
-      // exchange buffer of a CTA: [source rank][local unit][piece][token][4 fp32] - a warp stores (and later loads) 512
-      // contiguous bytes
-      const uint32_t xb = smem_base;                        // over the pipeline stages: dead once phase A completes
-      cluster_arrive();                                     // phase A: my MMAs have read their last stage
-      cluster_wait();
-      if (q < 2) {
-#pragma unroll 1
-        for (int u = u_lo; u < u_hi; ++u) {
-          uint32_t r[16], r2[16];
-          tmem_ld16(taddr + u * UNIT, r);
-          if (GATED) tmem_ld16(taddr + OUT_PER_TILE + u * UNIT, r2);
-          const int owner = u / units_per, lu = u - owner * units_per;
-          const uint32_t dst = mapa_u32(xb + (uint32_t)(((((crank * units_per + lu) * NJ) * WIDE_M) + tok) * 16), (uint32_t)owner);
-#pragma unroll
-          for (int j = 0; j < 4; ++j)
-            st_cluster_f4(dst + j * (WIDE_M * 16), __uint_as_float(r[4 * j]), __uint_as_float(r[4 * j + 1]), __uint_as_float(r[4 * j + 2]), __uint_as_float(r[4 * j + 3]));
-          if (GATED) {
-#pragma unroll
-            for (int j = 0; j < 4; ++j)
-              st_cluster_f4(dst + (4 + j) * (WIDE_M * 16), __uint_as_float(r2[4 * j]), __uint_as_float(r2[4 * j + 1]), __uint_as_float(r2[4 * j + 2]), __uint_as_float(r2[4 * j + 3]));
-          }
-        }
-      }
-      tc_fence_before();
-      if (et == 0) trace_stamp(p, 8);
-      cluster_arrive();                                     // phase B: my partials are in the owners' buffers
-      cluster_wait();
-      if (et == 0) trace_stamp(p, 9);
-      // my units, summed over the ranks in rank order; one item = one token's 16 outputs of one unit
-      const int u_begin = crank * units_per;
-      const int my_units = min(N_UNITS, u_begin + units_per) - u_begin;
-      for (int item = et; item < my_units * WIDE_M; item += 256) {
-        const int t = item & (WIDE_M - 1), lu = item / WIDE_M;
-        float a[16], up[16], o[16];
-#pragma unroll
-        for (int j = 0; j < 16; ++j) { a[j] = 0.f; up[j] = 0.f; }
-        for (int s2 = 0; s2 < S; ++s2) {
-          const uint32_t src = xb + (uint32_t)(((((s2 * units_per + lu) * NJ) * WIDE_M) + t) * 16);
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            const float4 v = lds_f4(src + j * (WIDE_M * 16));
-            a[4 * j] += v.x; a[4 * j + 1] += v.y; a[4 * j + 2] += v.z; a[4 * j + 3] += v.w;
-          }
-          if (GATED) {
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              const float4 v = lds_f4(src + (4 + j) * (WIDE_M * 16));
-              up[4 * j] += v.x; up[4 * j + 1] += v.y; up[4 * j + 2] += v.z; up[4 * j + 3] += v.w;
-            }
-          }
-        }
-        finish(u_begin + lu, a, up, o);
-        store16(t, u_begin + lu, o);
-      }
+      finish(u_begin + lu, a, o);
+      store16(t, u_begin + lu, o);
     }
     if (et == 0) trace_stamp(p, 10);
   }
-  if (SPLIT && warp < 4) {                       // non-epilogue warps take part in both cluster phases
+  if (warp < 4) {                       // non-epilogue warps take part in both cluster phases
     cluster_arrive();
     cluster_wait();
     cluster_arrive();
@@ -1217,7 +1160,7 @@ static int max_clusters(int tokn, int S) {
   return cache[ti][S];
 }
 
-struct GemmPlan { int tokn, m_tiles, n_tiles, splits, kb_total, kb_per_split; bool ws; int rows; bool pair = false; };
+struct GemmPlan { int tokn, m_tiles, n_tiles, splits, kb_total, kb_per_split; bool ws; bool pair = false; };
 
 constexpr int64_t kWsCounterBytes = 1024;        // per-tile arrival counters at the head of the workspace (<= 256 tiles)
 
@@ -1252,14 +1195,12 @@ static GemmPlan plan_gemm(int T, int N, int K, int rows_out = BLK_M, bool ws_ok 
   return g;
 }
 
-// ---- wide tiles (T <= 64): one tile of 256 weight rows per CTA / cluster
+// ---- wide tiles: one tile of 256 weight rows per cluster
 constexpr int kWideSmem = kWideStages * (int)WIDE_STAGE + 1024 /*align*/ + 2048 /*barriers*/;
 
-template <bool SPLIT, bool GATED>
 static int launch_wide(const CUtensorMap& tw, const CUtensorMap& tx, const GemmParams& p, cudaStream_t st) {
-  auto kern = gemm_wide_kernel<SPLIT, GATED>;
-  KGE_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kWideSmem));
-  prefer_max_shared(kern);
+  KGE_CUDA_OK(cudaFuncSetAttribute(gemm_wide_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kWideSmem));
+  prefer_max_shared(gemm_wide_kernel);
   cudaLaunchConfig_t cfg = {};
   cfg.blockDim = dim3(kWideThreads);
   cfg.dynamicSmemBytes = kWideSmem;
@@ -1268,13 +1209,10 @@ static int launch_wide(const CUtensorMap& tw, const CUtensorMap& tx, const GemmP
   cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = pdl_for_this_launch() ? 1 : 0;
-  cfg.attrs = attr; cfg.numAttrs = 1;
-  if (SPLIT) {
-    attr[1].id = cudaLaunchAttributeClusterDimension;
-    attr[1].val.clusterDim.x = p.splits; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = 1;
-    cfg.numAttrs = 2;
-  }
-  KGE_CUDA_OK(cudaLaunchKernelEx(&cfg, kern, tw, tx, p));
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = p.splits; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr; cfg.numAttrs = 2;
+  KGE_CUDA_OK(cudaLaunchKernelEx(&cfg, gemm_wide_kernel, tw, tx, p));
   return 0;
 }
 
@@ -1282,7 +1220,7 @@ static int max_clusters_wide(int S) {
   static int cache[9];
   static bool have[9];
   if (!have[S]) {
-    auto kern = gemm_wide_kernel<true, false>;
+    auto kern = gemm_wide_kernel;
     int n = 0;
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kWideSmem) == cudaSuccess) {
       cudaLaunchConfig_t cfg = {};
@@ -1298,50 +1236,25 @@ static int max_clusters_wide(int S) {
   return cache[S];
 }
 
-// Tile width (outputs per tile, a multiple of 16: up to 256, or 128 for the fused gate/up) and K split of the wide
-// kernel: full-width tiles with the largest cluster split that fits one round; where no split is possible (more than
-// 74 tiles) narrower tiles, down to 3/4 of the width, if that puts more CTAs to work (gate_up of Llama-8B: 128 tiles of
-// 112 outputs instead of 112 of 128).  A cost model over all widths and splits (k-block = max(MMA time, bytes at the
-// per-SM rate), price per split) picked plans that were faster alone and 0.35 ms per decode step SLOWER in the engine
-// (clusters of 3 and 5 next to the neighbouring kernels' CTAs); it was removed.
-// False: this problem keeps the 128-row kernels.
-static bool plan_wide(int T, int n_out, int K, bool gated, GemmPlan& g) {
-  if (!tunable(TUN_GEMM_WIDE) || T > WIDE_M) return false;
-  const int kb_total = (K + BLK_K - 1) / BLK_K;
-  const int max_rows = gated ? WIDE_N / 2 : WIDE_N;
-  const int max_by_k = kb_total / 4 > 0 ? kb_total / 4 : 1;   // >= 4 k-blocks (256 of K) per split
-  double best = 1e30;
-  int best_rows = 0, best_s = 0;
-  auto try_rows = [&](int rows) {               // largest split that fits one round; more CTAs win, then the wider tile
-    const int tiles = (n_out + rows - 1) / rows;
-    if (tiles > 148) return;
-    int sp = 148 / tiles;
-    if (sp > max_by_k) sp = max_by_k;
-    if (sp > 8) sp = 8;
-    while (sp > 1 && tiles > max_clusters_wide(sp)) --sp;
-    const double score = -(double)(tiles * sp) - rows * 1e-3;
-    if (score < best) { best = score; best_rows = rows; best_s = sp; }
-  };
-  try_rows(max_rows);
-  if (best_s == 1)                              // no split possible: spread the rows over more CTAs instead
-    for (int rows = max_rows - 16; rows >= (3 * max_rows) / 4; rows -= 16) try_rows(rows);
-  if (best_rows == 0) return false;
+// Whether a projection takes the wide tiles, and the K split: the largest whose clusters fit one round.  Only 33 to 64 tokens where
+// the 128-row plan splits K in two: us with wide and 128-row tiles, 64 tokens, 8192 x 8192 26.1 / 27.3, 7168 x 2048 9.9 / 10.2,
+// 6144 x 4096 13.6 / 13.8; up to 32 tokens a token tile is too small to matter (6144 x 4096 13.5 / 12.4), a split in three is finer
+// than what clusters of 256 rows leave (5120 x 5120 14.1 / 13.0), and more than 74 tiles need no split (16384 x 2048 15.4 / 13.4,
+// 28672 x 4096 42.0 / 40.2, gated 45.1 / 41.0, gated 16384 x 2048 16.8 / 13.9).
+static bool plan_wide(int T, int n_out, int K, GemmPlan& g) {
+  if (!tunable(TUN_GEMM_WIDE) || T > WIDE_M || T <= WIDE_M / 2 || plan_gemm(T, n_out, K).splits != 2) return false;
+  g.kb_total = (K + BLK_K - 1) / BLK_K;
+  g.m_tiles = (n_out + WIDE_N - 1) / WIDE_N;
+  int sp = 148 / g.m_tiles;
+  if (sp > g.kb_total / 4) sp = g.kb_total / 4;        // >= 4 k-blocks (256 of K) per split
+  if (sp > 8) sp = 8;
+  while (sp > 1 && g.m_tiles > max_clusters_wide(sp)) --sp;
+  if (sp < 2) return false;
   g.ws = false;
   g.tokn = WIDE_M; g.n_tiles = 1;
-  g.rows = best_rows;
-  g.m_tiles = (n_out + best_rows - 1) / best_rows;
-  g.kb_total = kb_total;
-  g.kb_per_split = (kb_total + best_s - 1) / best_s;
-  g.splits = (kb_total + g.kb_per_split - 1) / g.kb_per_split;
-  // only where it keeps at least as many CTAs streaming as the 128-row plan (measured: otherwise it loses)
-  const GemmPlan narrow = plan_gemm(T, n_out, K, gated ? 64 : BLK_M, false);
-  const int narrow_tiles = narrow.m_tiles * narrow.n_tiles;
-  int narrow_ctas = narrow_tiles * narrow.splits;
-  if (narrow_tiles > 148) {                                // persistent: the grid launch_gemm evens out
-    const int rounds = (narrow_tiles + 147) / 148;
-    narrow_ctas = tunable(TUN_GEMM_EVEN_GRID) ? (narrow_tiles + rounds - 1) / rounds : 148;
-  }
-  return g.m_tiles * g.splits >= narrow_ctas;
+  g.kb_per_split = (g.kb_total + sp - 1) / sp;
+  g.splits = (g.kb_total + g.kb_per_split - 1) / g.kb_per_split;
+  return true;
 }
 
 #include "gemm_rows.cuh"
@@ -1493,16 +1406,15 @@ extern "C" int KGE_GEMM_NAME(void* y, const void* x, const void* w, const void* 
       return launch_rows<false>((const bf16*)x, (const bf16*)w, p, (cudaStream_t)stream);
     }
     GemmPlan gw;
-    if (plan_wide(T, N, K, false, gw)) {
+    if (plan_wide(T, N, K, gw)) {
       GemmParams p;
       p.y = (bf16*)y; p.bias = (const bf16*)bias; p.T = T; p.N = N; p.K = K; p.act = act;
       p.l2_hints = 0; p.trace = g_gemm_trace; p.ws_count = nullptr; p.ws_part = nullptr;
       p.m_tiles = gw.m_tiles; p.n_tiles = 1; p.splits = gw.splits; p.kb_total = gw.kb_total; p.kb_per_split = gw.kb_per_split;
       CUtensorMap tw, tx;
-      p.rows = gw.rows;
-      if (int rc = make_tmap(&tw, w, N, K, gw.rows)) return rc;
+      if (int rc = make_tmap(&tw, w, N, K, WIDE_N)) return rc;
       if (int rc = make_tmap(&tx, x, T, K, WIDE_M)) return rc;
-      return gw.splits > 1 ? launch_wide<true, false>(tw, tx, p, (cudaStream_t)stream) : launch_wide<false, false>(tw, tx, p, (cudaStream_t)stream);
+      return launch_wide(tw, tx, p, (cudaStream_t)stream);
     }
   }
   GemmPlan g = plan_gemm(T, N, K, BLK_M, workspace != nullptr);
@@ -1541,18 +1453,6 @@ static int gemm_gated(void* y, const void* x, const void* w_gate_up, int T, int 
       GemmParams p;
       p.y = (bf16*)y; p.bias = (const bf16*)bias_gate_up; p.T = T; p.N = f; p.K = K; p.act = 2; p.glu = glu; p.glu_alpha = glu_alpha; p.glu_limit = glu_limit;
       return launch_rows<true>((const bf16*)x, (const bf16*)w_gate_up, p, (cudaStream_t)stream);
-    }
-    GemmPlan gw;
-    if (plan_wide(T, f, K, true, gw)) {
-      GemmParams p;
-      p.y = (bf16*)y; p.bias = (const bf16*)bias_gate_up; p.T = T; p.N = f; p.K = K; p.act = 2; p.glu = glu; p.glu_alpha = glu_alpha; p.glu_limit = glu_limit;
-      p.l2_hints = 0; p.trace = g_gemm_trace; p.ws_count = nullptr; p.ws_part = nullptr;
-      p.m_tiles = gw.m_tiles; p.n_tiles = 1; p.splits = gw.splits; p.kb_total = gw.kb_total; p.kb_per_split = gw.kb_per_split;
-      CUtensorMap tw, tx;
-      p.rows = gw.rows;
-      if (int rc = make_tmap(&tw, w_gate_up, 2 * (int64_t)f, K, gw.rows)) return rc;
-      if (int rc = make_tmap(&tx, x, T, K, WIDE_M)) return rc;
-      return gw.splits > 1 ? launch_wide<true, true>(tw, tx, p, (cudaStream_t)stream) : launch_wide<false, true>(tw, tx, p, (cudaStream_t)stream);
     }
   }
   GemmPlan g = plan_gemm(T, f, K, 64, workspace != nullptr);
