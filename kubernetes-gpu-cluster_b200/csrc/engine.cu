@@ -442,6 +442,7 @@ extern "C" int kge_engine_create(kge_engine** out, const char* model_dir, const 
   if (!e->h || !e->res || !e->xn || !e->qkv || !e->attn || !e->gu || !e->act || !e->xsel || !e->logits ||
       !e->d_out || !e->lp_vals || !e->lp_ids || !e->lp_rank || !e->mask_pairs || !e->ws_gemm || !e->ws_attn || !e->meta_dev)
     ENGINE_FAIL("kge_engine_create: activation arena allocation failed (%s)", cudaGetErrorString(cudaGetLastError()));
+  e->alloc_logits_host((int64_t)Rm * e->spec.vocab);
   if (cudaMallocHost((void**)&e->meta_host, e->meta_bytes) != cudaSuccess ||
       cudaMallocHost((void**)&e->out_host, (size_t)Rm * 4) != cudaSuccess ||
       cudaMallocHost((void**)&e->lp_vals_host, (size_t)Rm * 21 * 4) != cudaSuccess ||
@@ -506,6 +507,7 @@ extern "C" void kge_engine_destroy(kge_engine* e) {
   if (e->tpc) kge_tp_comm_destroy(e->tpc);
   if (e->meta_host) cudaFreeHost(e->meta_host);
   if (e->out_host) cudaFreeHost(e->out_host);
+  if (e->logits_host) cudaFreeHost(e->logits_host);
   if (e->lp_vals_host) cudaFreeHost(e->lp_vals_host);
   if (e->lp_ids_host) cudaFreeHost(e->lp_ids_host);
   if (e->lp_rank_host) cudaFreeHost(e->lp_rank_host);

@@ -213,6 +213,14 @@ struct kge_engine {
   uint8_t *meta_host = nullptr, *meta_dev = nullptr;
   int64_t meta_bytes = 0;
   int32_t* out_host = nullptr;               // pinned [max_num_seqs]
+  // Pinned landing place of logits that a caller reads back (up to 4 MiB of them; null if that could not be had): a copy into pageable
+  // memory waits for the device in between its pieces (one row of 50272: a decode step 357 us, 326 through here).
+  float* logits_host = nullptr;
+  int64_t logits_host_n = 0;
+  void alloc_logits_host(int64_t most) {
+    logits_host_n = most < (1 << 20) ? most : (1 << 20);
+    if (cudaMallocHost((void**)&logits_host, (size_t)logits_host_n * 4) != cudaSuccess) { (void)cudaGetLastError(); logits_host = nullptr; logits_host_n = 0; }
+  }
   // log-probabilities of the last step's sampled rows (only when a request asked): [max_num_seqs, 21] + ranks
   float* lp_vals = nullptr; int32_t* lp_ids = nullptr; int32_t* lp_rank = nullptr;        // device
   float* lp_vals_host = nullptr; int32_t* lp_ids_host = nullptr; int32_t* lp_rank_host = nullptr;   // pinned
@@ -220,7 +228,7 @@ struct kge_engine {
   std::unordered_map<int64_t, std::pair<int, int>> lp_last;    // request id -> (row of the last step, its own N)
 
   // CUDA graphs of pure decode steps, keyed by what is baked into the launches
-  struct DecodeGraph { int B, ns, stride; bool rnd; cudaGraphExec_t exec; int64_t launches; };
+  struct DecodeGraph { int B, ns, stride; bool rnd, logits; cudaGraphExec_t exec; int64_t launches; };
   std::vector<DecodeGraph> graphs;
   std::vector<std::pair<int64_t, int>> graph_seen;   // key hash -> eager runs so far
   bool use_graphs = true;

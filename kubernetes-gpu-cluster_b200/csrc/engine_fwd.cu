@@ -197,17 +197,19 @@ int engine_decode_step(kge_engine* e, int B, int stride, int max_seq_len, const 
   if (!e->use_graphs || e->timing || e->step_num_masks > 0 || e->layer_dump_host)      // a masked step is rare and its mask list is not part of a graph
     return forward();
   for (auto& g : e->graphs)
-    if (g.B == B && g.ns == ns && g.stride == stride && g.rnd == any_random) {
+    if (g.B == B && g.ns == ns && g.stride == stride && g.rnd == any_random && g.logits == e->want_logits32) {
       KGE_CUDA_OK(cudaGraphLaunch(g.exec, e->stream));
       e->launches += g.launches;
       return 0;
     }
-  const int64_t key = ((int64_t)B << 40) ^ ((int64_t)ns << 32) ^ ((int64_t)stride << 1) ^ (any_random ? 1 : 0);
+  const int64_t key = ((int64_t)B << 40) ^ ((int64_t)ns << 32) ^ ((int64_t)stride << 2) ^ (e->want_logits32 ? 2 : 0) ^ (any_random ? 1 : 0);
   int* seen = nullptr;
   for (auto& kv : e->graph_seen) if (kv.first == key) seen = &kv.second;
   if (!seen) { e->graph_seen.push_back({key, 0}); seen = &e->graph_seen.back().second; }
-  if ((*seen)++ == 0)     // first sight: run eagerly so every lazy initialisation happens outside a capture
-    return forward();
+  // First sight: eager, so that every lazy initialisation happens outside a capture.  Steps whose logits the caller reads back are
+  // captured later: they seldom come in great numbers, and a capture costs what eight replays save (opt-125m, one request: 0.95 ms,
+  // 490 us a step eager and 357 replayed).
+  if ((*seen)++ < (e->want_logits32 ? 8 : 1)) return forward();
   const int64_t l0 = e->launches;
   KGE_CUDA_OK(cudaStreamBeginCapture(e->stream, cudaStreamCaptureModeThreadLocal));
   const int rc = forward();
@@ -215,7 +217,7 @@ int engine_decode_step(kge_engine* e, int B, int stride, int max_seq_len, const 
   cudaError_t ce = cudaStreamEndCapture(e->stream, &graph);
   if (rc) { if (graph) cudaGraphDestroy(graph); return rc; }
   KGE_REQUIRE(ce == cudaSuccess && graph, "decode graph capture failed: %s", cudaGetErrorString(ce));
-  kge_engine::DecodeGraph g{B, ns, stride, any_random, nullptr, e->launches - l0};
+  kge_engine::DecodeGraph g{B, ns, stride, any_random, e->want_logits32, nullptr, e->launches - l0};
   ce = cudaGraphInstantiate(&g.exec, graph, 0);
   cudaGraphDestroy(graph);
   KGE_REQUIRE(ce == cudaSuccess, "cudaGraphInstantiate failed: %s", cudaGetErrorString(ce));
@@ -252,7 +254,7 @@ static int run_step(kge_engine* e, const kge_step_batch* b, const float* temp, c
   KGE_CUDA_OK(cudaSetDevice(e->cfg.device));
   // pure decode step with every row sampled: block-table rows at a bucketed stride so the captured
   // graph of this (B, splits, stride) can be replayed while contexts grow
-  bool decode_only = (T == B && R == B && !out_logits_host);
+  bool decode_only = (T == B && R == B && (!out_logits_host || e->tp_size == 1));
   for (int i = 0; decode_only && i < B; ++i) decode_only = (b->logits_rows[i] == i);
   const int stride = decode_only ? std::min(e->max_blocks_per_seq, (b->max_blocks + 31) / 32 * 32) : b->max_blocks;
   int64_t bytes = 0;
@@ -331,6 +333,8 @@ static int run_step(kge_engine* e, const kge_step_batch* b, const float* temp, c
   }
   ++e->step_count;
   e->lp_last_n = -1;
+  const int64_t logits_n = out_logits_host ? (int64_t)R * e->spec.vocab : 0;
+  float* const land = logits_n > 0 && logits_n <= e->logits_host_n ? e->logits_host : out_logits_host;
   if (R > 0) {
     if (sampled) KGE_CUDA_OK(cudaMemcpyAsync(e->out_host, e->d_out, (size_t)R * 4, cudaMemcpyDeviceToHost, e->stream));
     if (lp_n >= 0 && sampled) {
@@ -346,20 +350,21 @@ static int run_step(kge_engine* e, const kge_step_batch* b, const float* temp, c
     }
     if (out_logits_host && hybrid) {
       // layer-list models keep the logits of the step in fp32
-      KGE_CUDA_OK(cudaMemcpyAsync(out_logits_host, e->logits32, (size_t)R * e->spec.vocab * 4, cudaMemcpyDeviceToHost, e->stream));
+      KGE_CUDA_OK(cudaMemcpyAsync(land, e->logits32, (size_t)logits_n * 4, cudaMemcpyDeviceToHost, e->stream));
     } else if (out_logits_host) {
       // debug/parity path: logits as fp32 through a scratch carved from the (idle) gate_up buffer
       float* tmp = reinterpret_cast<float*>(e->gu);
-      const int64_t n = (int64_t)R * e->spec.vocab;
+      const int64_t n = logits_n;
       KGE_REQUIRE(n * 4 <= (int64_t)e->cfg.max_num_batched_tokens * e->layers[0].up.N * 2,
                   "kge_step: logits read-back needs R*vocab*4 <= gate_up buffer");
       elt_to_f32_kernel<<<148 * 4, 256, 0, e->stream>>>(tmp, e->logits, n, e->f16);
-      KGE_CUDA_OK(cudaMemcpyAsync(out_logits_host, tmp, (size_t)n * 4, cudaMemcpyDeviceToHost, e->stream));
+      KGE_CUDA_OK(cudaMemcpyAsync(land, tmp, (size_t)n * 4, cudaMemcpyDeviceToHost, e->stream));
     }
   }
   KGE_CUDA_OK(cudaStreamSynchronize(e->stream));
   if (e->timing) collect_timing(e);
   if (sampled && out_ids_host) memcpy(out_ids_host, e->out_host, (size_t)R * 4);
+  if (land != out_logits_host) memcpy(out_logits_host, land, (size_t)logits_n * 4);
   return 0;
 }
 

@@ -695,6 +695,7 @@ int hybrid_engine_build(kge_engine* e, const ModelDir& md, int64_t dummy_seed, s
   if (!e->res32 || !e->hx || !e->pbuf || !e->ubuf || !e->mixbuf || !e->obuf1 || !e->obuf2 || !e->ffbuf || !e->gates32 || !e->mo32 || !e->hsel ||
       !e->logits32 || !e->logits || !e->state || !e->d_out || !e->lp_vals || !e->lp_ids || !e->lp_rank || !e->mask_pairs || !e->meta_dev)
     return fail("activation arena allocation failed: " + b.err);
+  e->alloc_logits_host((int64_t)Rm * s.vocab);
   if (cudaMallocHost((void**)&e->meta_host, e->meta_bytes) != cudaSuccess ||
       cudaMallocHost((void**)&e->out_host, (size_t)Rm * 4) != cudaSuccess ||
       cudaMallocHost((void**)&e->lp_vals_host, (size_t)Rm * 21 * 4) != cudaSuccess ||
