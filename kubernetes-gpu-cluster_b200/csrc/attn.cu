@@ -70,12 +70,13 @@ struct KvLoader {
   uint32_t dst[NP];
   int row0, c8;
   const int32_t* btab;
+  int last;                                      // entries of the block-table row - 1
   int64_t head_off;                              // kvh * block_size * HD
   int64_t blk_stride;                            // KV * block_size * HD
   int bs_shift, bs_mask;
 
-  __device__ __forceinline__ void init(const int32_t* bt, int kvh, int KV, int shift, int tid) {
-    btab = bt; bs_shift = shift; bs_mask = (1 << shift) - 1;
+  __device__ __forceinline__ void init(const int32_t* bt, int max_blocks, int kvh, int KV, int shift, int tid) {
+    btab = bt; last = max_blocks - 1; bs_shift = shift; bs_mask = (1 << shift) - 1;
     row0 = tid / CH;
     const int c = tid % CH;
     c8 = c * 8;
@@ -84,6 +85,8 @@ struct KvLoader {
 #pragma unroll
     for (int j = 0; j < NP; ++j) dst[j] = swz<HD>(row0 + j * RP, c);
   }
+  // EARLY: the block id is read whether the key exists or not, so that it need not wait for the request's length
+  template <bool EARLY>
   __device__ __forceinline__ void load(uint32_t sK, uint32_t sV, const bf16* __restrict__ kc,
                                        const bf16* __restrict__ vc, int key0, int kv_len) const {
 #pragma unroll
@@ -91,7 +94,12 @@ struct KvLoader {
       const int key = key0 + row0 + j * RP;
       const bool ok = key < kv_len;
       int64_t off = 0;
-      if (ok) off = (int64_t)btab[key >> bs_shift] * blk_stride + head_off + (key & bs_mask) * HD + c8;
+      if (EARLY) {
+        const int blk = btab[min(key >> bs_shift, last)];
+        if (ok) off = (int64_t)blk * blk_stride + head_off + (key & bs_mask) * HD + c8;
+      } else if (ok) {
+        off = (int64_t)btab[key >> bs_shift] * blk_stride + head_off + (key & bs_mask) * HD + c8;
+      }
       cp_async16(sK + dst[j], kc + off, ok);
       cp_async16(sV + dst[j], vc + off, ok);
     }
@@ -120,7 +128,7 @@ attn_decode_kernel(bf16* __restrict__ out, float* __restrict__ part_o, float* __
   const int kv_len = seq_lens[b];
   const int ntiles_all = (kv_len + BN - 1) / BN;
   const int tps = (ntiles_all + nsplit - 1) / nsplit;
-  const int t_begin = split * tps, t_end = min(ntiles_all, t_begin + tps);
+  const int t_begin = nsplit == 1 ? 0 : split * tps, t_end = min(ntiles_all, t_begin + tps);
   const int32_t* btab = block_table + (int64_t)b * max_blocks;
   const int qrow = qsl[b];
 
@@ -140,12 +148,12 @@ attn_decode_kernel(bf16* __restrict__ out, float* __restrict__ part_o, float* __
     cp_async16(sQ + swz<HD>(r, c), src, ok);
   }
   KvLoader<HD, NT> ld;
-  ld.init(btab, kvh, KV, bs_shift, tid);
+  ld.init(btab, max_blocks, kvh, KV, bs_shift, tid);
   // prologue: STAGES-1 tiles in flight
 #pragma unroll
   for (int s = 0; s < STAGES - 1; ++s) {
     if (t_begin + s < t_end)
-      ld.load(sK + s * BN * HD * 2, sV + s * BN * HD * 2, k_cache, v_cache, (t_begin + s) * BN, kv_len);
+      ld.template load<true>(sK + s * BN * HD * 2, sV + s * BN * HD * 2, k_cache, v_cache, (t_begin + s) * BN, kv_len);
     cp_async_commit();
   }
 
@@ -162,7 +170,7 @@ attn_decode_kernel(bf16* __restrict__ out, float* __restrict__ part_o, float* __
     __syncthreads();             // tile `it` landed for all threads; stage (it-1)%STAGES is free
     if (nxt < t_end) {
       const int ns = (it + STAGES - 1) % STAGES;
-      ld.load(sK + ns * BN * HD * 2, sV + ns * BN * HD * 2, k_cache, v_cache, nxt * BN, kv_len);
+      ld.template load<false>(sK + ns * BN * HD * 2, sV + ns * BN * HD * 2, k_cache, v_cache, nxt * BN, kv_len);
     }
     cp_async_commit();
     if (it == 0) {
@@ -307,10 +315,13 @@ __global__ void attn_merge_kernel(bf16* __restrict__ out, const float* __restric
   out[(int64_t)qsl[b] * H * HD + head * HD + c] = f2bf(ll > 0.f ? acc / ll : 0.f);
 }
 
-constexpr int kDecodeStages = 3;
-template <int HD> constexpr int decode_smem() {
+// 64-key tiles in the ring: three, and five of 64-wide heads where two CTAs per SM are all there are, so that contexts of up to 256
+// tokens are all on their way at once (us with three and five: 190 keys, 12 heads of one request 3.9 / 3.5, 32 requests of 96 to 256
+// with 32 / 8 heads 7.6 / 5.4, one of 4000 9.8 / 8.7; but where more CTAs than that share an SM, 64 requests of up to 2000 45.7 / 60).
+constexpr int kDecodeStages = 3, kDecodeStagesFew = 5;
+template <int HD> constexpr int decode_smem(int stages) {
   static_assert(4 * 16 * (HD + 2) * 4 <= kDecodeStages * BN * HD * 2, "sRed must fit in the K stages");
-  return 16 * HD * 2 + 2 * kDecodeStages * BN * HD * 2;
+  return 16 * HD * 2 + 2 * stages * BN * HD * 2;
 }
 
 int attn_decode_splits(int B, int KV, int max_seq_len);
@@ -363,9 +374,9 @@ static int launch_attn(bf16* out, const bf16* q, int q_stride, const bf16* kc, c
       // kernel, but measured SLOWER than the merge kernel behind programmatic dependent launch (C3 decode step
       // 7.64 vs 7.38 ms): cluster co-scheduling costs more than the extra launch
       auto kern = attn_decode_kernel<HD, kDecodeStages, true>;
-      KGE_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, decode_smem<HD>()));
+      KGE_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, decode_smem<HD>(kDecodeStages)));
       cudaLaunchConfig_t cfg = {};
-      cfg.gridDim = dim3(ns, KV, B); cfg.blockDim = dim3(128); cfg.dynamicSmemBytes = decode_smem<HD>(); cfg.stream = st;
+      cfg.gridDim = dim3(ns, KV, B); cfg.blockDim = dim3(128); cfg.dynamicSmemBytes = decode_smem<HD>(kDecodeStages); cfg.stream = st;
       cudaLaunchAttribute attr[2];
       attr[0].id = cudaLaunchAttributeClusterDimension;
       attr[0].val.clusterDim.x = ns; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
@@ -391,9 +402,11 @@ static int launch_attn(bf16* out, const bf16* q, int q_stride, const bf16* kc, c
       return paged_attn_decode_tma(out, q, q_stride, kc, vc, bt, max_blocks, sl, qsl, B, H, KV, HD, bs, ns, sl2, po, pml, ws, ws_bytes,
                                    max_seq_len, cap_in2, cap_log2, sinks, st);
     KGE_REQUIRE(!extras, "paged attention: a soft cap or sink logits need the TMA-staged decode kernel (blocks of 32 tokens or more)");
-    auto kern = attn_decode_kernel<HD, kDecodeStages, false>;
-    KGE_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, decode_smem<HD>()));
-    KGE_CUDA_OK(launch_pdl(kern, dim3(ns, KV, B), dim3(128), decode_smem<HD>(), st, out, po, pml, q, q_stride, kc, vc, bt,
+    const bool few = HD == 64 && (int64_t)ns * KV * B <= 2 * 148;
+    auto kern = few ? attn_decode_kernel<HD, HD == 64 ? kDecodeStagesFew : kDecodeStages, false> : attn_decode_kernel<HD, kDecodeStages, false>;
+    const int smem = decode_smem<HD>(few ? kDecodeStagesFew : kDecodeStages);
+    KGE_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    KGE_CUDA_OK(launch_pdl(kern, dim3(ns, KV, B), dim3(128), smem, st, out, po, pml, q, q_stride, kc, vc, bt,
                            max_blocks, sl, qsl, H, KV, bs_shift, sl2));
     if (ns > 1)
       KGE_CUDA_OK(launch_pdl(attn_merge_kernel, dim3(H, B), dim3(HD), 0, st, out, (const float*)po, (const float*)pml, qsl, H, HD, ns));
