@@ -51,9 +51,19 @@ norm_kernel(bf16* __restrict__ y, bf16* __restrict__ residual, const bf16* __res
             const bf16* __restrict__ w, const bf16* __restrict__ b, int d, float eps) {
   __shared__ float red[33];
   pdl_launch_dependents();
-  pdl_wait();
   const int64_t base = (int64_t)blockIdx.x * d;
   const int nvec = d / 8;
+  // weights (no kernel's output) while the kernel before is still at work: behind the reduction they cost a trip to memory
+  uint4 wv[kMaxVecPerThread], bv[kMaxVecPerThread];
+#pragma unroll
+  for (int j = 0; j < kMaxVecPerThread; ++j) {
+    const int i = threadIdx.x + j * blockDim.x;
+    if (i < nvec && w) {
+      wv[j] = *reinterpret_cast<const uint4*>(w + i * 8);
+      if (MODE >= 2) bv[j] = *reinterpret_cast<const uint4*>(b + i * 8);
+    }
+  }
+  pdl_wait();
   float v[kMaxVecPerThread][8];
   float acc = 0.f;
 #pragma unroll
@@ -108,7 +118,7 @@ norm_kernel(bf16* __restrict__ y, bf16* __restrict__ residual, const bf16* __res
   for (int j = 0; j < kMaxVecPerThread; ++j) {
     const int i = threadIdx.x + j * blockDim.x;
     if (i < nvec) {
-      uint4 ww = *reinterpret_cast<const uint4*>(w + i * 8);
+      const uint4 ww = wv[j];
       float wf[8] = {bf_lo(ww.x), bf_hi(ww.x), bf_lo(ww.y), bf_hi(ww.y),
                      bf_lo(ww.z), bf_hi(ww.z), bf_lo(ww.w), bf_hi(ww.w)};
       float o[8];
@@ -116,7 +126,7 @@ norm_kernel(bf16* __restrict__ y, bf16* __restrict__ residual, const bf16* __res
 #pragma unroll
         for (int k = 0; k < 8; ++k) o[k] = rbf(v[j][k] * rstd) * wf[k];   // weight mul in bf16
       } else {
-        uint4 bb = *reinterpret_cast<const uint4*>(b + i * 8);
+        const uint4 bb = bv[j];
         float bfv[8] = {bf_lo(bb.x), bf_hi(bb.x), bf_lo(bb.y), bf_hi(bb.y),
                         bf_lo(bb.z), bf_hi(bb.z), bf_lo(bb.w), bf_hi(bb.w)};
 #pragma unroll
