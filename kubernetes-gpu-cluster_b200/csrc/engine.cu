@@ -14,10 +14,10 @@ namespace kge {
 
 const Ops kOpsBf16 = {kge_embed, kge_rmsnorm, kge_add_rmsnorm, kge_head_rmsnorm, kge_layernorm, kge_silu_mul, kge_gemm_bf16,
                       kge_gemm_silu_gate_ws_bf16, kge_rope_kvwrite, kge_rope_cache_host, kge_paged_attn, kge_argmax, kge_sample,
-                      kge_logprobs, kge_tp_reduce_add_norm};
+                      kge_logprobs, kge_tp_reduce_add_norm, kge_norm_gemm};
 const Ops kOpsF16 = {kge_embed_f16, kge_rmsnorm_f16, kge_add_rmsnorm_f16, kge_head_rmsnorm_f16, kge_layernorm_f16, kge_silu_mul_f16,
                      kge_gemm_f16, kge_gemm_silu_gate_ws_f16, kge_rope_kvwrite_f16, kge_rope_cache_host_f16, kge_paged_attn_f16,
-                     kge_argmax_f16, kge_sample_f16, kge_logprobs_f16, kge_tp_reduce_add_norm_f16};
+                     kge_argmax_f16, kge_sample_f16, kge_logprobs_f16, kge_tp_reduce_add_norm_f16, kge_norm_gemm_f16};
 
 // 16-bit pattern of v in the engine's element type
 __device__ __forceinline__ uint16_t to_elt_bits(float v, bool f16) {
@@ -421,6 +421,7 @@ extern "C" int kge_engine_create(kge_engine** out, const char* model_dir, const 
     e->logits = (bf16*)aalloc((int64_t)Rm * e->ld_logits, 2);
   }
   e->res = (bf16*)aalloc((int64_t)Tm * d, 2);
+  e->res_next = (bf16*)aalloc((int64_t)8 * d, 2);
   e->qkv = (bf16*)aalloc((int64_t)Tm * qkv_n, 2);
   e->attn = (bf16*)aalloc((int64_t)Tm * e->H_loc * s.hd, 2);
   e->gu = (bf16*)aalloc((int64_t)Tm * up_n, 2);
@@ -439,7 +440,7 @@ extern "C" int kge_engine_create(kge_engine** out, const char* model_dir, const 
   e->max_blocks_per_seq = (e->cfg.max_model_len + e->cfg.block_size - 1) / e->cfg.block_size;
   carve_meta(nullptr, Tm, Rm, Rm, e->max_blocks_per_seq, &e->meta_bytes);
   e->meta_dev = (uint8_t*)aalloc(e->meta_bytes, 1);
-  if (!e->h || !e->res || !e->xn || !e->qkv || !e->attn || !e->gu || !e->act || !e->xsel || !e->logits ||
+  if (!e->h || !e->res || !e->res_next || !e->xn || !e->qkv || !e->attn || !e->gu || !e->act || !e->xsel || !e->logits ||
       !e->d_out || !e->lp_vals || !e->lp_ids || !e->lp_rank || !e->mask_pairs || !e->ws_gemm || !e->ws_attn || !e->meta_dev)
     ENGINE_FAIL("kge_engine_create: activation arena allocation failed (%s)", cudaGetErrorString(cudaGetLastError()));
   e->alloc_logits_host((int64_t)Rm * e->spec.vocab);

@@ -11,6 +11,7 @@
 
 #include "common.cuh"
 #include "kge.h"
+#include "norm_gemm.h"
 #include "loader.h"
 #include "scheduler.h"
 
@@ -34,6 +35,7 @@ struct Ops {
   decltype(&kge_sample) sample;
   decltype(&kge_logprobs) logprobs;
   decltype(&kge_tp_reduce_add_norm) tp_reduce_add_norm;
+  decltype(&kge_norm_gemm) norm_gemm;
 };
 extern const Ops kOpsBf16, kOpsF16;     // engine.cu
 
@@ -202,6 +204,7 @@ struct kge_engine {
   int num_blocks = 0, max_blocks_per_seq = 0;
   int64_t weight_bytes = 0, kv_bytes = 0;
 
+  kge::bf16* res_next = nullptr;             // [8, d]: the residual stream's other buffer in small steps (norm_gemm.h)
   kge::bf16 *h = nullptr, *res = nullptr, *xn = nullptr, *qkv = nullptr, *attn = nullptr;
   kge::bf16 *gu = nullptr, *act = nullptr, *xsel = nullptr, *logits = nullptr;
   float* logits_f32 = nullptr;

@@ -67,12 +67,12 @@ int tp_all_gather_logits(kge_engine* e, int R);           // tp.cu (NCCL path)
 // all-reduce it, add it to the residual stream and normalise into e->xn.  Single GPU: the fused add + norm kernel.
 // TP over peer memory: ONE kernel does all three (tp_peer.cu) and keeps the residual for this rank's rows only.
 // TP over NCCL (--disable-custom-all-reduce): ncclAllReduce, then the norm kernel.
-static int reduce_add_norm(kge_engine* e, int T, const bf16* w, const bf16* b, bool layer_norm, float eps) {
+static int reduce_add_norm(kge_engine* e, bf16* res, int T, const bf16* w, const bf16* b, bool layer_norm, float eps) {
   const int d = e->spec.d;
   if (e->tp_peer())
-    return e->op->tp_reduce_add_norm(e->tpc, e->off_xn, e->res, e->off_h, w, b, T, d, eps, layer_norm ? 3 : 1, e->stream);
-  if (layer_norm) return e->op->layernorm(e->xn, e->res, e->h, w, b, T, d, eps, e->stream);
-  return e->op->add_rmsnorm(e->xn, e->res, e->h, w, T, d, eps, e->stream);
+    return e->op->tp_reduce_add_norm(e->tpc, e->off_xn, res, e->off_h, w, b, T, d, eps, layer_norm ? 3 : 1, e->stream);
+  if (layer_norm) return e->op->layernorm(e->xn, res, e->h, w, b, T, d, eps, e->stream);
+  return e->op->add_rmsnorm(e->xn, res, e->h, w, T, d, eps, e->stream);
 }
 
 int engine_forward(kge_engine* e, int T, int B, int R, int max_blocks, int max_q_len, int max_seq_len,
@@ -112,12 +112,35 @@ int engine_forward(kge_engine* e, int T, int B, int R, int max_blocks, int max_q
 #define REDUCE_NORM(w, b, ln, eps)                                                                      \
   do {                                                                                                  \
     if (e->tp_size > 1 && !peer) FWD(C_AR, ar_bytes, 0, tp_all_reduce(e, e->h, (int64_t)T * d));         \
-    FWD(peer ? C_AR : C_NORM, 4 * Td2, 0, reduce_add_norm(e, T, w, b, ln, eps));                        \
+    FWD(peer ? C_AR : C_NORM, 4 * Td2, 0, reduce_add_norm(e, res, T, w, b, ln, eps));                        \
   } while (0)
+  // A few tokens of an OPT model: norm and projection in one launch, the cache write in the projection (no rotation), the residual stream
+  // going back and forth between two buffers: five launches a layer in the place of eight.
+  bf16 *res = e->res, *res_next = e->res_next;
+  const bool fuse = s.is_opt() && e->tp_size == 1 && kge_norm_gemm_ok(T, e->layers[0].qkv.N, d) && kge_norm_gemm_ok(T, e->layers[0].up.N, d);
+  // y = act(norm(res [+ h]) W^T + b); the residual stream then is the sum
+  auto norm_linear = [&](bf16* y, bool add, const bf16* w, const bf16* b, const Linear& l, int act, const RowsKv& kv) -> int {
+    RowsNorm nm;
+    nm.res = res; nm.add = add ? e->h : nullptr; nm.res_out = add ? res_next : nullptr; nm.w = w; nm.b = b; nm.eps = 1e-5f;
+    FWD(C_GEMM_S, 2.0 * ((double)l.N * l.K + (double)T * (2 * l.K + l.N)), 2.0 * T * (double)l.N * l.K,
+        e->op->norm_gemm(y, nm, l.w, l.b, T, l.N, l.K, act, kv, st));
+    if (add) std::swap(res, res_next);
+    return 0;
+  };
   if (s.is_opt()) {
     FWD(C_EMBED, 2 * Td2, 0, e->op->embed(e->res, m.ids, e->embed, e->pos_embed, m.pos, 2, T, d, st));
     for (int i = 0; i < s.L; ++i) {
       const LayerW& L = e->layers[i];
+      if (fuse) {
+        RowsKv kv;
+        kv.kc = e->kc[i]; kv.vc = e->vc[i]; kv.slots = m.slots; kv.q_cols = Hl * hd; kv.KV = KVl; kv.hd = hd; kv.bs = bs;
+        if (int rc = norm_linear(e->qkv, i > 0, L.ln1_w, L.ln1_b, L.qkv, 0, kv)) return rc;
+        if (int rc = attend(i)) return rc;
+        LINEAR(e->h, e->attn, L.o, T, 0);
+        if (int rc = norm_linear(e->act, true, L.ln2_w, L.ln2_b, L.up, 1, RowsKv())) return rc;
+        LINEAR(e->h, e->act, L.down, T, 0);
+        continue;
+      }
       // first LN of the layer; for i > 0 it also folds in the previous layer's fc2 output
       if (i == 0) FWD(C_NORM, 2 * Td2, 0, e->op->layernorm(e->xn, e->res, nullptr, L.ln1_w, L.ln1_b, T, d, 1e-5f, st));
       else REDUCE_NORM(L.ln1_w, L.ln1_b, true, 1e-5f);

@@ -23,12 +23,92 @@ __device__ __forceinline__ void rows_mma(float (&c)[4], uint32_t a0, uint32_t a1
 
 constexpr int rows_smem(int warps, int nw, int tt, int s) { return warps * s * (nw + tt) * 1024; }
 
+// NORM: the rows are normalised first, each by one warp, in every CTA (a row of 768 is 1.5 KB from L2; a kernel of its own costs the
+// latency of one more launch in the chain of a step); their 16-bit values lie in shared memory behind the ring.
+constexpr int kNormVecs = 4;                           // 16-byte pieces of a row per lane: up to 1024 of K
+__host__ __device__ constexpr int norm_row_bytes(int K) { return 2 * K + 64; }      // the fragments of eight rows fall on different banks
+
+__device__ __forceinline__ void unpack8(uint4 a, float (&f)[8]) {
+  f[0] = bf_lo(a.x); f[1] = bf_hi(a.x); f[2] = bf_lo(a.y); f[3] = bf_hi(a.y);
+  f[4] = bf_lo(a.z); f[5] = bf_hi(a.z); f[6] = bf_lo(a.w); f[7] = bf_hi(a.w);
+}
+__device__ __forceinline__ uint4 pack8(const float (&f)[8]) {
+  return make_uint4(pack_bf2(f[0], f[1]), pack_bf2(f[2], f[3]), pack_bf2(f[4], f[5]), pack_bf2(f[6], f[7]));
+}
+
+__device__ __forceinline__ void norm_weights(uint4 (&wv)[kNormVecs], uint4 (&bv)[kNormVecs], const RowsNorm& nm, int K) {
+#pragma unroll
+  for (int j = 0; j < kNormVecs; ++j) {
+    const int i = (threadIdx.x & 31) + j * 32;
+    if (i < K / 8) {
+      wv[j] = *reinterpret_cast<const uint4*>((const bf16*)nm.w + i * 8);
+      bv[j] = *reinterpret_cast<const uint4*>((const bf16*)nm.b + i * 8);
+    }
+  }
+}
+// One row by one warp, with the roundings of norm_kernel (elementwise.cu)
+__device__ __forceinline__ void norm_row(uint8_t* dst, const RowsNorm& nm, const uint4 (&wv)[kNormVecs], const uint4 (&bv)[kNormVecs], int row, int K, bool store) {
+  const int lane = threadIdx.x & 31, nvec = K / 8;
+  const int64_t base = (int64_t)row * K;
+  const bf16 *res = (const bf16*)nm.res + base, *add = (const bf16*)nm.add + base;
+  // every load before the first store: behind a store to res_out the compiler keeps later loads back, and each costs a trip to L2
+  uint4 rv[kNormVecs], av[kNormVecs];
+#pragma unroll
+  for (int j = 0; j < kNormVecs; ++j) {
+    const int i = lane + j * 32;
+    if (i < nvec) {
+      rv[j] = *reinterpret_cast<const uint4*>(res + i * 8);
+      if (nm.add) av[j] = *reinterpret_cast<const uint4*>(add + i * 8);
+    }
+  }
+  float v[kNormVecs][8], acc = 0.f;
+#pragma unroll
+  for (int j = 0; j < kNormVecs; ++j) {
+    const int i = lane + j * 32;
+    if (i < nvec) {
+      unpack8(rv[j], v[j]);
+      if (nm.add) {
+        float r[8];
+        unpack8(av[j], r);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) v[j][k] += r[k];
+        const uint4 o = pack8(v[j]);
+        if (store) *reinterpret_cast<uint4*>((bf16*)nm.res_out + base + i * 8) = o;
+        unpack8(o, v[j]);
+      }
+#pragma unroll
+      for (int k = 0; k < 8; ++k) acc += v[j][k];
+    }
+  }
+  const float mean = warp_sum(acc) / (float)K;
+  float a2 = 0.f;
+#pragma unroll
+  for (int j = 0; j < kNormVecs; ++j)
+    if (lane + j * 32 < nvec)
+#pragma unroll
+      for (int k = 0; k < 8; ++k) { const float c = v[j][k] - mean; a2 += c * c; }
+  const float rstd = 1.0f / sqrtf(warp_sum(a2) / (float)K + nm.eps);
+#pragma unroll
+  for (int j = 0; j < kNormVecs; ++j) {
+    const int i = lane + j * 32;
+    if (i < nvec) {
+      float wf[8], bf[8], o[8];
+      unpack8(wv[j], wf);
+      unpack8(bv[j], bf);
+#pragma unroll
+      for (int k = 0; k < 8; ++k) o[k] = (v[j][k] - mean) * rstd * wf[k] + bf[k];
+      *reinterpret_cast<uint4*>(dst + i * 16) = pack8(o);
+    }
+  }
+}
+
 // W: warps per CTA; NT: 8-row weight tiles per CTA (GATED: NT of gate rows and NT of their up rows); TT: 8-token halves in
 // use; S: stages of 64 of K per warp
-template <int W, int NT, int TT, bool GATED, int S>
-__global__ void __launch_bounds__(W * 32)
-gemm_rows_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w, const GemmParams p) {
-  constexpr int NW = GATED ? 2 * NT : NT, PIECES = 2 * (NW + TT);
+template <int W, int NT, int TT, bool GATED, int S, bool NORM = false>
+__global__ void __launch_bounds__(W * 32, NORM ? 2 : 1)
+gemm_rows_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w, const GemmParams p, const RowsNorm nm, const RowsKv kv) {
+  static_assert(!NORM || TT == 1, "up to 8 normalised rows");
+  constexpr int NW = GATED ? 2 * NT : NT, PIECES = 2 * (NW + (NORM ? 0 : TT));
   extern __shared__ __align__(16) uint4 ring[];        // [warp][stage][piece][lane]
   __shared__ float part[W][TT * 8][NW * 8 + 2];
   pdl_launch_dependents();
@@ -72,11 +152,22 @@ gemm_rows_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w, const G
 #pragma unroll
   for (int i = 0; i < S - 1; ++i)
     if (i < mine) copy_w(i);
+  uint4 nw[kNormVecs], nb[kNormVecs];
+  if (NORM && warp < p.T) norm_weights(nw, nb, nm, p.K);
+  // the bias of this thread's first output: a trip to memory behind the sums otherwise
+  const int first_n = n0 + (int)threadIdx.x % (8 * NT);
+  const float first_bias = !GATED && p.bias && first_n < p.N ? bf2f(p.bias[first_n]) : 0.f;
   pdl_wait();                                          // the tokens are the previous kernel's output
 #pragma unroll
   for (int i = 0; i < S - 1; ++i) {
-    if (i < mine) copy_x(i);
+    if (!NORM && i < mine) copy_x(i);
     asm volatile("cp.async.commit_group;" ::: "memory");
+  }
+  uint8_t* rows = reinterpret_cast<uint8_t*>(ring + W * S * PIECES * 32);
+  const uint8_t* my_row = rows + min(g, p.T - 1) * norm_row_bytes(p.K) + t * 16;      // what rows beyond T hold is not stored
+  if (NORM) {
+    if (warp < p.T) norm_row(rows + warp * norm_row_bytes(p.K), nm, nw, nb, warp, p.K, blockIdx.x == 0);
+    __syncthreads();
   }
 #pragma unroll 1
   for (int i = 0; i < mine; ++i) {
@@ -87,10 +178,18 @@ gemm_rows_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w, const G
     for (int h = 0; h < 2; ++h) {
 #pragma unroll
       for (int j = 0; j < NW; ++j) wv[j][h] = src[(2 * j + h) * 32];
+      if (NORM) {
+        const int k = (warp + i * W) * 64 + h * 32;
+        xv[0][h] = k + t * 8 < p.K ? *reinterpret_cast<const uint4*>(my_row + 2 * k) : make_uint4(0, 0, 0, 0);
+      } else {
 #pragma unroll
-      for (int j = 0; j < TT; ++j) xv[j][h] = src[(2 * (NW + j) + h) * 32];
+        for (int j = 0; j < TT; ++j) xv[j][h] = src[(2 * (NW + j) + h) * 32];
+      }
     }
-    if (i + S - 1 < mine) { copy_w(i + S - 1); copy_x(i + S - 1); }      // into the stage that the previous turn read
+    if (i + S - 1 < mine) {                            // into the stage that the previous turn read
+      copy_w(i + S - 1);
+      if (!NORM) copy_x(i + S - 1);
+    }
     asm volatile("cp.async.commit_group;" ::: "memory");
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
@@ -121,8 +220,14 @@ gemm_rows_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w, const G
     }
     float v;
     if (GATED) v = silu_gate_bf16(p, a, b, n);
-    else v = apply_act(p.bias ? a + bf2f(p.bias[n]) : a, p.act);
+    else v = apply_act(p.bias ? a + first_bias : a, p.act);             // W * 32 is a multiple of 8 NT: every trip has the same column
     p.y[(int64_t)tok * p.N + n] = f2bf(v);
+    if (NORM && kv.kc && n >= kv.q_cols) {             // a key or a value: into the cache too
+      const int64_t slot = kv.slots[tok];
+      const int c = n - kv.q_cols, width = kv.KV * kv.hd, u = c < width ? c : c - width;
+      if (slot >= 0)
+        (c < width ? (bf16*)kv.kc : (bf16*)kv.vc)[(((slot / kv.bs) * kv.KV + u / kv.hd) * kv.bs + slot % kv.bs) * kv.hd + u % kv.hd] = f2bf(v);
+    }
   }
 }
 
@@ -131,7 +236,15 @@ static int launch_rows_as(const bf16* x, const bf16* w, const GemmParams& p, cud
   auto kern = gemm_rows_kernel<W, NT, TT, GATED, S>;
   constexpr int smem = rows_smem(W, GATED ? 2 * NT : NT, TT, S);
   KGE_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-  KGE_CUDA_OK(launch_pdl(kern, dim3((p.N + 8 * NT - 1) / (8 * NT)), dim3(W * 32), smem, st, x, w, p));
+  KGE_CUDA_OK(launch_pdl(kern, dim3((p.N + 8 * NT - 1) / (8 * NT)), dim3(W * 32), smem, st, x, w, p, RowsNorm(), RowsKv()));
+  return 0;
+}
+template <int NT, int S>
+static int launch_norm_rows(const bf16* w, const GemmParams& p, const RowsNorm& nm, const RowsKv& kv, cudaStream_t st) {
+  auto kern = gemm_rows_kernel<8, NT, 1, false, S, true>;
+  const int smem = rows_smem(8, NT, 0, S) + p.T * norm_row_bytes(p.K);
+  KGE_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  KGE_CUDA_OK(launch_pdl(kern, dim3((p.N + 8 * NT - 1) / (8 * NT)), dim3(8 * 32), smem, st, nullptr, w, p, nm, kv));
   return 0;
 }
 template <bool GATED>

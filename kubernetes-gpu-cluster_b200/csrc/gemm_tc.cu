@@ -39,6 +39,7 @@
 
 #include "common.cuh"
 #include "kge.h"
+#include "norm_gemm.h"
 
 namespace kge {
 inline namespace KGE_ELT_NS {
@@ -1387,6 +1388,21 @@ extern "C" int64_t kge_gemm_workspace_bytes(int T, int N, int K) {
 #define KGE_GEMM_GATE_WS_NAME kge_gemm_silu_gate_ws_bf16
 #define KGE_GEMM_GLU_NAME kge_gemm_clamped_glu_bf16
 #endif
+// Up to 8 rows of up to 1024, and outputs for no more CTAs than are resident at once: norm and projection in two launches and in one,
+// us, 768 x 2304 at 1 and 8 tokens 4.0 / 3.2 and 4.7 / 3.7, 768 x 3072 3.6 / 3.3 and 4.2 / 3.9, 1024 x 4096 3.7 / 3.5 and 4.25 / 4.25.
+// Longer rows and more CTAs pay for a norm in each CTA (2048 x 3072 4.9 / 6.4, 2048 x 6144 8.7 / 15.0).
+#ifndef KGE_HALF
+extern "C" bool kge_norm_gemm_ok(int T, int N, int K) {
+  return T > 0 && T <= 8 && K % 8 == 0 && K <= 32 * 8 * kNormVecs && N <= 2 * 148 * 16 && use_rows(T, N, K);
+}
+#endif
+extern "C" int KGE_API(kge_norm_gemm)(void* y, const RowsNorm& nm, const void* w, const void* bias, int T, int N, int K, int act, const RowsKv& kv, void* stream) {
+  KGE_REQUIRE(kge_norm_gemm_ok(T, N, K) && (!nm.add || (nm.res_out && nm.res_out != nm.res)), "kge_norm_gemm: sizes");
+  GemmParams p;
+  p.y = (bf16*)y; p.bias = (const bf16*)bias; p.T = T; p.N = N; p.K = K; p.act = act;
+  return N < 16 * 148 ? launch_norm_rows<1, 4>((const bf16*)w, p, nm, kv, (cudaStream_t)stream) : launch_norm_rows<2, 3>((const bf16*)w, p, nm, kv, (cudaStream_t)stream);
+}
+
 extern "C" int KGE_GEMM_NAME(void* y, const void* x, const void* w, const void* bias, int T, int N, int K,
                              int act, void* workspace, int64_t workspace_bytes, void* stream) {
   KGE_REQUIRE(y && x && w, "kge_gemm_bf16: null pointer");
