@@ -2,6 +2,8 @@
 // sink logit per head in the softmax denominator, for any key / value head size, in bfloat16 or float32 storage.  One warp per (query row, head): 32 keys at a time, one key per lane for the scores (q in shared
 // memory), softmax statistics in fp32 across the warp, then the lanes split the value columns.  Only keys of the
 // query's own chunk are read, so the cost per query is bounded by the chunk size whatever the context length.
+#include <algorithm>
+
 #include "common.cuh"
 #include "elt_access.cuh"
 #include "hybrid_ops.h"
@@ -137,17 +139,21 @@ __device__ __forceinline__ void ab_ldsm_t(uint32_t (&r)[4], const void* p) {
   asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"((uint32_t)__cvta_generic_to_shared(p)) : "memory");
 }
 
-// ROWS = false: a CTA owns 16 rows and its warps split the key tiles (decoding, short pieces).  ROWS = true: a CTA owns
-// 64 rows, 16 per warp, and every key tile is staged once for all four warps (prompts).
+// ROWS = false: a CTA owns 16 rows and its warps split the key tiles (decoding, short pieces); where that leaves most of the chip idle,
+// the warps of a cluster do, and its CTAs' sums meet over distributed shared memory.  A tile's keys and values are asked for at once
+// (cp.async): with a round trip per eight pieces and one CTA per (request, group) two requests of 1160 keys in chunks of 1024 took 27 us
+// (cold caches), 14.5 with clusters of eight.  ROWS = true: a CTA owns 64 rows, 16 per warp, and every key tile is staged once for all four warps (prompts).
 template <bool ROWS>
 __global__ void __launch_bounds__(AM_WARPS * 32) attn_bias_mma_kernel(AttnBiasArgs a, int req0) {
   pdl_launch_dependents();
   pdl_wait();
   typedef __nv_bfloat16 E;
   extern __shared__ __align__(16) unsigned char am_smem[];
+  // CTAs of a cluster (1 or more; ROWS: 1) share the rows
+  const int S = ROWS ? 1 : (int)cluster_nctarank(), crank = ROWS ? 0 : (int)cluster_ctarank();
   const int b = req0 + blockIdx.z, g = blockIdx.y, hpg = a.H / a.G;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, qr = lane >> 2, qc = (lane & 3) * 2;
-  const int rs = a.qsl[b], nrows = (a.qsl[b + 1] - rs) * hpg, Rc = blockIdx.x * (ROWS ? 16 * AM_WARPS : 16);
+  const int rs = a.qsl[b], nrows = (a.qsl[b + 1] - rs) * hpg, Rc = (int)(blockIdx.x / S) * (ROWS ? 16 * AM_WARPS : 16);
   if (Rc >= nrows) return;
   const int R0 = ROWS ? Rc + warp * 16 : Rc;               // may lie beyond the request's rows: such a warp only helps staging
   const int dim = a.dim, vdim = a.vdim, ksteps = dim >> 4, vtiles = vdim >> 3;
@@ -203,7 +209,7 @@ __global__ void __launch_bounds__(AM_WARPS * 32) attn_bias_mma_kernel(AttnBiasAr
   float m[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f};
   const int32_t* bt = a.block_table + (int64_t)b * a.max_blocks;
   const int kseg = dim >> 3, vseg = vdim >> 3, vld = a.v_ld > 0 ? a.v_ld : vdim;
-  for (int kt = ROWS ? 0 : warp; kt < ntiles; kt += ROWS ? 1 : AM_WARPS) {
+  for (int kt = ROWS ? 0 : crank * AM_WARPS + warp; kt < ntiles; kt += ROWS ? 1 : AM_WARPS * S) {
     const bool ptile = kt < ptiles;                         // a tile of prefix keys: j0 counts them from 0
     const int j0 = ptile ? kt * AM_KT : lo_min + (kt - ptiles) * AM_KT;
     const E* kc = (const E*)(ptile && a.pool > 0 ? a.pk_cache : a.k_cache);
@@ -214,37 +220,50 @@ __global__ void __launch_bounds__(AM_WARPS * 32) attn_bias_mma_kernel(AttnBiasAr
     int64_t myrow = -1;
     if (ptile) { if (jl < pre_cta) myrow = prefix_row(a, bt, g, jl); }
     else if (jl <= pos_last) myrow = ((int64_t)bt[jl / a.block_size] * a.G + g) * a.block_size + jl % a.block_size;
-    const int sid = ROWS ? threadIdx.x : lane, sstep = ROWS ? AM_WARPS * 32 : 32;
-    // four 16-byte pieces (eight where one warp stages a whole tile: decoding) are requested before the first is stored, so
-    // a tile costs a few memory round trips, not one per piece (whole warps run the loops: the shuffle needs every lane)
-    constexpr int SU = ROWS ? 4 : 8;
-    for (int idx0 = 0; idx0 < AM_KT * kseg; idx0 += SU * sstep) {
-      uint4 v[SU]; int dst[SU];
+    // (whole warps run the loops: the shuffle needs every lane)
+    if constexpr (!ROWS) {
+      auto stage = [&](E* dst, const E* src, int segs, int st, int64_t ld) {
+        for (int idx = lane; idx < AM_KT * segs; idx += 32) {
+          const int key = idx / segs, seg = idx % segs;
+          const int64_t row = __shfl_sync(0xffffffffu, myrow, key);
+          asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst + key * st + seg * 8)),
+                       "l"(src + (row >= 0 ? row * ld + seg * 8 : 0)), "r"(row >= 0 ? 16 : 0) : "memory");
+        }
+      };
+      stage(Ks, kc, kseg, kst, dim);
+      stage(Vs, vc, vseg, vst, vld);
+      asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;" ::: "memory");
+    } else {
+      // four 16-byte pieces are requested before the first is stored, so a tile costs a few memory round trips, not one per piece
+      constexpr int SU = 4, sstep = AM_WARPS * 32;
+      for (int idx0 = 0; idx0 < AM_KT * kseg; idx0 += SU * sstep) {
+        uint4 v[SU]; int dst[SU];
 #pragma unroll
-      for (int u = 0; u < SU; ++u) {
-        const int idx = min(idx0 + u * sstep + sid, AM_KT * kseg - 1);
-        const int key = idx / kseg, seg = idx % kseg;
-        const int64_t row = __shfl_sync(0xffffffffu, myrow, key);
-        v[u] = make_uint4(0u, 0u, 0u, 0u);
-        if (row >= 0) v[u] = *reinterpret_cast<const uint4*>(kc + row * dim + seg * 8);
-        dst[u] = key * kst + seg * 8;
+        for (int u = 0; u < SU; ++u) {
+          const int idx = min(idx0 + u * sstep + (int)threadIdx.x, AM_KT * kseg - 1);
+          const int key = idx / kseg, seg = idx % kseg;
+          const int64_t row = __shfl_sync(0xffffffffu, myrow, key);
+          v[u] = make_uint4(0u, 0u, 0u, 0u);
+          if (row >= 0) v[u] = *reinterpret_cast<const uint4*>(kc + row * dim + seg * 8);
+          dst[u] = key * kst + seg * 8;
+        }
+#pragma unroll
+        for (int u = 0; u < SU; ++u) *reinterpret_cast<uint4*>(Ks + dst[u]) = v[u];
       }
+      for (int idx0 = 0; idx0 < AM_KT * vseg; idx0 += SU * sstep) {
+        uint4 v[SU]; int dst[SU];
 #pragma unroll
-      for (int u = 0; u < SU; ++u) *reinterpret_cast<uint4*>(Ks + dst[u]) = v[u];
-    }
-    for (int idx0 = 0; idx0 < AM_KT * vseg; idx0 += SU * sstep) {
-      uint4 v[SU]; int dst[SU];
+        for (int u = 0; u < SU; ++u) {
+          const int idx = min(idx0 + u * sstep + (int)threadIdx.x, AM_KT * vseg - 1);
+          const int key = idx / vseg, seg = idx % vseg;
+          const int64_t row = __shfl_sync(0xffffffffu, myrow, key);
+          v[u] = make_uint4(0u, 0u, 0u, 0u);
+          if (row >= 0) v[u] = *reinterpret_cast<const uint4*>(vc + row * vld + seg * 8);
+          dst[u] = key * vst + seg * 8;
+        }
 #pragma unroll
-      for (int u = 0; u < SU; ++u) {
-        const int idx = min(idx0 + u * sstep + sid, AM_KT * vseg - 1);
-        const int key = idx / vseg, seg = idx % vseg;
-        const int64_t row = __shfl_sync(0xffffffffu, myrow, key);
-        v[u] = make_uint4(0u, 0u, 0u, 0u);
-        if (row >= 0) v[u] = *reinterpret_cast<const uint4*>(vc + row * vld + seg * 8);
-        dst[u] = key * vst + seg * 8;
+        for (int u = 0; u < SU; ++u) *reinterpret_cast<uint4*>(Vs + dst[u]) = v[u];
       }
-#pragma unroll
-      for (int u = 0; u < SU; ++u) *reinterpret_cast<uint4*>(Vs + dst[u]) = v[u];
     }
     if (ROWS) __syncthreads(); else __syncwarp();
     if (ROWS && (ptile ? j0 >= own_pre : (j0 > own_hi || j0 + AM_KT <= own_lo))) continue;
@@ -360,12 +379,8 @@ __global__ void __launch_bounds__(AM_WARPS * 32) attn_bias_mma_kernel(AttnBiasAr
     ML[(warp * 2 + 1) * 16 + qr] = l[0]; ML[(warp * 2 + 1) * 16 + qr + 8] = l[1];
   }
   __syncthreads();
-  for (int idx = threadIdx.x; idx < 16 * vdim; idx += AM_WARPS * 32) {
-    const int r = idx / vdim, c = idx % vdim;
-    if (R0 + r >= nrows) continue;
-    float M = -INFINITY;
-#pragma unroll
-    for (int w = 0; w < AM_WARPS; ++w) M = fmaxf(M, ML[(w * 2) * 16 + r]);
+  // a row's largest score and, relative to it, its sums: over this CTA's warps, then over the cluster's CTAs in rank order
+  auto finish = [&](int r, int c, float M, auto&& sums) {
     const int row = R0 + r;
     float num = 0.f, den = 0.f;
     if (a.sinks) {
@@ -373,6 +388,17 @@ __global__ void __launch_bounds__(AM_WARPS * 32) attn_bias_mma_kernel(AttnBiasAr
       M = fmaxf(M, sk);
       den = exp2f(sk - M);
     }
+    sums(M, num, den);
+    E* out = (E*)a.out + (int64_t)(rs + row / hpg) * a.ldo + (g * hpg + row % hpg) * vdim + c;
+    *out = __float2bfloat16_rn(num / den * a.out_scale);
+  };
+  auto warps_max = [&](int r) {
+    float M = -INFINITY;
+#pragma unroll
+    for (int w = 0; w < AM_WARPS; ++w) M = fmaxf(M, ML[(w * 2) * 16 + r]);
+    return M;
+  };
+  auto warps_sum = [&](int r, int c, float M, float& num, float& den) {
 #pragma unroll
     for (int w = 0; w < AM_WARPS; ++w) {
       const float mw = ML[(w * 2) * 16 + r];
@@ -380,9 +406,75 @@ __global__ void __launch_bounds__(AM_WARPS * 32) attn_bias_mma_kernel(AttnBiasAr
       num = fmaf(f, reinterpret_cast<const float*>(am_smem + w * region)[r * vdim + c], num);
       den = fmaf(f, ML[(w * 2 + 1) * 16 + r], den);
     }
-    E* out = (E*)a.out + (int64_t)(rs + row / hpg) * a.ldo + (g * hpg + row % hpg) * vdim + c;
-    *out = __float2bfloat16_rn(num / den * a.out_scale);
+  };
+  if (S == 1) {
+    for (int idx = threadIdx.x; idx < 16 * vdim; idx += AM_WARPS * 32) {
+      const int r = idx / vdim, c = idx % vdim;
+      if (R0 + r >= nrows) continue;
+      finish(r, c, warps_max(r), [&](float M, float& num, float& den) { warps_sum(r, c, M, num, den); });
+    }
+    return;
   }
+  float* part = ML + AM_WARPS * 2 * 16;                     // this CTA's sums: [16][vdim], then [2][16]: largest scores, weights
+  for (int idx = threadIdx.x; idx < 16 * vdim; idx += AM_WARPS * 32) {
+    const int r = idx / vdim, c = idx % vdim;
+    const float M = warps_max(r);
+    float num = 0.f, den = 0.f;
+    if (M != -INFINITY) warps_sum(r, c, M, num, den);
+    part[idx] = num;
+    if (c == 0) { part[16 * vdim + r] = M; part[16 * vdim + 16 + r] = den; }
+  }
+  cluster_arrive();                                         // every CTA's sums are in its shared memory
+  cluster_wait();
+  const uint32_t mine = (uint32_t)__cvta_generic_to_shared(part);
+  auto remote = [&](int rank, int i) {
+    float v;
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(mapa_u32(mine + i * 4, (uint32_t)rank)) : "memory");
+    return v;
+  };
+  for (int idx = crank * AM_WARPS * 32 + threadIdx.x; idx < 16 * vdim; idx += S * AM_WARPS * 32) {
+    const int r = idx / vdim, c = idx % vdim;
+    if (R0 + r >= nrows) continue;
+    float mr[8], M = -INFINITY;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      mr[k] = k < S ? remote(k, 16 * vdim + r) : -INFINITY;
+      M = fmaxf(M, mr[k]);
+    }
+    finish(r, c, M, [&](float Mall, float& num, float& den) {
+#pragma unroll
+      for (int k = 0; k < 8; ++k)
+        if (k < S) {
+          const float f = mr[k] == -INFINITY ? 0.f : exp2f(mr[k] - Mall);
+          num = fmaf(f, remote(k, idx), num);
+          den = fmaf(f, remote(k, 16 * vdim + 16 + r), den);
+        }
+    });
+  }
+  cluster_arrive();                                         // nobody leaves while a peer reads its sums
+  cluster_wait();
+}
+
+// CTAs per cluster for `ctas` CTAs whose rows see up to `tiles` key tiles: as many as a round of one CTA per SM has room for, while each
+// warp keeps a tile
+static int bias_cluster(int64_t ctas, int tiles) {
+  int S = 8;
+  while (S > 1 && (ctas * S > 148 || tiles < AM_WARPS * S)) S /= 2;
+  return S;
+}
+static cudaError_t launch_bias_split(dim3 grid, int S, size_t smem, cudaStream_t st, const AttnBiasArgs& a, int req0) {
+  grid.x *= S;
+  if (S == 1) return launch_pdl(attn_bias_mma_kernel<false>, grid, dim3(AM_WARPS * 32), smem, st, a, req0);
+  prefer_max_shared(attn_bias_mma_kernel<false>);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid; cfg.blockDim = dim3(AM_WARPS * 32); cfg.dynamicSmemBytes = smem; cfg.stream = st;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = S; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr; cfg.numAttrs = pdl_for_this_launch() ? 2 : 1;
+  return cudaLaunchKernelEx(&cfg, attn_bias_mma_kernel<false>, a, req0);
 }
 
 int attn_bias_chunk(const AttnBiasArgs& a, cudaStream_t st) {
@@ -393,22 +485,27 @@ int attn_bias_chunk(const AttnBiasArgs& a, cudaStream_t st) {
   if (a.elt == KGE_ELT_BF16 && a.max_q > 0 && a.dim % 16 == 0 && a.dim <= AM_MAXD && a.vdim % 8 == 0 && a.vdim <= AM_MAXD && a.ldq % 2 == 0 &&
       a.H % a.G == 0 && a.v_ld % 8 == 0 && (reinterpret_cast<uintptr_t>(a.q) & 3) == 0 && a.B <= 65535 && a.G <= 65535) {
     const int hpg = a.H / a.G;
-    const size_t smem = (size_t)AM_WARPS * AM_KT * (a.dim + a.vdim + 2 * AM_PAD) * 2 + (size_t)AM_WARPS * 2 * 16 * 4;
+    // a tile for all warps (ROWS), or one each, their statistics and, in a cluster, the CTA's sums
+    const size_t tile = (size_t)AM_KT * (a.dim + a.vdim + 2 * AM_PAD) * 2, split = AM_WARPS * tile + (size_t)AM_WARPS * 2 * 16 * 4, sums = (size_t)16 * (a.vdim + 2) * 4;
     static size_t smem_set = 0;                       // opt in once per size that needs more than the default 48 KB
-    if (smem > 48 * 1024 && smem > smem_set) {
-      KGE_CUDA_OK(cudaFuncSetAttribute(attn_bias_mma_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-      KGE_CUDA_OK(cudaFuncSetAttribute(attn_bias_mma_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-      smem_set = smem;
+    if (split + sums > 48 * 1024 && split + sums > smem_set) {
+      KGE_CUDA_OK(cudaFuncSetAttribute(attn_bias_mma_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(split + sums)));
+      smem_set = split + sums;
     }
     // the leading one-token requests, then the rest; 64-row CTAs where a request has that many rows and its output
     // pairs can be stored as 32-bit words
     const int D = std::min(std::max(a.num_decode, 0), a.B);
-    if (D > 0) KGE_CUDA_OK(launch_pdl(attn_bias_mma_kernel<false>, dim3((hpg + 15) / 16, a.G, D), dim3(AM_WARPS * 32), smem, st, a, 0));
+    // the keys of a row that the launch can know of: its chunk, its window, or the block table's reach
+    const int reach = std::min(a.max_blocks * a.block_size, a.window > 0 ? a.window + a.keep_first : a.chunk > 0 ? a.chunk : 1 << 30);
+    if (D > 0) {
+      const int S = bias_cluster((int64_t)((hpg + 15) / 16) * a.G * D, reach / AM_KT);
+      KGE_CUDA_OK(launch_bias_split(dim3((hpg + 15) / 16, a.G, D), S, S > 1 ? split + sums : split, st, a, 0));
+    }
     if (D < a.B) {
       const int rows = a.max_q * hpg;
       const bool wide = rows > 32 && a.ldo % 2 == 0 && a.vdim % 2 == 0 && (reinterpret_cast<uintptr_t>(a.out) & 3) == 0;
-      if (wide) KGE_CUDA_OK(launch_pdl(attn_bias_mma_kernel<true>, dim3((rows + 16 * AM_WARPS - 1) / (16 * AM_WARPS), a.G, a.B - D), dim3(AM_WARPS * 32), smem, st, a, D));
-      else KGE_CUDA_OK(launch_pdl(attn_bias_mma_kernel<false>, dim3((rows + 15) / 16, a.G, a.B - D), dim3(AM_WARPS * 32), smem, st, a, D));
+      if (wide) KGE_CUDA_OK(launch_pdl(attn_bias_mma_kernel<true>, dim3((rows + 16 * AM_WARPS - 1) / (16 * AM_WARPS), a.G, a.B - D), dim3(AM_WARPS * 32), tile, st, a, D));
+      else KGE_CUDA_OK(launch_bias_split(dim3((rows + 15) / 16, a.G, a.B - D), 1, split, st, a, D));
     }
     return 0;
   }
@@ -425,32 +522,40 @@ int attn_bias_chunk(const AttnBiasArgs& a, cudaStream_t st) {
   return 0;
 }
 
-template <typename E>
+// W: numbers per thread and pass, 16 bytes of them where rows, heads and caches allow
+template <typename E, int W>
 __global__ void kv_write_any_kernel(const E* k, int ldk, const E* v, int ldv, const int64_t* slots, E* kc, E* vc, int G, int dim, int vdim, int bs) {
+  struct __align__(W * sizeof(E)) Piece { E e[W]; };
   pdl_launch_dependents();
   pdl_wait();
   const int t = blockIdx.x;
   const int64_t slot = slots[t];
   if (slot < 0) return;
   const int64_t blk = slot / bs, off = slot % bs;
-  for (int c = threadIdx.x; c < G * dim; c += blockDim.x) {
-    const int g = c / dim, d = c % dim;
-    kc[((blk * G + g) * bs + off) * dim + d] = k[(int64_t)t * ldk + c];
-  }
-  for (int c = threadIdx.x; c < G * vdim; c += blockDim.x) {
-    const int g = c / vdim, d = c % vdim;
-    vc[((blk * G + g) * bs + off) * vdim + d] = v[(int64_t)t * ldv + c];
+  const int nk = G * dim / W, n = nk + G * vdim / W;          // keys, then values
+  for (int i = threadIdx.x; i < n; i += blockDim.x) {
+    const bool key = i < nk;
+    const int c = (key ? i : i - nk) * W, hd = key ? dim : vdim, g = c / hd, d = c % hd;
+    const E* src = (key ? k + (int64_t)t * ldk : v + (int64_t)t * ldv) + c;
+    E* dst = (key ? kc : vc) + ((blk * G + g) * bs + off) * hd + d;
+    *reinterpret_cast<Piece*>(dst) = *reinterpret_cast<const Piece*>(src);
   }
 }
 
+template <typename E, int W>
+static cudaError_t launch_kv_write(const void* k, int ldk, const void* v, int ldv, const int64_t* slots, void* kc, void* vc, int T, int G, int dim, int vdim, int bs, cudaStream_t st) {
+  const int n = (G * dim + G * vdim) / W, th = std::max(32, std::min(256, (n + 31) / 32 * 32));
+  return launch_pdl(kv_write_any_kernel<E, W>, dim3(T), dim3(th), 0, st, (const E*)k, ldk, (const E*)v, ldv, slots, (E*)kc, (E*)vc, G, dim, vdim, bs);
+}
 int kv_write_any(const void* k, int ldk, const void* v, int ldv, const int64_t* slots, void* k_cache, void* v_cache, int T, int G,
                  int dim, int vdim, int block_size, int elt, cudaStream_t st) {
   if (T <= 0) return 0;
-  cudaError_t ce = elt == KGE_ELT_F32
-      ? launch_pdl(kv_write_any_kernel<float>, dim3(T), dim3(128), 0, st, (const float*)k, ldk, (const float*)v, ldv, slots, (float*)k_cache, (float*)v_cache, G, dim, vdim, block_size)
-      : launch_pdl(kv_write_any_kernel<__nv_bfloat16>, dim3(T), dim3(128), 0, st, (const __nv_bfloat16*)k, ldk, (const __nv_bfloat16*)v, ldv, slots,
-                   (__nv_bfloat16*)k_cache, (__nv_bfloat16*)v_cache, G, dim, vdim, block_size);
-  KGE_CUDA_OK(ce);
+  const int per = elt == KGE_ELT_F32 ? 4 : 8;
+  const bool wide = dim % per == 0 && vdim % per == 0 && ldk % per == 0 && ldv % per == 0 &&
+                    ((reinterpret_cast<uintptr_t>(k) | reinterpret_cast<uintptr_t>(v) | reinterpret_cast<uintptr_t>(k_cache) | reinterpret_cast<uintptr_t>(v_cache)) & 15) == 0;
+  auto run = elt == KGE_ELT_F32 ? (wide ? launch_kv_write<float, 4> : launch_kv_write<float, 1>)
+                                : (wide ? launch_kv_write<__nv_bfloat16, 8> : launch_kv_write<__nv_bfloat16, 1>);
+  KGE_CUDA_OK(run(k, ldk, v, ldv, slots, k_cache, v_cache, T, G, dim, vdim, block_size, st));
   return 0;
 }
 
