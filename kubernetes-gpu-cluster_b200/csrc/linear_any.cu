@@ -531,6 +531,141 @@ static int launch_linear_narrow(const LinearArgs& a, cudaStream_t st) {
   return 0;
 }
 
+// A few rows (up to 8 in all slices together): every weight is used once or twice, so a warp streams its own weight rows as in gemm_rows.cuh:
+// mma.m16n8k16 with the rows as M, a lane copies 16 consecutive bytes of each 32-number piece of the weights by cp.async into slots that only
+// it reads, the eight warps of a CTA interleave over K in chunks of 64 and add their sums in warp order.  A CTA has 8 outputs (gated pairs:
+// 8 of either matrix) of one slice; of groups only as many as there are rows are launched.  Strided slices ask for their first weights before the wait; which
+// groups have rows is the previous kernel's result.  us on cold weights in the ring of linear_stream_kernel or the tiles of
+// linear_mma_kernel and here: 4 rows in 4 of 16 experts, gated 2 x 1024 x 2048 25.8 / 11.4, 2048 x 1024 15.5 / 9.6, 2 rows by 16 blocks of
+// 160 x 160 7.8 / 4.4.
+constexpr int FEW_ROWS = 8, FEW_S = 4;
+template <typename O, bool DUAL>
+__global__ void __launch_bounds__(256) linear_few_kernel(LinearArgs a) {
+  constexpr int NW = DUAL ? 2 : 1, PIECES = 2 * (NW + 1);
+  typedef __nv_bfloat16 E;
+  pdl_launch_dependents();
+  extern __shared__ __align__(16) uint4 lf_ring[];             // [warp][stage][piece][lane]
+  __shared__ float part[8][FEW_ROWS][NW * 8 + 1];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3, n0 = blockIdx.x * 8;
+  const int chunks = (a.K + 63) / 64, mine = chunks > warp ? (chunks - warp + 7) / 8 : 0;
+  int z = a.group_off ? 0 : blockIdx.y;
+  const E* wrow[NW];
+  auto rows_of = [&] {
+#pragma unroll
+    for (int j = 0; j < NW; ++j) wrow[j] = (const E*)(j ? a.w2 : a.w) + z * a.w_zs + (int64_t)min(n0 + g, a.N - 1) * a.K + t * 8;
+  };
+  rows_of();
+  uint4* slot0 = lf_ring + (warp * FEW_S * PIECES) * 32 + lane;
+  auto copy = [&](uint4* dst, const E* src, bool in) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(in ? src : (const E*)a.w), "r"(in ? 16u : 0u) : "memory");
+  };
+  auto copy_w = [&](int i) {
+    uint4* dst = slot0 + (i % FEW_S) * PIECES * 32;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int k = (warp + i * 8) * 64 + h * 32;
+#pragma unroll
+      for (int j = 0; j < NW; ++j) copy(dst + (2 * j + h) * 32, wrow[j] + k, k + t * 8 < a.K && n0 + g < a.N);
+    }
+  };
+  if (!a.group_off) {
+#pragma unroll
+    for (int i = 0; i < FEW_S - 1; ++i)
+      if (i < mine) copy_w(i);
+  }
+  pdl_wait();
+  int r0 = 0, rows = a.T;
+  if (a.group_off) {
+    // group number blockIdx.y of those that have rows
+    int left = blockIdx.y, found = -1;
+    for (int z0 = 0; z0 < a.nz && found < 0; z0 += 32) {
+      const int i = z0 + lane, lo = i < a.nz ? a.group_off[i] : 0, hi = i < a.nz ? a.group_off[i + 1] : 0;
+      uint32_t some = __ballot_sync(0xffffffffu, hi > lo);
+      if (left < __popc(some)) {
+        for (; left > 0; --left) some &= some - 1;
+        found = __ffs(some) - 1;
+        z = z0 + found;
+        r0 = __shfl_sync(0xffffffffu, lo, found);
+        rows = __shfl_sync(0xffffffffu, hi, found) - r0;
+      }
+      left -= __popc(some);
+    }
+    if (found < 0) return;                                     // (no copy is under way)
+    rows_of();
+  }
+  const int r = r0 + min(g, rows - 1);
+  const E* xrow = (const E*)a.x + z * a.x_zs + (int64_t)(a.xrows ? a.xrows[r] : r) * a.ldx + t * 8;
+  auto copy_x = [&](int i) {
+    uint4* dst = slot0 + ((i % FEW_S) * PIECES + 2 * NW) * 32;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int k = (warp + i * 8) * 64 + h * 32;
+      copy(dst + h * 32, xrow + k, k + t * 8 < a.K && g < rows);
+    }
+  };
+#pragma unroll
+  for (int i = 0; i < FEW_S - 1; ++i) {
+    if (i < mine) {
+      if (a.group_off) copy_w(i);
+      copy_x(i);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  }
+  float acc[NW][4] = {};
+#pragma unroll 1
+  for (int i = 0; i < mine; ++i) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(FEW_S - 2) : "memory");
+    const uint4* src = slot0 + (i % FEW_S) * PIECES * 32;
+    uint4 wv[NW][2], xv[2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+#pragma unroll
+      for (int j = 0; j < NW; ++j) wv[j][h] = src[(2 * j + h) * 32];
+      xv[h] = src[(2 * NW + h) * 32];
+    }
+    if (i + FEW_S - 1 < mine) { copy_w(i + FEW_S - 1); copy_x(i + FEW_S - 1); }      // into the stage that the previous turn read
+    asm volatile("cp.async.commit_group;" ::: "memory");
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const uint32_t a0[4] = {xv[h].x, 0u, xv[h].y, 0u}, a1[4] = {xv[h].z, 0u, xv[h].w, 0u};
+#pragma unroll
+      for (int j = 0; j < NW; ++j) {
+        mma_bf16_16816(acc[j], a0, wv[j][h].x, wv[j][h].y);
+        mma_bf16_16816(acc[j], a1, wv[j][h].z, wv[j][h].w);
+      }
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < NW; ++j)
+#pragma unroll
+    for (int q = 0; q < 2; ++q) part[warp][g][j * 8 + t * 2 + q] = acc[j][q];
+  __syncthreads();
+  const int row = threadIdx.x >> 3, col = threadIdx.x & 7, n = n0 + col;
+  if (row < rows && n < a.N) {
+    float s1 = 0.f, s2 = 0.f;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) {
+      s1 += part[w][row][col];
+      if (DUAL) s2 += part[w][row][8 + col];
+    }
+    const float sc = a.row_scale ? a.row_scale[r0 + row] : 1.f;
+    const int yr = a.yrows ? a.yrows[r0 + row] : r0 + row;
+    linear_store(a, (O*)a.y + z * a.y_zs + (int64_t)yr * a.ldy + n, a.bias ? (const E*)a.bias + z * a.b_zs : nullptr, n, sc * s1, sc * s2);
+  }
+}
+static bool linear_few_ok(const LinearArgs& a) {
+  return a.elt == KGE_ELT_BF16 && a.T <= FEW_ROWS && a.K % 8 == 0 && a.K >= 64 && a.N <= 32768 && a.ldx % 8 == 0 && a.x_zs % 8 == 0 && a.w_zs % 8 == 0 && a.nz <= 65535 &&
+         ((reinterpret_cast<uintptr_t>(a.x) | reinterpret_cast<uintptr_t>(a.w) | reinterpret_cast<uintptr_t>(a.w2)) & 15) == 0;
+}
+static int launch_linear_few(const LinearArgs& a, cudaStream_t st) {
+  auto kern = a.out_f32 ? (a.w2 ? linear_few_kernel<float, true> : linear_few_kernel<float, false>)
+                        : (a.w2 ? linear_few_kernel<__nv_bfloat16, true> : linear_few_kernel<__nv_bfloat16, false>);
+  const int smem = 8 * FEW_S * 2 * (a.w2 ? 3 : 2) * 512;
+  KGE_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  KGE_CUDA_OK(launch_pdl(kern, dim3((a.N + 7) / 8, a.group_off ? std::min(a.nz, a.T) : a.nz), dim3(256), smem, st, a));
+  return 0;
+}
+
 static bool linear_short_ok(const LinearArgs& a) {
   return a.elt == KGE_ELT_BF16 && a.out_f32 && !a.w2 && !a.group_off && !a.xrows && !a.yrows && !a.row_scale && !a.accumulate && a.nz == 1 && a.T > 256 && a.K % 16 == 0 && a.K <= WMAXK &&
          a.N % 2 == 0 && a.ldy % 2 == 0 && a.ldx % 8 == 0 && (a.T + WBM - 1) / WBM <= 65535 && (a.act == ACT_NONE || a.act == ACT_SOFTPLUS || a.act == ACT_EXP_DECAY) &&
@@ -542,6 +677,7 @@ int linear_any(const LinearArgs& a, cudaStream_t st) {
   KGE_REQUIRE(a.act != ACT_EXP_DECAY || (a.act_coef && !a.w2), "linear_any: the decay needs its coefficients");
   if (a.T <= 0) return 0;
   if (linear_narrow_ok(a)) return a.N <= 8 ? launch_linear_narrow<1>(a, st) : a.N <= 16 ? launch_linear_narrow<2>(a, st) : launch_linear_narrow<4>(a, st);
+  if (linear_few_ok(a)) return launch_linear_few(a, st);
   if (linear_short_ok(a)) {
     const size_t smem = (size_t)(WBM + WBN) * (a.K + MPAD) * 2;
     auto kern = a.act == ACT_SOFTPLUS ? linear_short_kernel<ACT_SOFTPLUS> : a.act == ACT_EXP_DECAY ? linear_short_kernel<ACT_EXP_DECAY> : linear_short_kernel<ACT_NONE>;
@@ -573,18 +709,30 @@ int linear_any(const LinearArgs& a, cudaStream_t st) {
 }
 
 // ------------------------------------------------------------------------------------------------ small row kernels
-template <typename E>
+template <typename E, bool VEC>      // VEC: four columns per thread and pass (the rows of a step are a trip to memory each)
 __global__ void embed_f32_kernel(float* res, const int32_t* ids, const E* table, int d) {
   pdl_launch_dependents();
   pdl_wait();
   const int t = blockIdx.x;
   const E* src = table + (int64_t)ids[t] * d;
+  if (VEC) {
+    for (int c = threadIdx.x * 4; c < d; c += blockDim.x * 4) {
+      float v[4];
+      ld4(src + c, v);
+      st4(res + (int64_t)t * d + c, v);
+    }
+    return;
+  }
   for (int c = threadIdx.x; c < d; c += blockDim.x) res[(int64_t)t * d + c] = ldf(src + c);
 }
 int embed_f32(float* res, const int32_t* ids, const void* table, int T, int d, int elt, cudaStream_t st) {
   if (T <= 0) return 0;
-  cudaError_t ce = elt == KGE_ELT_F32 ? launch_pdl(embed_f32_kernel<float>, dim3(T), dim3(128), 0, st, res, ids, (const float*)table, d)
-                                      : launch_pdl(embed_f32_kernel<__nv_bfloat16>, dim3(T), dim3(128), 0, st, res, ids, (const __nv_bfloat16*)table, d);
+  const bool vec = d % 4 == 0 && ((reinterpret_cast<uintptr_t>(res) | reinterpret_cast<uintptr_t>(table)) & 15) == 0;
+  const dim3 block(vec ? std::min(1024, (d / 4 + 31) / 32 * 32) : 128);
+  cudaError_t ce;
+  if (elt == KGE_ELT_F32) ce = vec ? launch_pdl(embed_f32_kernel<float, true>, dim3(T), block, 0, st, res, ids, (const float*)table, d) : launch_pdl(embed_f32_kernel<float, false>, dim3(T), block, 0, st, res, ids, (const float*)table, d);
+  else ce = vec ? launch_pdl(embed_f32_kernel<__nv_bfloat16, true>, dim3(T), block, 0, st, res, ids, (const __nv_bfloat16*)table, d)
+                : launch_pdl(embed_f32_kernel<__nv_bfloat16, false>, dim3(T), block, 0, st, res, ids, (const __nv_bfloat16*)table, d);
   KGE_CUDA_OK(ce);
   return 0;
 }

@@ -1,0 +1,42 @@
+"""Decode steps of layer-list models: grouped and strided projections of up to 8 rows (linear_few_kernel) and distance-biased attention with
+its keys split over clusters, against the float64 oracle."""
+import pytest
+
+from oracle import hybrid as oh
+from test_hybrid_gpu import check, make_engine, prompt, run_pieces
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("experts,top,width,eff,r_width", [
+    (40, 3, 264, 72, 192),         # groups found in the second 32; K that ends inside a piece; blocks of 64 (one chunk for eight warps)
+    (5, 1, 64, 136, 216),          # K of one chunk; blocks of 72
+    (8, 4, 520, 64, 600),          # two tokens are eight rows, three are more
+    (3, 3, 72, 1000, 768),         # every expert has rows; blocks of 256
+])
+def test_few_rows(kge, tmp_path, experts, top, width, eff, r_width):
+    cfg = oh.make_config(width=width, layers=("parallel", "rglru"), mlps=("moe", "moe"), experts=experts, top=top, expert_ff=eff, r_width=r_width)
+    W = oh.make_weights(cfg, seed=26)        # a choice of experts that rounding to bfloat16 does not turn
+    toks = prompt(cfg, 40)
+    want = oh.forward(cfg, W, toks)
+    llm = make_engine(kge, tmp_path, cfg, W, "bfloat16")
+    check(run_pieces(llm, 0, toks, [1, 2, 3, 4, 7, 8, 9, 1, 1, 1, 1, 2]), want, "bfloat16")
+    llm.close()
+
+
+@pytest.mark.parametrize("chunk,kv,hd,n", [(1024, 2, 64, 1100), (520, 1, 32, 700), (300, 4, 128, 420)])      # clusters of 8, 4 and 2; chunk edges inside
+def test_decode_over_clusters(kge, tmp_path, chunk, kv, hd, n):
+    cfg = oh.make_config(layers=("parallel",), mlps=(None,), right_scale=0.0, chunk=chunk, scale=3.0 / hd ** 0.5, heads=4, kv_heads=kv, dim=hd, vdim=hd)
+    W = oh.make_weights(cfg, seed=31)
+    toks = prompt(cfg, n)
+    want = oh.forward(cfg, W, toks)
+    llm = make_engine(kge, tmp_path, cfg, W, "bfloat16", tokens=2 * n + 64, bs=16)
+    head = max(1, chunk - 3)        # decoding from just before the chunk's end into the next chunk (few keys: most CTAs of a cluster have none)
+    check(run_pieces(llm, 0, toks, [head] + [1] * 12 + [n - head - 32] + [1] * 20), want, "bfloat16", "decoding over the edge")
+    # two requests at once, one of them with a single key
+    llm.trace_add(1, toks)
+    llm.trace_step([(1, n - 1, [])])
+    llm.trace_add(2, toks[:1])
+    got = llm.trace_step([(1, 1, [0]), (2, 1, [0])])
+    llm.close()
+    check(got, want[[n - 1, 0]], "bfloat16", "two requests")
