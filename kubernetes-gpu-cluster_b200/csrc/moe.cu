@@ -15,6 +15,7 @@ namespace kge {
 __device__ __forceinline__ float dot_part(const __nv_bfloat16* h, const __nv_bfloat16* w, int d, int lane, bool vec) {
   float acc = 0.f;
   if (vec) {
+#pragma unroll 8
     for (int k = lane * 8; k < d; k += 256) {
       const uint4 a = *reinterpret_cast<const uint4*>(h + k), b = *reinterpret_cast<const uint4*>(w + k);
       const __nv_bfloat162* a2 = reinterpret_cast<const __nv_bfloat162*>(&a);

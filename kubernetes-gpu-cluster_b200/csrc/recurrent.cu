@@ -38,14 +38,19 @@ __global__ void rglru_conv_kernel(RglruArgs a) {
 }
 
 // The same for bfloat16 rows in 16-byte pieces: a thread takes eight channels of four tokens, so that all its loads (taps x tokens,
-// and the taps' weights once) are in flight together.  Same order of summation.  2312 tokens x 2560: 28 us (43 with a
-// channel per thread and pass), 2 tokens: 10 us (27).
+// and the taps' weights once) are in flight together.  Same order of summation.  2312 tokens x 2560 by 4 taps: 20 us (28 with
+// the taps' weights one by one, 43 with a channel per thread and pass), 2 tokens: 8.6 us (11, 27).
+// TAPS 4: a channel's taps lie side by side, so those of eight channels are 64 bytes, read (like the bias) before the wait; 0: any number.
 constexpr int RC_TOK = 4;
+template <int TAPS>
 __global__ void __launch_bounds__(128) rglru_conv_vec_kernel(RglruArgs a) {
   pdl_launch_dependents();
-  pdl_wait();
   const int c = (blockIdx.y * 128 + threadIdx.x) * 8, t0 = blockIdx.x * RC_TOK;
   if (c >= a.width) return;
+  const int taps = TAPS ? TAPS : a.taps;
+  uint4 wq[TAPS ? TAPS : 1];
+#pragma unroll
+  for (int i = 0; i < TAPS; ++i) wq[i] = *reinterpret_cast<const uint4*>((const __nv_bfloat16*)a.conv_w + (int64_t)c * TAPS + i * 8);
   const __nv_bfloat16* yx = (const __nv_bfloat16*)a.yx + a.width + c;
   float acc[RC_TOK][8], bias[8];
   int back_rows[RC_TOK], back_pos[RC_TOK], p0s[RC_TOK];
@@ -56,6 +61,7 @@ __global__ void __launch_bounds__(128) rglru_conv_vec_kernel(RglruArgs a) {
 #pragma unroll
     for (int i = 0; i < 8; ++i) bias[i] = (i & 1) ? bf_hi(w[i / 2]) : bf_lo(w[i / 2]);
   }
+  pdl_wait();
 #pragma unroll
   for (int k = 0; k < RC_TOK; ++k) {
     const int t = min(t0 + k, a.T - 1), b = a.token_req[t], rs = a.qsl[b];
@@ -67,11 +73,19 @@ __global__ void __launch_bounds__(128) rglru_conv_vec_kernel(RglruArgs a) {
     for (int i = 0; i < 8; ++i) acc[k][i] = bias[i];
   }
 #pragma unroll 4
-  for (int j = 0; j < a.taps; ++j) {
-    const int back = a.taps - 1 - j;
+  for (int j = 0; j < taps; ++j) {
+    const int back = taps - 1 - j;
     float w[8];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) w[i] = ldf((const __nv_bfloat16*)a.conv_w + (int64_t)(c + i) * a.taps + j);
+    for (int i = 0; i < 8; ++i) {
+      if (TAPS) {
+        const uint32_t q[4] = {wq[(i * TAPS + j) / 8 % (TAPS ? TAPS : 1)].x, wq[(i * TAPS + j) / 8 % (TAPS ? TAPS : 1)].y, wq[(i * TAPS + j) / 8 % (TAPS ? TAPS : 1)].z, wq[(i * TAPS + j) / 8 % (TAPS ? TAPS : 1)].w};
+        const uint32_t pair = q[(i * TAPS + j) % 8 / 2];
+        w[i] = (j & 1) ? bf_hi(pair) : bf_lo(pair);
+      } else {
+        w[i] = ldf((const __nv_bfloat16*)a.conv_w + (int64_t)(c + i) * taps + j);
+      }
+    }
 #pragma unroll
     for (int k = 0; k < RC_TOK; ++k) {
       const int sp = back_pos[k] - back;
@@ -83,7 +97,7 @@ __global__ void __launch_bounds__(128) rglru_conv_vec_kernel(RglruArgs a) {
         for (int i = 0; i < 8; ++i) x[i] = (i & 1) ? bf_hi(u[i / 2]) : bf_lo(u[i / 2]);
       } else {
 #pragma unroll
-        for (int i = 0; i < 8; ++i) x[i] = sp >= 0 ? tails[k][(int64_t)(sp - p0s[k] + a.taps - 1) * a.width + i] : 0.f;
+        for (int i = 0; i < 8; ++i) x[i] = sp >= 0 ? tails[k][(int64_t)(sp - p0s[k] + taps - 1) * a.width + i] : 0.f;
       }
 #pragma unroll
       for (int i = 0; i < 8; ++i) acc[k][i] = fmaf(w[i], x[i], acc[k][i]);
@@ -102,7 +116,8 @@ int rglru_conv(const RglruArgs& a, cudaStream_t st) {
   // few rows of few channels leave its threads a chain of loads each where the other kernel has a thread for every channel (64 rows of
   // 64 channels 5.1 us here and 2.6 there, of 264 5.6 and 3.6; 64 of 1024 6.3 and 6.1, 256 of 1024 6.4 and 7.0, 2312 of 64 4.3 and 4.7)
   if (a.elt == KGE_ELT_BF16 && (a.width >= 1024 || a.T > 1024) && a.width % 8 == 0 && ((reinterpret_cast<uintptr_t>(a.yx) | reinterpret_cast<uintptr_t>(a.u) | reinterpret_cast<uintptr_t>(a.conv_b)) & 15) == 0) {
-    KGE_CUDA_OK(launch_pdl(rglru_conv_vec_kernel, dim3((a.T + RC_TOK - 1) / RC_TOK, (a.width / 8 + 127) / 128), dim3(128), 0, st, a));
+    auto kern = a.taps == 4 && (reinterpret_cast<uintptr_t>(a.conv_w) & 15) == 0 ? rglru_conv_vec_kernel<4> : rglru_conv_vec_kernel<0>;
+    KGE_CUDA_OK(launch_pdl(kern, dim3((a.T + RC_TOK - 1) / RC_TOK, (a.width / 8 + 127) / 128), dim3(128), 0, st, a));
     return 0;
   }
   cudaError_t ce = a.elt == KGE_ELT_F32 ? launch_pdl(rglru_conv_kernel<float>, dim3(a.T), dim3(256), 0, st, a)
