@@ -477,6 +477,19 @@ static cudaError_t launch_bias_split(dim3 grid, int S, size_t smem, cudaStream_t
   return cudaLaunchKernelEx(&cfg, attn_bias_mma_kernel<false>, a, req0);
 }
 
+inline namespace KGE_ELT_NS {
+int paged_attn_bias_pair(void* out, int ldo, const void* q, int ldq, const void* kc, const void* vc, const int32_t* bt, int max_blocks, const int32_t* sl,
+                         const int32_t* qsl, int B, int T, int max_q_len, int H, int KV, int hd, int bs, float scale, int chunk, float span, float out_scale, cudaStream_t st);      // attn_tc.cu
+}
+// What the tcgen05 kernel of attn_pair.cuh takes: plain chunked attention with distance biases, keys and values of 64 or 128, pages of a
+// power of two of at least 8 tokens, aligned rows.  Two prompts of 1150 tokens, 16 / 4 heads of 128 in chunks of 1024: 162 us in the
+// kernel above, 34 there.
+static bool bias_pair_ok(const AttnBiasArgs& a) {
+  return a.elt == KGE_ELT_BF16 && (a.dim == 64 || a.dim == 128) && a.vdim == a.dim && (a.v_ld == 0 || a.v_ld == a.vdim) && a.softcap == 0.f && !a.sinks && a.window == 0 &&
+         a.seq_lens && a.H % a.G == 0 && a.H / a.G <= 128 && a.block_size >= 8 && (a.block_size & (a.block_size - 1)) == 0 && a.ldq % 8 == 0 && a.ldo % 8 == 0 && a.scale > 0.f &&
+         ((reinterpret_cast<uintptr_t>(a.q) | reinterpret_cast<uintptr_t>(a.out) | reinterpret_cast<uintptr_t>(a.k_cache) | reinterpret_cast<uintptr_t>(a.v_cache)) & 15) == 0;
+}
+
 int attn_bias_chunk(const AttnBiasArgs& a, cudaStream_t st) {
   if (a.T <= 0) return 0;
   KGE_REQUIRE(a.window >= 0 && (a.window > 0 || (a.keep_first == 0 && a.pool == 0)) && !(a.keep_first > 0 && a.pool > 0) && (a.window == 0 || a.bias_span == 0.f) &&
@@ -501,6 +514,9 @@ int attn_bias_chunk(const AttnBiasArgs& a, cudaStream_t st) {
       const int S = bias_cluster((int64_t)((hpg + 15) / 16) * a.G * D, reach / AM_KT);
       KGE_CUDA_OK(launch_bias_split(dim3((hpg + 15) / 16, a.G, D), S, S > 1 ? split + sums : split, st, a, 0));
     }
+    if (D < a.B && a.max_q * hpg > 32 && bias_pair_ok(a))
+      return paged_attn_bias_pair(a.out, a.ldo, a.q, a.ldq, a.k_cache, a.v_cache, a.block_table + (int64_t)D * a.max_blocks, a.max_blocks, a.seq_lens + D, a.qsl + D, a.B - D, a.T - D,
+                                  a.max_q, a.H, a.G, a.dim, a.block_size, a.scale, a.chunk, a.bias_span, a.out_scale, st);
     if (D < a.B) {
       const int rows = a.max_q * hpg;
       const bool wide = rows > 32 && a.ldo % 2 == 0 && a.vdim % 2 == 0 && (reinterpret_cast<uintptr_t>(a.out) & 3) == 0;

@@ -27,7 +27,12 @@ template <int HD> constexpr int pair_smem() { return (2 * 128 + 2 * kPairStages 
 
 // n0, n1: key tiles of the two query tiles; n1 < 0: no more work.  split: there is one query tile, the even key tiles are the first
 // one's and the odd ones the second one's.
-struct __align__(16) Item { int q0, tok0, ntok0, ntok1, ctx0, kvh, n0, n1, split; };
+struct __align__(16) Item { int q0, tok0, ntok0, ntok1, ctx0, kvh, n0, n1, split, tile_lo; };
+
+// Outputs `ldo` apart and multiplied by out_scale.  BIAS kernels: a query at position i sees the keys j of its own chunk (chunk > 0; all up to i
+// otherwise) with -slope (i - j) added to the scaled score, slope 2^(-span (head + 1) / H) (span > 0).  What is the same for a whole row drops
+// out of the softmax but for the growth of its maximum, so distances are counted from the row's own position.
+struct PairArgs { int ldo; float out_scale; int chunk; float span; };
 
 __device__ __forceinline__ void tmem_ld32_nowait(uint32_t taddr, uint32_t* r) {
   asm volatile(
@@ -58,13 +63,13 @@ __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map
   asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
                ::"r"(dst), "l"(map), "r"(bar), "r"(c0), "r"(c1), "r"(c2) : "memory");
 }
-template <int HD>
+template <int HD, bool BIAS>
 __global__ void __launch_bounds__(kPairThreads, 1)
 attn_pair_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_q8,
                  const __grid_constant__ CUtensorMap tm_q1, bf16* __restrict__ out, const bf16* __restrict__ k_cache, const bf16* __restrict__ v_cache,
                  const int32_t* __restrict__ block_table, int max_blocks,
                  const int32_t* __restrict__ seq_lens, const int32_t* __restrict__ qsl, int flat, int per, int H, int KV, int bs_shift, float scale_log2,
-                 const float* __restrict__ sinks) {
+                 const float* __restrict__ sinks, const PairArgs pa) {
   constexpr int NST = kPairStages;
   constexpr uint32_t Q_TILE = 128 * HD * 2, TILE = BNK * HD * 2;
   // TMEM: O0 and O1, then per query tile the scores (64 columns) and two buffers of probabilities (32 columns each)
@@ -172,13 +177,15 @@ attn_pair_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant
       if (tok0 >= 0) {
         const int ctx0 = seq_len - q_len;
         const int ntok0 = min(TT, q_len - tok0), ntok1 = max(0, min(TI - TT, q_len - tok0 - TT));
-        const int kv_len = ctx0 + tok0 + ntok0 + ntok1, n = (kv_len + BNK - 1) / BNK, split = ntok1 == 0 && n > 1;
-        const int n0 = split ? (n + 1) / 2 : (ctx0 + tok0 + ntok0 + BNK - 1) / BNK, n1 = split ? n / 2 : (ntok1 ? n : 0);
+        const int kv_len = ctx0 + tok0 + ntok0 + ntok1;
+        const int tile_lo = BIAS && pa.chunk > 0 ? (ctx0 + tok0) / pa.chunk * pa.chunk / BNK : 0;      // where the first query's chunk begins
+        const int n = (kv_len + BNK - 1) / BNK - tile_lo, split = ntok1 == 0 && n > 1;
+        const int n0 = split ? (n + 1) / 2 : (ctx0 + tok0 + ntok0 + BNK - 1) / BNK - tile_lo, n1 = split ? n / 2 : (ntok1 ? n : 0);
         const int slot = ni & 1;
         if (ni >= 2) mbar_wait(item_empty(slot), ((ni >> 1) - 1) & 1);
         if (leader) {
           Item it;
-          it.q0 = q0; it.tok0 = tok0; it.ntok0 = ntok0; it.ntok1 = ntok1; it.ctx0 = ctx0; it.kvh = kvh; it.n0 = n0; it.n1 = n1; it.split = split;
+          it.q0 = q0; it.tok0 = tok0; it.ntok0 = ntok0; it.ntok1 = ntok1; it.ctx0 = ctx0; it.kvh = kvh; it.n0 = n0; it.n1 = n1; it.split = split; it.tile_lo = tile_lo;
           items[slot] = it;
           mbar_arrive(item_full(slot));
         }
@@ -237,8 +244,8 @@ attn_pair_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant
         }
         __syncwarp();
         for (int j = 0; j < n; ++j) {
-          fetch(j, true);
-          fetch(j, false);
+          fetch(tile_lo + j, true);
+          fetch(tile_lo + j, false);
           ++nk;
         }
         hand_over(0);
@@ -346,6 +353,9 @@ attn_pair_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant
       const bool row_ok = tk < (qt ? it.ntok1 : it.ntok0);
       const int row_tok = it.tok0 + qt * TT + tk;
       const int lim = row_ok ? it.ctx0 + row_tok : -1;                 // last visible key of this row
+      const int head = it.kvh * G + hh;
+      const int lo_row = BIAS && row_ok && pa.chunk > 0 ? lim / pa.chunk * pa.chunk : 0;      // its first key
+      const float slope2 = BIAS && pa.span > 0.f ? exp2f(-pa.span * (float)(head + 1) / (float)H) * kLog2e : 0.f;
       float m_ref = -INFINITY, l = 0.f;
       // the second group's exponentials start when the first's of its first tile are done.  From three tiles of the second group on: then
       // the first group cannot come to its next item's handshake before the second has passed this one (it needs Q, which waits for the
@@ -361,17 +371,26 @@ attn_pair_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant
         tc_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(s_read(a));                         // the next tile's scores may be written
-        const int vis = lim - (it.split ? 2 * j + a : j) * BNK;        // columns 0 .. vis are visible
+        const int kbase = (it.tile_lo + (it.split ? 2 * j + a : j)) * BNK, vis = lim - kbase, from = lo_row - kbase;      // columns from .. vis are visible
         float mxa[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
-        if (!__all_sync(0xffffffffu, vis >= BNK - 1)) {
+        if (BIAS) {
+          const f2 sl2 = pk(slope2, slope2), b2 = pk(-slope2 * (float)vis, -slope2 * (float)vis);
 #pragma unroll
-          for (int i = 0; i < BNK; ++i) sv[i] = i <= vis ? sv[i] : 0xff800000u;
+          for (int i = 0; i < BNK; i += 2) {
+            float x0, x1;
+            upk(fma2(pk(__uint_as_float(sv[i]), __uint_as_float(sv[i + 1])), sc2, fma2(pk((float)i, (float)(i + 1)), sl2, b2)), x0, x1);
+            sv[i] = __float_as_uint(x0); sv[i + 1] = __float_as_uint(x1);
+          }
+        }
+        if (!__all_sync(0xffffffffu, vis >= BNK - 1 && (!BIAS || from <= 0))) {
+#pragma unroll
+          for (int i = 0; i < BNK; ++i) sv[i] = i <= vis && (!BIAS || i >= from) ? sv[i] : 0xff800000u;
         }
 #pragma unroll
         for (int i = 0; i < BNK; i += 8)
 #pragma unroll
           for (int k = 0; k < 4; ++k) mxa[k] = max3(mxa[k], __uint_as_float(sv[i + 2 * k]), __uint_as_float(sv[i + 2 * k + 1]));
-        const float mx = max3(fmaxf(mxa[0], mxa[1]), mxa[2], mxa[3]) * scale_log2;      // -inf stays -inf
+        const float mx = max3(fmaxf(mxa[0], mxa[1]), mxa[2], mxa[3]) * (BIAS ? 1.f : scale_log2);      // -inf stays -inf
         const bool grow = mx > m_ref + kRescaleThreshold;              // includes the first finite maximum
         if (__any_sync(0xffffffffu, grow)) {
           float alpha = 1.f;
@@ -408,7 +427,8 @@ attn_pair_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant
 #pragma unroll
           for (int i = 0; i < 16; ++i) {
             float p0, p1;
-            upk(fma2(pk(__uint_as_float(sv[c + 2 * i]), __uint_as_float(sv[c + 2 * i + 1])), sc2, nb2), p0, p1);
+            const f2 x = pk(__uint_as_float(sv[c + 2 * i]), __uint_as_float(sv[c + 2 * i + 1]));
+            upk(BIAS ? add2(x, nb2) : fma2(x, sc2, nb2), p0, p1);
             p0 = ex2_ftz(p0); p1 = ex2_ftz(p1);                        // masked: -inf -> 0
             rs[i & 1] = add2(rs[i & 1], pk(p0, p1));
             pkd[i] = pack_bf2(p0, p1);
@@ -425,7 +445,6 @@ attn_pair_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant
       }
       mbar_wait(o_full(a, ns - 1), ((ns - 1) >> 1) & 1);
       tc_after();
-      const int head = it.kvh * G + hh;
       float2* part = reinterpret_cast<float2*>(smem_raw + 2 * Q_TILE + 2 * NST * TILE + 512 + 8 * 4096);
       float mine = 1.f, other = 0.f;                                   // weights of the two halves of a split row
       if (it.split) {
@@ -445,7 +464,7 @@ attn_pair_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant
         }
       }
       if (sinks && row_ok && m_ref != -INFINITY) l += exp2f(sinks[head] * kLog2e - m_ref);
-      const float inv = l > 0.f ? 1.f / l : 0.f;
+      const float inv = l > 0.f ? pa.out_scale / l : 0.f;
       // a warp turns its 32 rows in shared memory, 64 columns at a time, and stores 128 contiguous bytes of four rows at once (16 bytes
       // of each row by its own thread: a third of the time of a short item)
       uint8_t* stage = smem_raw + 2 * Q_TILE + 2 * NST * TILE + 512 + warp * 4096;
@@ -484,7 +503,7 @@ attn_pair_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant
           const int row = i + srow, rr = (warp & 3) * 32 + row, t2 = rr / G;
           const uint4 w = *reinterpret_cast<const uint4*>(stage + row * 128 + ((schunk ^ (row & 7)) << 4));
           if ((rows_ok >> row) & 1)
-            *reinterpret_cast<uint4*>(out + (int64_t)(it.q0 + it.tok0 + qt * TT + t2) * H * HD + (it.kvh * G + rr - t2 * G) * HD + c + schunk * 8) = w;
+            *reinterpret_cast<uint4*>(out + (int64_t)(it.q0 + it.tok0 + qt * TT + t2) * pa.ldo + (it.kvh * G + rr - t2 * G) * HD + c + schunk * 8) = w;
         }
       }
       if (it.split) {                                                  // O1 and the sums are read
@@ -504,8 +523,8 @@ attn_pair_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant
 int make_tmap(CUtensorMap* m, const void* ptr, int64_t rows, int64_t cols, int box_rows);   // gemm_tc.cu (cached)
 int encode_tmap_q(CUtensorMap* m, const void* ptr, int64_t stride, int hd, int heads, int box_heads, int box_tokens);     // gemm_tc.cu
 
-template <int HD>
-static int launch_pair(bf16* out, const bf16* q, int q_stride, const bf16* kc, const bf16* vc, const int32_t* bt, int max_blocks, const int32_t* sl,
+template <int HD, bool BIAS>
+static int launch_pair(const atc2::PairArgs& pa, bf16* out, const bf16* q, int q_stride, const bf16* kc, const bf16* vc, const int32_t* bt, int max_blocks, const int32_t* sl,
                        const int32_t* qsl, int B, int T, int max_q_len, int max_seq_len, int H, int KV, int bs, int bs_shift, float scale, const float* sinks, cudaStream_t st) {
   const int G = H / KV, TT = atc::BM / G, box_rows = bs < atc::BNK ? bs : atc::BNK;
   // Query tiles per item: two, sharing the K and V tiles (us with two / one and its key tiles split: 4 x 2048 tokens 125 / 169, two of
@@ -527,9 +546,9 @@ static int launch_pair(bf16* out, const bf16* q, int q_stride, const bf16* kc, c
   if (int rc = encode_tmap_q(&tq8, q, q_stride, HD, H, G, TT >= 8 ? 8 : 1)) return rc;
   if (int rc = encode_tmap_q(&tq1, q, q_stride, HD, H, G, 1)) return rc;
   if (!tunable(TUN_ATTN_TMA)) { gk = kc; gv = vc; }
-  auto kern = atc2::attn_pair_kernel<HD>;
+  auto kern = atc2::attn_pair_kernel<HD, BIAS>;
   KGE_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, atc2::pair_smem<HD>()));
   KGE_CUDA_OK(launch_pdl(kern, grid, dim3(atc2::kPairThreads), atc2::pair_smem<HD>(), st, tk, tv, tq8, tq1, out, gk, gv, bt, max_blocks, sl, qsl, by_request ? B : 0, per, H, KV,
-                         bs_shift, scale * atc::kLog2e, sinks));
+                         bs_shift, scale * atc::kLog2e, sinks, pa));
   return 0;
 }

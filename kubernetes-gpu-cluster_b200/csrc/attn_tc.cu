@@ -537,7 +537,7 @@ static int launch_tc(bf16* out, const bf16* q, int q_stride, const bf16* kc, con
   // TMEM and 226 KB start later than two of these CTAs per SM (us here / there: 8 x 128 tokens 10.3 / 11.4, 2 x 300 10.3 / 11.5, 64 tokens
   // 5.6 / 7.0; but 8 x 300 26.5 / 23.3, one of 512 14.2 / 11.3; 32 / 8 heads of 128).
   if (bs >= 8 && !cap && B <= 65535 && !(max_seq_len <= 320 && (int64_t)T * KV <= 256 * TT))
-    return launch_pair<HD>(out, q, q_stride, kc, vc, bt, max_blocks, sl, qsl, B, T, max_q_len, max_seq_len, H, KV, bs, bs_shift, scale, sinks, st);
+    return launch_pair<HD, false>(atc2::PairArgs{H * HD, 1.f, 0, 0.f}, out, q, q_stride, kc, vc, bt, max_blocks, sl, qsl, B, T, max_q_len, max_seq_len, H, KV, bs, bs_shift, scale, sinks, st);
   if (tma) {
     const int box_rows = bs < atc::BNK ? bs : atc::BNK;
     const int64_t rows = (int64_t)1 << 30;      // the pool's extent is not known here; it only bounds out-of-range handling, never relied on
@@ -614,6 +614,20 @@ int paged_attn_prefill_tc(bf16* out, const bf16* q, int q_stride, const bf16* kc
   if (hd == 128) return launch_tc<128>(out, q, q_stride, kc, vc, bt, max_blocks, sl, qsl, B, T, max_q_len, max_seq_len, H, KV, bs, scale, softcap, sinks, st);
   return launch_tc<64>(out, q, q_stride, kc, vc, bt, max_blocks, sl, qsl, B, T, max_q_len, max_seq_len, H, KV, bs, scale, softcap, sinks, st);
 }
+
+#ifndef KGE_HALF
+// Prompts of a distance-biased, chunked attention (attn_bias.cu) with keys and values of 64 or 128, in the pair kernel.
+int paged_attn_bias_pair(void* out, int ldo, const void* q, int ldq, const void* kc, const void* vc, const int32_t* bt, int max_blocks, const int32_t* sl,
+                         const int32_t* qsl, int B, int T, int max_q_len, int H, int KV, int hd, int bs, float scale, int chunk, float span, float out_scale, cudaStream_t st) {
+  int bs_shift = 0;
+  while ((1 << bs_shift) < bs) ++bs_shift;
+  const atc2::PairArgs pa{ldo, out_scale, chunk, span};
+  const int64_t reach = (int64_t)max_blocks * bs;
+  const int seen = (int)(chunk > 0 && chunk < reach ? chunk : reach);
+  auto run = hd == 128 ? launch_pair<128, true> : launch_pair<64, true>;
+  return run(pa, (bf16*)out, (const bf16*)q, ldq, (const bf16*)kc, (const bf16*)vc, bt, max_blocks, sl, qsl, B, T, max_q_len, seen, H, KV, bs, bs_shift, scale, nullptr, st);
+}
+#endif
 
 }  // namespace KGE_ELT_NS
 }  // namespace kge

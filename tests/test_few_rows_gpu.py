@@ -1,5 +1,5 @@
-"""Decode steps of layer-list models: grouped and strided projections of up to 8 rows (linear_few_kernel) and distance-biased attention with
-its keys split over clusters, against the float64 oracle."""
+"""Small steps of layer-list models: grouped and strided projections of up to 8 rows (linear_few_kernel), distance-biased attention with
+its keys split over clusters and (64 and 128 wide, prompts) in the tcgen05 kernel, against the float64 oracle."""
 import pytest
 
 from oracle import hybrid as oh
@@ -24,7 +24,7 @@ def test_few_rows(kge, tmp_path, experts, top, width, eff, r_width):
     llm.close()
 
 
-@pytest.mark.parametrize("chunk,kv,hd,n", [(1024, 2, 64, 1100), (520, 1, 32, 700), (300, 4, 128, 420)])      # clusters of 8, 4 and 2; chunk edges inside
+@pytest.mark.parametrize("chunk,kv,hd,n", [(1024, 2, 64, 1100), (520, 1, 32, 700), (300, 4, 128, 420), (200, 1, 128, 450)])      # clusters of 8, 4, 2 and 1; chunk edges inside pieces
 def test_decode_over_clusters(kge, tmp_path, chunk, kv, hd, n):
     cfg = oh.make_config(layers=("parallel",), mlps=(None,), right_scale=0.0, chunk=chunk, scale=3.0 / hd ** 0.5, heads=4, kv_heads=kv, dim=hd, vdim=hd)
     W = oh.make_weights(cfg, seed=31)
