@@ -848,6 +848,7 @@ int hybrid_forward(kge_engine* e, int T, int B, int R, int max_blocks, const Ste
     if (hyper) { if (!hx_ready) HFWD(C_NORM, Td * (4.0 * S + es), 0, stream_read(e->hx, L.hc_in[0], nullptr, L.norm1, T, 1.f, nullptr)); hx_ready = false; }
     else if (!hx_ready) HFWD(C_NORM, Td * (4 + es), 0, layer_norm(e->hx, nullptr, L.norm1, T, 1.f));
     hx_ready = false;
+    bool pair_ready = false;                           // the mixer's write of the stream formed the feed-forward's normed input
     CombineArgs cb;
     const void* inner_w[2] = {nullptr, nullptr};      // a norm of a source's own before the sources are summed (models with normed results)
     const void* pair_src = nullptr;                    // the experts' rows a post-norm model gathers by (token, choice) pair
@@ -899,11 +900,19 @@ int hybrid_forward(kge_engine* e, int T, int B, int R, int max_blocks, const Ste
         cb = CombineArgs(); inner_w[0] = inner_w[1] = nullptr;
         return dyt_combine(da, st);
       }
-      if (!hyper) return flush_more();
+      const bool mixer_done = sub == 0 && h.mlp != HybridLayerSpec::NONE;
+      if (!hyper) {
+        const bool before_ff = mixer_done && s.hyb_prenorm_pair;
+        const void* next = before_ff ? L.norm2 : i + 1 < s.L ? e->hyb[i + 1].norm1 : nullptr;
+        if (!next || !combine_norm_ok(e->res32, cb, e->hx, next, d)) return flush_more();
+        (before_ff ? pair_ready : hx_ready) = true;
+        const int rc = combine_norm(e->res32, cb, e->hx, next, T, d, s.eps, s.hyb_layernorm, elt, st);
+        cb = CombineArgs();
+        return rc;
+      }
       StreamCombineArgs sc;
       sc.xs = e->res32; sc.src = cb; sc.y32 = y32_used ? e->y32 : nullptr; sc.col_scale = L.col_scale[sub]; sc.mix = L.hc_mix[sub]; sc.out_w = L.hc_out[sub];
       sc.mult = s.residual_mult; sc.T = T; sc.d = d; sc.S = S; sc.elt = elt; sc.eps = s.eps;
-      const bool mixer_done = sub == 0 && h.mlp != HybridLayerSpec::NONE;
       if (mixer_done) { sc.next_in = L.hc_in[1]; sc.next_w = L.norm2; sc.next_y = e->hx; }
       else if (i + 1 < s.L) { sc.next_in = e->hyb[i + 1].hc_in[0]; sc.next_w = e->hyb[i + 1].norm1; sc.next_y = e->hx; hx_ready = true; }
       cb = CombineArgs(); y32_used = false;
@@ -1318,7 +1327,7 @@ int hybrid_forward(kge_engine* e, int T, int B, int R, int max_blocks, const Ste
       // the feed-forward reads a norm of the stream that already holds the mixer's output
       { const double nsrc = cb.n + (s.hyb_postnorm || s.hyb_dyt ? 1 : 0); HFWD(C_ACT, Td * (8.0 * S + nsrc * es), 0, flush()); }      // post-norm models also write the next normed row
       sub = 1;
-      if (!hyper && !s.hyb_postnorm && !s.hyb_dyt) HFWD(C_NORM, Td * (4 + es), 0, layer_norm(e->hx, nullptr, L.norm2, T, 1.f));
+      if (!hyper && !s.hyb_postnorm && !s.hyb_dyt && !pair_ready) HFWD(C_NORM, Td * (4 + es), 0, layer_norm(e->hx, nullptr, L.norm2, T, 1.f));
     }
     if (h.mlp == HybridLayerSpec::DENSE && h.ff_silu_bias) {
       // silu(gate h + b) * (up h + b): one product over [gate | up] with the biases, the pair formed from its rows

@@ -95,6 +95,9 @@ struct CombineArgs {
   int n = 0;
 };
 int residual_combine(float* res, const CombineArgs& a, int T, int d, int elt, cudaStream_t st);
+// residual_combine, and y = the RMS norm (weight 1 + w) or weight-only layer norm of the new rows, in one pass
+bool combine_norm_ok(const float* res, const CombineArgs& a, const void* y, const void* w, int d);
+int combine_norm(float* res, const CombineArgs& a, void* y, const void* w, int T, int d, float eps, bool layer_norm, int elt, cudaStream_t st);
 // RMS norm in groups: the row is cut into `groups` equal consecutive parts, each divided by its own
 // sqrt(mean(part^2) + eps); the whole is multiplied by w (as it is) and out_scale.  x fp32, y in elt.
 int group_rmsnorm_f32in(void* y, const float* x, const int32_t* rows, const void* w, int R, int d, int groups, float eps, float out_scale, int elt,

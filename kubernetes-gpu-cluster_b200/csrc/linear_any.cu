@@ -956,6 +956,89 @@ int residual_combine(float* res, const CombineArgs& a, int T, int d, int elt, cu
   return 0;
 }
 
+// The sum above and the next sublayer's norm of the new row in one pass: the row stays in registers, so it is not read back, and the loads of
+// all sources are under way together.  The same arithmetic as residual_combine and norm_f32in_vec_kernel one after the other.
+// NV: four-column pieces per thread.  2312 rows of 2048, one to four sources: 36 us in two launches, 16 here.
+template <typename E, bool LN, int NV>
+__global__ void __launch_bounds__(256) combine_norm_kernel(float* res, CombineArgs a, E* y, const E* w, int d, float eps, float offset) {
+  pdl_launch_dependents();
+  __shared__ float red[33];
+  const int64_t t = blockIdx.x;
+  const int nvec = d >> 2;
+  float4 g[NV];
+#pragma unroll
+  for (int i = 0; i < NV; ++i) {
+    const int c = threadIdx.x + i * 256;
+    if (c < nvec) g[i] = ldw4(w + 4 * c);
+  }
+  pdl_wait();
+  float4* row = reinterpret_cast<float4*>(res + t * d);
+  float4 v[NV], src[4][NV];
+  float f[4];
+#pragma unroll
+  for (int i = 0; i < NV; ++i) {
+    const int c = threadIdx.x + i * 256;
+    v[i] = c < nvec ? row[c] : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      if (k < a.n && c < nvec) src[k][i] = ldw4((const E*)a.src[k] + t * a.ld[k] + 4 * c);
+  }
+#pragma unroll
+  for (int k = 0; k < 4; ++k) f[k] = k < a.n ? (a.rscale[k] ? a.scale[k] * a.rscale[k][t * a.rs_stride[k]] : a.scale[k]) : 0.f;
+  float s = 0.f;
+#pragma unroll
+  for (int i = 0; i < NV; ++i) {
+    const int c = threadIdx.x + i * 256;
+    if (c < nvec) {
+      float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        if (k < a.n) {
+          const float4 x = src[k][i];
+          o.x = fmaf(f[k], x.x, o.x); o.y = fmaf(f[k], x.y, o.y); o.z = fmaf(f[k], x.z, o.z); o.w = fmaf(f[k], x.w, o.w);
+        }
+      v[i].x += o.x; v[i].y += o.y; v[i].z += o.z; v[i].w += o.w;
+      row[c] = v[i];
+    }
+    if (LN) s += (v[i].x + v[i].y) + (v[i].z + v[i].w);
+  }
+  float mean = 0.f;
+  if (LN) { mean = block_sum(s, red) / (float)d; __syncthreads(); }
+  float ss = 0.f;
+#pragma unroll
+  for (int i = 0; i < NV; ++i)
+    if (threadIdx.x + i * 256 < nvec) {
+      v[i].x -= mean; v[i].y -= mean; v[i].z -= mean; v[i].w -= mean;
+      ss = fmaf(v[i].x, v[i].x, ss); ss = fmaf(v[i].y, v[i].y, ss); ss = fmaf(v[i].z, v[i].z, ss); ss = fmaf(v[i].w, v[i].w, ss);
+    }
+  ss = block_sum(ss, red);
+  const float inv = 1.f / sqrtf(ss / (float)d + eps);
+#pragma unroll
+  for (int i = 0; i < NV; ++i) {
+    const int c = threadIdx.x + i * 256;
+    if (c < nvec)
+      st4(y + t * d + 4 * c, make_float4(v[i].x * inv * (offset + g[i].x), v[i].y * inv * (offset + g[i].y), v[i].z * inv * (offset + g[i].z), v[i].w * inv * (offset + g[i].w)));
+  }
+}
+template <typename E, bool LN>
+static cudaError_t launch_combine_norm(float* res, const CombineArgs& a, void* y, const void* w, int T, int d, float eps, float offset, cudaStream_t st) {
+  auto kern = d <= 1024 ? combine_norm_kernel<E, LN, 1> : d <= 2048 ? combine_norm_kernel<E, LN, 2> : combine_norm_kernel<E, LN, 4>;
+  return launch_pdl(kern, dim3(T), dim3(256), 0, st, res, a, (E*)y, (const E*)w, d, eps, offset);
+}
+bool combine_norm_ok(const float* res, const CombineArgs& a, const void* y, const void* w, int d) {
+  bool ok = a.n > 0 && d % 4 == 0 && d <= 4096 && ((reinterpret_cast<uintptr_t>(res) | reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(w)) & 15) == 0;
+  for (int k = 0; k < a.n; ++k) ok = ok && a.ld[k] % 4 == 0 && (reinterpret_cast<uintptr_t>(a.src[k]) & 15) == 0;
+  return ok;
+}
+int combine_norm(float* res, const CombineArgs& a, void* y, const void* w, int T, int d, float eps, bool layer_norm, int elt, cudaStream_t st) {
+  KGE_REQUIRE(combine_norm_ok(res, a, y, w, d), "combine_norm: sizes");
+  if (T <= 0) return 0;
+  // RMS weights apply as 1 + w, those of the layer norm as they are
+  KGE_CUDA_OK(elt == KGE_ELT_F32 ? (layer_norm ? launch_combine_norm<float, true>(res, a, y, w, T, d, eps, 0.f, st) : launch_combine_norm<float, false>(res, a, y, w, T, d, eps, 1.f, st))
+                                 : (layer_norm ? launch_combine_norm<__nv_bfloat16, true>(res, a, y, w, T, d, eps, 0.f, st) : launch_combine_norm<__nv_bfloat16, false>(res, a, y, w, T, d, eps, 1.f, st)));
+  return 0;
+}
+
 __global__ void logits_to_elt16_kernel(uint16_t* out, const float* in, int R, int V, int ld, bool f16) {
   pdl_launch_dependents();
   pdl_wait();

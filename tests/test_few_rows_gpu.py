@@ -40,3 +40,15 @@ def test_decode_over_clusters(kge, tmp_path, chunk, kv, hd, n):
     got = llm.trace_step([(1, 1, [0]), (2, 1, [0])])
     llm.close()
     check(got, want[[n - 1, 0]], "bfloat16", "two requests")
+
+
+@pytest.mark.parametrize("width", [1024, 1028, 2048, 2052, 4096, 4100])
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+def test_sum_and_norm_by_width(kge, tmp_path, dtype, width):
+    """The stream's sum and the next layer's norm in one pass: each number of pieces per thread, the first width beyond it."""
+    cfg = oh.make_config(width=width, layers=("rglru", "rglru", "rglru"), mlps=("dense", "moe", None), experts=3, top=3)
+    W = oh.make_weights(cfg, seed=5)
+    toks = prompt(cfg, 11)
+    llm = make_engine(kge, tmp_path, cfg, W, dtype)
+    check(run_pieces(llm, 0, toks, [9, 1, 1]), oh.forward(cfg, W, toks), dtype)
+    llm.close()
