@@ -368,7 +368,8 @@ __global__ void __launch_bounds__(256) linear_stream_kernel(LinearArgs a) {
 
 // Many rows, a short sum, fp32 output (the second half of a low-rank pair): the output is the traffic.  128 x 128 tiles whose operands
 // are staged whole (K <= 256) with cp.async; eight warps of 64 rows x 32 outputs, fragments by ldmatrix, the same order of summation
-// as above, two outputs per store.
+// as above, two outputs per store.  Strided slices (block-diagonal gates) are the grid's third dimension: 2312 rows by 16 blocks of 160 x 160
+// 38 us in the 64-row tiles of linear_mma_kernel, 23 here.
 constexpr int WBM = 128, WBN = 128, WMAXK = 256;
 
 __device__ __forceinline__ void la_ldsm4(uint32_t (&r)[4], const void* p) {
@@ -384,13 +385,14 @@ __global__ void __launch_bounds__(256) linear_short_kernel(LinearArgs a) {
   const int pitch = a.K + MPAD, pieces = a.K / 8;
   E* xs = reinterpret_cast<E*>(lw_raw);                       // [WBM][pitch]
   E* ws = xs + WBM * pitch;                                   // [WBN][pitch]
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, m0 = blockIdx.y * WBM, n0 = blockIdx.x * WBN;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, m0 = blockIdx.y * WBM, n0 = blockIdx.x * WBN, z = blockIdx.z;
+  const E *x = (const E*)a.x + z * a.x_zs, *w = (const E*)a.w + z * a.w_zs, *b = a.bias ? (const E*)a.bias + z * a.b_zs : nullptr;
   for (int i = tid; i < (WBM + WBN) * pieces; i += 256) {
     const int r = i / pieces, k = i % pieces * 8;
     const bool isx = r < WBM;
     const int g = isx ? m0 + r : n0 + r - WBM;
     const bool ok = isx ? g < a.T : g < a.N;
-    const E* src = isx ? (const E*)a.x + (ok ? (int64_t)g * a.ldx + k : 0) : (const E*)a.w + (ok ? (int64_t)g * a.K + k : 0);
+    const E* src = isx ? x + (ok ? (int64_t)g * a.ldx + k : 0) : w + (ok ? (int64_t)g * a.K + k : 0);
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(xs + r * pitch + k)), "l"(src), "r"(ok ? 16 : 0));
   }
   asm volatile("cp.async.commit_group;");
@@ -399,11 +401,12 @@ __global__ void __launch_bounds__(256) linear_short_kernel(LinearArgs a) {
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
     const int n = n0 + wn + j * 8 + (lane & 3) * 2;
-    bias[j] = make_float2(a.bias && n < a.N ? ldf((const E*)a.bias + n) : 0.f, a.bias && n + 1 < a.N ? ldf((const E*)a.bias + n + 1) : 0.f);
+    bias[j] = make_float2(b && n < a.N ? ldf(b + n) : 0.f, b && n + 1 < a.N ? ldf(b + n + 1) : 0.f);
   }
   float acc[4][4][4] = {};
   asm volatile("cp.async.wait_group 0;" ::: "memory");
   __syncthreads();
+  if (n0 + wn >= a.N) return;                                 // no outputs, and no barrier behind
   for (int k = 0; k < a.K; k += 16) {
     uint32_t bf[2][4];
 #pragma unroll
@@ -416,7 +419,7 @@ __global__ void __launch_bounds__(256) linear_short_kernel(LinearArgs a) {
       for (int j = 0; j < 4; ++j) mma_bf16_16816(acc[i][j], af, bf[j >> 1][(j & 1) * 2], bf[j >> 1][(j & 1) * 2 + 1]);
     }
   }
-  float* y = (float*)a.y;
+  float* y = (float*)a.y + z * a.y_zs;
 #pragma unroll
   for (int i = 0; i < 4; ++i)
 #pragma unroll
@@ -667,7 +670,7 @@ static int launch_linear_few(const LinearArgs& a, cudaStream_t st) {
 }
 
 static bool linear_short_ok(const LinearArgs& a) {
-  return a.elt == KGE_ELT_BF16 && a.out_f32 && !a.w2 && !a.group_off && !a.xrows && !a.yrows && !a.row_scale && !a.accumulate && a.nz == 1 && a.T > 256 && a.K % 16 == 0 && a.K <= WMAXK &&
+  return a.elt == KGE_ELT_BF16 && a.out_f32 && !a.w2 && !a.group_off && !a.xrows && !a.yrows && !a.row_scale && !a.accumulate && a.nz <= 65535 && (a.nz == 1 || (a.act == ACT_NONE && a.x_zs % 8 == 0 && a.w_zs % 8 == 0 && a.y_zs % 2 == 0)) && a.T > 256 && a.K % 16 == 0 && a.K <= WMAXK &&
          a.N % 2 == 0 && a.ldy % 2 == 0 && a.ldx % 8 == 0 && (a.T + WBM - 1) / WBM <= 65535 && (a.act == ACT_NONE || a.act == ACT_SOFTPLUS || a.act == ACT_EXP_DECAY) &&
          ((reinterpret_cast<uintptr_t>(a.x) | reinterpret_cast<uintptr_t>(a.w)) & 15) == 0 && (reinterpret_cast<uintptr_t>(a.y) & 7) == 0;
 }
@@ -682,7 +685,7 @@ int linear_any(const LinearArgs& a, cudaStream_t st) {
     const size_t smem = (size_t)(WBM + WBN) * (a.K + MPAD) * 2;
     auto kern = a.act == ACT_SOFTPLUS ? linear_short_kernel<ACT_SOFTPLUS> : a.act == ACT_EXP_DECAY ? linear_short_kernel<ACT_EXP_DECAY> : linear_short_kernel<ACT_NONE>;
     KGE_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    KGE_CUDA_OK(launch_pdl(kern, dim3((a.N + WBN - 1) / WBN, (a.T + WBM - 1) / WBM), dim3(256), smem, st, a));
+    KGE_CUDA_OK(launch_pdl(kern, dim3((a.N + WBN - 1) / WBN, (a.T + WBM - 1) / WBM, a.nz), dim3(256), smem, st, a));
     return 0;
   }
   const int rows = a.group_off ? (a.max_rows > 0 ? a.max_rows : a.T) : a.T;

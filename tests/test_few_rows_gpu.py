@@ -52,3 +52,15 @@ def test_sum_and_norm_by_width(kge, tmp_path, dtype, width):
     llm = make_engine(kge, tmp_path, cfg, W, dtype)
     check(run_pieces(llm, 0, toks, [9, 1, 1]), oh.forward(cfg, W, toks), dtype)
     llm.close()
+
+
+@pytest.mark.parametrize("width,blocks,rows", [(480, 3, 257), (512, 2, 300), (48, 3, 400), (288, 2, 385)])
+def test_block_diagonal_gates_of_many_rows(kge, tmp_path, width, blocks, rows):
+    """Strided slices in 128 x 128 tiles: blocks that end inside a tile (160), fill two (256), leave most warps without outputs (16), and end
+    inside a warp's columns (144); rows that end inside a tile."""
+    cfg = oh.make_config(layers=("rglru",), mlps=(None,), r_width=width, r_blocks=blocks)
+    W = oh.make_weights(cfg, seed=41)
+    toks = prompt(cfg, rows)
+    llm = make_engine(kge, tmp_path, cfg, W, "bfloat16")
+    check(run_pieces(llm, 0, toks, [rows]), oh.forward(cfg, W, toks), "bfloat16")
+    llm.close()
