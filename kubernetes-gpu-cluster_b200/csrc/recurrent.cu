@@ -192,9 +192,12 @@ __global__ void __launch_bounds__(128) rglru_scan_kernel(RglruArgs a) {
 // rglru_ab_kernel turns the gate pre-activations, in place, into the recurrence's coefficients (a_t, b_t = sqrt(1 - a_t^2)
 // i_t u_t); rglru_chain_kernel is then one fma per token and channel (S_t written over a_t) plus the state hand-over; and
 // rglru_out_kernel multiplies by gelu(y).  Same arithmetic per element as the fused kernel.  A thread keeps its channel and walks
-// over tokens (no divisions by the width).  2312 tokens x 2560: 92 us back to back (162 with a chain that loads into registers); 200
+// over tokens (no divisions by the width).  2312 tokens x 2560: 84 us back to back (92 before that, 162 with a chain that loads into registers); 200
 // tokens beside 64 single ones 21 (31).  All three in one kernel, with seven warps of a block feeding the chain, took 422: too few
 // warps for the exponentials' latency.
+// RG_AT tokens at a time in the first and the last of them: behind a store to the gates the compiler keeps later loads back, and a token
+// at a time each costs a trip to memory (2312 tokens x 2560: 40 and 17 us; 32 and 15 now).
+constexpr int RG_AT = 4;
 template <typename E>
 __global__ void __launch_bounds__(256) rglru_ab_kernel(RglruArgs a, float* gates) {
   pdl_launch_dependents();
@@ -202,12 +205,24 @@ __global__ void __launch_bounds__(256) rglru_ab_kernel(RglruArgs a, float* gates
   const int c = blockIdx.y * 256 + threadIdx.x;
   if (c >= a.width) return;
   const float sp = a.decay_c * softplusf_(ldf((const E*)a.lam + c));
-  for (int t = blockIdx.x; t < a.T; t += gridDim.x) {
-    float* gt = gates + (int64_t)t * 2 * a.width + c;
-    const float r = sigmoidf_(gt[0]), ig = sigmoidf_(gt[a.width]);
-    const float log_a = -sp * r;
-    gt[0] = expf(log_a);
-    gt[a.width] = sqrtf(-expm1f(2.f * log_a)) * ig * ldf((const E*)a.u + (int64_t)t * a.width + c);
+  for (int t0 = blockIdx.x; t0 < a.T; t0 += RG_AT * gridDim.x) {
+    float gr[RG_AT], gi[RG_AT], uv[RG_AT];
+#pragma unroll
+    for (int k = 0; k < RG_AT; ++k) {
+      const int t = min(t0 + k * (int)gridDim.x, a.T - 1);
+      const float* gt = gates + (int64_t)t * 2 * a.width + c;
+      gr[k] = gt[0]; gi[k] = gt[a.width];
+      uv[k] = ldf((const E*)a.u + (int64_t)t * a.width + c);
+    }
+#pragma unroll
+    for (int k = 0; k < RG_AT; ++k) {
+      const int t = t0 + k * (int)gridDim.x;
+      if (t >= a.T) break;
+      float* gt = gates + (int64_t)t * 2 * a.width + c;
+      const float log_a = -sp * sigmoidf_(gr[k]);
+      gt[0] = expf(log_a);
+      gt[a.width] = sqrtf(-expm1f(2.f * log_a)) * sigmoidf_(gi[k]) * uv[k];
+    }
   }
 }
 
@@ -302,8 +317,20 @@ __global__ void __launch_bounds__(256) rglru_out_kernel(RglruArgs a, const float
   pdl_wait();
   const int c = blockIdx.y * 256 + threadIdx.x;
   if (c >= a.width) return;
-  for (int t = blockIdx.x; t < a.T; t += gridDim.x)
-    stf((E*)a.out + (int64_t)t * a.width + c, gates[(int64_t)t * 2 * a.width + c] * gelu_tanhf_(ldf((const E*)a.yx + (int64_t)t * 2 * a.width + c)));
+  for (int t0 = blockIdx.x; t0 < a.T; t0 += RG_AT * gridDim.x) {
+    float sv[RG_AT], yv[RG_AT];
+#pragma unroll
+    for (int k = 0; k < RG_AT; ++k) {
+      const int64_t at = (int64_t)min(t0 + k * (int)gridDim.x, a.T - 1) * 2 * a.width + c;
+      sv[k] = gates[at];
+      yv[k] = ldf((const E*)a.yx + at);
+    }
+#pragma unroll
+    for (int k = 0; k < RG_AT; ++k) {
+      const int t = t0 + k * (int)gridDim.x;
+      if (t < a.T) stf((E*)a.out + (int64_t)t * a.width + c, sv[k] * gelu_tanhf_(yv[k]));
+    }
+  }
 }
 
 template <typename E, int N, int TOK>
