@@ -461,7 +461,8 @@ static int norm_common(int mode, void* y, void* residual, const void* x, const v
          : mode == 2 ? launch_norm_rows<2>(gt, y, residual, x, w, b, T, d, eps, s) : launch_norm_rows<3>(gt, y, residual, x, w, b, T, d, eps, s);
   }
   // weights early up to two rows an SM: 64 x 4096 1.95 us, 2.12 with them behind the reduction, 256 x 4096 3.25 / 3.7; 1339 x 2048 5.8 / 5.0
-  const bool early = T <= 2 * 148;
+  // (plain RMSNorm of rows up to 2048 keeps them there: one of 32 x 2048, its projection to 128256 and sampling 136.7 early, 136.1 so)
+  const bool early = T <= 2 * 148 && (mode != 0 || d > 2048);
   auto kern = early ? (mode == 0 ? norm_kernel<0, true> : mode == 1 ? norm_kernel<1, true> : mode == 2 ? norm_kernel<2, true> : norm_kernel<3, true>)
                     : (mode == 0 ? norm_kernel<0, false> : mode == 1 ? norm_kernel<1, false> : mode == 2 ? norm_kernel<2, false> : norm_kernel<3, false>);
   KGE_CUDA_OK(launch_pdl(kern, dim3(T), dim3(th), 0, s, (bf16*)y, (bf16*)residual, (const bf16*)x, (const bf16*)w,
