@@ -26,8 +26,8 @@ constexpr int kPairStages = 4;                 // K tiles and as many V tiles
 template <int HD> constexpr int pair_smem() { return (2 * 128 + 2 * kPairStages * BNK) * HD * 2 + 512 + 8 * 4096 + 128 * 8; }
 
 // n0, n1: key tiles of the two query tiles; n1 < 0: no more work.  split: there is one query tile, the even key tiles are the first
-// one's and the odd ones the second one's.
-struct __align__(16) Item { int q0, tok0, ntok0, ntok1, ctx0, kvh, n0, n1, split, tile_lo; };
+// one's and the odd ones the second one's.  tail: rows of the last tile that hold keys; 0: all of them, or the rest is zeros.
+struct __align__(16) Item { int q0, tok0, ntok0, ntok1, ctx0, kvh, n0, n1, split, tile_lo, tail; };
 
 // Outputs `ldo` apart and multiplied by out_scale.  BIAS kernels: a query at position i sees the keys j of its own chunk (chunk > 0; all up to i
 // otherwise) with -slope (i - j) added to the scaled score, slope 2^(-span (head + 1) / H) (span > 0).  What is the same for a whole row drops
@@ -84,6 +84,7 @@ attn_pair_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant
   Item* items = reinterpret_cast<Item*>(tail + 288);                   // 2 slots of 48 bytes
   const uint32_t clc_resp = bar0 + 384;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tail + 400);
+  static_assert(sizeof(Item) == 48, "two items lie between the barriers and the answers to requests for work");
   // Barriers; tiles are counted over all items of the CTA.  A parity wait holds only while no later phase of its barrier can complete:
   // what completes the next phase needs something that the waiter does after the wait (p_full and o_full, which may run a tile ahead of
   // their waiters, are pairs for that).  No stage is handed back before it was filled: an issuer without work for a tile waits for it too.
@@ -98,12 +99,13 @@ attn_pair_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant
   auto item_full = [&](int s) { return bar0 + 224u + 8u * s; };
   auto item_empty = [&](int s) { return bar0 + 240u + 8u * s; };
   const uint32_t q_full = bar0 + 256u, q_empty = bar0 + 264u, clc_full = bar0 + 272u;
+  auto v_clean = [&](int s) { return bar0 + 408u + 8u * s; };
   const int warp = uniform_warp(), lane = threadIdx.x & 31;
   const int G = H / KV, TT = BM / G, TI = per * TT;     // tokens of a query tile, of an item
 
   if (warp == 8) {
     if (lane == 0) {
-      for (int s = 0; s < NST; ++s) { mbar_init(k_full(s), 1); mbar_init(k_empty(s), 2); mbar_init(v_full(s), 1); mbar_init(v_empty(s), 2); }
+      for (int s = 0; s < NST; ++s) { mbar_init(k_full(s), 1); mbar_init(k_empty(s), 2); mbar_init(v_full(s), 1); mbar_init(v_empty(s), 2); mbar_init(v_clean(s), 1); }
       for (int a = 0; a < 2; ++a) {
         mbar_init(s_full(a), 1); mbar_init(s_read(a), 4);
         for (int t = 0; t < 2; ++t) { mbar_init(p_full(a, t), 4); mbar_init(o_full(a, t), 1); }
@@ -185,7 +187,7 @@ attn_pair_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant
         if (ni >= 2) mbar_wait(item_empty(slot), ((ni >> 1) - 1) & 1);
         if (leader) {
           Item it;
-          it.q0 = q0; it.tok0 = tok0; it.ntok0 = ntok0; it.ntok1 = ntok1; it.ctx0 = ctx0; it.kvh = kvh; it.n0 = n0; it.n1 = n1; it.split = split; it.tile_lo = tile_lo;
+          it.q0 = q0; it.tok0 = tok0; it.ntok0 = ntok0; it.ntok1 = ntok1; it.ctx0 = ctx0; it.kvh = kvh; it.n0 = n0; it.n1 = n1; it.split = split; it.tile_lo = tile_lo; it.tail = k_cache ? 0 : kv_len % BNK;
           items[slot] = it;
           mbar_arrive(item_full(slot));
         }
@@ -206,14 +208,15 @@ attn_pair_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant
             ids = key < kv_len ? btab[min(key >> bs_shift, max_blocks - 1)] : block0;
           }
           if (k_cache) {
-            // knob "attn_tma" 0: the same tiles gathered by the lanes; a tile is handed over when the next one's copies are under way
+            // knob "attn_tma" 0: the same tiles gathered by the lanes (zeros beyond the keys); a tile is handed over when the next one's
+            // copies are under way
             constexpr int CH = HD / 8;
 #pragma unroll 4
             for (int i = lane; i < BNK * CH; i += 32) {
               const int row = i / CH, chunk = i % CH;
               const int blk = __shfl_sync(0xffffffffu, ids, (first + row / box_rows) & 31);
               const bf16* src = (is_k ? k_cache : v_cache) + ((int64_t)(blk * KV + kvh) * bs + ((j * BNK + row) & (bs - 1))) * HD + chunk * 8;
-              cp16(dst + tile_off<BNK>(row, chunk), src, true);
+              cp16(dst + tile_off<BNK>(row, chunk), src, j * BNK + row < kv_len);
             }
             cp_commit();
             hand_over(bar);
@@ -284,11 +287,13 @@ attn_pair_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant
       const int a = warp - 8;
       const uint32_t t_s = tmem + S_COL + a * 128, t_o = tmem + a * 128;
       uint32_t ns = 0, np = 0, nk = 0;                 // score tiles and products P V issued so far, key tiles
+      uint32_t cleaned = 0;                            // parities of the stages' next v_clean
       for (uint32_t ni = 0;; ++ni) {
         mbar_wait(item_full(ni & 1), (ni >> 1) & 1);
-        const int n0 = items[ni & 1].n0, n1 = items[ni & 1].n1, split = items[ni & 1].split;
+        const int n0 = items[ni & 1].n0, n1 = items[ni & 1].n1, split = items[ni & 1].split, tail = items[ni & 1].tail;
         mbar_arrive(item_empty(ni & 1));
         if (n1 < 0) break;
+        const bool shared_tail = !split && n0 == n1;   // both query tiles see the last key tile
         const int n = split ? n0 + n1 : max(n0, n1), na = a ? n1 : n0, ahead = 1 + split;
         const uint64_t qd = desc_kmajor(sQ + (split ? 0 : a) * Q_TILE);
         mbar_wait(q_full, ni & 1);
@@ -317,13 +322,33 @@ attn_pair_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant
             const int st = (nk + j) % NST;
             mbar_wait(v_full(st), ((nk + j) / NST) & 1);
             if (split ? (j & 1) == a : j < na) {
+              // The page that holds the item's last key has the values of a former owner behind it.  Their weights are zero, but infinity
+              // times zero is none: groups of 16 keys without a key are left out, and the rest of the last group is cleared first, by one
+              // issuer where both use the tile.  (Cleared before the tile is handed over, by the producer or a warp of its own, 200 decode
+              // rows beside 300 tokens took 125 us; here 124.4, 123.8 without.)
+              int groups = BNK / 16;
+              if (tail && j + 1 == n) {
+                groups = (tail + 15) / 16;
+                if (shared_tail && a == 1) {
+                  mbar_wait(v_clean(st), (cleaned >> st) & 1);
+                  cleaned ^= 1u << st;
+                } else {
+                  for (int at = sV + st * TILE + tail * 128; at < (int)(sV + st * TILE + groups * 16 * 128); at += 16)
+#pragma unroll
+                    for (int h = 0; h < HD / 64; ++h)
+                      asm volatile("st.shared.v4.b32 [%0], {%1, %1, %1, %1};" ::"r"(at + h * BNK * 128), "r"(0) : "memory");
+                  fence_async_smem();
+                  if (shared_tail) mbar_arrive(v_clean(st));
+                }
+              }
               mbar_wait(p_full(a, np), (np >> 1) & 1);
               tc_after();
               const uint64_t vd = desc_mnmajor(sV + st * TILE);
               const uint32_t t_p = t_s + 64 + (np & 1) * 32;
 #pragma unroll
               for (int k = 0; k < BNK / 16; ++k)
-                tc_mma_ts(t_o, t_p + k * 8, vd + (uint32_t)((k * 16 * 128) >> 4), IDESC_O, (!first || k > 0) ? 1u : 0u);
+                if (k < groups)
+                  tc_mma_ts(t_o, t_p + k * 8, vd + (uint32_t)((k * 16 * 128) >> 4), IDESC_O, (!first || k > 0) ? 1u : 0u);
               tc_commit(o_full(a, np));
               ++np;
               first = false;

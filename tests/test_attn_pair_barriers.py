@@ -17,7 +17,7 @@ OPS = [
     # issuers
     "wait item_full(ni & 1), (ni >> 1) & 1", "arrive item_empty(ni & 1)", "wait q_full, ni & 1",
     "wait k_full(st), ((nk + js) / NST) & 1", "wait s_read(a), (ns - 1) & 1", "commit s_full(a)", "commit k_empty(st)", "commit q_empty",
-    "wait v_full(st), ((nk + j) / NST) & 1", "wait p_full(a, np), (np >> 1) & 1", "commit o_full(a, np)", "commit v_empty(st)",
+    "wait v_full(st), ((nk + j) / NST) & 1", "wait v_clean(st), (cleaned >> st) & 1", "arrive v_clean(st)", "wait p_full(a, np), (np >> 1) & 1", "commit o_full(a, np)", "commit v_empty(st)",
     # softmax warps
     "wait item_full(ni & 1), (ni >> 1) & 1", "arrive item_empty(ni & 1)", "wait s_full(a), ns & 1", "arrive s_read(a)",
     "wait o_full(a, ns - 1), ((ns - 1) >> 1) & 1", "wait o_full(a, ns), ((ns - 2) >> 1) & 1", "arrive p_full(a, ns)",
@@ -45,12 +45,12 @@ def test_transcription_matches_the_kernel():
 
 def programs(items, nst):
     """Instruction lists of the roles.  items: (key tiles of the first query tile, of the second[, whether they share the key tiles of one
-    query tile between them]).  BAR: a barrier of the two groups of softmax threads.  An MMA is ("mma", barriers that it
-    commits to, buffers it reads, buffers it writes); a copy ("load", barrier, buffer)."""
+    query tile between them[, whether values beyond the last key are cleared]]).  BAR: a barrier of the two groups of softmax threads.  An
+    MMA is ("mma", barriers that it commits to, buffers it reads, buffers it writes); a copy ("load", barrier, buffer)."""
     def wait(bar, k, optional=False):
         return ("maybe" if optional else "wait", bar, k)
     prod, nk, end = [], 0, len(items)
-    items = [(*i, 0)[:3] for i in items]
+    items = [(*i, 0, 0)[:4] for i in items]
     tiles = [i[0] + i[1] if i[2] else max(i) for i in items]
     for ni in range(end + 1):
         if ni >= 2:
@@ -69,7 +69,7 @@ def programs(items, nst):
             nk += 1
     roles = [prod]
     for a in range(2):
-        issue, ns, np, nk = [], 0, 0, 0
+        issue, ns, np, nk, cleaned = [], 0, 0, 0, [0] * nst
         for ni, nn in enumerate(items):
             n, ahead = tiles[ni], 1 + nn[2]
             issue += [wait(("item_full", ni & 1), ni >> 1), ("arrive", ("item_empty", ni & 1)), wait(("q_full",), ni)]
@@ -88,6 +88,12 @@ def programs(items, nst):
                     st = (nk + j) % nst
                     issue.append(wait(("v_full", st), (nk + j) // nst))
                     if j % 2 == a if nn[2] else j < nn[a]:
+                        both = not nn[2] and nn[0] == nn[1]
+                        if nn[3] and j + 1 == n and both and a:
+                            issue.append(wait(("v_clean", st), cleaned[st]))
+                            cleaned[st] += 1
+                        elif nn[3] and j + 1 == n:
+                            issue += [("write", ("v", st))] + ([("arrive", ("v_clean", st))] if both else [])
                         issue += [wait(("p_full", a, np & 1), np >> 1),
                                   ("mma", [("o_full", a, np & 1)], [("p", a, np & 1), ("v", st)], [("o", a)])]
                         np += 1
@@ -130,7 +136,7 @@ def explore(items, nst, only=None, drop=None):
     if only is not None:
         roles = [roles[0], roles[1 + only], roles[3 + only]]
         need = {"item_empty": 2}
-        roles = [[op for op in r if op[0] == "mma" or op[1][0][:3] != "bar"] for r in roles]
+        roles = [[op for op in r if op[0] == "mma" or op[1][0][:3] != "bar" and op[1][0] != "v_clean"] for r in roles]
     if drop:
         roles = [[op for op in r if not (op[0] == "wait" and op[1][0] == drop)] for r in roles]
     bars = sorted({b for r in roles for op in r for b in (op[1] if op[0] == "mma" else [op[1]] if op[0] in ("wait", "maybe", "arrive", "load") else [])}, key=str)
@@ -169,11 +175,13 @@ def explore(items, nst, only=None, drop=None):
             elif op[0] == "load":
                 if any(op[2] in f[2] for f in flight):           # a copy into what an MMA reads
                     return True
-                succ.append((nxt, state, done_mma, tuple(sorted(loads + (op[1],), key=str))))
+                succ.append((nxt, state, done_mma, tuple(sorted(loads + (op[1:],), key=str))))
             else:
                 # threads: what an MMA in flight writes may not be read, what it reads may not be written
                 if op[0] == "read" and any(op[1] in f[3] for f in flight) or op[0] == "write" and any(op[1] in f[2] for f in flight):
                     return True
+                if op[0] == "write" and any(op[1] == buf for _, buf in loads):
+                    return True                                  # nor what a copy in flight writes
                 succ.append((nxt, state, done_mma, loads))
         for r, m in enumerate(mmas):
             if done_mma[r] < before[r][pcs[r]]:
@@ -181,7 +189,7 @@ def explore(items, nst, only=None, drop=None):
                 for b in m[done_mma[r]][1]:
                     s = arrive(s, b)
                 succ.append((pcs, s, done_mma[:r] + (done_mma[r] + 1,) + done_mma[r + 1:], loads))
-        for i, b in enumerate(loads):
+        for i, (b, _) in enumerate(loads):
             succ.append((pcs, arrive(state, b), done_mma, loads[:i] + loads[i + 1:]))
         if not succ and any(pcs[r] < len(prog) for r, prog in enumerate(roles)):
             return True
@@ -207,3 +215,20 @@ def test_every_wait_of_one_query_tile_ends_in_every_order(items, nst, only):
 @pytest.mark.parametrize("drop", ["o_full", "p_full", "s_read", "k_empty", "q_empty"])
 def test_the_exploration_finds_a_missing_wait(drop):
     assert explore([(3, 3), (2, 1)], 2, 0, drop)
+
+
+@pytest.mark.parametrize("items", [[(1, 0, 0, 1)], [(1, 1, 0, 1)], [(1, 2, 0, 1)], [(2, 1, 1, 1)], [(1, 1, 0, 1), (1, 1, 0, 1)], [(3, 3, 0, 1)]], ids=str)
+def test_cleared_values_in_every_order(items):
+    assert not explore(items, 2)
+
+
+@pytest.mark.parametrize("nst", [2, 4])
+@pytest.mark.parametrize("items", [[(5, 6, 0, 1)], [(2, 3, 0, 1), (1, 0, 0, 1), (3, 3)], [(3, 2, 1, 1), (1, 2, 0, 1)], [(1, 1, 1, 1)] * 3], ids=str)
+@pytest.mark.parametrize("only", [0, 1])
+def test_cleared_values_of_one_query_tile_in_every_order(items, nst, only):
+    assert not explore(items, nst, only)
+
+
+def test_the_exploration_finds_values_that_are_cleared_too_early_or_not_waited_for():
+    assert explore([(3, 3, 0, 1)], 2, 0, "v_full")
+    assert explore([(1, 1, 0, 1)], 2, None, "v_clean")
