@@ -167,7 +167,7 @@ attn_pair_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant
           } else {
             rank -= __shfl_sync(0xffffffffu, upto, 31);
             by += 32;
-            if (by >= flat) { b = 0; rank = 1 << 24; }                 // more CTAs than work
+            if (by >= flat) { b = 0; rank = -1; }                      // more CTAs than work
           }
         }
       }
@@ -175,7 +175,7 @@ attn_pair_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant
       const int32_t* btab = block_table + (int64_t)b * max_blocks;
       const int q0 = qsl[b], q1 = qsl[b + 1], seq_len = seq_lens[b], id0 = btab[min((lane * box_rows) >> bs_shift, max_blocks - 1)];
       const int q_len = q1 - q0;
-      const int tok0 = ((q_len + TI - 1) / TI - 1 - rank) * TI;
+      const int tok0 = rank < 0 ? -1 : ((q_len + TI - 1) / TI - 1 - rank) * TI;
       if (tok0 >= 0) {
         const int ctx0 = seq_len - q_len;
         const int ntok0 = min(TT, q_len - tok0), ntok1 = max(0, min(TI - TT, q_len - tok0 - TT));
