@@ -325,7 +325,8 @@ attn_pair_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant
               // The page that holds the item's last key has the values of a former owner behind it.  Their weights are zero, but infinity
               // times zero is none: groups of 16 keys without a key are left out, and the rest of the last group is cleared first, by one
               // issuer where both use the tile.  (Cleared before the tile is handed over, by the producer or a warp of its own, 200 decode
-              // rows beside 300 tokens took 125 us; here 124.4, 123.8 without.)
+              // rows beside 300 tokens took 126 us, 119.8 here and 121.0 without; 14 rows of 128 cleared 16 bytes at a time cost this
+              // thread 0.8 us.)
               int groups = BNK / 16;
               if (tail && j + 1 == n) {
                 groups = (tail + 15) / 16;
@@ -333,10 +334,10 @@ attn_pair_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant
                   mbar_wait(v_clean(st), (cleaned >> st) & 1);
                   cleaned ^= 1u << st;
                 } else {
-                  for (int at = sV + st * TILE + tail * 128; at < (int)(sV + st * TILE + groups * 16 * 128); at += 16)
+                  if (tail & 15)
 #pragma unroll
                     for (int h = 0; h < HD / 64; ++h)
-                      asm volatile("st.shared.v4.b32 [%0], {%1, %1, %1, %1};" ::"r"(at + h * BNK * 128), "r"(0) : "memory");
+                      asm volatile("st.bulk.weak.shared::cta [%0], %1, 0;" ::"r"(sV + st * TILE + (uint32_t)(h * BNK * 128 + tail * 128)), "l"((uint64_t)(groups * 16 - tail) * 128) : "memory");
                   fence_async_smem();
                   if (shared_tail) mbar_arrive(v_clean(st));
                 }
