@@ -322,23 +322,16 @@ attn_pair_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant
             const int st = (nk + j) % NST;
             mbar_wait(v_full(st), ((nk + j) / NST) & 1);
             if (split ? (j & 1) == a : j < na) {
-              // The page that holds the item's last key has the values of a former owner behind it.  Their weights are zero, but infinity
-              // times zero is none: groups of 16 keys without a key are left out, and the rest of the last group is cleared first, by one
-              // issuer where both use the tile.  (Cleared before the tile is handed over, by the producer or a warp of its own, 200 decode
-              // rows beside 300 tokens took 126 us, 119.8 here and 121.0 without; 14 rows of 128 cleared 16 bytes at a time cost this
-              // thread 0.8 us.)
+              // values beyond the last key (clean_tail), by one issuer where both use the tile.  (Cleared before the tile is handed over, by the
+              // producer or a warp of its own, 200 decode rows beside 300 tokens took 126 us, 119.8 here and 121.0 without.)
               int groups = BNK / 16;
               if (tail && j + 1 == n) {
-                groups = (tail + 15) / 16;
                 if (shared_tail && a == 1) {
                   mbar_wait(v_clean(st), (cleaned >> st) & 1);
                   cleaned ^= 1u << st;
+                  groups = (tail + 15) / 16;
                 } else {
-                  if (tail & 15)
-#pragma unroll
-                    for (int h = 0; h < HD / 64; ++h)
-                      asm volatile("st.bulk.weak.shared::cta [%0], %1, 0;" ::"r"(sV + st * TILE + (uint32_t)(h * BNK * 128 + tail * 128)), "l"((uint64_t)(groups * 16 - tail) * 128) : "memory");
-                  fence_async_smem();
+                  groups = clean_tail<HD>(sV + st * TILE, tail);
                   if (shared_tail) mbar_arrive(v_clean(st));
                 }
               }

@@ -96,6 +96,20 @@ __device__ __forceinline__ uint64_t desc_mnmajor(uint32_t saddr) {
          ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
 }
 
+// The page that holds the last key has the values of a former owner behind it.  Their weights are zero, but infinity times zero is none:
+// of the last value tile, with `rows` rows of keys, the product takes the groups of 16 that have any (returned), and what the last of
+// them has beyond the keys is cleared first.  (14 rows of 128 cleared 16 bytes at a time cost the issuing thread 0.8 us.)
+template <int HD>
+__device__ __forceinline__ int clean_tail(uint32_t v_tile, int rows) {
+  const int groups = (rows + 15) / 16;
+  if (rows & 15)
+#pragma unroll
+    for (int h = 0; h < HD / 64; ++h)
+      asm volatile("st.bulk.weak.shared::cta [%0], %1, 0;" ::"r"(v_tile + (uint32_t)(h * BNK * 128 + rows * 128)), "l"((uint64_t)(groups * 16 - rows) * 128) : "memory");
+  fence_async_smem();
+  return groups;
+}
+
 __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&r)[32]) {
   asm volatile(
       "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
@@ -269,14 +283,15 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
           if (j > 0) { wait_o(j - 1); tc_after(); }
           issue_s(j + 1);
         }
-        mbar_wait(p_full(j & 1), (uint32_t)((j >> 1) & 1));
         mbar_wait(v_full(j & 1), (uint32_t)((j >> 1) & 1));
+        const int tail = TMA && j + 1 == ntiles ? kv_len % BNK : 0, groups = tail ? clean_tail<HD>(sV + (j & 1) * TILE_BYTES, tail) : BNK / 16;
+        mbar_wait(p_full(j & 1), (uint32_t)((j >> 1) & 1));
         tc_after();
         const uint64_t vd = desc_mnmajor(sV + (j & 1) * TILE_BYTES);
 #pragma unroll
         for (int k = 0; k < BNK / 16; ++k) {
           const uint32_t boff = (uint32_t)(k * 16 * 128);                             // V: 16 keys = 16 rows of 128 B
-          tc_mma_ts(tmem + O_COL, tmem + (j & 1) * BNK + k * 8, vd + (boff >> 4), IDESC_O, (j > 0 || k > 0) ? 1u : 0u);
+          if (k < groups) tc_mma_ts(tmem + O_COL, tmem + (j & 1) * BNK + k * 8, vd + (boff >> 4), IDESC_O, (j > 0 || k > 0) ? 1u : 0u);
         }
         tc_commit(o_full(j & 1));
         if (TMA) tc_commit(v_empty(j & 1));      // PV_j has read V stage j&1: the producer may refill it

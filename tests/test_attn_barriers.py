@@ -12,7 +12,7 @@ OPS = [
     "wait o_full(j & 1), (uint32_t)((j >> 1) & 1)",                  # wait_o
     # issuer
     "wait k_full(st), (uint32_t)((j >> 1) & 1)", "commit s_full(st)",
-    "wait q_full, 0u", "wait_o j - 1", "wait p_full(j & 1), (uint32_t)((j >> 1) & 1)", "wait v_full(j & 1), (uint32_t)((j >> 1) & 1)",
+    "wait q_full, 0u", "wait_o j - 1", "wait v_full(j & 1), (uint32_t)((j >> 1) & 1)", "wait p_full(j & 1), (uint32_t)((j >> 1) & 1)",
     "commit o_full(j & 1)", "commit v_empty(j & 1)",
     # producer
     "wait s_full(j & 1), (uint32_t)((j >> 1) & 1)", "wait v_empty(j & 1), (uint32_t)((j >> 1) & 1)",
@@ -60,7 +60,7 @@ def programs(n, tma, o_bars, last):
             if j > 0:
                 issuer.append(wait_o(j - 1))
             issue_s(j + 1)
-        issuer += [wait("p", j), wait("v", j), ("mma", (("o", j % o_bars),) + ((("e", j % 2),) if tma else ()))]
+        issuer += [wait("v", j), wait("p", j), ("mma", (("o", j % o_bars),) + ((("e", j % 2),) if tma else ()))]
     if tma:
         for t in range(min(n, 2)):
             producer.append(("load", ("k", t)))

@@ -18,7 +18,13 @@ def staging(kge, request):
     kge.check(kge.lib().kge_set_tunable(b"attn_tma", 1), "tunable")
 
 
-@pytest.mark.parametrize("c", CASES, ids=lambda c: f"{c[0]}-{c[1]}x{c[2]}x{c[3]}-{c[4]}-{max(c[5])}")
+# prompts of small launches (attn_tc_kernel): a piece of a tile, ends inside and at groups of 16 keys
+SMALL = [
+    ("bf16", 32, 8, 128, 64, [17], [0]), ("bf16", 8, 8, 64, 16, [64, 50, 3], [0, 30, 77]), ("fp16", 16, 4, 128, 32, [40, 1, 48, 47], [0, 100, 17, 0]),
+]
+
+
+@pytest.mark.parametrize("c", CASES + SMALL, ids=lambda c: f"{c[0]}-{c[1]}x{c[2]}x{c[3]}-{c[4]}-{max(c[5])}")
 def test_prompts(kge, staging, c):
     dtype, H, KV, hd, bs, q, prior = c
     dt = torch.bfloat16 if dtype == "bf16" else torch.float16
