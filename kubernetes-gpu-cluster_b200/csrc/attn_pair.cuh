@@ -540,7 +540,7 @@ attn_pair_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant
 }  // namespace atc2
 
 int make_tmap(CUtensorMap* m, const void* ptr, int64_t rows, int64_t cols, int box_rows);   // gemm_tc.cu (cached)
-int encode_tmap_q(CUtensorMap* m, const void* ptr, int64_t stride, int hd, int heads, int box_heads, int box_tokens);     // gemm_tc.cu
+int make_tmap_q(CUtensorMap* m, const void* ptr, int64_t stride, int hd, int heads, int box_heads, int box_tokens);     // gemm_tc.cu (cached)
 
 template <int HD, bool BIAS>
 static int launch_pair(const atc2::PairArgs& pa, bf16* out, const bf16* q, int q_stride, const bf16* kc, const bf16* vc, const int32_t* bt, int max_blocks, const int32_t* sl,
@@ -562,8 +562,9 @@ static int launch_pair(const atc2::PairArgs& pa, bf16* out, const bf16* q, int q
   const int64_t rows = (int64_t)1 << 30;
   if (int rc = make_tmap(&tk, kc, rows, HD, box_rows)) return rc;
   if (int rc = make_tmap(&tv, vc, rows, HD, box_rows)) return rc;
-  if (int rc = encode_tmap_q(&tq8, q, q_stride, HD, H, G, TT >= 8 ? 8 : 1)) return rc;
-  if (int rc = encode_tmap_q(&tq1, q, q_stride, HD, H, G, 1)) return rc;
+  if (int rc = make_tmap_q(&tq1, q, q_stride, HD, H, G, 1)) return rc;
+  tq8 = tq1;
+  if (TT >= 8) { if (int rc = make_tmap_q(&tq8, q, q_stride, HD, H, G, 8)) return rc; }
   if (!tunable(TUN_ATTN_TMA)) { gk = kc; gv = vc; }
   auto kern = atc2::attn_pair_kernel<HD, BIAS>;
   KGE_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, atc2::pair_smem<HD>()));

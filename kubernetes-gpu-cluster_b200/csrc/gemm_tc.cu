@@ -1042,22 +1042,26 @@ struct TmapKeyHash {
     return (size_t)(h ^ (h >> 29));
   }
 };
-int make_tmap(CUtensorMap* m, const void* ptr, int64_t rows, int64_t cols, int box_rows) {
+// Tensor maps by what they are made of, for all threads.  Callers that cycle through fresh buffers (tests) stay bounded.
+template <class Key, class Hash, class Encode>
+static int cached_tmap(CUtensorMap* m, const Key& key, Encode&& encode) {
   static std::mutex mu;
-  static std::unordered_map<TmapKey, CUtensorMap, TmapKeyHash> cache;
-  const TmapKey key{ptr, rows, cols, box_rows};
+  static std::unordered_map<Key, CUtensorMap, Hash> cache;
   std::lock_guard<std::mutex> lock(mu);
   auto it = cache.find(key);
   if (it != cache.end()) { *m = it->second; return 0; }
-  if (int rc = encode_tmap(m, ptr, rows, cols, box_rows)) return rc;
-  if (cache.size() >= 16384) cache.clear();       // callers that cycle through fresh buffers (tests) stay bounded
+  if (int rc = encode(m)) return rc;
+  if (cache.size() >= 16384) cache.clear();
   cache.emplace(key, *m);
   return 0;
+}
+int make_tmap(CUtensorMap* m, const void* ptr, int64_t rows, int64_t cols, int box_rows) {
+  return cached_tmap<TmapKey, TmapKeyHash>(m, TmapKey{ptr, rows, cols, box_rows}, [&](CUtensorMap* t) { return encode_tmap(t, ptr, rows, cols, box_rows); });
 }
 
 // Queries of a packed projection, [tokens][heads][hd] with tokens `stride` numbers apart: boxes of 64 columns x box_heads x
 // box_tokens, 128B swizzle.  The number of tokens is not known to the callers: a box must lie within the rows they may read.
-int encode_tmap_q(CUtensorMap* m, const void* ptr, int64_t stride, int hd, int heads, int box_heads, int box_tokens) {
+static int encode_tmap_q(CUtensorMap* m, const void* ptr, int64_t stride, int hd, int heads, int box_heads, int box_tokens) {
   EncodeTiledFn enc = get_encode_fn();
   KGE_REQUIRE(enc, "cuTensorMapEncodeTiled unavailable (no CUDA driver?)");
   cuuint64_t dims[3] = {(cuuint64_t)hd, (cuuint64_t)heads, (cuuint64_t)1 << 30};
@@ -1073,6 +1077,22 @@ int encode_tmap_q(CUtensorMap* m, const void* ptr, int64_t stride, int hd, int h
                    CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   KGE_REQUIRE(r == CUDA_SUCCESS, "cuTensorMapEncodeTiled failed (%d) stride=%lld heads=%d", (int)r, (long long)stride, heads);
   return 0;
+}
+
+struct TmapQKey {
+  const void* p; int64_t stride; int hd, heads, box_heads, box_tokens;
+  bool operator==(const TmapQKey& o) const { return p == o.p && stride == o.stride && hd == o.hd && heads == o.heads && box_heads == o.box_heads && box_tokens == o.box_tokens; }
+};
+struct TmapQKeyHash {
+  size_t operator()(const TmapQKey& k) const {
+    uint64_t h = (uint64_t)(uintptr_t)k.p * 0x9E3779B97F4A7C15ull;
+    h ^= ((uint64_t)k.stride * 0xBF58476D1CE4E5B9ull) ^ ((uint64_t)k.heads << 40) ^ ((uint64_t)k.hd << 24) ^ ((uint64_t)k.box_heads << 8) ^ (uint64_t)k.box_tokens;
+    return (size_t)(h ^ (h >> 29));
+  }
+};
+int make_tmap_q(CUtensorMap* m, const void* ptr, int64_t stride, int hd, int heads, int box_heads, int box_tokens) {
+  return cached_tmap<TmapQKey, TmapQKeyHash>(m, TmapQKey{ptr, stride, hd, heads, box_heads, box_tokens},
+                                             [&](CUtensorMap* t) { return encode_tmap_q(t, ptr, stride, hd, heads, box_heads, box_tokens); });
 }
 
 constexpr int kGemmSmemBudget = 224 * 1024;
