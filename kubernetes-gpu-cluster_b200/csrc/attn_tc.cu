@@ -20,6 +20,8 @@
 #include <cuda.h>
 #include <string.h>
 
+#include <algorithm>
+
 #include "common.cuh"
 #include "f32x2.cuh"
 #include "kge.h"
@@ -548,10 +550,22 @@ static int launch_tc(bf16* out, const bf16* q, int q_stride, const bf16* kc, con
   const dim3 grid = tc_grid(B, T, max_q_len, TT, KV, by_request);
   CUtensorMap tk, tv;
   const bool tma = tunable(TUN_ATTN_TMA) != 0 && bs >= 8;
-  // Two query tiles per CTA (attn_pair.cuh) but for launches of short contexts that do not fill the chip: there its 384 threads, all of
-  // TMEM and 226 KB start later than two of these CTAs per SM (us here / there: 8 x 128 tokens 10.3 / 11.4, 2 x 300 10.3 / 11.5, 64 tokens
-  // 5.6 / 7.0; but 8 x 300 26.5 / 23.3, one of 512 14.2 / 11.3; 32 / 8 heads of 128).
-  if (bs >= 8 && !cap && B <= 65535 && !(max_seq_len <= 320 && (int64_t)T * KV <= 256 * TT))
+  // Two query tiles per CTA (attn_pair.cuh) but for small launches: there its 384 threads, all of TMEM and 226 KB start later than two of
+  // these CTAs per SM.  Measured over 9238 launches (1 to 64 requests, 1 to 12 kv heads, groups of 1 to 8, heads of 64 and 128, contexts up to
+  // 3600), time there over time here, by query tiles and longest context:
+  //     tiles        to 320    to 640   to 1280   to 2560    beyond
+  //     to 37          1.37      1.15      1.06      1.01      0.97
+  //     to 148         1.24      1.08      1.00      0.91      0.90
+  //     to 296         1.26      1.06      0.99      0.99      0.95
+  //     beyond         0.95      0.80      0.81      0.90      0.93
+  // Up to 37 tiles little but the start counts; up to 148 an item there has an SM and two groups of warps for its keys; up to 296 they take two
+  // rounds there and one here.  CTAs without a query tile (short requests beside long ones) cost this kernel their start: up to 1000 CTAs.  Short
+  // contexts are nearly all start: those of at most 296 tiles' tokens stay here up to six CTAs an SM.  So 2 % of the launches are more than 3 %
+  // slower there than here would be, 21 % with a line of T * KV <= 256 tiles' tokens and contexts up to 320.
+  const int64_t launched = (int64_t)grid.x * grid.y * grid.z, tiles = std::min(launched, KV * ((int64_t)T / TT + B));
+  const bool small = (launched <= 1000 && tiles <= 296 && max_seq_len <= (tiles <= 37 ? 2048 : tiles <= 148 ? 1024 : 1800)) ||
+                     (launched <= 888 && max_seq_len <= 320 && (int64_t)T * KV <= 296 * TT);
+  if (bs >= 8 && !cap && B <= 65535 && !small)
     return launch_pair<HD, false>(atc2::PairArgs{H * HD, 1.f, 0, 0.f}, out, q, q_stride, kc, vc, bt, max_blocks, sl, qsl, B, T, max_q_len, max_seq_len, H, KV, bs, bs_shift, scale, sinks, st);
   if (tma) {
     const int box_rows = bs < atc::BNK ? bs : atc::BNK;

@@ -18,6 +18,14 @@ CASES = [   # dtype, heads, kv heads, head size, block, query lengths, tokens ca
     ("bf16", 32, 8, 128, 64, [1] * 33 + [300], [5 + 64 * i for i in range(33)] + [0]),
     ("bf16", 128, 1, 128, 64, [1] * 5 + [3], [2000, 0, 63, 64, 65] + [500]),     # groups of 128: a token a query tile
 ]
+# the same over contexts that no small launch has (launch_tc in csrc/attn_tc.cu keeps those for its own kernel)
+LONG = [
+    ("bf16", 32, 8, 128, 64, [512], [600]),
+    ("bf16", 32, 8, 128, 64, [64, 63, 65, 1], [1089, 1090, 1088, 0]),
+    ("fp16", 24, 8, 128, 64, [400, 43, 700], [0, 2600, 100]),
+    ("bf16", 64, 2, 64, 8, [333, 5, 1], [2300, 800, 1200]),
+    ("bf16", 128, 1, 128, 64, [1] * 5 + [3], [2700, 0, 63, 64, 65] + [500]),
+]
 
 
 def case(kge, dtype, H, KV, hd, bs, q, prior, ramp):
@@ -61,7 +69,7 @@ def case(kge, dtype, H, KV, hd, bs, q, prior, ramp):
 
 
 @pytest.mark.parametrize("ramp", [False, True])
-@pytest.mark.parametrize("c", CASES, ids=lambda c: f"{c[0]}-{c[1]}x{c[2]}x{c[3]}-{c[4]}-{max(c[5])}")
+@pytest.mark.parametrize("c", CASES + LONG, ids=lambda c: f"{c[0]}-{c[1]}x{c[2]}x{c[3]}-{c[4]}-{max(c[5])}-{max(c[6])}")
 def test_against_float64(kge, c, ramp):
     out, ref, dt = case(kge, *c, ramp)
     assert torch.isfinite(out).all()

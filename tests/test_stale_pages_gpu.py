@@ -5,7 +5,7 @@ import pytest
 import torch
 
 from oracle import hybrid as oh
-from test_attn_pair_gpu import CASES
+from test_attn_pair_gpu import CASES, LONG
 from test_hybrid_gpu import check, make_engine, prompt, run_pieces
 
 pytestmark = pytest.mark.gpu
@@ -24,7 +24,7 @@ SMALL = [
 ]
 
 
-@pytest.mark.parametrize("c", CASES + SMALL, ids=lambda c: f"{c[0]}-{c[1]}x{c[2]}x{c[3]}-{c[4]}-{max(c[5])}")
+@pytest.mark.parametrize("c", CASES + LONG + SMALL, ids=lambda c: f"{c[0]}-{c[1]}x{c[2]}x{c[3]}-{c[4]}-{max(c[5])}-{max(c[6])}")
 def test_prompts(kge, staging, c):
     dtype, H, KV, hd, bs, q, prior = c
     dt = torch.bfloat16 if dtype == "bf16" else torch.float16
