@@ -479,7 +479,7 @@ static cudaError_t launch_bias_split(dim3 grid, int S, size_t smem, cudaStream_t
 
 inline namespace KGE_ELT_NS {
 int paged_attn_bias_pair(void* out, int ldo, const void* q, int ldq, const void* kc, const void* vc, const int32_t* bt, int max_blocks, const int32_t* sl,
-                         const int32_t* qsl, int B, int T, int max_q_len, int H, int KV, int hd, int bs, float scale, int chunk, float span, float out_scale, cudaStream_t st);      // attn_tc.cu
+                         const int32_t* qsl, int B, int T, int max_q_len, int max_seq_len, int H, int KV, int hd, int bs, float scale, int chunk, float span, float out_scale, cudaStream_t st);      // attn_tc.cu
 }
 // What the tcgen05 kernel of attn_pair.cuh takes: plain chunked attention with distance biases, keys and values of 64 or 128, pages of a
 // power of two of at least 8 tokens, aligned rows.  Two prompts of 1150 tokens, 16 / 4 heads of 128 in chunks of 1024: 162 us in the
@@ -514,9 +514,12 @@ int attn_bias_chunk(const AttnBiasArgs& a, cudaStream_t st) {
       const int S = bias_cluster((int64_t)((hpg + 15) / 16) * a.G * D, reach / AM_KT);
       KGE_CUDA_OK(launch_bias_split(dim3((hpg + 15) / 16, a.G, D), S, S > 1 ? split + sums : split, st, a, 0));
     }
-    if (D < a.B && a.max_q * hpg > 32 && bias_pair_ok(a))
+    // the tcgen05 kernel's start shows where all keys are one tile of this kernel: 32 / 8 heads of 128, one piece of 9 tokens 6.25 us here and 7.2
+    // there, of 32 7.1 and 7.4, eight of 17 7.1 and 7.4 (eight of 20 behind 8 keys 8.9 and 7.6, heads of 64 level)
+    const int max_seq = a.max_seq > 0 ? a.max_seq : (int)std::min<int64_t>((int64_t)a.max_blocks * a.block_size, INT32_MAX);
+    if (D < a.B && a.max_q * hpg > 32 && max_seq > AM_KT && bias_pair_ok(a))
       return paged_attn_bias_pair(a.out, a.ldo, a.q, a.ldq, a.k_cache, a.v_cache, a.block_table + (int64_t)D * a.max_blocks, a.max_blocks, a.seq_lens + D, a.qsl + D, a.B - D, a.T - D,
-                                  a.max_q, a.H, a.G, a.dim, a.block_size, a.scale, a.chunk, a.bias_span, a.out_scale, st);
+                                  a.max_q, max_seq, a.H, a.G, a.dim, a.block_size, a.scale, a.chunk, a.bias_span, a.out_scale, st);
     if (D < a.B) {
       const int rows = a.max_q * hpg;
       const bool wide = rows > 32 && a.ldo % 2 == 0 && a.vdim % 2 == 0 && (reinterpret_cast<uintptr_t>(a.out) & 3) == 0;

@@ -647,12 +647,11 @@ int paged_attn_prefill_tc(bf16* out, const bf16* q, int q_stride, const bf16* kc
 #ifndef KGE_HALF
 // Prompts of a distance-biased, chunked attention (attn_bias.cu) with keys and values of 64 or 128, in the pair kernel.
 int paged_attn_bias_pair(void* out, int ldo, const void* q, int ldq, const void* kc, const void* vc, const int32_t* bt, int max_blocks, const int32_t* sl,
-                         const int32_t* qsl, int B, int T, int max_q_len, int H, int KV, int hd, int bs, float scale, int chunk, float span, float out_scale, cudaStream_t st) {
+                         const int32_t* qsl, int B, int T, int max_q_len, int max_seq_len, int H, int KV, int hd, int bs, float scale, int chunk, float span, float out_scale, cudaStream_t st) {
   int bs_shift = 0;
   while ((1 << bs_shift) < bs) ++bs_shift;
   const atc2::PairArgs pa{ldo, out_scale, chunk, span};
-  const int64_t reach = (int64_t)max_blocks * bs;
-  const int seen = (int)(chunk > 0 && chunk < reach ? chunk : reach);
+  const int seen = chunk > 0 && chunk < max_seq_len ? chunk : max_seq_len;
   auto run = hd == 128 ? launch_pair<128, true> : launch_pair<64, true>;
   return run(pa, (bf16*)out, (const bf16*)q, ldq, (const bf16*)kc, (const bf16*)vc, bt, max_blocks, sl, qsl, B, T, max_q_len, seen, H, KV, bs, bs_shift, scale, nullptr, st);
 }

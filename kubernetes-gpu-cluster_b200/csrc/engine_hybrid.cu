@@ -963,10 +963,10 @@ int hybrid_forward(kge_engine* e, int T, int B, int R, int max_blocks, const Ste
                       h.heads / h.kv_heads <= 128 && ((uintptr_t)e->pbuf & 15) == 0 &&
                       (!decode_only || (e->ws_attn && paged_attn_extras_decode_ok(B, h.heads, h.kv_heads, h.dim, bs)));
       // a decode step may be replayed as a graph while its contexts grow: sized for the longest context its block-table stride holds
-      const int max_seq_bound = decode_only ? max_blocks * bs : 0;
+      const int max_seq_bound = decode_only ? max_blocks * bs : *std::max_element(hm.seq_lens, hm.seq_lens + B);
       HFWD(decode_only ? C_ATT_DEC : C_ATT_GEN, (decode_only ? keys : (double)T) * h.kv_heads * (h.dim + h.vdim) * es + (double)T * h.heads * (h.dim + h.vdim) * es,
            2.0 * keys * h.heads * (h.dim + h.vdim),
-           tc ? paged_attn_extras(e->mixbuf, e->pbuf, ldp, L.kc, L.vc, m.btab, max_blocks, m.seq_lens, m.qsl, B, T, aa.max_q, std::max(max_seq_bound, 1),
+           tc ? paged_attn_extras(e->mixbuf, e->pbuf, ldp, L.kc, L.vc, m.btab, max_blocks, m.seq_lens, m.qsl, B, T, aa.max_q, max_seq_bound,
                                   h.heads, h.kv_heads, h.dim, bs, h.scale, h.softcap, L.sinks, e->ws_attn, e->ws_attn_bytes, st)
               : attn_bias_chunk(aa, st));
       DENSE(e->obuf1, d, e->mixbuf, ko, L.o, T, ACT_NONE);
@@ -1281,10 +1281,10 @@ int hybrid_forward(kge_engine* e, int T, int B, int R, int max_blocks, const Ste
       // Llama family (every head its own key/value head); everything else: the mma.sync / per-row kernels
       const bool tc = !e->f32 && (h.dim == 64 || h.dim == 128) && h.vdim == h.dim && ldq % 8 == 0 && (bs & (bs - 1)) == 0 && ((uintptr_t)q & 15) == 0 &&
                       (!decode_only || (e->ws_attn && paged_attn_extras_decode_ok(B, H, H, h.dim, bs)));
-      const int max_seq_bound = decode_only ? max_blocks * bs : 0;
+      const int max_seq_bound = decode_only ? max_blocks * bs : *std::max_element(hm.seq_lens, hm.seq_lens + B);
       HFWD(decode_only ? C_ATT_DEC : C_ATT_GEN, (decode_only ? keys : (double)T) * H * (h.dim + h.vdim) * es + (double)T * H * (h.dim + h.vdim) * es,
            2.0 * keys * H * (h.dim + h.vdim),
-           tc ? paged_attn_extras(e->mixbuf, q, ldq, L.kc, L.vc, m.btab, max_blocks, m.seq_lens, m.qsl, B, T, aa.max_q, std::max(max_seq_bound, 1), H, H, h.dim, bs,
+           tc ? paged_attn_extras(e->mixbuf, q, ldq, L.kc, L.vc, m.btab, max_blocks, m.seq_lens, m.qsl, B, T, aa.max_q, max_seq_bound, H, H, h.dim, bs,
                                   h.scale, 0.f, nullptr, e->ws_attn, e->ws_attn_bytes, st)
               : attn_bias_chunk(aa, st));
       if (h.out_gate) HFWD(C_ACT, (double)T * nv * 3 * es, 0, sigmoid_gate_mul(e->mixbuf, nv, at(e->pbuf, L.lat_g), ldp, T, nv, elt, st));
@@ -1306,7 +1306,7 @@ int hybrid_forward(kge_engine* e, int T, int B, int R, int max_blocks, const Ste
       aa.block_table = m.btab; aa.max_blocks = max_blocks; aa.seq_lens = m.seq_lens; aa.qsl = m.qsl; aa.positions = m.pos; aa.token_req = m.treq;
       aa.B = B; aa.T = T; aa.H = h.heads; aa.G = h.kv_heads; aa.dim = h.dim; aa.vdim = h.vdim; aa.block_size = bs; aa.chunk = h.chunk;
       aa.scale = h.scale; aa.bias_span = 8.f; aa.out_scale = h.left_scale; aa.elt = elt;
-      for (int r = 0; r < B; ++r) aa.max_q = std::max(aa.max_q, hm.qsl[r + 1] - hm.qsl[r]);
+      for (int r = 0; r < B; ++r) { aa.max_q = std::max(aa.max_q, hm.qsl[r + 1] - hm.qsl[r]); aa.max_seq = std::max(aa.max_seq, hm.seq_lens[r]); }
       while (aa.num_decode < B && hm.qsl[aa.num_decode + 1] - hm.qsl[aa.num_decode] == 1) ++aa.num_decode;
       double keys = 0;                                   // visible keys over all rows
       for (int t = 0; t < T; ++t) keys += h.chunk > 0 ? hm.pos[t] % h.chunk + 1 : hm.pos[t] + 1;
