@@ -44,14 +44,6 @@ __device__ __forceinline__ void tmem_ld32_nowait(uint32_t taddr, uint32_t* r) {
         "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
       : "r"(taddr));
 }
-__device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
-// keeps the registers' readers behind the wait
-__device__ __forceinline__ void tmem_tie32(uint32_t* r) {
-  asm volatile("" : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]), "+r"(r[8]), "+r"(r[9]), "+r"(r[10]), "+r"(r[11]),
-               "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15]));
-  asm volatile("" : "+r"(r[16]), "+r"(r[17]), "+r"(r[18]), "+r"(r[19]), "+r"(r[20]), "+r"(r[21]), "+r"(r[22]), "+r"(r[23]), "+r"(r[24]), "+r"(r[25]), "+r"(r[26]),
-               "+r"(r[27]), "+r"(r[28]), "+r"(r[29]), "+r"(r[30]), "+r"(r[31]));
-}
 __device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
   asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
@@ -386,7 +378,7 @@ attn_pair_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant
         uint32_t sv[BNK];
 #pragma unroll
         for (int c = 0; c < BNK; c += 32) tmem_ld32_nowait(t_s + c, &sv[c]);
-        tmem_wait_ld();
+        tmem_wait_ld(sv);
         tc_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(s_read(a));                         // the next tile's scores may be written
@@ -427,7 +419,7 @@ attn_pair_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant
               asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
                            : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]),
                              "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]) : "r"(t_o + c));
-              tmem_wait_ld();
+              tmem_wait_ld(v);
 #pragma unroll
               for (int i = 0; i < 16; ++i) v[i] = __float_as_uint(__uint_as_float(v[i]) * alpha);
               tmem_st16(t_o + c, v);
@@ -494,13 +486,13 @@ attn_pair_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant
         uint32_t v[64];
         tmem_ld32_nowait(t_o + c, v);
         tmem_ld32_nowait(t_o + c + 32, v + 32);
-        tmem_wait_ld();
+        tmem_wait_ld(v);
         if (it.split) {
 #pragma unroll
           for (int h = 0; h < 64; h += 32) {
             uint32_t u[32];
             tmem_ld32_nowait(t_o + 128 + c + h, u);
-            tmem_wait_ld();
+            tmem_wait_ld(u);
 #pragma unroll
             for (int i = 0; i < 32; ++i) v[h + i] = __float_as_uint(__uint_as_float(v[h + i]) * mine + __uint_as_float(u[i]) * other);
           }

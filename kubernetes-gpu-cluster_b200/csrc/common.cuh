@@ -160,6 +160,18 @@ inline cudaError_t launch_pdl(void (*kern)(KArgs...), dim3 grid, dim3 block, siz
   return cudaLaunchKernelEx(&cfg, kern, KArgs(args)...);
 }
 
+// Waits for this thread's loads from TMEM into the registers `r`, and keeps what reads them behind the wait: the loads only name registers
+// that are filled some time later, and arithmetic on them is not held back by a wait that does not name them.
+template <int... N>
+__device__ __forceinline__ void tmem_wait_ld(uint32_t (&...r)[N]) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+  auto hold = [](auto& a) {
+#pragma unroll
+    for (uint32_t& v : a) asm volatile("" : "+r"(v));
+  };
+  (hold(r), ...);
+}
+
 // One lane of a converged warp, for the instructions that one thread issues (TMA copies, tcgen05.mma, commits).  Behind this
 // branch the compiler knows that a single lane runs and keeps descriptors and addresses in uniform registers, where those
 // instructions want them; behind `lane == 0` it moves them there before each one, which paced the MMA loops: 88 cycles to issue

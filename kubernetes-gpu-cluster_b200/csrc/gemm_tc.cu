@@ -92,7 +92,7 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
                  "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
                : "r"(taddr));
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+  tmem_wait_ld(r);
 }
 
 // 16 TMEM lanes x 8 G columns as MMA accumulator fragments: register 4 k + i holds lane (l / 4) + 8 (i / 2), column 8 k + 2 (l % 4) + i % 2.
@@ -109,7 +109,6 @@ __device__ __forceinline__ void tmem_ld_frag(uint32_t taddr, uint32_t (&r)[4 * G
     asm volatile("tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]) : "r"(taddr));
 }
-__device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void stsm_trans(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
   asm volatile("stmatrix.sync.aligned.m8n8.x4.trans.shared.b16 [%0], {%1,%2,%3,%4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
 }
@@ -591,7 +590,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant
             uint32_t r[2][4 * G];
             tmem_ld_frag<G>(taddr + c, r[0]);
             tmem_ld_frag<G>(taddr + c + (16u << 16), r[1]);
-            tmem_wait_ld();
+            tmem_wait_ld(r[0], r[1]);
 #pragma unroll
             for (int quad = 0; quad < 8; ++quad) {
               const uint32_t* v = &r[quad >> 2][(quad & 3) * 4];
@@ -608,7 +607,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant
           uint32_t r[2][4 * G];
           tmem_ld_frag<G>(taddr + c, r[0]);
           tmem_ld_frag<G>(taddr + c + (16u << 16), r[1]);
-          tmem_wait_ld();
+          tmem_wait_ld(r[0], r[1]);
           if constexpr (SPLIT) {
             float sum[2][4 * G];
 #pragma unroll

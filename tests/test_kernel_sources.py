@@ -44,3 +44,15 @@ def test_barrier_waits_are_bounded_by_the_clock():
     assert users == {"common.cuh"}
     src = open(os.path.join(CSRC, "common.cuh")).read()
     assert 1e9 <= int(re.search(r"kBarrierCycles = (\d+)ll", src).group(1)) <= 2e10
+
+
+def test_waits_for_tensor_memory_hold_back_what_reads_it():
+    """A load from tensor memory names registers that are filled later: a wait that does not name them holds back no arithmetic on them."""
+    waits = 0
+    for path in sorted(glob.glob(os.path.join(CSRC, "*.cu*"))):
+        src = re.sub(r"//[^\n]*", "", open(path).read())
+        assert ("tcgen05.wait::ld" in src) == path.endswith("common.cuh"), path
+        for call in re.findall(r"tmem_wait_ld\(([^()]*)\);", src):
+            assert call, path
+            waits += 1
+    assert waits >= 8
