@@ -144,7 +144,7 @@ norm_kernel(bf16* __restrict__ y, bf16* __restrict__ residual, const bf16* __res
 // The same for many rows: a CTA goes through rows with the next two of each thread group on their way (cp.async into pieces of shared
 // memory that the same thread reads back), weights in registers.  GT threads a row, four 16-byte pieces each; one barrier a sum.
 // The kernel above is a chain of load, sum and store per CTA and keeps 60 KB an SM in flight at best.  us above and here: RMSNorm of
-// 8192 x 4096 35.1 / 30.9 (20.5 at the rate of a copy), of 8192 x 768 10.7 / 8.3, LayerNorm of 8192 x 2048 31.7 / 16.9.
+// 8192 x 4096 35.1 / 30.0 (20.5 at the rate of a copy), of 8192 x 768 10.7 / 8.3, LayerNorm of 8192 x 2048 31.7 / 16.9.
 constexpr int kNormStages = 3, kNormThreads = 256;
 template <int MODE> constexpr int norm_rows_smem() { return kNormStages * (MODE == 1 || MODE == 3 ? 2 : 1) * kMaxVecPerThread * kNormThreads * 16; }
 
@@ -460,9 +460,10 @@ static int norm_common(int mode, void* y, void* residual, const void* x, const v
     return mode == 0 ? launch_norm_rows<0>(gt, y, residual, x, w, b, T, d, eps, s) : mode == 1 ? launch_norm_rows<1>(gt, y, residual, x, w, b, T, d, eps, s)
          : mode == 2 ? launch_norm_rows<2>(gt, y, residual, x, w, b, T, d, eps, s) : launch_norm_rows<3>(gt, y, residual, x, w, b, T, d, eps, s);
   }
-  // weights early up to two rows an SM: 64 x 4096 1.95 us, 2.12 with them behind the reduction, 256 x 4096 3.25 / 3.7; 1339 x 2048 5.8 / 5.0
-  // (plain RMSNorm of rows up to 2048 keeps them there: one of 32 x 2048, its projection to 128256 and sampling 136.7 early, 136.1 so)
-  const bool early = T <= 2 * 148 && (mode != 0 || d > 2048);
+  // weights early up to two rows an SM, us there and behind the reduction: RMSNorm of 1 x 512 1.25 / 1.36, 32 x 2048 1.54 / 1.64, 296 x 2048
+  // 1.69 / 2.28 (with the projection behind it 7.27 / 7.35 at 32 x 2048, faster or level at all of 512 to 4096 by 1 to 296; only
+  // with the head's projection and sampling behind it 136.0 / 135.7); 1339 x 2048 5.8 / 5.0
+  const bool early = T <= 2 * 148;
   auto kern = early ? (mode == 0 ? norm_kernel<0, true> : mode == 1 ? norm_kernel<1, true> : mode == 2 ? norm_kernel<2, true> : norm_kernel<3, true>)
                     : (mode == 0 ? norm_kernel<0, false> : mode == 1 ? norm_kernel<1, false> : mode == 2 ? norm_kernel<2, false> : norm_kernel<3, false>);
   KGE_CUDA_OK(launch_pdl(kern, dim3(T), dim3(th), 0, s, (bf16*)y, (bf16*)residual, (const bf16*)x, (const bf16*)w,
