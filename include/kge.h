@@ -295,6 +295,7 @@ int kge_engine_eos_token_id(const kge_engine* e);
 int kge_engine_max_model_len(const kge_engine* e);
 int64_t kge_engine_weight_bytes(const kge_engine* e);
 int64_t kge_engine_launches(const kge_engine* e);
+int kge_engine_decode_graphs(const kge_engine* e);      /* captured decode steps that the engine keeps */
 
 /* Host-only view of a model directory - what kge_engine_create reads, without a GPU (tests, tooling):
  * config.json -> the model description as JSON; *.safetensors tensors (all shards, BF16 / F16 / F32) sliced and

@@ -113,6 +113,7 @@ SIGNATURES = {
     "kge_engine_max_model_len": (_I, [_P]),
     "kge_engine_weight_bytes": (_L, [_P]),
     "kge_engine_launches": (_L, [_P]),
+    "kge_engine_decode_graphs": (_I, [_P]),
     "kge_step": (_I, [_P, C.POINTER(StepBatch), _P, _P]),
     "kge_engine_set_timing": (_I, [_P, _I]),
     "kge_engine_get_timing": (_I, [_P, _P]),
@@ -351,6 +352,10 @@ class LLM:
     @property
     def kernel_launches(self) -> int:
         return lib().kge_engine_launches(self._h)
+
+    @property
+    def decode_graphs(self) -> int:
+        return lib().kge_engine_decode_graphs(self._h)
 
     def set_timing(self, enable: bool):
         check(lib().kge_engine_set_timing(self._h, int(enable)), "kge_engine_set_timing")

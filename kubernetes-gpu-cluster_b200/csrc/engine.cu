@@ -525,3 +525,4 @@ extern "C" int kge_engine_eos_token_id(const kge_engine* e) { return e ? e->spec
 extern "C" int kge_engine_max_model_len(const kge_engine* e) { return e ? e->cfg.max_model_len : 0; }
 extern "C" int64_t kge_engine_weight_bytes(const kge_engine* e) { return e ? e->weight_bytes : 0; }
 extern "C" int64_t kge_engine_launches(const kge_engine* e) { return e ? e->launches : 0; }
+extern "C" int kge_engine_decode_graphs(const kge_engine* e) { return e ? (int)e->graphs.size() : 0; }

@@ -131,6 +131,7 @@ extern "C" int kge_engine_run_resident(kge_engine* e, const int32_t* prompts_hos
   cudaEventCreate(&ev0); cudaEventCreate(&ev1); cudaEventCreate(&ev2);
   KGE_CUDA_OK(cudaStreamSynchronize(e->stream));
 
+  e->want_logits32 = false;                  // whatever the last step's caller asked for
   // ---- timed region: nothing but kernel launches and device-to-device id hand-offs
   int rc = 0;
   cudaEventRecord(ev0, e->stream);
@@ -232,6 +233,7 @@ extern "C" int kge_engine_replay_recorded(kge_engine* e, int32_t* out_tokens_hos
   cudaEvent_t ev0, ev1, ev2;
   cudaEventCreate(&ev0); cudaEventCreate(&ev1); cudaEventCreate(&ev2);
   KGE_CUDA_OK(cudaStreamSynchronize(e->stream));
+  e->want_logits32 = false;                  // whatever the last step's caller asked for
   // ---- timed region: device-to-device metadata moves, the id patch, and the step's kernels
   int rc = 0;
   cudaEventRecord(ev0, e->stream);

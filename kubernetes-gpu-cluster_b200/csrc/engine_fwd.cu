@@ -219,13 +219,14 @@ int engine_decode_step(kge_engine* e, int B, int stride, int max_seq_len, const 
   };
   if (!e->use_graphs || e->timing || e->step_num_masks > 0 || e->layer_dump_host)      // a masked step is rare and its mask list is not part of a graph
     return forward();
+  const bool logits = hybrid && e->want_logits32;      // only layer-list models launch anything for logits that are read back
   for (auto& g : e->graphs)
-    if (g.B == B && g.ns == ns && g.stride == stride && g.rnd == any_random && g.logits == e->want_logits32) {
+    if (g.B == B && g.ns == ns && g.stride == stride && g.rnd == any_random && g.logits == logits) {
       KGE_CUDA_OK(cudaGraphLaunch(g.exec, e->stream));
       e->launches += g.launches;
       return 0;
     }
-  const int64_t key = ((int64_t)B << 40) ^ ((int64_t)ns << 32) ^ ((int64_t)stride << 2) ^ (e->want_logits32 ? 2 : 0) ^ (any_random ? 1 : 0);
+  const int64_t key = ((int64_t)B << 40) ^ ((int64_t)ns << 32) ^ ((int64_t)stride << 2) ^ (logits ? 2 : 0) ^ (any_random ? 1 : 0);
   int* seen = nullptr;
   for (auto& kv : e->graph_seen) if (kv.first == key) seen = &kv.second;
   if (!seen) { e->graph_seen.push_back({key, 0}); seen = &e->graph_seen.back().second; }
@@ -240,7 +241,7 @@ int engine_decode_step(kge_engine* e, int B, int stride, int max_seq_len, const 
   cudaError_t ce = cudaStreamEndCapture(e->stream, &graph);
   if (rc) { if (graph) cudaGraphDestroy(graph); return rc; }
   KGE_REQUIRE(ce == cudaSuccess && graph, "decode graph capture failed: %s", cudaGetErrorString(ce));
-  kge_engine::DecodeGraph g{B, ns, stride, any_random, e->want_logits32, nullptr, e->launches - l0};
+  kge_engine::DecodeGraph g{B, ns, stride, any_random, logits, nullptr, e->launches - l0};
   ce = cudaGraphInstantiate(&g.exec, graph, 0);
   cudaGraphDestroy(graph);
   KGE_REQUIRE(ce == cudaSuccess, "cudaGraphInstantiate failed: %s", cudaGetErrorString(ce));

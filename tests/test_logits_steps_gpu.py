@@ -3,6 +3,7 @@ import numpy as np
 import pytest
 import torch
 
+from oracle import hybrid as oh
 from oracle import model as om
 
 pytestmark = pytest.mark.gpu
@@ -42,3 +43,36 @@ def test_replayed_steps_return_the_logits_of_eager_ones(kge, tmp_path, B):
         assert np.array_equal(tokens, once[0][0]) and np.array_equal(logits, once[0][1])
     for (t0, l0), (t1, l1) in zip(once[1:], often[11:]):       # replayed in one engine from here on, eager in the other up to the eighth
         assert np.array_equal(t0, t1) and np.array_equal(l0, l1)
+
+
+def decode_llm(kge, path, B, bs=16, per=4):
+    """An engine and a function that runs the same decode step of B requests again."""
+    llm = kge.LLM(str(path), max_model_len=64, max_num_seqs=4, max_num_batched_tokens=128, block_size=bs, num_gpu_blocks_override=B * per + 1, enable_prefix_caching=False)
+    table = 1 + np.arange(B * per, dtype=np.int32).reshape(B, per)
+    at = np.arange(B + 1, dtype=np.int32)
+
+    def step(want):
+        return llm.raw_step(np.full(B, 5, dtype=np.int32), np.zeros(B, dtype=np.int32), at, np.ones(B, dtype=np.int32), table, per, table[:, 0].astype(np.int64) * bs, at[:B], want_logits=want)
+    return llm, step
+
+
+def test_steps_that_launch_the_same_share_a_graph(kge, tmp_path):
+    cfg = om.CONFIGS["tiny-llama"]
+    om.save_model_dir(tmp_path, cfg, om.make_weights(cfg, seed=0))
+    llm, step = decode_llm(kge, tmp_path, 2)
+    eager = step(True)
+    for want in [False] * 2 + [True] * 12:
+        got = step(want)
+        assert llm.decode_graphs <= 1
+    assert llm.decode_graphs == 1 and all(np.array_equal(a, b) for a, b in zip(eager, got))
+    llm.close()
+
+
+def test_layer_list_steps_with_logits_have_a_graph_of_their_own(kge, tmp_path):
+    cfg = oh.make_config()
+    oh.save_model_dir(str(tmp_path), cfg, oh.make_weights(cfg, seed=0))
+    llm, step = decode_llm(kge, tmp_path, 2)
+    for want, graphs in [(False, 0), (False, 1), (True, 1)] + [(True, 1)] * 7 + [(True, 2)] * 2 + [(False, 2)]:
+        step(want)
+        assert llm.decode_graphs == graphs
+    llm.close()
