@@ -64,3 +64,17 @@ def test_block_diagonal_gates_of_many_rows(kge, tmp_path, width, blocks, rows):
     llm = make_engine(kge, tmp_path, cfg, W, "bfloat16")
     check(run_pieces(llm, 0, toks, [rows]), oh.forward(cfg, W, toks), "bfloat16")
     llm.close()
+
+
+@pytest.mark.parametrize("hd", [64, 128])
+def test_short_biased_pieces(kge, tmp_path, hd):
+    """Pieces around the length from which on prompts run in the tcgen05 kernel: the last whose keys are one tile of the other, and the next."""
+    cfg = oh.make_config(layers=("parallel",), mlps=(None,), right_scale=0.0, chunk=1024, scale=3.0 / hd ** 0.5, dim=hd, vdim=hd)
+    W = oh.make_weights(cfg, seed=37)
+    toks = prompt(cfg, 70)
+    want = oh.forward(cfg, W, toks)
+    llm = make_engine(kge, tmp_path, cfg, W, "bfloat16", tokens=160)
+    for rid, pieces in enumerate([[32, 33, 5], [31, 1, 38], [33, 37], [20, 20, 30]]):
+        check(run_pieces(llm, rid, toks, pieces), want, "bfloat16", f"pieces {pieces}")
+        llm.trace_end(rid)
+    llm.close()
