@@ -499,12 +499,13 @@ int attn_bias_chunk(const AttnBiasArgs& a, cudaStream_t st) {
       a.H % a.G == 0 && a.v_ld % 8 == 0 && (reinterpret_cast<uintptr_t>(a.q) & 3) == 0 && a.B <= 65535 && a.G <= 65535) {
     const int hpg = a.H / a.G;
     // a tile for all warps (ROWS), or one each, their statistics and, in a cluster, the CTA's sums
-    const size_t tile = (size_t)AM_KT * (a.dim + a.vdim + 2 * AM_PAD) * 2, split = AM_WARPS * tile + (size_t)AM_WARPS * 2 * 16 * 4, sums = (size_t)16 * (a.vdim + 2) * 4;
-    static size_t smem_set = 0;                       // opt in once per size that needs more than the default 48 KB
-    if (split + sums > 48 * 1024 && split + sums > smem_set) {
-      KGE_CUDA_OK(cudaFuncSetAttribute(attn_bias_mma_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(split + sums)));
-      smem_set = split + sums;
-    }
+    auto tile_of = [](int dim, int vdim) { return (size_t)AM_KT * (dim + vdim + 2 * AM_PAD) * 2; };
+    auto split_of = [&](int dim, int vdim) { return AM_WARPS * tile_of(dim, vdim) + (size_t)AM_WARPS * 2 * 16 * 4; };
+    auto sums_of = [](int vdim) { return (size_t)16 * (vdim + 2) * 4; };
+    const size_t tile = tile_of(a.dim, a.vdim), split = split_of(a.dim, a.vdim), sums = sums_of(a.vdim);
+    // the function's limit on this device, for every size
+    if (split + sums > 48 * 1024)
+      KGE_CUDA_OK(cudaFuncSetAttribute(attn_bias_mma_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(split_of(AM_MAXD, AM_MAXD) + sums_of(AM_MAXD))));
     // the leading one-token requests, then the rest; 64-row CTAs where a request has that many rows and its output
     // pairs can be stored as 32-bit words
     const int D = std::min(std::max(a.num_decode, 0), a.B);

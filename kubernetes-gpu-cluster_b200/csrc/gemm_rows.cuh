@@ -243,7 +243,8 @@ template <int NT, int S>
 static int launch_norm_rows(const bf16* w, const GemmParams& p, const RowsNorm& nm, const RowsKv& kv, cudaStream_t st) {
   auto kern = gemm_rows_kernel<8, NT, 1, false, S, true>;
   const int smem = rows_smem(8, NT, 0, S) + p.T * norm_row_bytes(p.K);
-  KGE_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  // the function's limit, for every size: one set for this call could be lowered by another thread's before the launch
+  KGE_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, rows_smem(8, NT, 0, S) + 8 * norm_row_bytes(32 * 8 * kNormVecs)));
   KGE_CUDA_OK(launch_pdl(kern, dim3((p.N + 8 * NT - 1) / (8 * NT)), dim3(8 * 32), smem, st, nullptr, w, p, nm, kv));
   return 0;
 }

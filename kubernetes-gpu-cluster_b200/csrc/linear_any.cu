@@ -684,7 +684,7 @@ int linear_any(const LinearArgs& a, cudaStream_t st) {
   if (linear_short_ok(a)) {
     const size_t smem = (size_t)(WBM + WBN) * (a.K + MPAD) * 2;
     auto kern = a.act == ACT_SOFTPLUS ? linear_short_kernel<ACT_SOFTPLUS> : a.act == ACT_EXP_DECAY ? linear_short_kernel<ACT_EXP_DECAY> : linear_short_kernel<ACT_NONE>;
-    KGE_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    KGE_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (WBM + WBN) * (WMAXK + MPAD) * 2));      // for every K
     KGE_CUDA_OK(launch_pdl(kern, dim3((a.N + WBN - 1) / WBN, (a.T + WBM - 1) / WBM, a.nz), dim3(256), smem, st, a));
     return 0;
   }
