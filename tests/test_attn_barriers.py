@@ -5,6 +5,8 @@ import re
 
 import pytest
 
+import barrier_explorer
+
 SRC = os.path.join(os.path.dirname(__file__), "..", "kubernetes-gpu-cluster_b200", "csrc", "attn_tc.cu")
 
 # every barrier operation of the kernel after the barriers' set-up, in the order of the source: what the programs below transcribe
@@ -88,57 +90,12 @@ def programs(n, tma, o_bars, last):
 
 
 def explore(n, tma, o_bars=2, last=None):
-    """Whether some order leaves a role waiting for ever.  Two softmax threads; MMAs complete in order, copies in any."""
+    """What can go wrong (barrier_explorer), with two softmax threads."""
     issuer, producer, soft = programs(n, tma, o_bars, [n - 1] if last is None else last)
     roles = [issuer, producer, soft, soft]
     need = {"q": 2, "p": 2, "k": 1 if tma else 2, "v": 1 if tma else 2}
-    bars = sorted({b for r in roles for op in r for b in (op[1] if op[0] == "mma" else (op[1],))})
-    index = {b: i for i, b in enumerate(bars)}
-
-    def arrive(state, bar):
-        done, got = state[index[bar]]
-        got += 1
-        if got == need.get(bar[0], 1):
-            done, got = done + 1, 0
-        return state[:index[bar]] + ((done, got),) + state[index[bar] + 1:]
-
-    start = ((0,) * 4, ((0, 0),) * len(bars), (), ())
-    seen, todo, stuck = {start}, [start], False
-    while todo:
-        pcs, state, pipe, loads = todo.pop()
-        succ = []
-        for r, prog in enumerate(roles):
-            if pcs[r] == len(prog):
-                continue
-            op = prog[pcs[r]]
-            nxt = pcs[:r] + (pcs[r] + 1,) + pcs[r + 1:]
-            if op[0] in ("wait", "maybe"):
-                if op[0] == "maybe":
-                    succ.append((nxt, state, pipe, loads))
-                done = state[index[op[1]]][0]
-                if (done & 1) != (op[2] & 1):                # mbarrier.try_wait.parity
-                    assert done > op[2], "a wait passed before its phase"
-                    succ.append((nxt, state, pipe, loads))
-            elif op[0] == "arrive":
-                succ.append((nxt, arrive(state, op[1]), pipe, loads))
-            elif op[0] == "mma":
-                succ.append((nxt, state, pipe + (op[1],), loads))
-            else:
-                succ.append((nxt, state, pipe, tuple(sorted(loads + (op[1],)))))
-        if pipe:
-            s = state
-            for b in pipe[0]:
-                s = arrive(s, b)
-            succ.append((pcs, s, pipe[1:], loads))
-        for i, b in enumerate(loads):
-            succ.append((pcs, arrive(state, b), pipe, loads[:i] + loads[i + 1:]))
-        if not succ and any(pcs[r] < len(prog) for r, prog in enumerate(roles)):
-            stuck = True
-        for s in succ:
-            if s not in seen:
-                seen.add(s)
-                todo.append(s)
-    return stuck
+    roles = [[(*op, (), ()) if op[0] == "mma" else (*op, None) if op[0] == "load" else op for op in r] for r in roles]
+    return barrier_explorer.explore(roles, need)
 
 
 @pytest.mark.parametrize("tma", [True, False])

@@ -6,6 +6,8 @@ import re
 
 import pytest
 
+import barrier_explorer
+
 SRC = os.path.join(os.path.dirname(__file__), "..", "kubernetes-gpu-cluster_b200", "csrc", "attn_pair.cuh")
 
 # every barrier operation of the kernel after the barriers' set-up, in the order of the source: what the programs below transcribe
@@ -43,10 +45,10 @@ def test_transcription_matches_the_kernel():
     assert barrier_ops() == OPS
 
 
-def programs(items, nst):
+def programs(items, nst, turns_from=3):
     """Instruction lists of the roles.  items: (key tiles of the first query tile, of the second[, whether they share the key tiles of one
-    query tile between them[, whether values beyond the last key are cleared]]).  BAR: a barrier of the two groups of softmax threads.  An
-    MMA is ("mma", barriers that it commits to, buffers it reads, buffers it writes); a copy ("load", barrier, buffer)."""
+    query tile between them[, whether values beyond the last key are cleared]]).  turns_from: key tiles of the second query tile from
+    which on the two groups of softmax threads take turns."""
     def wait(bar, k, optional=False):
         return ("maybe" if optional else "wait", bar, k)
     prod, nk, end = [], 0, len(items)
@@ -102,102 +104,59 @@ def programs(items, nst):
         issue.append(wait(("item_full", end & 1), end >> 1))
         roles.append(issue)
     for a in range(2):
-        s, ns, nb, nt = [], 0, 0, 0
+        s, ns, joined = [], 0, {}
+
+        def join(bar, meet):
+            s.append(("join", (bar,), a))
+            if meet:                                             # bar.sync
+                s.append(("meet", (bar,), joined.get(bar, 0)))
+            joined[bar] = joined.get(bar, 0) + 1
         for ni, nn in enumerate(items):
             s += [wait(("item_full", ni & 1), ni >> 1), ("arrive", ("item_empty", ni & 1))]
-            turns = nn[1] >= 3
             for j in range(nn[a]):
                 s += [wait(("s_full", a), ns), ("read", ("s", a)), ("arrive", ("s_read", a))]
                 if j:
                     s += [wait(("o_full", a, (ns - 1) & 1), (ns - 1) >> 1, True)]        # only where a row's maximum has grown
                 if ns >= 2:
                     s.append(wait(("o_full", a, ns & 1), (ns - 2) >> 1))
-                if turns and j == 0:
-                    s += [("arrive", ("bar1",))] + ([wait(("bar1",), nt)] if a else [])
-                    nt += 1
-                s += [("write", ("p", a, ns & 1)), ("arrive", ("p_full", a, ns & 1))]
+                turn = nn[1] >= turns_from and j == 0
+                if turn and a:
+                    join("bar1", True)
+                s.append(("write", ("p", a, ns & 1)))
+                if turn and not a:
+                    join("bar1", False)
+                s.append(("arrive", ("p_full", a, ns & 1)))
                 ns += 1
             if nn[a]:
                 s += [wait(("o_full", a, (ns - 1) & 1), (ns - 1) >> 1), ("read", ("o", a))]
             if nn[2]:
-                s += [("arrive", ("bar2",)), wait(("bar2",), nb)] + ([] if a else [("read", ("o", 1))]) + [("arrive", ("bar3",)), wait(("bar3",), nb)]
-                nb += 1
+                join("bar2", True)
+                if not a:
+                    s.append(("read", ("o", 1)))
+                join("bar3", True)
         s.append(wait(("item_full", end & 1), end >> 1))
         roles.append(s)
     return roles
 
 
-def explore(items, nst, only=None, drop=None):
-    """True if some order leaves a role waiting for ever, or lets a buffer be written while an MMA in flight uses it.  An issuer's MMAs
-    complete in the order of issue, copies in any.  only: the query tile whose roles are run (the other's arrivals are taken out), which
-    keeps the number of states small; drop: a wait that is left out."""
-    roles = programs(items, nst)
-    need = {"item_empty": 4, "k_empty": 2, "v_empty": 2, "q_empty": 2, "bar1": 2, "bar2": 2, "bar3": 2}
+def explore(items, nst, only=None, drop=None, turns_from=3, rings=True):
+    """What can go wrong (barrier_explorer).  only: the query tile whose roles are run (the other's arrivals are taken out), which keeps the
+    number of states small; so does rings: False, keys and values are always there (more orders than there are, of fewer roles' steps).
+    drop: a wait that is left out."""
+    roles = programs(items, nst, turns_from)
+    need = {"item_empty": 4, "k_empty": 2, "v_empty": 2, "q_empty": 2}
     if only is not None:
         roles = [roles[0], roles[1 + only], roles[3 + only]]
         need = {"item_empty": 2}
         roles = [[op for op in r if op[0] == "mma" or op[1][0][:3] != "bar" and op[1][0] != "v_clean"] for r in roles]
     if drop:
         roles = [[op for op in r if not (op[0] == "wait" and op[1][0] == drop)] for r in roles]
-    bars = sorted({b for r in roles for op in r for b in (op[1] if op[0] == "mma" else [op[1]] if op[0] in ("wait", "maybe", "arrive", "load") else [])}, key=str)
-    index = {b: i for i, b in enumerate(bars)}
-    mmas = [[op for op in r if op[0] == "mma"] for r in roles]
-    before = [[sum(op[0] == "mma" for op in r[:i]) for i in range(len(r) + 1)] for r in roles]
-
-    def arrive(state, bar):
-        done, got = state[index[bar]]
-        got += 1
-        if got == need.get(bar[0], 1):
-            done, got = done + 1, 0
-        return state[:index[bar]] + ((done, got),) + state[index[bar] + 1:]
-
-    start = ((0,) * len(roles), ((0, 0),) * len(bars), (0,) * len(roles), ())            # positions, barriers, MMAs done, copies in flight
-    seen, todo = {start}, [start]
-    while todo:
-        pcs, state, done_mma, loads = todo.pop()
-        flight = [f for m, d, b, pc in zip(mmas, done_mma, before, pcs) for f in m[d:b[pc]]]
-        succ = []
-        for r, prog in enumerate(roles):
-            if pcs[r] == len(prog):
-                continue
-            op = prog[pcs[r]]
-            nxt = pcs[:r] + (pcs[r] + 1,) + pcs[r + 1:]
-            if op[0] in ("wait", "maybe"):
-                if op[0] == "maybe":
-                    succ.append((nxt, state, done_mma, loads))
-                done = state[index[op[1]]][0]
-                if (done & 1) != (op[2] & 1):                    # mbarrier.try_wait.parity
-                    if done != op[2] + 1:
-                        return True
-                    succ.append((nxt, state, done_mma, loads))
-            elif op[0] == "arrive":
-                succ.append((nxt, arrive(state, op[1]), done_mma, loads))
-            elif op[0] == "load":
-                if any(op[2] in f[2] for f in flight):           # a copy into what an MMA reads
-                    return True
-                succ.append((nxt, state, done_mma, tuple(sorted(loads + (op[1:],), key=str))))
-            else:
-                # threads: what an MMA in flight writes may not be read, what it reads may not be written
-                if op[0] == "read" and any(op[1] in f[3] for f in flight) or op[0] == "write" and any(op[1] in f[2] for f in flight):
-                    return True
-                if op[0] == "write" and any(op[1] == buf for _, buf in loads):
-                    return True                                  # nor what a copy in flight writes
-                succ.append((nxt, state, done_mma, loads))
-        for r, m in enumerate(mmas):
-            if done_mma[r] < before[r][pcs[r]]:
-                s = state
-                for b in m[done_mma[r]][1]:
-                    s = arrive(s, b)
-                succ.append((pcs, s, done_mma[:r] + (done_mma[r] + 1,) + done_mma[r + 1:], loads))
-        for i, (b, _) in enumerate(loads):
-            succ.append((pcs, arrive(state, b), done_mma, loads[:i] + loads[i + 1:]))
-        if not succ and any(pcs[r] < len(prog) for r, prog in enumerate(roles)):
-            return True
-        for s in succ:
-            if s not in seen:
-                seen.add(s)
-                todo.append(s)
-    return False
+    if not rings:
+        ring = {"k_full", "k_empty", "v_full", "v_empty", "v_clean"}
+        roles = [[("mma", [b for b in op[1] if b[0] not in ring], *op[2:]) if op[0] == "mma" else op for op in r
+                  if op[0] == "mma" or not (op[1][0] in ring or op[0] == "write" and op[1][0] == "v")] for r in roles]
+        roles = [[op for op in r if op[0] != "mma" or op[1]] for r in roles]
+    return barrier_explorer.explore(roles, need)
 
 
 @pytest.mark.parametrize("items", [[(1, 0)], [(1, 1)], [(1, 2)], [(1, 0), (1, 1)], [(1, 1, 1), (1, 0)], [(2, 1, 1)], [(3, 3)]], ids=str)
@@ -232,3 +191,15 @@ def test_cleared_values_of_one_query_tile_in_every_order(items, nst, only):
 def test_the_exploration_finds_values_that_are_cleared_too_early_or_not_waited_for():
     assert explore([(3, 3, 0, 1)], 2, 0, "v_full")
     assert explore([(1, 1, 0, 1)], 2, None, "v_clean")
+
+
+@pytest.mark.parametrize("items", [[(3, 3), (3, 3)], [(1, 3), (4, 3)], [(3, 3), (1, 1), (3, 3)], [(1, 1, 1), (3, 3), (2, 1, 1)], [(1, 1, 1), (1, 1, 1)]], ids=str)
+def test_turns_of_items_in_sequence(items):
+    assert not explore(items, 4, rings=False)
+
+
+@pytest.mark.parametrize("turns_from", [1, 2])
+def test_the_exploration_finds_turns_that_begin_too_early(turns_from):
+    """The first group must not come to its next item's handshake before the second has passed this one."""
+    n = turns_from
+    assert "arrives twice" in explore([(n, n), (n, n)], 4, turns_from=n, rings=False)
