@@ -551,19 +551,19 @@ static int launch_tc(bf16* out, const bf16* q, int q_stride, const bf16* kc, con
   CUtensorMap tk, tv;
   const bool tma = tunable(TUN_ATTN_TMA) != 0 && bs >= 8;
   // Two query tiles per CTA (attn_pair.cuh) but for small launches: there its 384 threads, all of TMEM and 226 KB start later than two of
-  // these CTAs per SM.  Measured over 9238 launches (1 to 64 requests, 1 to 12 kv heads, groups of 1 to 8, heads of 64 and 128, contexts up to
-  // 3600), time there over time here, by query tiles and longest context:
-  //     tiles        to 320    to 640   to 1280   to 2560    beyond
-  //     to 37          1.37      1.15      1.06      1.01      0.97
-  //     to 148         1.24      1.08      1.00      0.91      0.90
-  //     to 296         1.26      1.06      0.99      0.99      0.95
-  //     beyond         0.95      0.80      0.81      0.90      0.93
-  // Up to 37 tiles little but the start counts; up to 148 an item there has an SM and two groups of warps for its keys; up to 296 they take two
-  // rounds there and one here.  CTAs without a query tile (short requests beside long ones) cost this kernel their start: up to 1000 CTAs.  Short
-  // contexts are nearly all start: those of at most 296 tiles' tokens stay here up to six CTAs an SM.  So 2 % of the launches are more than 3 %
-  // slower there than here would be, 21 % with a line of T * KV <= 256 tiles' tokens and contexts up to 320.
+  // these CTAs per SM, and small blocks are more copies for its one producer.  Measured over 15007 launches (1 to 64 requests, 1 to 12 kv heads,
+  // groups of 1 to 8, heads of 64 and 128, up to 1000 CTAs here), time there over time here, by longest context:
+  //                                      to 320    to 640   to 1280   to 2048    beyond
+  //     to 296 query tiles, blocks of 64+   1.34      1.07      0.96      0.87      0.84
+  //                                   32    1.35      1.11      1.03      0.97      0.93
+  //                                   16    1.33      1.15      1.08      1.03      1.03
+  //                                    8    1.37      1.18      1.11      1.08      1.05
+  //     more tiles                          1.05      0.95      0.93      0.92      0.92
+  // CTAs without a query tile (short requests beside long ones) cost this kernel their start: up to 1000 CTAs.  Short contexts are nearly all
+  // start: those of at most 296 tiles' tokens stay here up to six CTAs an SM.  3 % of these launches are more than 3 % slower there than here
+  // would be, and 2 % here than there.
   const int64_t launched = (int64_t)grid.x * grid.y * grid.z, tiles = std::min(launched, KV * ((int64_t)T / TT + B));
-  const bool small = (launched <= 1000 && tiles <= 296 && max_seq_len <= (tiles <= 37 ? 2048 : tiles <= 148 ? 1024 : 1800)) ||
+  const bool small = (launched <= 1000 && tiles <= 296 && max_seq_len <= (bs <= 16 ? 2048 : bs == 32 ? 1280 : 640)) ||
                      (launched <= 888 && max_seq_len <= 320 && (int64_t)T * KV <= 296 * TT);
   if (bs >= 8 && !cap && B <= 65535 && !small)
     return launch_pair<HD, false>(atc2::PairArgs{H * HD, 1.f, 0, 0.f}, out, q, q_stride, kc, vc, bt, max_blocks, sl, qsl, B, T, max_q_len, max_seq_len, H, KV, bs, bs_shift, scale, sinks, st);

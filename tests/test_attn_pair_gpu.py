@@ -24,6 +24,7 @@ LONG = [
     ("bf16", 32, 8, 128, 64, [64, 63, 65, 1], [1089, 1090, 1088, 0]),
     ("fp16", 24, 8, 128, 64, [400, 43, 700], [0, 2600, 100]),
     ("bf16", 64, 2, 64, 8, [333, 5, 1], [2300, 800, 1200]),
+    ("bf16", 4, 4, 128, 16, [1300, 257], [800, 255]),
     ("bf16", 128, 1, 128, 64, [1] * 5 + [3], [2700, 0, 63, 64, 65] + [500]),
 ]
 
