@@ -29,7 +29,9 @@ int kge_device_sm_count(void);
 /* Launch-shape knobs for tuning and diagnostics (no counterpart in the reference): they change how work is
  * partitioned over the 148 SMs, never the results.  Process-wide; set them before creating an engine
  * (captured decode graphs keep the shape they were captured with).
- *   "pdl" 0/1                 programmatic dependent launch between the kernels of a step
+ *   "pdl" 0/1                 programmatic dependent launch between the kernels of a step: a kernel reads what a model fixes (weights,
+ *                             biases, norm weights) while the kernel before it is still at work, so these must not be the output
+ *                             of work that is in flight on the stream
  *   "gemm_even_grid" 0/1      persistent weight-streaming GEMM: size the grid so every CTA gets the same tile count
  *   "attn_decode_splits" n    force the split-KV factor of decode attention (0 = heuristic)
  *   "attn_split_balance" 0/1  heuristic picks the split factor that fills whole waves of resident CTAs

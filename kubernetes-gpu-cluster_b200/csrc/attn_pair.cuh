@@ -16,8 +16,8 @@
 //     tiles between the two groups of warps, which merge at the end: half the serial walk of a decode row over its context
 //   * outputs turned in shared memory so that rows leave in full lines (16 bytes of 32 rows per store took 3500 cycles an item).
 // us before (128-row CTAs, two per SM) and now, 32 / 8 heads of 128: 4 x 2048 tokens 152 -> 125 (1097 TFLOP/s), one of 8192 467 -> 411
-// (1337), 4 x 1000 61 -> 48, one of 512 14.2 -> 11.3, 37 decode rows of up to 3000 keys beside 2 x 1011 tokens behind 2777 181 -> 146,
-// 200 decode rows beside 300 tokens 128 -> 69.
+// (1337), 4 x 1000 61 -> 48, 37 decode rows of up to 3000 keys beside 2 x 1011 tokens behind 2777 181 -> 146, 200 decode rows beside 300
+// tokens 128 -> 69.  Small launches stay with the other kernel (launch_tc).
 namespace atc2 {
 using namespace atc;
 

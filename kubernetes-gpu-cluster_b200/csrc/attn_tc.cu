@@ -14,8 +14,8 @@
 // mbarriers; tcgen05.commit tells it when a stage is free.  The softmax warps issue no loads.
 // TMA = false (knob "attn_tma" 0, block sizes below 8): tiles gathered by the softmax threads with
 // 16-byte cp.async (K two tiles ahead, V one; block-table lookup once per row) and published with fence.proxy.async.
-// Which kernel takes what: attn_pair.cuh has the plain prompts (see launch_tc); this one short contexts in small launches, soft caps,
-// windows with prefix keys and block sizes below 8.
+// Which kernel takes what: attn_pair.cuh has the plain prompts (see launch_tc); this one small launches, soft caps, windows with prefix
+// keys and block sizes below 8.
 // Tensor-bound: 4 * hd * sum_b q_b (ctx0_b + (q_b+1)/2) flop per q head.
 #include <cuda.h>
 #include <string.h>

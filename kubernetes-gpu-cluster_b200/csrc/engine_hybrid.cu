@@ -663,7 +663,7 @@ int hybrid_engine_build(kge_engine* e, const ModelDir& md, int64_t dummy_seed, s
     e->moe_out = aalloc(np * d, es);
     if (!e->f32) {
       e->moe_xperm = aalloc(np * d, 2); e->moe_operm = aalloc(np * d, 2);
-      if (!e->moe_xperm || !e->moe_operm || cudaMallocHost((void**)&e->moe_goff_host, (size_t)(max_E + 1) * 4) != cudaSuccess) return fail("expert staging allocation failed: " + b.err);
+      if (!e->moe_xperm || !e->moe_operm) return fail("expert staging allocation failed: " + b.err);
     }
     e->moe_goff = (int32_t*)aalloc(max_E + 1, 4);
     e->moe_prow = (int32_t*)aalloc(np, 4);

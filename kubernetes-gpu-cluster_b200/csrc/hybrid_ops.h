@@ -32,7 +32,8 @@ inline size_t elt_size(int elt) { return elt == KGE_ELT_F32 ? 4 : 2; }
 // Rows r run over [0, T), or - with group_off - over [group_off[z], group_off[z+1]) for each z < nz, where slice z
 // reads x at column offset z * x_zs, weights at w + z * w_zs (elements), bias at z * b_zs and writes y at column offset
 // z * y_zs.  xrows / yrows (null = identity) gather the input row and scatter the output row; row_scale (null = 1) is
-// indexed by r.  Sums run over k in ascending order in fp32, whatever else is in the launch.
+// indexed by r.  Sums are fp32: over k in ascending order in float32 storage, whatever else is in the launch; in bfloat16 storage the kernel
+// goes by the launch's sizes, and with it the order (ascending in steps of 16, or interleaved over eight warps: up to 8 rows, up to 32 outputs).
 struct LinearArgs {
   const void* x = nullptr; int ldx = 0;
   const void* w = nullptr; const void* w2 = nullptr; const void* bias = nullptr;

@@ -1,5 +1,6 @@
 // Shape-agnostic linear layer for layer-list models: any T / N / K and alignment, bfloat16 or float32 storage, fp32
-// accumulation in a fixed k order (so a row's result does not depend on what else is in the launch), optional row
+// accumulation (float32 storage: in a fixed k order, so that a row's result does not depend on what else is in the launch; bfloat16: in the
+// order of the kernel that the launch's sizes choose), optional row
 // gather / scatter, per-row input scale, grouped rows (one weight slice per group: mixture-of-experts) or strided slices
 // (block-diagonal projections), gated pairs (silu(x.w) * (x.w2)) and fp32 output or accumulation.  Tiles of 64 x 64
 // outputs and 256 threads: float32 storage multiplies on the fp32 pipes (4 x 4 outputs per thread, operands staged in
