@@ -806,9 +806,8 @@ int hybrid_forward(kge_engine* e, int T, int B, int R, int max_blocks, const Ste
   const StepMeta hm = carve_meta(const_cast<uint8_t*>(hostm), T, B, R, max_blocks, nullptr);
   bool decode_only = true;
   for (int i = 0; i < B; ++i) decode_only &= hm.qsl[i + 1] - hm.qsl[i] == 1;
-  // Steps that carry prompt pieces run their kernels in plain stream order: they are tens of milliseconds long, early
-  // launch buys nothing there, and hundreds of long-running CTAs of one kernel waiting on the previous one would only
-  // hold shared memory.  Decode steps keep programmatic dependent launch (and run as CUDA graphs).
+  // Steps that carry prompt pieces run their kernels in plain stream order: with dependent launch, steps of the benchmark's models
+  // have stood still, for a cause that is not known.  Decode steps keep programmatic dependent launch (and run as CUDA graphs).
   struct PdlOff { bool on; explicit PdlOff(bool o) : on(o) { if (on) pdl_suspend(true); } ~PdlOff() { if (on) pdl_suspend(false); } } pdl_off(!decode_only);
   // the model's norm of residual rows: RMS with the weight applied as 1 + w, the weight-only layer norm, or Dynamic Tanh
   auto layer_norm = [&](void* y, const int32_t* rows, const void* w, int R, float out_scale) -> int {

@@ -1,9 +1,9 @@
-"""Third opinion (oracle plan item 3): the installed vLLM 0.22.0 running its own CUDA
+"""Third opinion: the installed vLLM 0.22.0 running its own CUDA
 kernels on a B200, on the oracle's seeded tiny models (identical safetensors) and token-id prompts, greedy.
 NOT the pinned version (v0.8.x) and not vLLM's CPU backend - but it is the dependency the reference deploys,
 executing the same model graph, so its tokens and logprobs pin the oracle and the product end to end.
 
-Runs ONLY on a GPU box (gpurun); needs vllm.  Writes gpurun_out/vllm_cuda.json, which is then committed as
+Runs ONLY on a GPU box; needs vllm.  Writes vllm_cuda.json into $KGE_OUT (the working folder otherwise), which is then committed as
 tests/golden/vllm_cuda.json.  Nothing reads vllm at test time.
 
   python tests/golden/make_vllm_cuda_golden.py            # parity fixtures, one subprocess per model
@@ -19,7 +19,7 @@ import time
 HERE = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.join(HERE, "..", "..")
 sys.path.insert(0, ROOT)
-OUT = os.path.join(ROOT, "gpurun_out")
+OUT = os.environ.get("KGE_OUT", os.getcwd())
 MODELS = ["tiny-llama-hd128", "tiny-qwen3", "tiny-opt", "tiny-qwen2", "tiny-llama"]
 DEFAULT_MODELS = MODELS[:3]
 PROMPT_LENS = (5, 17, 33, 64)
@@ -148,7 +148,7 @@ def main():
                 ok = True
                 break
         if i == 0 and not ok:
-            print("vLLM did not start on this box with either attention backend; see gpurun_out/vllm_cuda_*.log")
+            print("vLLM did not start on this box with either attention backend; see vllm_cuda_*.log")
             sys.exit(3)
     merged = [json.load(open(os.path.join(OUT, f"vllm_cuda_{m}.json"))) for m in MODELS
               if os.path.exists(os.path.join(OUT, f"vllm_cuda_{m}.json"))]

@@ -149,10 +149,10 @@ BASELINE_CASES = {
 
 
 def _record(name, **kw):
-    """Measured parity figures, kept next to the run's other outputs when that directory exists."""
-    d = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "gpurun_out")
+    """Measured parity figures, kept in $KGE_OUT if that is a directory."""
+    d = os.environ.get("KGE_OUT", "")
     if os.path.isdir(d):
-        with open(os.path.join(d, "parity_r02.jsonl"), "a") as fh:
+        with open(os.path.join(d, "parity.jsonl"), "a") as fh:
             fh.write(json.dumps(dict(case=name, **kw)) + "\n")
 
 

@@ -4,7 +4,7 @@
   decode  attn_decode_kernel vs FlashInfer's trtllm-gen decode (trtllm_batch_decode_with_kv_cache)
 CUDA events on the launching (default) stream, buffers rotated past L2 for the HBM-bound cases.  The library calls are
 comparison points only (tools/, never the product).  Writes one JSON document to --out.
-  python tools/bench_vs_libs.py --out gpurun_out/r02_vs_libs.json"""
+  python tools/bench_vs_libs.py --out vs_libs.json"""
 import argparse
 import json
 import os
@@ -201,7 +201,7 @@ def decode_rows():
 
 if __name__ == "__main__":
     ap = argparse.ArgumentParser()
-    ap.add_argument("--out", default="gpurun_out/r02_vs_libs.json")
+    ap.add_argument("--out", default="vs_libs.json")
     ap.add_argument("--skip", default="")
     a = ap.parse_args()
     kge.require_cuda()

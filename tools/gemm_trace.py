@@ -1,7 +1,7 @@
 """Where a decode-sized GEMM launch spends its time: per-CTA %globaltimer stamps written by the kernel itself
 (kge_gemm_set_trace, csrc/gemm_tc.cu) for back-to-back launches on one stream, weights rotated through HBM.
 
-  python tools/gemm_trace.py [--T 64] [--knob gemm_ws=1] [--out gpurun_out/trace.jsonl]
+  python tools/gemm_trace.py [--T 64] [--knob gemm_ws=1] [--out trace.jsonl]
 
 Slots (ns, relative to the earliest CTA entry of the launch):
   0 entry            first instruction of the CTA (thread 0)
