@@ -856,6 +856,64 @@ def test_sample_vocabularies_by_shared_memory(kge, L, V):
         test_sample_row_split_over_a_cluster(kge, L, B, V, V)
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("V", [1003, 50272])
+@pytest.mark.parametrize("shape", ["near_zero", "every_scale", "negative", "zeros", "one_value", "nan", "masked"])
+def test_sample_thresholds_wherever_they_lie(kge, L, shape, V, dtype):
+    """Thresholds in the first counted keys, among the values near zero that share a counter, and below the first 8192 keys; logits
+    without a finite neighbour, equal ones, NaN (the largest logit alone is kept) and rows that are mostly masked."""
+    g = torch.Generator().manual_seed(V)
+    B = 6
+    x = torch.randn(B, V, generator=g)
+    if shape == "near_zero":
+        x = x * 2.0 ** -13
+    elif shape == "every_scale":
+        x = x.sign() * torch.exp2(torch.rand(B, V, generator=g) * 20 - 14)
+    elif shape == "negative":
+        x = -torch.exp2(torch.rand(B, V, generator=g) * 4) - 0.1
+    elif shape == "zeros":
+        x = torch.where(torch.rand(B, V, generator=g) < 0.7, torch.zeros(B, V), x)
+    elif shape == "one_value":
+        x = torch.full((B, V), -1.5)
+    elif shape == "nan":
+        x[:, V // 3] = float("nan")
+    elif shape == "masked":
+        x = torch.where(torch.rand(B, V, generator=g) < 0.95, torch.full((B, V), -float("inf")), x * 3)
+    lg = x.to(dtype)
+    temp = torch.tensor([0.8, 1.0, 1.0, 2.0, 0.7, 1.0])
+    k = torch.tensor([V // 2, V - 3, 0, 0, V // 3, 9], dtype=torch.int32)
+    pp = torch.tensor([1.0, 0.9, 0.4, 0.97, 0.6, 0.8])
+    fn = L.kge_sample_f16 if dtype == torch.float16 else L.kge_sample
+    lgd, td, kd, ppd = dev(lg), dev(temp), dev(k), dev(pp)
+    # where a NaN is in the row only its largest other logit can be drawn, and the oracle has no rule for it
+    finite = torch.nan_to_num(lg.float(), nan=-float("inf"), neginf=-float("inf"))
+    for noise in (torch.empty(B, V).exponential_(generator=g), edge_noise(finite, temp)):
+        out, qd = torch.empty(B, dtype=torch.int32, device="cuda"), dev(noise)
+        check_ok(kge, fn(p(out), p(lgd), B, V, V, p(td), p(kd), p(ppd), p(qd), None, 0, None, 0, None), "sample")
+        sync()
+        got = out.cpu().long()
+        if shape == "nan":
+            for b in range(B):
+                if pp[b] < 1:
+                    assert finite[b, got[b]] == finite[b].max()
+        else:
+            check_draws(got, lg.float(), V, temp, k, pp, noise)
+
+
+def test_sample_a_draw_whose_noise_is_none(kge, L):
+    """A seed whose uniform number at index 2 is 1 exactly: its noise is -0 and its score the lowest there is, below the bound under
+    which elements are left out, so the draw is repeated without that bound."""
+    lg = torch.tensor([[0.0, 1.0, 30.0, -2.0]]).to(BF)
+    lgd, td, ppd = dev(lg), dev(torch.ones(1)), dev(torch.ones(1))
+    for seed in (20971202, 24200764):
+        for k, want in ((1, [2]), (2, [1]), (0, [0, 1, 3])):
+            kd, sd = dev(torch.tensor([k], dtype=torch.int32)), dev(torch.tensor([seed]))
+            out = torch.empty(1, dtype=torch.int32, device="cuda")
+            check_ok(kge, L.kge_sample(p(out), p(lgd), 1, 4, 4, p(td), p(kd), p(ppd), None, p(sd), 0, None, 0, None), "sample")
+            sync()
+            assert out.item() in want, (seed, k, out.item())
+
+
 def test_sample_philox_is_deterministic_and_in_support(kge, L):
     g = torch.Generator().manual_seed(2)
     B, V = 4, 2048
