@@ -151,7 +151,7 @@ struct kge_engine {
   bool f32 = false;                          // float32 storage and arithmetic (--dtype float32; layer-list models only)
   // layer-list ("hybrid") models: fp32 residual stream, their own activation arena and the recurrent-state pool
   std::vector<kge::HybridLayerW> hyb;
-  float *res32 = nullptr, *gates32 = nullptr, *logits32 = nullptr, *state = nullptr, *mo32 = nullptr;
+  float *res32 = nullptr, *gates32 = nullptr, *rglru_tiles = nullptr, *logits32 = nullptr, *state = nullptr, *mo32 = nullptr;
   float final_alpha = 0.f;                   // Dynamic Tanh in the place of the final norm (weight final_w, shift final_b)
   float* sgate32 = nullptr;                  // [tokens]: the shared expert's per-token gate where the router's logits come from a matrix product
   float* dt32 = nullptr;                     // [tokens, channels]: step sizes of a selective scan

@@ -199,7 +199,7 @@ int hybrid_engine_build(kge_engine* e, const ModelDir& md, int64_t dummy_seed, s
   int max_mo = 1, max_nm = 0;
   int max_proj = 1, max_mix = 1, max_ff = 1, max_gate = 1, max_u = 1, max_top = 0, max_eff = 1, max_E = 1;
   int max_hd = 0, max_qr = 0, max_kvr = 0, max_lkv = 0, max_lq = 0;      // WKV heads * dim; latent ranks, [k | v] and query widths
-  int max_mix2 = 0, max_bc = 0, max_dt = 0;
+  int max_mix2 = 0, max_bc = 0, max_dt = 0, max_rglru = 0;
   for (int i = 0; i < s.L; ++i) {
     const HybridLayerSpec& h = s.hybrid[i];
     HybridLayerW& L = e->hyb[i];
@@ -246,7 +246,7 @@ int hybrid_engine_build(kge_engine* e, const ModelDir& md, int64_t dummy_seed, s
       L.o.N = d; L.o.K = w;
       HB_OK(L.o.w = b.mat({mx + "o"}, {d}, w, ws));
       state_floats += rglru_state_floats(w, h.conv);
-      max_proj = std::max(max_proj, 2 * w); max_mix = std::max(max_mix, w); max_gate = std::max(max_gate, 2 * w); max_u = std::max(max_u, w);
+      max_proj = std::max(max_proj, 2 * w); max_mix = std::max(max_mix, w); max_gate = std::max(max_gate, 2 * w); max_u = std::max(max_u, w); max_rglru = std::max(max_rglru, w);
     } else if (h.mixer == HybridLayerSpec::ATTENTION) {
       const int nq = h.heads * h.dim, nk = h.kv_heads * h.dim;
       if (!h.v_from_k) return fail("an attention mixer with a value projection of its own is not built");
@@ -647,6 +647,7 @@ int hybrid_engine_build(kge_engine* e, const ModelDir& md, int64_t dummy_seed, s
   e->obuf2 = aalloc((int64_t)Tm * d, es);
   e->ffbuf = aalloc((int64_t)Tm * max_ff, es);
   e->gates32 = (float*)aalloc((int64_t)Tm * max_gate, 4);
+  e->rglru_tiles = (float*)aalloc(std::max<int64_t>(4, rglru_tile_floats(Tm, max_rglru)), 4);
   e->mo32 = (float*)aalloc((int64_t)Tm * max_mo + (int64_t)Rm * max_nm, 4);      // read-outs of a step's tokens, and behind them new normalisers of its requests
   e->hsel = aalloc((int64_t)std::max(Rm, Tm) * d, es);
   // logits rows: the sampled rows of a step, or every row a trace asks for
@@ -692,7 +693,7 @@ int hybrid_engine_build(kge_engine* e, const ModelDir& md, int64_t dummy_seed, s
   e->max_blocks_per_seq = (e->cfg.max_model_len + e->cfg.block_size - 1) / e->cfg.block_size;
   carve_meta(nullptr, Tm, Rm, std::max(Rm, Tm), e->max_blocks_per_seq, &e->meta_bytes);
   e->meta_dev = (uint8_t*)aalloc(e->meta_bytes, 1);
-  if (!e->res32 || !e->hx || !e->pbuf || !e->ubuf || !e->mixbuf || !e->obuf1 || !e->obuf2 || !e->ffbuf || !e->gates32 || !e->mo32 || !e->hsel ||
+  if (!e->res32 || !e->hx || !e->pbuf || !e->ubuf || !e->mixbuf || !e->obuf1 || !e->obuf2 || !e->ffbuf || !e->gates32 || !e->rglru_tiles || !e->mo32 || !e->hsel ||
       !e->logits32 || !e->logits || !e->state || !e->d_out || !e->lp_vals || !e->lp_ids || !e->lp_rank || !e->mask_pairs || !e->meta_dev)
     return fail("activation arena allocation failed: " + b.err);
   e->alloc_logits_host((int64_t)Rm * s.vocab);
@@ -926,7 +927,14 @@ int hybrid_forward(kge_engine* e, int T, int B, int R, int max_blocks, const Ste
       ra.state = e->state + L.state_off; ra.slot_stride = e->slot_stride;
       ra.slots = m.sslot; ra.qsl = m.qsl; ra.positions = m.pos; ra.token_req = m.treq;
       ra.B = B; ra.T = T; ra.width = w; ra.taps = h.conv; ra.decay_c = 8.f; ra.elt = elt;
-      const double Tw = (double)T * w;
+      ra.w_r = L.ra.w; ra.b_r = L.ra.b; ra.w_i = L.ri.w; ra.b_i = L.ri.b; ra.blocks = h.blocks; ra.tiles = e->rglru_tiles;
+      const double Tw = (double)T * w, wbytes = 2.0 * w * bw * es, sbytes = 2.0 * B * rglru_state_floats(w, h.conv) * 4;
+      if (decode_only && rglru_step_ok(ra)) {
+        HFWD(C_RGLRU, Tw * 3 * es + wbytes + sbytes, 4.0 * Tw * bw, rglru_step(ra, st));
+      } else if (!decode_only && rglru_gates_ok(ra)) {
+        HFWD(C_RGLRU, Tw * (es + 8) + wbytes, 4.0 * Tw * bw, rglru_gates(ra, st));
+        HFWD(C_RGLRU, Tw * (2 * es + 8) + sbytes, 0, rglru_walk(ra, st));
+      } else {
       HFWD(C_RGLRU, Tw * 2 * es, 0, rglru_conv(ra, st));
       for (int gsel = 0; gsel < 2; ++gsel) {           // block-diagonal gate projections of u, kept in fp32
         const HybMat& gm = gsel ? L.ri : L.ra;
@@ -936,7 +944,8 @@ int hybrid_forward(kge_engine* e, int T, int B, int R, int max_blocks, const Ste
         a.elt = elt; a.out_f32 = true;
         HFWD(C_RGLRU, Tw * (es + 4) + (double)w * bw * es, 2.0 * Tw * bw, linear_any(a, st));
       }
-      HFWD(C_RGLRU, Tw * (3 * es + 8) + 2.0 * B * rglru_state_floats(w, h.conv) * 4, 0, rglru_scan(ra, st));
+      HFWD(C_RGLRU, Tw * (3 * es + 8) + sbytes, 0, rglru_scan(ra, st));
+      }
       DENSE(e->obuf1, d, e->mixbuf, w, L.o, T, ACT_NONE);
       add_src(e->obuf1, d, 1.f);
     } else if (h.mixer == HybridLayerSpec::ATTENTION) {

@@ -265,9 +265,21 @@ struct RglruArgs {
   int B = 0, T = 0, width = 0, taps = 1;
   float decay_c = 8.f;
   int elt = KGE_ELT_BF16;
+  // block-diagonal gate projections ([blocks, width / blocks, width / blocks], biases [width] or none) for rglru_gates and rglru_step
+  const void* w_r = nullptr; const void* b_r = nullptr; const void* w_i = nullptr; const void* b_i = nullptr; int blocks = 0;
+  float* tiles = nullptr;                  // scratch of steps with prompt pieces: rglru_tile_floats(T, width)
 };
 int rglru_conv(const RglruArgs& a, cudaStream_t st);
 int rglru_scan(const RglruArgs& a, cudaStream_t st);
+// Both and the gate projections together.  Decode steps (one row a request; rglru_step_ok): one launch, u and gates unused.  Other steps
+// (rglru_gates_ok): rglru_gates turns x into the coefficients a, b (in `gates`), rglru_walk those into out and state.
+bool rglru_step_ok(const RglruArgs& a);
+bool rglru_gates_ok(const RglruArgs& a);
+int rglru_step(const RglruArgs& a, cudaStream_t st);
+int rglru_gates(const RglruArgs& a, cudaStream_t st);
+int rglru_coefficients(const RglruArgs& a, cudaStream_t st);     // gate pre-activations -> a, b, in place
+int rglru_walk(const RglruArgs& a, cudaStream_t st);
+inline int64_t rglru_tile_floats(int64_t T, int width) { return (T + 31) / 32 * 2 * width; }
 inline int64_t rglru_state_floats(int width, int taps) { return (int64_t)width * taps; }   // S + (taps - 1) conv inputs
 
 // Matrix memory (mLSTM) with a running maximum m that starts at 0.

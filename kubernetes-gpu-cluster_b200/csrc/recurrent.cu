@@ -188,175 +188,13 @@ __global__ void __launch_bounds__(128) rglru_scan_kernel(RglruArgs a) {
   }
 }
 
-// Prompt steps: everything of the recurrence that does not depend on the previous token is done for all tokens at once.
-// rglru_ab_kernel turns the gate pre-activations, in place, into the recurrence's coefficients (a_t, b_t = sqrt(1 - a_t^2)
-// i_t u_t); rglru_chain_kernel is then one fma per token and channel (S_t written over a_t) plus the state hand-over; and
-// rglru_out_kernel multiplies by gelu(y).  Same arithmetic per element as the fused kernel.  A thread keeps its channel and walks
-// over tokens (no divisions by the width).  2312 tokens x 2560: 84 us back to back (92 before that, 162 with a chain that loads into registers); 200
-// tokens beside 64 single ones 21 (31).  All three in one kernel, with seven warps of a block feeding the chain, took 422: too few
-// warps for the exponentials' latency.
-// RG_AT tokens at a time in the first and the last of them: behind a store to the gates the compiler keeps later loads back, and a token
-// at a time each costs a trip to memory (2312 tokens x 2560: 40 and 17 us; 32 and 15 now).
-constexpr int RG_AT = 4;
-template <typename E>
-__global__ void __launch_bounds__(256) rglru_ab_kernel(RglruArgs a, float* gates) {
-  pdl_launch_dependents();
-  pdl_wait();
-  const int c = blockIdx.y * 256 + threadIdx.x;
-  if (c >= a.width) return;
-  const float sp = a.decay_c * softplusf_(ldf((const E*)a.lam + c));
-  for (int t0 = blockIdx.x; t0 < a.T; t0 += RG_AT * gridDim.x) {
-    float gr[RG_AT], gi[RG_AT], uv[RG_AT];
-#pragma unroll
-    for (int k = 0; k < RG_AT; ++k) {
-      const int t = min(t0 + k * (int)gridDim.x, a.T - 1);
-      const float* gt = gates + (int64_t)t * 2 * a.width + c;
-      gr[k] = gt[0]; gi[k] = gt[a.width];
-      uv[k] = ldf((const E*)a.u + (int64_t)t * a.width + c);
-    }
-#pragma unroll
-    for (int k = 0; k < RG_AT; ++k) {
-      const int t = t0 + k * (int)gridDim.x;
-      if (t >= a.T) break;
-      float* gt = gates + (int64_t)t * 2 * a.width + c;
-      const float log_a = -sp * sigmoidf_(gr[k]);
-      gt[0] = expf(log_a);
-      gt[a.width] = sqrtf(-expm1f(2.f * log_a)) * sigmoidf_(gi[k]) * uv[k];
-    }
-  }
-}
-
-// One warp per 32 channels of a request: the coefficients of TOK tokens at a time arrive by cp.async, two stages ahead, so that the
-// chain waits for its fma's and not for memory.  What bounds steps with many requests is how many of these one-warp blocks fit at
-// once: stages of 16 tokens (12 KB a block) and four of 64 (64 KB) take 92 and 101 us for 2 x 1160 tokens, 28 and 64 for 60 and 200 single
-// ones, us of the whole recurrence at width 2560; stages of 8, where requests bring less than 8 tokens on average, 26.
-// N: numbers per copy, four where the rows are aligned for it, one elsewhere (widths that are no multiple of four).
-constexpr int RS_STAGES = 3;
-template <typename E, int N, int TOK>
-__global__ void __launch_bounds__(32) rglru_chain_kernel(RglruArgs a, float* gates) {
-  pdl_launch_dependents();
-  pdl_wait();
-  extern __shared__ __align__(16) float rs_sm[];          // [stage][a | b][token][channel]
-  const int b = blockIdx.x, lane = threadIdx.x, c0 = blockIdx.y * 32, c = c0 + lane;
-  const bool in = c < a.width;
-  const int rs = a.qsl[b], re = a.qsl[b + 1], n = re - rs;
-  if (n <= 0) return;
-  const int p0 = a.positions[rs], tiles = (n + TOK - 1) / TOK;
-  float* slot = a.state + (int64_t)a.slots[b] * a.slot_stride;
-  const E* yx = (const E*)a.yx;
-  auto fetch = [&](int tile) {
-    if (tile < tiles) {
-      float* dst = rs_sm + (tile % RS_STAGES) * (2 * TOK * 32);
-      constexpr int LANES = 32 / N;                        // lanes that copy a token's 32 channels
-      const int len = min(TOK, n - tile * TOK), piece = (lane % LANES) * N;
-      const int bytes = c0 + piece < a.width ? N * 4 : 0;
-      for (int k = lane / LANES; k < len; k += N) {
-        const float* src = gates + (int64_t)(rs + tile * TOK + k) * 2 * a.width + (bytes > 0 ? c0 + piece : 0);
-#pragma unroll
-        for (int w = 0; w < 2; ++w) {
-          const uint32_t to = (uint32_t)__cvta_generic_to_shared(dst + (w * TOK + k) * 32 + piece);
-          if constexpr (N == 4) asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(to), "l"(src + w * a.width), "r"(bytes) : "memory");
-          else asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(to), "l"(src + w * a.width), "r"(bytes) : "memory");
-        }
-      }
-    }
-    asm volatile("cp.async.commit_group;" ::: "memory");
-  };
-  float S = in && p0 > 0 ? slot[c] : 0.f;
-#pragma unroll
-  for (int i = 0; i < RS_STAGES - 1; ++i) fetch(i);
-  for (int tile = 0; tile < tiles; ++tile) {
-    asm volatile("cp.async.wait_group %0;" ::"n"(RS_STAGES - 2) : "memory");
-    __syncwarp();
-    fetch(tile + RS_STAGES - 1);                           // the stage that the previous turn has read
-    const float* av = rs_sm + (tile % RS_STAGES) * (2 * TOK * 32) + lane;
-    const float* bv = av + TOK * 32;
-    const int len = min(TOK, n - tile * TOK);
-    float* out = gates + (int64_t)(rs + tile * TOK) * 2 * a.width + c;
-    if (len == TOK) {
-      float x[TOK], y[TOK];
-#pragma unroll
-      for (int i = 0; i < TOK; ++i) { x[i] = av[i * 32]; y[i] = bv[i * 32]; }
-#pragma unroll
-      for (int i = 0; i < TOK; ++i) {
-        S = fmaf(x[i], S, y[i]);
-        if (in) out[(int64_t)i * 2 * a.width] = S;
-      }
-    } else {
-      for (int k = 0; k < len; ++k) {
-        S = fmaf(av[k * 32], S, bv[k * 32]);
-        if (in) out[(int64_t)k * 2 * a.width] = S;
-      }
-    }
-    __syncwarp();
-  }
-  if (!in) return;
-  slot[c] = S;
-  // the convolution's next inputs: the last taps - 1 rows of this step, or of the old tail
-  float nt[MAX_TAPS];
-  float* tail = slot + a.width;
-#pragma unroll
-  for (int k = 0; k < MAX_TAPS; ++k) {
-    if (k >= a.taps - 1) break;
-    const int sp2 = p0 + n - (a.taps - 1) + k;
-    float v = 0.f;
-    if (sp2 >= p0) v = ldf(yx + (int64_t)(rs + sp2 - p0) * 2 * a.width + a.width + c);
-    else if (sp2 >= 0) v = tail[(int64_t)(sp2 - p0 + a.taps - 1) * a.width + c];
-    nt[k] = v;
-  }
-#pragma unroll
-  for (int k = 0; k < MAX_TAPS; ++k) {
-    if (k >= a.taps - 1) break;
-    tail[(int64_t)k * a.width + c] = nt[k];
-  }
-}
-
-template <typename E>
-__global__ void __launch_bounds__(256) rglru_out_kernel(RglruArgs a, const float* gates) {
-  pdl_launch_dependents();
-  pdl_wait();
-  const int c = blockIdx.y * 256 + threadIdx.x;
-  if (c >= a.width) return;
-  for (int t0 = blockIdx.x; t0 < a.T; t0 += RG_AT * gridDim.x) {
-    float sv[RG_AT], yv[RG_AT];
-#pragma unroll
-    for (int k = 0; k < RG_AT; ++k) {
-      const int64_t at = (int64_t)min(t0 + k * (int)gridDim.x, a.T - 1) * 2 * a.width + c;
-      sv[k] = gates[at];
-      yv[k] = ldf((const E*)a.yx + at);
-    }
-#pragma unroll
-    for (int k = 0; k < RG_AT; ++k) {
-      const int t = t0 + k * (int)gridDim.x;
-      if (t < a.T) stf((E*)a.out + (int64_t)t * a.width + c, sv[k] * gelu_tanhf_(yv[k]));
-    }
-  }
-}
-
-template <typename E, int N, int TOK>
-static int rglru_prompt_as(const RglruArgs& a, cudaStream_t st) {
-  float* gates = const_cast<float*>(a.gates);
-  const int slices = (a.width + 255) / 256;
-  const dim3 eg(std::min(a.T, std::max(1, 148 * 8 / slices)), slices), cg(a.B, (a.width + 31) / 32);
-  KGE_REQUIRE(cg.y <= 65535, "rglru_scan: width %d", a.width);
-  KGE_CUDA_OK(launch_pdl(rglru_ab_kernel<E>, eg, dim3(256), 0, st, a, gates));
-  KGE_CUDA_OK(launch_pdl(rglru_chain_kernel<E, N, TOK>, cg, dim3(32), RS_STAGES * 2 * TOK * 32 * 4, st, a, gates));
-  KGE_CUDA_OK(launch_pdl(rglru_out_kernel<E>, eg, dim3(256), 0, st, a, (const float*)gates));
-  return 0;
-}
-
-template <typename E, int N>
-static int rglru_prompt(const RglruArgs& a, cudaStream_t st) {
-  return a.T < 8 * a.B ? rglru_prompt_as<E, N, 8>(a, st) : rglru_prompt_as<E, N, 16>(a, st);
-}
-
 int rglru_scan(const RglruArgs& a, cudaStream_t st) {
   if (a.T <= 0 || a.B <= 0) return 0;
   KGE_REQUIRE(a.taps >= 1 && a.taps <= MAX_TAPS, "rglru_scan: %d taps (1..%d)", a.taps, MAX_TAPS);
   const dim3 grid(a.B, (a.width + 127) / 128), block(128);
   if (a.T > a.B) {                       // some request brings several rows
-    if (a.width % 4 == 0 && (reinterpret_cast<uintptr_t>(a.gates) & 15) == 0) return a.elt == KGE_ELT_F32 ? rglru_prompt<float, 4>(a, st) : rglru_prompt<__nv_bfloat16, 4>(a, st);
-    return a.elt == KGE_ELT_F32 ? rglru_prompt<float, 1>(a, st) : rglru_prompt<__nv_bfloat16, 1>(a, st);
+    const int rc = rglru_coefficients(a, st);
+    return rc ? rc : rglru_walk(a, st);
   }
   cudaError_t ce = a.elt == KGE_ELT_F32 ? launch_pdl(rglru_scan_kernel<float>, grid, block, 0, st, a)
                                         : launch_pdl(rglru_scan_kernel<__nv_bfloat16>, grid, block, 0, st, a);

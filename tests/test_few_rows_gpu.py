@@ -66,6 +66,38 @@ def test_block_diagonal_gates_of_many_rows(kge, tmp_path, width, blocks, rows):
     llm.close()
 
 
+@pytest.mark.parametrize("width,blocks,taps", [(64, 2, 4), (192, 3, 3), (256, 2, 4), (480, 3, 4), (320, 2, 2), (512, 2, 4), (66, 2, 4)])
+def test_recurrence_by_tiles(kge, tmp_path, width, blocks, taps):
+    """Convolution, gates and coefficients in one kernel (blocks of 32, 64, 128 and 160 channels; 256 and 33 take the general ones), the
+    recurrence by tiles of 32 rows: pieces that end before, at and behind a tile's edge and span more tiles than are composed at once;
+    many requests that begin and end inside one tile, beside decode rows; then decode steps of more requests than a block has rows."""
+    cfg = oh.make_config(layers=("rglru",), mlps=(None,), r_width=width, r_blocks=blocks, r_conv=taps)
+    W = oh.make_weights(cfg, seed=43)
+    toks = prompt(cfg, 420)
+    want = oh.forward(cfg, W, toks)
+    llm = make_engine(kge, tmp_path, cfg, W, "bfloat16", tokens=2048, seqs=24)
+    for rid, pieces in enumerate([[420], [31, 1, 32, 33, 2, 64, 65, 127, 62, 3]]):
+        check(run_pieces(llm, rid, toks, pieces), want, "bfloat16", f"pieces {pieces}")
+        llm.trace_end(rid)
+    n = 18
+    lens = [1 + 3 * rid for rid in range(n)]
+    for rid in range(n):
+        llm.trace_add(rid, toks[:lens[rid]])
+    got = llm.trace_step([(rid, lens[rid], list(range(lens[rid]))) for rid in range(n)])
+    check(got, want[[i for m in lens for i in range(m)]], "bfloat16", "prompts side by side")
+    for turn in range(3):
+        for rid in range(n):
+            llm.trace_add(rid, [toks[lens[rid] + turn]])
+        got = llm.trace_step([(rid, 1, [0]) for rid in range(n)])
+        check(got, want[[m + turn for m in lens]], "bfloat16", f"decode step {turn}")
+    for rid in range(n):                                   # pieces of some beside single tokens of others
+        m = 1 + (rid % 3) * 20
+        llm.trace_add(rid, toks[lens[rid] + 3:lens[rid] + 3 + m])
+    got = llm.trace_step([(rid, 1 + (rid % 3) * 20, list(range(1 + (rid % 3) * 20))) for rid in range(n)])
+    check(got, want[[lens[rid] + 3 + i for rid in range(n) for i in range(1 + (rid % 3) * 20)]], "bfloat16", "mixed step")
+    llm.close()
+
+
 @pytest.mark.parametrize("hd", [64, 128])
 def test_short_biased_pieces(kge, tmp_path, hd):
     """Pieces around the length from which on prompts run in the tcgen05 kernel: the last whose keys are one tile of the other, and the next."""
