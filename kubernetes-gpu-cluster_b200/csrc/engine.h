@@ -203,6 +203,7 @@ struct kge_engine {
   int num_blocks = 0, max_blocks_per_seq = 0;
   int64_t weight_bytes = 0, kv_bytes = 0;
 
+  bool step_rows_all = false;                // the step's logits rows are its tokens, in order: nothing to gather
   kge::bf16* res_next = nullptr;             // [8, d]: the residual stream's other buffer in small steps (norm_gemm.h)
   kge::bf16 *h = nullptr, *res = nullptr, *xn = nullptr, *qkv = nullptr, *attn = nullptr;
   kge::bf16 *gu = nullptr, *act = nullptr, *xsel = nullptr, *logits = nullptr;

@@ -181,14 +181,16 @@ int engine_forward(kge_engine* e, int T, int B, int R, int max_blocks, int max_q
 #undef REDUCE_NORM
   if (R > 0) {
     // logits only for the last token of each sampled request (logits_processor.py:54-99)
-    FWD(C_EMBED, 2.0 * R * d * 2, 0, e->op->embed(e->xsel, m.rows, e->xn, nullptr, nullptr, 0, R, d, st));
+    const bool gather = !e->step_rows_all || e->tp_size > 1;
+    const bf16* xsel = gather ? e->xsel : e->xn;
+    if (gather) FWD(C_EMBED, 2.0 * R * d * 2, 0, e->op->embed(e->xsel, m.rows, e->xn, nullptr, nullptr, 0, R, d, st));
     Linear head;
     head.w = e->lm_head; head.b = nullptr; head.N = e->vocab_loc; head.K = d;
     if (e->tp_size == 1) {
-      LINEAR(e->logits, e->xsel, head, R, 0);
+      LINEAR(e->logits, xsel, head, R, 0);
     } else {
       // this rank's vocabulary columns, then the all-gather of vllm:model_executor/layers/logits_processor.py:83
-      LINEAR(e->logits_loc, e->xsel, head, R, 0);
+      LINEAR(e->logits_loc, xsel, head, R, 0);
       if (peer)
         FWD(C_AR, 2.0 * R * s.vocab, 0, kge_tp_all_gather_cols(e->tpc, e->off_logits, e->logits_loc, R, e->vocab_loc, s.vocab, e->vocab_col0, st));
       else
@@ -214,8 +216,11 @@ int engine_decode_step(kge_engine* e, int B, int stride, int max_seq_len, const 
   const bool hybrid = e->spec.is_hybrid();
   const int ns = hybrid ? 0 : attn_decode_splits(B, e->KV_loc, max_seq_len);
   auto forward = [&]() -> int {
-    return hybrid ? hybrid_forward(e, B, B, B, stride, dm, any_random)
-                  : engine_forward(e, B, B, B, stride, 1, max_seq_len, dm, any_random, sum_seq, attn_flops);
+    if (hybrid) return hybrid_forward(e, B, B, B, stride, dm, any_random);
+    e->step_rows_all = true;
+    const int rc = engine_forward(e, B, B, B, stride, 1, max_seq_len, dm, any_random, sum_seq, attn_flops);
+    e->step_rows_all = false;
+    return rc;
   };
   if (!e->use_graphs || e->timing || e->step_num_masks > 0 || e->layer_dump_host)      // a masked step is rare and its mask list is not part of a graph
     return forward();
