@@ -913,6 +913,75 @@ __global__ void mlstm_norm_gate_kernel(MlstmArgs a) {
   }
 }
 
+// Decode steps, one row a request, in one launch: log gates, state, read-out, its norm over the head and the output gate.  A block has 32
+// value columns of a head, a warp 16 of the key dimensions (DIM / 8); the blocks of a head form a cluster, which adds up the head's
+// squares and holds the new normaliser back until all have read the old one.  4 heads of 128 x 256, us back to back (cold caches), in
+// three launches (mlstm_log_gates, mlstm_cols, mlstm_norm_gate) and here: 1 request 12.5 (18.5) and 4.0 (10.3), 2 requests 12.5 and 4.2,
+// 8 requests 13.4 and 6.4, 64 requests 25.0 and 21.6, 200 requests 75.3 and 63.5 (HBM: the state is read and written).
+template <typename E>
+__global__ void __launch_bounds__(256) mlstm_token_kernel(MlstmArgs a) {
+  cluster_arrive_relaxed();                                    // waited for before the first remote store
+  pdl_launch_dependents();
+  pdl_wait();
+  __shared__ __align__(16) float qs[ML_MAXD], ks[ML_MAXD], part[8][33], np_s[8], squares[8];
+  const int b = blockIdx.x, h = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, c = blockIdx.z * 32 + lane;
+  const int dim = a.dim, vdim = a.vdim, per = (dim + 7) / 8, d0 = warp * per, d1 = min(dim, d0 + per);
+  const bool in = c < vdim, fresh = a.positions[b] == 0;
+  float* slot = a.state + (int64_t)a.slots[b] * a.slot_stride + (int64_t)h * ((int64_t)dim * vdim + dim + 1);
+  const float ip = a.gates[(int64_t)b * 2 * a.H + h], fp = a.gates[(int64_t)b * 2 * a.H + a.H + h];
+  const float vv0 = in ? ldf((const E*)a.v + (int64_t)b * a.ld + h * vdim + c) : 0.f;
+  float gate = 0.f, w = 0.f;
+  if (warp == 0 && in) { gate = ldf((const E*)a.g + (int64_t)b * a.ld + h * vdim + c); w = ldf((const E*)a.norm_w + h * vdim + c); }
+  float nk = 0.f, nq = 0.f, nv = 0.f;
+  if (tid < dim) {
+    nk = ldf((const E*)a.k + (int64_t)b * a.ld + h * dim + tid);
+    nq = ldf((const E*)a.q + (int64_t)b * a.ld + h * dim + tid) * a.q_scale;
+    nv = fresh ? 0.f : slot[(int64_t)dim * vdim + tid];
+    ks[tid] = nk; qs[tid] = nq;
+  }
+  const float m0 = fresh ? 0.f : slot[(int64_t)dim * vdim + dim];
+  float S[ML_MAXD / 8];
+#pragma unroll
+  for (int k = 0; k < ML_MAXD / 8; ++k) S[k] = d0 + k < d1 && in && !fresh ? slot[(int64_t)(d0 + k) * vdim + c] : 0.f;
+  const float it = a.cap * tanhf(ip / a.cap), fc = a.cap * tanhf(fp / a.cap), ft = fminf(fc, 0.f) - log1pf(expf(-fabsf(fc)));
+  const float mn = fmaxf(ft + m0, it), fa = expf(ft + m0 - mn), ia = expf(it - mn), vv = ia * vv0;
+  __syncthreads();
+  float num = 0.f;
+#pragma unroll
+  for (int k = 0; k < ML_MAXD / 8; ++k)
+    if (d0 + k < d1) {
+      S[k] = fmaf(fa, S[k], ks[d0 + k] * vv);
+      num = fmaf(S[k], qs[d0 + k], num);
+      if (in) slot[(int64_t)(d0 + k) * vdim + c] = S[k];
+    }
+  part[warp][lane] = num;
+  const float nn = fmaf(fa, nv, ia * nk), np = warp_sum(tid < dim ? nn * nq : 0.f);
+  if (lane == 0) np_s[warp] = np;
+  cluster_wait();
+  __syncthreads();
+  float o = 0.f;
+  if (warp == 0) {
+    float den = 0.f;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) { o += part[k][lane]; den += np_s[k]; }
+    o = in ? o / (fmaxf(fabsf(den), expf(-mn)) + a.den_eps) : 0.f;
+    const float sq = warp_sum(o * o);
+    if (lane < (int)gridDim.z)
+      asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(mapa_u32((uint32_t)__cvta_generic_to_shared(&squares[blockIdx.z]), (uint32_t)lane)), "f"(sq) : "memory");
+  }
+  cluster_arrive(); cluster_wait();                            // the squares are there, and all have read n and m
+  if (warp == 0 && in) {
+    float ss = 0.f;
+    for (int k = 0; k < (int)gridDim.z; ++k) ss += squares[k];
+    const float inv = a.out_scale / sqrtf(ss / (float)vdim + a.eps);
+    stf((E*)a.out + (int64_t)b * a.ldo + h * vdim + c, o * inv * w * (1.f / (1.f + expf(-gate))));
+  }
+  if (blockIdx.z == 0) {
+    if (tid < dim) slot[(int64_t)dim * vdim + tid] = nn;
+    if (tid == 0) slot[(int64_t)dim * vdim + dim] = mn;
+  }
+}
+
 // Tensor-core chunks or the fp32 ones, by estimates (us) from measurements at 8 x 32 x 32 to 4 x 128 x 256 and 1 to 256 requests: a
 // tensor-core block fills an SM and takes 9 us beside 7 per 64 tokens of the longest request, an fp32 one shares it with two others,
 // 8 us and 1.1 per token (0.6 to 1.1 by head size).  4 x 128 x 256, tensor cores and fp32: 2 x 1150 tokens 152 / 1278, 200 and 64
@@ -925,6 +994,20 @@ static bool mlstm_use_mma(const MlstmArgs& a) {
 int mlstm_step(const MlstmArgs& a, cudaStream_t st) {
   if (a.T <= 0 || a.B <= 0) return 0;
   if (a.o_scratch && a.nm_scratch && a.dim <= ML_MAXD && a.dim % 4 == 0 && a.H <= 65535) {
+    if (a.T == a.B && a.vdim <= 8 * 32) {
+      auto kern = a.elt == KGE_ELT_F32 ? mlstm_token_kernel<float> : mlstm_token_kernel<__nv_bfloat16>;
+      prefer_max_shared(kern);
+      cudaLaunchConfig_t cfg = {};
+      cfg.gridDim = dim3(a.B, a.H, (a.vdim + 31) / 32); cfg.blockDim = dim3(256); cfg.stream = st;
+      cudaLaunchAttribute attr[2];
+      attr[0].id = cudaLaunchAttributeClusterDimension;
+      attr[0].val.clusterDim.x = 1; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = cfg.gridDim.z;
+      attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+      attr[1].val.programmaticStreamSerializationAllowed = 1;
+      cfg.attrs = attr; cfg.numAttrs = pdl_for_this_launch() ? 2 : 1;
+      KGE_CUDA_OK(cudaLaunchKernelEx(&cfg, kern, a));
+      return 0;
+    }
     const dim3 grid(a.B, a.H, (a.vdim + ML_COLS - 1) / ML_COLS), g2(a.T + a.B, a.H);
     const int nt = std::min(256, (a.vdim + 31) / 32 * 32);
     KGE_CUDA_OK(launch_pdl(mlstm_log_gates_kernel, dim3((a.T * 2 * a.H + 255) / 256), dim3(256), 0, st, const_cast<float*>(a.gates), a.T, a.H, a.cap));

@@ -98,6 +98,41 @@ def test_recurrence_by_tiles(kge, tmp_path, width, blocks, taps):
     llm.close()
 
 
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+@pytest.mark.parametrize("heads,dim,vdim,requests", [(3, 128, 256, 3), (1, 4, 8, 9), (2, 36, 40, 5), (2, 128, 33, 2), (1, 16, 264, 2)])
+def test_matrix_memory_token_by_token(kge, tmp_path, heads, dim, vdim, requests, dtype):
+    """Decode steps in one launch: key dimensions that do not fill their warps, value columns that end inside a block and take one to eight
+    blocks, the first width beyond (264); requests that start at different steps, so that some states are fresh."""
+    cfg = oh.make_config(layers=("parallel",), mlps=(None,), left_scale=0.0, m_heads=heads, m_dim=dim, m_vdim=vdim)
+    W = oh.make_weights(cfg, seed=47)
+    toks = prompt(cfg, 24)
+    want = oh.forward(cfg, W, toks)
+    llm = make_engine(kge, tmp_path, cfg, W, dtype, tokens=1024, seqs=16)
+    at = [0] * requests
+    for turn in range(16):
+        live = [r for r in range(requests) if r <= turn and at[r] < 24]
+        for r in live:
+            llm.trace_add(r, [toks[at[r]]])
+        got = llm.trace_step([(r, 1, [0]) for r in live])
+        check(got, want[[at[r] for r in live]], dtype, f"step {turn}")
+        for r in live:
+            at[r] += 1
+    llm.close()
+
+
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+@pytest.mark.parametrize("experts,top,width", [(16, 2, 512), (17, 4, 2056), (33, 3, 40), (128, 5, 136), (129, 2, 136)])
+def test_routing_of_a_few_tokens(kge, tmp_path, experts, top, width, dtype):
+    """Scores, choice and grouping in one launch: one row a warp, several, the last count of experts it takes and the first it does not, rows
+    longer than what is asked for ahead; one to five tokens (four are the most)."""
+    cfg = oh.make_config(width=width, layers=("rglru",), mlps=("moe",), experts=experts, top=top, expert_ff=16)
+    W = oh.make_weights(cfg, seed=53)
+    toks = prompt(cfg, 15)
+    llm = make_engine(kge, tmp_path, cfg, W, dtype)
+    check(run_pieces(llm, 0, toks, [1, 2, 3, 4, 5]), oh.forward(cfg, W, toks), dtype)
+    llm.close()
+
+
 @pytest.mark.parametrize("hd", [64, 128])
 def test_short_biased_pieces(kge, tmp_path, hd):
     """Pieces around the length from which on prompts run in the tcgen05 kernel: the last whose keys are one tile of the other, and the next."""
