@@ -168,10 +168,8 @@ __global__ void __launch_bounds__(256) moe_pick_kernel(MoeRouteArgs a, int per_w
   moe_pick(a, t, sc, lane);
 }
 
-__global__ void __launch_bounds__(1024) moe_group_kernel(MoeRouteArgs a) {
-  pdl_launch_dependents();
-  pdl_wait();
-  extern __shared__ int cnt[];            // [E] counts, then [E] cursors
+// The pairs by expert, by one block.  cnt: [E] counts, then [E] cursors, in shared memory
+__device__ __forceinline__ void moe_group(const MoeRouteArgs& a, int* cnt) {
   int* cur = cnt + a.E;
   const int n = a.T * a.top, En = a.E - a.identity;      // experts with tensors
   for (int e = threadIdx.x; e < a.E; e += blockDim.x) cnt[e] = 0;
@@ -207,6 +205,77 @@ __global__ void __launch_bounds__(1024) moe_group_kernel(MoeRouteArgs a) {
     a.perm_weight[p] = a.choice_weight[i];
     a.perm_dest[p] = i;
   }
+}
+__global__ void __launch_bounds__(1024) moe_group_kernel(MoeRouteArgs a) {
+  pdl_launch_dependents();
+  pdl_wait();
+  extern __shared__ int cnt[];
+  moe_group(a, cnt);
+}
+
+// Decode steps of a few tokens: scores, choice and grouping in one launch of one block.  A warp has a row of the router at a time, the
+// first one asked for before the kernel before has ended: what this costs is latency.  Same order of summation as dot_part.  16 experts of
+// 2048, top 2, us back to back (with cold caches), in two launches and here: 1 token 7.2 (18.5) and 4.2 (10.3), 2 tokens 7.3 (16.4) and
+// 5.1 (12.3), 4 tokens 7.4 (16.4) and 6.8 (12.3); 8 tokens 7.5 and 10.4: one block's arithmetic, so they stay with a block a token.
+constexpr int MF_WARPS = 16, MF_TOKENS = 4, MF_AHEAD = 8;
+template <typename E>
+__global__ void __launch_bounds__(MF_WARPS * 32) moe_few_kernel(MoeRouteArgs a, int per) {
+  pdl_launch_dependents();
+  extern __shared__ __align__(16) uint4 hs[];      // [token][d], then [token][per] scores and the grouping's counters
+  float* sc_all = reinterpret_cast<float*>(hs + a.T * (a.d * (int)sizeof(E) / 16));
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  constexpr int N = 16 / (int)sizeof(E);
+  const int nrows = a.E + (a.w_extra ? 1 : 0);
+  auto row_of = [&](int e) { return e < a.E ? (const E*)a.w_router + (int64_t)e * a.d : (const E*)a.w_extra; };
+  uint4 ahead[MF_AHEAD];
+  if (warp < nrows)
+#pragma unroll
+    for (int i = 0; i < MF_AHEAD; ++i)
+      if ((lane + i * 32) * N < a.d) ahead[i] = *reinterpret_cast<const uint4*>(row_of(warp) + (lane + i * 32) * N);
+  pdl_wait();
+  const int pieces = a.d / N;
+  for (int i = threadIdx.x; i < a.T * pieces; i += MF_WARPS * 32) {
+    const int t = i / pieces, p = i - t * pieces;
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(hs + i)), "l"((const E*)a.h + (int64_t)t * a.ldh + p * N) : "memory");
+  }
+  asm volatile("cp.async.wait_all;" ::: "memory");
+  __syncthreads();
+  auto term = [](float acc, uint4 x, uint4 y) {
+    if constexpr (sizeof(E) == 2) {
+      const uint32_t u[4] = {x.x, x.y, x.z, x.w}, v[4] = {y.x, y.y, y.z, y.w};
+#pragma unroll
+      for (int j = 0; j < 4; ++j) { acc = fmaf(bf_lo(u[j]), bf_lo(v[j]), acc); acc = fmaf(bf_hi(u[j]), bf_hi(v[j]), acc); }
+    } else {
+      acc = fmaf(__uint_as_float(x.x), __uint_as_float(y.x), acc); acc = fmaf(__uint_as_float(x.y), __uint_as_float(y.y), acc);
+      acc = fmaf(__uint_as_float(x.z), __uint_as_float(y.z), acc); acc = fmaf(__uint_as_float(x.w), __uint_as_float(y.w), acc);
+    }
+    return acc;
+  };
+  for (int e = warp; e < nrows; e += MF_WARPS) {
+    const E* w = row_of(e);
+    if (e != warp)
+#pragma unroll
+      for (int i = 0; i < MF_AHEAD; ++i)
+        if ((lane + i * 32) * N < a.d) ahead[i] = *reinterpret_cast<const uint4*>(w + (lane + i * 32) * N);
+#pragma unroll 2
+    for (int t = 0; t < a.T; ++t) {
+      const uint4* h = hs + t * pieces;
+      float acc = 0.f;
+#pragma unroll
+      for (int i = 0; i < MF_AHEAD; ++i)
+        if (lane + i * 32 < pieces) acc = term(acc, h[lane + i * 32], ahead[i]);
+      for (int k = lane + MF_AHEAD * 32; k < pieces; k += 32) acc = term(acc, h[k], *reinterpret_cast<const uint4*>(w + k * N));
+      acc = warp_sum(acc);
+      if (lane == 0) {
+        if (e < a.E) sc_all[t * per + e] = a.b_router ? acc + ldf((const E*)a.b_router + e) : acc;
+        else a.extra_sigmoid[t] = 1.f / (1.f + expf(-acc));
+      }
+    }
+  }
+  __syncthreads();
+  if (warp < a.T) moe_pick(a, warp, sc_all + warp * per, lane);
+  __syncthreads();                        // the choices are there
+  moe_group(a, reinterpret_cast<int*>(sc_all + a.T * per));
 }
 
 // Bound by its bytes: 16 of them at a time, be the row zeros, a plain copy or weighted.  4480 padded rows of 2048 with weights, number by
@@ -265,6 +334,14 @@ int moe_route(const MoeRouteArgs& a, cudaStream_t st) {
   const size_t smem = (size_t)per * 4;
   KGE_REQUIRE(!a.logits || ((!a.extra_sigmoid || a.ld_logits > a.E) && smem * 8 <= 48 * 1024), "moe_route: %d router outputs with ready logits", a.E);
   cudaError_t ce;
+  const int row = 16 / (a.elt == KGE_ELT_F32 ? 4 : 2);
+  const size_t few = (size_t)a.T * a.d * (16 / row) + smem * a.T + (size_t)2 * a.E * 4;
+  if (!a.logits && a.T <= MF_TOKENS && a.E <= 128 && few <= 48 * 1024 && a.d % row == 0 && a.ldh % row == 0 &&
+      ((reinterpret_cast<uintptr_t>(a.h) | reinterpret_cast<uintptr_t>(a.w_router) | reinterpret_cast<uintptr_t>(a.w_extra)) & 15) == 0) {
+    if (a.elt == KGE_ELT_F32) KGE_CUDA_OK(launch_pdl(moe_few_kernel<float>, dim3(1), dim3(MF_WARPS * 32), few, st, a, per));
+    else KGE_CUDA_OK(launch_pdl(moe_few_kernel<__nv_bfloat16>, dim3(1), dim3(MF_WARPS * 32), few, st, a, per));
+    return 0;
+  }
   if (a.logits) ce = launch_pdl(moe_pick_kernel, dim3((a.T + 7) / 8), dim3(256), smem * 8, st, a, per);
   else ce = a.elt == KGE_ELT_F32 ? launch_pdl(moe_score_kernel<float>, dim3(a.T), dim3(256), smem, st, a)
                                         : launch_pdl(moe_score_kernel<__nv_bfloat16>, dim3(a.T), dim3(256), smem, st, a);
