@@ -70,6 +70,8 @@ int dyt_combine(const DytCombineArgs& a, cudaStream_t st);
 
 // res[t, :] = float(table[ids[t], :])
 int embed_f32(float* res, const int32_t* ids, const void* table, int T, int d, int elt, cudaStream_t st);
+// rows `rows[0] < rows[1] < ...` (n <= 256) of three row-major buffers, rows of the given byte counts (multiples of 2), to their first n rows
+int rows_to_front(const int32_t* rows, int n, void* a, int64_t a_bytes, void* b, int64_t b_bytes, void* c, int64_t c_bytes, cudaStream_t st);
 // Token embedding plus a row of a second table picked by the token and the one before it: with p the previous token of the
 // sequence, res[t, :] = float(table[ids[t], :]) + float(bigram[(p * mul_prev + ids[t] * mul_cur) mod buckets, :]), a sequence's
 // first token (position 0) taking row `buckets` (bigram null: the token's row alone, no state); y (elt, optional) receives the same row.  The token before a request's

@@ -741,6 +741,36 @@ int embed_f32(float* res, const int32_t* ids, const void* table, int T, int d, i
   return 0;
 }
 
+// Ascending rows of up to three buffers to their front, in place.  A thread owns one piece (16 bytes, or 2 where a row or a base is not a
+// multiple of 16) of every row and takes the rows in order, 16 at a time: it reads them all before it writes, and a row written is never
+// one that is still to be read, since row k lies at rows[k] >= k.
+struct FrontRows { uint8_t* p[3]; int64_t bytes[3]; };
+template <class V>
+__global__ void __launch_bounds__(128) rows_to_front_kernel(FrontRows f, const int32_t* rows, int n) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, row = f.bytes[blockIdx.y];
+  if (c >= row / (int64_t)sizeof(V)) return;
+  uint8_t* p = f.p[blockIdx.y] + c * sizeof(V);
+  for (int r0 = 0; r0 < n; r0 += 16) {
+    V v[16];
+#pragma unroll
+    for (int j = 0; j < 16; ++j) if (r0 + j < n) v[j] = *reinterpret_cast<const V*>(p + rows[r0 + j] * row);
+#pragma unroll
+    for (int j = 0; j < 16; ++j) if (r0 + j < n) *reinterpret_cast<V*>(p + (r0 + j) * row) = v[j];
+  }
+}
+int rows_to_front(const int32_t* rows, int n, void* a, int64_t a_bytes, void* b, int64_t b_bytes, void* c, int64_t c_bytes, cudaStream_t st) {
+  if (n <= 0) return 0;
+  const FrontRows f = {{(uint8_t*)a, (uint8_t*)b, (uint8_t*)c}, {a_bytes, b_bytes, c_bytes}};
+  const uintptr_t any = (uintptr_t)a | (uintptr_t)b | (uintptr_t)c | (uintptr_t)a_bytes | (uintptr_t)b_bytes | (uintptr_t)c_bytes;
+  const int64_t longest = std::max(a_bytes, std::max(b_bytes, c_bytes));
+  auto blocks = [&](int piece) { return dim3((unsigned)((longest / piece + 127) / 128), 3); };
+  KGE_CUDA_OK((any & 15) == 0 ? launch_pdl(rows_to_front_kernel<uint4>, blocks(16), dim3(128), 0, st, f, rows, n)
+                              : launch_pdl(rows_to_front_kernel<uint16_t>, blocks(2), dim3(128), 0, st, f, rows, n));
+  return 0;
+}
+
 // one block per token; the row's four-column pieces when the tables allow
 template <typename E, bool VEC>
 __global__ void __launch_bounds__(256) embed_bigram_kernel(BigramArgs a) {

@@ -454,3 +454,42 @@ def test_trace_runner_command_line(kge, tmp_path):
                         "--max-tokens", "128"], input="", capture_output=True, text=True, timeout=600)
     assert r.returncode == 3, (r.returncode, r.stderr[-500:])
 
+
+
+def last_layer_designs():
+    """A last layer of every kind whose rows behind the mixer run for the asked tokens only, with and without a feed-forward, one and
+    several residual streams, plain and normed results."""
+    from oracle import girolorn as og, kogonex as okg, nosolix as on, zezilix as oz
+    out = {f"{mixer}-{mlp}": (oh, oh.make_config(layers=("rglru", mixer), mlps=("dense", mlp))) for mixer in ("rglru", "parallel") for mlp in ("dense", "moe", None)}
+    out["attention-moe"] = og, og.make_config(n_layers=2)
+    out["delta-moe"] = okg, okg.make_config([okg.latent_layer(), okg.delta_layer()], width=96)
+    out["shared-latent"] = okg, okg.make_config([okg.latent_layer(), okg.latent_layer(size=9, kv_from=0, mlp=None)], width=96)
+    out["scan-dense"] = on, on.make_config([on.mamba_layer(mlp=on.dense_mlp()), on.mamba_layer(mlp=on.dense_mlp(28))], width=96)
+    out["scan-moe"] = on, on.make_config([on.mamba_layer(), on.mamba_layer()], width=96)
+    out["wkv-streams"] = oz, oz.make_config([oz.latent_layer(mlp="moe"), oz.wkv_layer(mlp="dense")])
+    out["latent-streams"] = oz, oz.make_config([oz.wkv_layer(mlp="dense"), oz.latent_layer(gated=True, mlp="moe")], loop=(0, 2, 2))
+    return out
+
+
+@pytest.mark.parametrize("design", ["rglru-dense", "rglru-moe", "rglru-None", "parallel-dense", "parallel-moe", "parallel-None", "attention-moe", "delta-moe",
+                                    "shared-latent", "scan-dense", "scan-moe", "wkv-streams", "latent-streams"])
+def test_last_layer_of_the_asked_rows(kge, tmp_path, design):
+    """Prompt steps that ask for few of their tokens' logits: none (the next piece stands on its caches and states), the first row, rows
+    side by side, more than one turn of the copying kernel, one row for four tokens, and places out of order."""
+    o, cfg = last_layer_designs()[design]
+    W = o.make_weights(cfg, seed=31)
+    toks = prompt(cfg, 150, 32)
+    want = o.forward(cfg, W, toks).numpy()
+    d = str(tmp_path / "m")
+    o.save_model_dir(d, cfg, W)
+    llm = kge.LLM(d, dtype="float32", block_size=16, num_gpu_blocks_override=33, max_model_len=513, max_num_seqs=64, max_num_batched_tokens=512, enable_prefix_caching=False)
+    at = 0
+    for n, places in ((9, []), (21, [20]), (12, [0, 1, 11]), (80, list(range(0, 80, 4))), (20, [7, 3]), (8, [7])):
+        llm.trace_add(0, toks[at:at + n])
+        got = llm.trace_step([(0, n, places)])
+        if places: check(got, want[[at + p for p in places]], "float32", f"{n} tokens, places {places}")
+        at += n
+    # beside other requests, one of which wants nothing
+    llm.trace_add(1, toks[:40]); llm.trace_add(2, toks[:33]); llm.trace_add(3, toks[:1])
+    check(llm.trace_step([(3, 1, [0]), (1, 40, []), (2, 33, [5, 32])]), want[[0, 5, 32]], "float32", "three requests")
+    llm.close()
