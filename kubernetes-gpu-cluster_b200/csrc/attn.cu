@@ -369,14 +369,20 @@ static int launch_attn(bf16* out, const bf16* q, int q_stride, const bf16* kc, c
   const int G = H / KV;
   if (max_q_len == 1 && G <= 16) {
     const int ns = decode_splits(B, KV, max_seq_len);
-    if (ns > 1 && ns <= 8 && tunable(TUN_ATTN_CLUSTER_MERGE) && !extras) {
-      // opt-in: split-KV CTAs of one (request, kv head) as a cluster, merged over DSMEM - no workspace and one
-      // kernel, but measured SLOWER than the merge kernel behind programmatic dependent launch (C3 decode step
-      // 7.64 vs 7.38 ms): cluster co-scheduling costs more than the extra launch
-      auto kern = attn_decode_kernel<HD, kDecodeStages, true>;
-      KGE_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, decode_smem<HD>(kDecodeStages)));
+    constexpr int kFew = HD == 64 ? kDecodeStagesFew : kDecodeStages;
+    const bool few = HD == 64 && (int64_t)ns * KV * B <= 2 * 148;
+    const bool tma = tunable(TUN_ATTN_TMA) && bs >= 32 && decode_tma_supported(B, KV, bs);
+    if (ns > 1 && ns <= 8 && !extras && (tunable(TUN_ATTN_CLUSTER_MERGE) || (few && !tma))) {
+      // split-KV CTAs of one (request, kv head) as a cluster, merged over DSMEM: no workspace and one kernel.  By itself for small
+      // launches of 64-wide heads (the line of kDecodeStagesFew): 32 / 8 heads, one request of 500 keys 6.7 us with the merge kernel and
+      // 6.2 so, 4 of 2000 8.9 and 8.0, 16 of 300 7.5 and 6.7, 8 of 2000 level; but 128-wide heads 8.2 and 8.5 (one of 500; 8 of 500 with
+      // 4 kv heads 9.0 and 10.6), and where the SMs are full co-scheduling costs more than the merge kernel behind programmatic
+      // dependent launch (a decode step of 64 requests 7.64 and 7.38 ms): there only where asked for.
+      auto kern = few ? attn_decode_kernel<HD, kFew, true> : attn_decode_kernel<HD, kDecodeStages, true>;
+      const int smem = decode_smem<HD>(few ? kFew : kDecodeStages);
+      KGE_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
       cudaLaunchConfig_t cfg = {};
-      cfg.gridDim = dim3(ns, KV, B); cfg.blockDim = dim3(128); cfg.dynamicSmemBytes = decode_smem<HD>(kDecodeStages); cfg.stream = st;
+      cfg.gridDim = dim3(ns, KV, B); cfg.blockDim = dim3(128); cfg.dynamicSmemBytes = smem; cfg.stream = st;
       cudaLaunchAttribute attr[2];
       attr[0].id = cudaLaunchAttributeClusterDimension;
       attr[0].val.clusterDim.x = ns; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
@@ -398,13 +404,12 @@ static int launch_attn(bf16* out, const bf16* q, int q_stride, const bf16* kc, c
     // (measured: with 16-token blocks a TMA box is 2 KB and the TMA unit's request
     // rate, not HBM, bounds the kernel - 107 us against 102 us for the cp.async gathers; from 32-token blocks on the
     // boxes are large enough and TMA wins, 96 us at 64)
-    if (tunable(TUN_ATTN_TMA) && bs >= 32 && decode_tma_supported(B, KV, bs))
+    if (tma)
       return paged_attn_decode_tma(out, q, q_stride, kc, vc, bt, max_blocks, sl, qsl, B, H, KV, HD, bs, ns, sl2, po, pml, ws, ws_bytes,
                                    max_seq_len, cap_in2, cap_log2, sinks, st);
     KGE_REQUIRE(!extras, "paged attention: a soft cap or sink logits need the TMA-staged decode kernel (blocks of 32 tokens or more)");
-    const bool few = HD == 64 && (int64_t)ns * KV * B <= 2 * 148;
-    auto kern = few ? attn_decode_kernel<HD, HD == 64 ? kDecodeStagesFew : kDecodeStages, false> : attn_decode_kernel<HD, kDecodeStages, false>;
-    const int smem = decode_smem<HD>(few ? kDecodeStagesFew : kDecodeStages);
+    auto kern = few ? attn_decode_kernel<HD, kFew, false> : attn_decode_kernel<HD, kDecodeStages, false>;
+    const int smem = decode_smem<HD>(few ? kFew : kDecodeStages);
     KGE_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     KGE_CUDA_OK(launch_pdl(kern, dim3(ns, KV, B), dim3(128), smem, st, out, po, pml, q, q_stride, kc, vc, bt,
                            max_blocks, sl, qsl, H, KV, bs_shift, sl2));

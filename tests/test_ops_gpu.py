@@ -613,6 +613,9 @@ DECODE_SPLIT_CASES = [
     (64, 8, 128, [1, 1], [900, 33], 3),
     (28, 4, 128, [1] * 2, [300, 2000], 5),
     (32, 8, 128, [1], [6000], 0),                # heuristic picks > 8 splits: workspace + merge kernel path
+    (32, 8, 64, [1] * 2, [1900, 300], 8),        # 64-wide heads, small launches: clusters of eight, most of them without keys
+    (4, 4, 64, [1] * 3, [1, 257, 2040], 0),
+    (32, 8, 64, [1] * 19, [257 + 13 * i for i in range(19)], 0),      # ... and one CTA too many for it: the merge kernel
 ]
 
 
