@@ -25,6 +25,10 @@ __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, bool v
   const int sz = valid ? 16 : 0;   // src-size 0 => zero fill
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(sz));
 }
+// the same unless `skip`; straight-line code, so that the block ids of all rows are read together
+__device__ __forceinline__ void cp_async16_unless(uint32_t dst, const void* src, bool valid, bool skip) {
+  asm volatile("{\n.reg .pred p;\nsetp.eq.u32 p, %3, 0;\n@p cp.async.cg.shared.global [%0], [%1], 16, %2;\n}" ::"r"(dst), "l"(src), "r"(valid ? 16 : 0), "r"((uint32_t)skip));
+}
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;"); }
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N)); }
@@ -86,9 +90,10 @@ struct KvLoader {
     for (int j = 0; j < NP; ++j) dst[j] = swz<HD>(row0 + j * RP, c);
   }
   // EARLY: the block id is read whether the key exists or not, so that it need not wait for the request's length
-  template <bool EARLY>
+  // SKIP: the row of key `skip` is left as it is (own() brings it)
+  template <bool EARLY, bool SKIP = false>
   __device__ __forceinline__ void load(uint32_t sK, uint32_t sV, const bf16* __restrict__ kc,
-                                       const bf16* __restrict__ vc, int key0, int kv_len) const {
+                                       const bf16* __restrict__ vc, int key0, int kv_len, int skip = -1) const {
 #pragma unroll
     for (int j = 0; j < NP; ++j) {
       const int key = key0 + row0 + j * RP;
@@ -100,9 +105,21 @@ struct KvLoader {
       } else if (ok) {
         off = (int64_t)btab[key >> bs_shift] * blk_stride + head_off + (key & bs_mask) * HD + c8;
       }
-      cp_async16(sK + dst[j], kc + off, ok);
-      cp_async16(sV + dst[j], vc + off, ok);
+      if (SKIP) {
+        cp_async16_unless(sK + dst[j], kc + off, ok, key == skip);
+        cp_async16_unless(sV + dst[j], vc + off, ok, key == skip);
+      } else {
+        cp_async16(sK + dst[j], kc + off, ok);
+        cp_async16(sV + dst[j], vc + off, ok);
+      }
     }
+  }
+  // the row of one key, which is there
+  __device__ __forceinline__ void own(uint32_t sK, uint32_t sV, const bf16* __restrict__ kc, const bf16* __restrict__ vc, int key0, int key) const {
+    const int64_t off = (int64_t)btab[key >> bs_shift] * blk_stride + head_off + (key & bs_mask) * HD + c8;
+#pragma unroll
+    for (int j = 0; j < NP; ++j)
+      if (key0 + row0 + j * RP == key) { cp_async16(sK + dst[j], kc + off, true); cp_async16(sV + dst[j], vc + off, true); }
   }
 };
 
@@ -113,7 +130,10 @@ struct KvLoader {
 // CLUSTER: the `splits` CTAs of one (request, kv head) form a thread-block cluster; each leaves its partial in
 // its own shared memory and every rank finishes a slice of the output columns by reading its peers' partials
 // over DSMEM - same arithmetic and summation order as attn_merge_kernel, no workspace, no second kernel.
-template <int HD, int STAGES, bool CLUSTER>
+// EARLY: all keys but each request's last, the lengths and the block table were there before the launch's step began (the caller's
+// word), so that they are fetched while the kernel before still runs; only q and the last key wait for it.  A decode step of opt-125m
+// (12 layers), one request of 190 keys: 262 us without, 246 with; of 32 keys 243 and 233; 8 requests of up to 60 keys 403 and 393.
+template <int HD, int STAGES, bool CLUSTER, bool EARLY>
 __global__ void __launch_bounds__(128)
 attn_decode_kernel(bf16* __restrict__ out, float* __restrict__ part_o, float* __restrict__ part_ml,
                    const bf16* __restrict__ q, int q_stride, const bf16* __restrict__ k_cache,
@@ -122,7 +142,7 @@ attn_decode_kernel(bf16* __restrict__ out, float* __restrict__ part_o, float* __
                    const int32_t* __restrict__ qsl, int H, int KV, int bs_shift, float scale_log2) {
   constexpr int CH = HD / 8, NT = 128;
   pdl_launch_dependents();
-  pdl_wait();
+  if (!EARLY) pdl_wait();
   const int b = blockIdx.z, kvh = blockIdx.y, split = blockIdx.x, nsplit = gridDim.x;
   const int G = H / KV;
   const int kv_len = seq_lens[b];
@@ -141,20 +161,32 @@ attn_decode_kernel(bf16* __restrict__ out, float* __restrict__ part_o, float* __
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int g = lane >> 2, tg = lane & 3;
 
-  for (int i = tid; i < 16 * CH; i += NT) {
-    const int r = i / CH, c = i % CH;
-    const bool ok = r < G;
-    const bf16* src = ok ? q + (int64_t)qrow * q_stride + (kvh * G + r) * HD + c * 8 : q;
-    cp_async16(sQ + swz<HD>(r, c), src, ok);
-  }
+  auto load_q = [&]() {
+    for (int i = tid; i < 16 * CH; i += NT) {
+      const int r = i / CH, c = i % CH;
+      const bool ok = r < G;
+      const bf16* src = ok ? q + (int64_t)qrow * q_stride + (kvh * G + r) * HD + c * 8 : q;
+      cp_async16(sQ + swz<HD>(r, c), src, ok);
+    }
+  };
+  if (!EARLY) load_q();
   KvLoader<HD, NT> ld;
   ld.init(btab, max_blocks, kvh, KV, bs_shift, tid);
   // prologue: STAGES-1 tiles in flight
 #pragma unroll
   for (int s = 0; s < STAGES - 1; ++s) {
     if (t_begin + s < t_end)
-      ld.template load<true>(sK + s * BN * HD * 2, sV + s * BN * HD * 2, k_cache, v_cache, (t_begin + s) * BN, kv_len);
+      ld.template load<true, EARLY>(sK + s * BN * HD * 2, sV + s * BN * HD * 2, k_cache, v_cache, (t_begin + s) * BN, kv_len, kv_len - 1);
     cp_async_commit();
+  }
+  if (EARLY) {
+    pdl_wait();
+    load_q();
+    const int s = ntiles_all - 1 - t_begin;                      // the stage of the last key's tile, where the prologue has it
+    if (t_end == ntiles_all && s >= 0 && s < STAGES - 1)
+      ld.own(sK + s * BN * HD * 2, sV + s * BN * HD * 2, k_cache, v_cache, (ntiles_all - 1) * BN, kv_len - 1);
+    cp_async_commit();
+    cp_async_wait<0>();
   }
 
   uint32_t qf[HD / 16][4];
@@ -360,7 +392,7 @@ template <int HD>
 static int launch_attn(bf16* out, const bf16* q, int q_stride, const bf16* kc, const bf16* vc,
                        const int32_t* bt, int max_blocks, const int32_t* sl, const int32_t* qsl, int B,
                        int max_q_len, int max_seq_len, int H, int KV, int bs, float scale, void* ws,
-                       int64_t ws_bytes, float softcap, const float* sinks, cudaStream_t st) {
+                       int64_t ws_bytes, float softcap, const float* sinks, bool early, cudaStream_t st) {
   const float sl2 = scale * kLog2e;
   const bool extras = softcap > 0.f || sinks;      // soft cap / sink logits: the TMA-staged kernels have them
   const float cap_in2 = softcap > 0.f ? 2.f * kLog2e * scale / softcap : 0.f, cap_log2 = softcap * kLog2e;
@@ -371,6 +403,7 @@ static int launch_attn(bf16* out, const bf16* q, int q_stride, const bf16* kc, c
     const int ns = decode_splits(B, KV, max_seq_len);
     constexpr int kFew = HD == 64 ? kDecodeStagesFew : kDecodeStages;
     const bool few = HD == 64 && (int64_t)ns * KV * B <= 2 * 148;
+    auto pick = [&](auto plain, auto ahead) { return early ? ahead : plain; };      // (128-wide heads have one form)
     const bool tma = tunable(TUN_ATTN_TMA) && bs >= 32 && decode_tma_supported(B, KV, bs);
     if (ns > 1 && ns <= 8 && !extras && (tunable(TUN_ATTN_CLUSTER_MERGE) || (few && !tma))) {
       // split-KV CTAs of one (request, kv head) as a cluster, merged over DSMEM: no workspace and one kernel.  By itself for small
@@ -378,7 +411,7 @@ static int launch_attn(bf16* out, const bf16* q, int q_stride, const bf16* kc, c
       // 6.2 so, 4 of 2000 8.9 and 8.0, 16 of 300 7.5 and 6.7, 8 of 2000 level; but 128-wide heads 8.2 and 8.5 (one of 500; 8 of 500 with
       // 4 kv heads 9.0 and 10.6), and where the SMs are full co-scheduling costs more than the merge kernel behind programmatic
       // dependent launch (a decode step of 64 requests 7.64 and 7.38 ms): there only where asked for.
-      auto kern = few ? attn_decode_kernel<HD, kFew, true> : attn_decode_kernel<HD, kDecodeStages, true>;
+      auto kern = few ? pick(attn_decode_kernel<HD, kFew, true, false>, attn_decode_kernel<HD, kFew, true, HD == 64>) : attn_decode_kernel<HD, kDecodeStages, true, false>;
       const int smem = decode_smem<HD>(few ? kFew : kDecodeStages);
       KGE_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
       cudaLaunchConfig_t cfg = {};
@@ -408,7 +441,8 @@ static int launch_attn(bf16* out, const bf16* q, int q_stride, const bf16* kc, c
       return paged_attn_decode_tma(out, q, q_stride, kc, vc, bt, max_blocks, sl, qsl, B, H, KV, HD, bs, ns, sl2, po, pml, ws, ws_bytes,
                                    max_seq_len, cap_in2, cap_log2, sinks, st);
     KGE_REQUIRE(!extras, "paged attention: a soft cap or sink logits need the TMA-staged decode kernel (blocks of 32 tokens or more)");
-    auto kern = few ? attn_decode_kernel<HD, kFew, false> : attn_decode_kernel<HD, kDecodeStages, false>;
+    auto kern = few ? pick(attn_decode_kernel<HD, kFew, false, false>, attn_decode_kernel<HD, kFew, false, HD == 64>)
+                    : pick(attn_decode_kernel<HD, kDecodeStages, false, false>, attn_decode_kernel<HD, kDecodeStages, false, HD == 64>);
     const int smem = decode_smem<HD>(few ? kFew : kDecodeStages);
     KGE_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     KGE_CUDA_OK(launch_pdl(kern, dim3(ns, KV, B), dim3(128), smem, st, out, po, pml, q, q_stride, kc, vc, bt,
@@ -445,7 +479,7 @@ inline namespace KGE_ELT_NS {
 int paged_attn_extras(void* out, const void* q, int q_stride, const void* k_cache, const void* v_cache, const int32_t* block_table,
                       int max_blocks_per_seq, const int32_t* seq_lens, const int32_t* query_start_loc, int B, int T, int max_q_len,
                       int max_seq_len, int H, int KV, int hd, int block_size, float scale, float softcap, const float* sinks, void* workspace,
-                      int64_t workspace_bytes, void* stream) {
+                      int64_t workspace_bytes, void* stream, bool early) {
   KGE_REQUIRE(out && q && k_cache && v_cache && block_table && seq_lens && query_start_loc,
               "kge_paged_attn: null pointer");
   KGE_REQUIRE(H > 0 && KV > 0 && H % KV == 0, "kge_paged_attn: H=%d must be a multiple of KV=%d", H, KV);
@@ -461,13 +495,21 @@ int paged_attn_extras(void* out, const void* q, int q_stride, const void* k_cach
   if (hd == 64)
     return launch_attn<64>((bf16*)out, (const bf16*)q, q_stride, (const bf16*)k_cache, (const bf16*)v_cache,
                            block_table, max_blocks_per_seq, seq_lens, query_start_loc, B, max_q_len,
-                           max_seq_len, H, KV, block_size, scale, workspace, workspace_bytes, softcap, sinks, st);
+                           max_seq_len, H, KV, block_size, scale, workspace, workspace_bytes, softcap, sinks, early, st);
   if (hd == 128)
     return launch_attn<128>((bf16*)out, (const bf16*)q, q_stride, (const bf16*)k_cache, (const bf16*)v_cache,
                             block_table, max_blocks_per_seq, seq_lens, query_start_loc, B, max_q_len,
-                            max_seq_len, H, KV, block_size, scale, workspace, workspace_bytes, softcap, sinks, st);
+                            max_seq_len, H, KV, block_size, scale, workspace, workspace_bytes, softcap, sinks, early, st);
   kge::set_error("kge_paged_attn: head_dim=%d unsupported (64, 128)", hd);
   return -1;
+}
+// kge_paged_attn of a step's one-token requests, for callers whose lengths, block table and keys before each request's last were written
+// before the first kernel of the step was launched, and that kernel in plain stream order behind them
+int paged_attn_step(void* out, const void* q, int q_stride, const void* k_cache, const void* v_cache, const int32_t* block_table,
+                    int max_blocks_per_seq, const int32_t* seq_lens, const int32_t* query_start_loc, int B, int T, int max_q_len,
+                    int max_seq_len, int H, int KV, int hd, int block_size, float scale, void* workspace, int64_t workspace_bytes, void* stream) {
+  return paged_attn_extras(out, q, q_stride, k_cache, v_cache, block_table, max_blocks_per_seq, seq_lens, query_start_loc, B, T, max_q_len,
+                           max_seq_len, H, KV, hd, block_size, scale, 0.f, nullptr, workspace, workspace_bytes, stream, max_q_len == 1);
 }
 // whether a pure decode step with these sizes reaches a kernel that has the cap and the sinks
 bool paged_attn_extras_decode_ok(int B, int H, int KV, int hd, int block_size) {
@@ -483,7 +525,7 @@ extern "C" int KGE_API(kge_paged_attn)(void* out, const void* q, int q_stride, c
                               int max_q_len, int max_seq_len, int H, int KV, int hd, int block_size,
                               float scale, void* workspace, int64_t workspace_bytes, void* stream) {
   return paged_attn_extras(out, q, q_stride, k_cache, v_cache, block_table, max_blocks_per_seq, seq_lens, query_start_loc, B, T, max_q_len,
-                           max_seq_len, H, KV, hd, block_size, scale, 0.f, nullptr, workspace, workspace_bytes, stream);
+                           max_seq_len, H, KV, hd, block_size, scale, 0.f, nullptr, workspace, workspace_bytes, stream, false);
 }
 
 #ifndef KGE_HALF      // bfloat16 only: one scratch array per library image
@@ -564,9 +606,9 @@ extern "C" int kge_paged_attn_decode_noalloc(void* out, const void* q, int q_str
   if (hd == 64)
     return launch_attn<64>((bf16*)out, (const bf16*)q, q_stride, (const bf16*)k_cache, (const bf16*)v_cache, block_table,
                            max_blocks_per_seq, seq_lens, query_start_loc, B, 1, max_seq_len, H, KV, block_size, scale,
-                           ws, kNoAllocScratchBytes, 0.f, nullptr, st);
+                           ws, kNoAllocScratchBytes, 0.f, nullptr, false, st);
   return launch_attn<128>((bf16*)out, (const bf16*)q, q_stride, (const bf16*)k_cache, (const bf16*)v_cache, block_table,
                           max_blocks_per_seq, seq_lens, query_start_loc, B, 1, max_seq_len, H, KV, block_size, scale,
-                          ws, kNoAllocScratchBytes, 0.f, nullptr, st);
+                          ws, kNoAllocScratchBytes, 0.f, nullptr, false, st);
 }
 #endif

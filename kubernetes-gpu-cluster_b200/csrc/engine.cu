@@ -12,12 +12,20 @@ using namespace kge;
 
 namespace kge {
 
+#define PAGED_ATTN_STEP                                                                                                                            \
+  int paged_attn_step(void* out, const void* q, int q_stride, const void* k_cache, const void* v_cache, const int32_t* block_table,                \
+                      int max_blocks_per_seq, const int32_t* seq_lens, const int32_t* query_start_loc, int B, int T, int max_q_len, int max_seq_len, \
+                      int H, int KV, int hd, int block_size, float scale, void* workspace, int64_t workspace_bytes, void* stream)
+inline namespace b16 { PAGED_ATTN_STEP; }
+namespace h16 { PAGED_ATTN_STEP; }
+#undef PAGED_ATTN_STEP
+
 const Ops kOpsBf16 = {kge_embed, kge_rmsnorm, kge_add_rmsnorm, kge_head_rmsnorm, kge_layernorm, kge_silu_mul, kge_gemm_bf16,
                       kge_gemm_silu_gate_ws_bf16, kge_rope_kvwrite, kge_rope_cache_host, kge_paged_attn, kge_argmax, kge_sample,
-                      kge_logprobs, kge_tp_reduce_add_norm, kge_norm_gemm};
+                      kge_logprobs, kge_tp_reduce_add_norm, kge_norm_gemm, b16::paged_attn_step};
 const Ops kOpsF16 = {kge_embed_f16, kge_rmsnorm_f16, kge_add_rmsnorm_f16, kge_head_rmsnorm_f16, kge_layernorm_f16, kge_silu_mul_f16,
                      kge_gemm_f16, kge_gemm_silu_gate_ws_f16, kge_rope_kvwrite_f16, kge_rope_cache_host_f16, kge_paged_attn_f16,
-                     kge_argmax_f16, kge_sample_f16, kge_logprobs_f16, kge_tp_reduce_add_norm_f16, kge_norm_gemm_f16};
+                     kge_argmax_f16, kge_sample_f16, kge_logprobs_f16, kge_tp_reduce_add_norm_f16, kge_norm_gemm_f16, h16::paged_attn_step};
 
 // 16-bit pattern of v in the engine's element type
 __device__ __forceinline__ uint16_t to_elt_bits(float v, bool f16) {

@@ -36,6 +36,7 @@ struct Ops {
   decltype(&kge_logprobs) logprobs;
   decltype(&kge_tp_reduce_add_norm) tp_reduce_add_norm;
   decltype(&kge_norm_gemm) norm_gemm;
+  decltype(&kge_paged_attn) paged_attn_step;      // one-token requests whose keys but the last are from before the step (attn.cu)
 };
 extern const Ops kOpsBf16, kOpsF16;     // engine.cu
 
@@ -203,6 +204,9 @@ struct kge_engine {
   int num_blocks = 0, max_blocks_per_seq = 0;
   int64_t weight_bytes = 0, kv_bytes = 0;
 
+  // a decode step in which no request's keys before its last are written: they can be read while the kernel that writes the last still runs
+  bool step_keys_before = false;
+  std::vector<int32_t> block_writer;         // [num_blocks] request of the step that writes to the block + 1 (all zero between steps)
   bool step_rows_all = false;                // the step's logits rows are its tokens, in order: nothing to gather
   kge::bf16* res_next = nullptr;             // [8, d]: the residual stream's other buffer in small steps (norm_gemm.h)
   kge::bf16 *h = nullptr, *res = nullptr, *xn = nullptr, *qkv = nullptr, *attn = nullptr;
@@ -231,7 +235,7 @@ struct kge_engine {
   std::unordered_map<int64_t, std::pair<int, int>> lp_last;    // request id -> (row of the last step, its own N)
 
   // CUDA graphs of pure decode steps, keyed by what is baked into the launches
-  struct DecodeGraph { int B, ns, stride; bool rnd, logits; cudaGraphExec_t exec; int64_t launches; };
+  struct DecodeGraph { int B, ns, stride; bool rnd, logits, before; cudaGraphExec_t exec; int64_t launches; };
   std::vector<DecodeGraph> graphs;
   std::vector<std::pair<int64_t, int>> graph_seen;   // key hash -> eager runs so far
   bool use_graphs = true;
@@ -254,7 +258,7 @@ struct kge_engine {
   struct RecordedStep {
     int T, B, R, stride, max_q, max_seq, num_decode, dec_max_seq;
     double sum_seq, attn_flops, dec_sum_seq;
-    bool decode_only, any_random;
+    bool decode_only, any_random, keys_before;
     int64_t bytes;
     int sample0;                               // index of this step's first sampled row in the job's sample log
     std::vector<uint8_t> meta;

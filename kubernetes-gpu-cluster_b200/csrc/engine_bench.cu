@@ -59,6 +59,7 @@ extern "C" int kge_engine_run_resident(kge_engine* e, const int32_t* prompts_hos
   const bool was_timing = e->timing;
   e->timing = false;
   e->step_num_decode = 0;                 // resident steps are pure prefill or pure decode
+  e->step_keys_before = true;             // (each request in blocks of its own)
   e->step_num_masks = 0;
 
   // ---- build every step's metadata on the host (untimed)
@@ -243,7 +244,7 @@ extern "C" int kge_engine_replay_recorded(kge_engine* e, int32_t* out_tokens_hos
     StepMeta dm = carve_meta(e->meta_dev, st.T, st.B, st.R, st.stride, nullptr);
     cudaMemcpyAsync(e->meta_dev, d_arena + off_meta[i], (size_t)st.bytes, cudaMemcpyDeviceToDevice, e->stream);
     patch_ids_kernel<<<(st.T + 255) / 256, 256, 0, e->stream>>>(dm.ids, (const int32_t*)(d_arena + off_src[i]), d_log, st.T);
-    e->step_num_decode = st.num_decode; e->step_dec_max_seq = st.dec_max_seq; e->step_dec_sum_seq = st.dec_sum_seq;
+    e->step_keys_before = st.keys_before; e->step_num_decode = st.num_decode; e->step_dec_max_seq = st.dec_max_seq; e->step_dec_sum_seq = st.dec_sum_seq;
     if (st.decode_only) rc = engine_decode_step(e, st.B, st.stride, st.max_seq, dm, st.any_random, st.sum_seq);
     else rc = engine_forward(e, st.T, st.B, st.R, st.stride, st.max_q, st.max_seq, dm, st.any_random, st.sum_seq, st.attn_flops);
     if (rc) break;

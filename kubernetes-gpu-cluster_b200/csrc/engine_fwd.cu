@@ -93,7 +93,7 @@ int engine_forward(kge_engine* e, int T, int B, int R, int max_blocks, int max_q
   // offset the per-request arrays
   auto attend = [&](int i) -> int {
     if (D == 0) {
-      FWD(c_att, att_bytes, att_fl, e->op->paged_attn(e->attn, e->qkv, qkv_n, e->kc[i], e->vc[i], m.btab, max_blocks, m.seq_lens, m.qsl, B, T,
+      FWD(c_att, att_bytes, att_fl, (e->step_keys_before && max_q_len == 1 ? e->op->paged_attn_step : e->op->paged_attn)(e->attn, e->qkv, qkv_n, e->kc[i], e->vc[i], m.btab, max_blocks, m.seq_lens, m.qsl, B, T,
                          max_q_len, max_seq_len, Hl, KVl, hd, bs, scale, e->ws_attn, e->ws_attn_bytes, st));
       return 0;
     }
@@ -226,12 +226,12 @@ int engine_decode_step(kge_engine* e, int B, int stride, int max_seq_len, const 
     return forward();
   const bool logits = hybrid && e->want_logits32;      // only layer-list models launch anything for logits that are read back
   for (auto& g : e->graphs)
-    if (g.B == B && g.ns == ns && g.stride == stride && g.rnd == any_random && g.logits == logits) {
+    if (g.B == B && g.ns == ns && g.stride == stride && g.rnd == any_random && g.logits == logits && g.before == e->step_keys_before) {
       KGE_CUDA_OK(cudaGraphLaunch(g.exec, e->stream));
       e->launches += g.launches;
       return 0;
     }
-  const int64_t key = ((int64_t)B << 40) ^ ((int64_t)ns << 32) ^ ((int64_t)stride << 2) ^ (logits ? 2 : 0) ^ (any_random ? 1 : 0);
+  const int64_t key = ((int64_t)B << 40) ^ ((int64_t)ns << 32) ^ ((int64_t)stride << 2) ^ (logits ? 2 : 0) ^ (any_random ? 1 : 0) ^ (e->step_keys_before ? (int64_t)1 << 62 : 0);
   int* seen = nullptr;
   for (auto& kv : e->graph_seen) if (kv.first == key) seen = &kv.second;
   if (!seen) { e->graph_seen.push_back({key, 0}); seen = &e->graph_seen.back().second; }
@@ -246,7 +246,7 @@ int engine_decode_step(kge_engine* e, int B, int stride, int max_seq_len, const 
   cudaError_t ce = cudaStreamEndCapture(e->stream, &graph);
   if (rc) { if (graph) cudaGraphDestroy(graph); return rc; }
   KGE_REQUIRE(ce == cudaSuccess && graph, "decode graph capture failed: %s", cudaGetErrorString(ce));
-  kge_engine::DecodeGraph g{B, ns, stride, any_random, logits, nullptr, e->launches - l0};
+  kge_engine::DecodeGraph g{B, ns, stride, any_random, logits, e->step_keys_before, nullptr, e->launches - l0};
   ce = cudaGraphInstantiate(&g.exec, graph, 0);
   cudaGraphDestroy(graph);
   KGE_REQUIRE(ce == cudaSuccess, "cudaGraphInstantiate failed: %s", cudaGetErrorString(ce));
@@ -266,6 +266,36 @@ __global__ void mask_logits_kernel(bf16* logits, const int32_t* pairs, int n, in
 __global__ void elt_to_f32_kernel(float* o, const bf16* x, int64_t n, bool f16) {
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
     o[i] = f16 ? __half2float(reinterpret_cast<const __half*>(x)[i]) : bf2f(x[i]);
+}
+
+// Whether the keys before each request's last were all there before this decode step: no block of a request's table is written by another
+// request of the step (one may find a full block in the prefix cache that another is about to fill, and a scripted step may hold two rows
+// of one sequence).  The step's metadata is copied in stream order ahead of its first kernel, so that the steps before are complete when
+// that starts.  Tables of more than 4096 blocks are not looked through: 5 us of host time, and steps of that size gain less.
+static bool keys_before_step(kge_engine* e, const kge_step_batch* b) {
+  const int bs = e->cfg.block_size, nb = e->num_blocks;
+  int64_t blocks = 0;
+  for (int i = 0; i < b->B; ++i) blocks += (b->seq_lens[i] + bs - 1) / bs;
+  if (b->B > 1 && blocks > 4096) return false;
+  e->block_writer.resize((size_t)nb, 0);
+  bool ok = true;
+  int marked = 0;
+  for (; marked < b->B && ok; ++marked) {
+    const int64_t blk = b->slot_mapping[marked] / bs;
+    ok = b->slot_mapping[marked] >= 0 && blk < nb && e->block_writer[blk] == 0;
+    if (!ok) break;
+    e->block_writer[blk] = marked + 1;
+  }
+  for (int i = 0; i < b->B && ok; ++i) {
+    const int32_t* t = b->block_table + (size_t)i * b->max_blocks;
+    for (int j = 0, n = (b->seq_lens[i] + bs - 1) / bs; j < n && ok; ++j) {
+      ok = t[j] >= 0 && t[j] < nb && (e->block_writer[t[j]] == 0 || e->block_writer[t[j]] == i + 1);
+    }
+    // ... and it writes its last key where its table has it
+    ok = ok && b->slot_mapping[i] == (int64_t)t[(b->seq_lens[i] - 1) / bs] * bs + (b->seq_lens[i] - 1) % bs;
+  }
+  for (int i = 0; i < marked; ++i) e->block_writer[b->slot_mapping[i] / bs] = 0;
+  return ok;
 }
 
 // Copy the caller's host metadata into the pinned block, ship it, run, read the ids back.
@@ -337,11 +367,12 @@ static int run_step(kge_engine* e, const kge_step_batch* b, const float* temp, c
     max_seq = std::max(max_seq, b->seq_lens[i]);
   }
   KGE_REQUIRE(b->query_start_loc[B] == T, "kge_step: query_start_loc[B]=%d != T=%d", b->query_start_loc[B], T);
+  e->step_keys_before = decode_only && max_q == 1 && keys_before_step(e, b);
   if (e->recording) {
     kge_engine::RecordedStep rs{};
     rs.T = T; rs.B = B; rs.R = R; rs.stride = stride; rs.max_q = max_q; rs.max_seq = max_seq;
     rs.num_decode = e->step_num_decode; rs.dec_max_seq = e->step_dec_max_seq; rs.dec_sum_seq = e->step_dec_sum_seq;
-    rs.sum_seq = sum_seq; rs.attn_flops = attn_flops; rs.decode_only = decode_only && max_q == 1; rs.any_random = any_random;
+    rs.sum_seq = sum_seq; rs.attn_flops = attn_flops; rs.decode_only = decode_only && max_q == 1; rs.any_random = any_random; rs.keys_before = e->step_keys_before;
     rs.bytes = bytes; rs.sample0 = (int)e->rec_sample_req.size();
     rs.meta.assign(e->meta_host, e->meta_host + bytes);
     rs.src = e->rec_pending_src;

@@ -27,7 +27,7 @@ inline namespace b16 {
 int paged_attn_extras(void* out, const void* q, int q_stride, const void* k_cache, const void* v_cache, const int32_t* block_table,
                       int max_blocks_per_seq, const int32_t* seq_lens, const int32_t* query_start_loc, int B, int T, int max_q_len,
                       int max_seq_len, int H, int KV, int hd, int block_size, float scale, float softcap, const float* sinks, void* workspace,
-                      int64_t workspace_bytes, void* stream);
+                      int64_t workspace_bytes, void* stream, bool early = false);
 bool paged_attn_extras_decode_ok(int B, int H, int KV, int hd, int block_size);
 // attn_tc.cu: the tcgen05 prompt kernel with a sliding window and kept first tokens or pooled blocks (64- / 128-wide heads)
 bool paged_attn_window_tc_ok(int H, int KV, int hd, int vd, int bs, int pool, int pool_slots);

@@ -76,3 +76,51 @@ def test_layer_list_steps_with_logits_have_a_graph_of_their_own(kge, tmp_path):
         step(want)
         assert llm.decode_graphs == graphs
     llm.close()
+
+
+@pytest.mark.parametrize("name,lengths", [
+    ("tiny-opt", [1, 62, 63, 64, 65, 127]),                  # one to three tiles; the last key alone in its tile, at its start and at its end
+    ("tiny-opt", [250]),
+    ("tiny-llama", [255, 256, 318, 321, 40, 511]),           # two splits merged in a cluster, one of them empty; a last key behind the tiles of the start
+    ("tiny-llama", [700, 3]),
+    ("tiny-llama", [200 + (i % 17) for i in range(160)]),    # more CTAs than two an SM: three tiles under way
+])
+def test_keys_before_the_step_read_ahead(kge, tmp_path, name, lengths):
+    """A decode step whose attention fetches the keys before each request's last while the projection still runs: eager and replayed against
+    the oracle; and a step of two rows of one sequence, where a row's earlier key is written by the other, which must wait for it."""
+    cfg = om.CONFIGS[name]
+    w = om.make_weights(cfg, seed=0)
+    om.save_model_dir(tmp_path, cfg, w)
+    lengths = [min(n, 240) for n in lengths] if name == "tiny-opt" else lengths      # (its positions end at 256)
+    prompts = [om.make_prompts(cfg, 1, n, seed=11 + i)[0] for i, n in enumerate(lengths)]
+    ids, ref = om.OracleModel(cfg, w, torch.bfloat16, max_pos=1024).generate_greedy(prompts, 2, return_logits=True)
+    bs, per, B = 16, (max(lengths) + 2 + 15) // 16, len(lengths)
+    llm = kge.LLM(str(tmp_path), max_model_len=per * bs, max_num_seqs=B + 1, max_num_batched_tokens=max(256, sum(lengths)), block_size=bs,
+                  num_gpu_blocks_override=B * per + 1, enable_prefix_caching=False)
+    table = 1 + np.arange(B * per, dtype=np.int32).reshape(B, per)
+
+    def step(rows, want=True):
+        """rows: (request, first position, tokens)"""
+        tok = np.concatenate([np.asarray(t, dtype=np.int32) for _, _, t in rows])
+        pos = np.concatenate([np.arange(a, a + len(t), dtype=np.int32) for _, a, t in rows])
+        slots = np.concatenate([table[r, np.arange(a, a + len(t)) // bs].astype(np.int64) * bs + np.arange(a, a + len(t)) % bs for r, a, t in rows])
+        qsl = np.concatenate([[0], np.cumsum([len(t) for _, _, t in rows])]).astype(np.int32)
+        return llm.raw_step(tok, pos, qsl, np.asarray([a + len(t) for _, a, t in rows], dtype=np.int32), table[[r for r, _, _ in rows]], per, slots, qsl[1:] - 1, want_logits=want)
+
+    def close(got, want, what):
+        want = want.numpy() if isinstance(want, torch.Tensor) else want
+        err, scale = np.abs(got - want), np.abs(want).max()
+        assert (err <= 3e-2 * scale + 1.6e-2 * np.abs(want)).all(), f"{what}: {err.max():.4g} of {scale:.3g}"
+
+    step([(r, 0, p) for r, p in enumerate(prompts)], False)
+    turns = [step([(r, len(p), [ids[r][0]]) for r, p in enumerate(prompts)])[1] for _ in range(11)]
+    close(turns[0], ref[1], "decode step")
+    for t in turns[1:]:                                       # eager, captured, replayed
+        assert np.array_equal(t, turns[0])
+    long = int(np.argmax(lengths))
+    n = lengths[long]
+    step([(long, 0, [7] * (n + 1))], False)                   # other keys where the two rows' will be
+    step([(long, 0, prompts[long][:n - 1])], False) if n > 1 else None
+    both = step([(long, n - 1, prompts[long][n - 1:]), (long, n, [ids[long][0]])])[1]
+    close(both, np.stack([ref[0][long], ref[1][long]]), "two rows of one sequence")
+    llm.close()
