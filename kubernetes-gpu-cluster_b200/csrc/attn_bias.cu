@@ -143,10 +143,13 @@ __device__ __forceinline__ void ab_ldsm_t(uint32_t (&r)[4], const void* p) {
 // the warps of a cluster do, and its CTAs' sums meet over distributed shared memory.  A tile's keys and values are asked for at once
 // (cp.async): with a round trip per eight pieces and one CTA per (request, group) two requests of 1160 keys in chunks of 1024 took 27 us
 // (cold caches), 14.5 with clusters of eight.  ROWS = true: a CTA owns 64 rows, 16 per warp, and every key tile is staged once for all four warps (prompts).
-template <bool ROWS>
+// AHEAD (one row a request): what is there before the step - positions, block ids and a warp's first tile, all keys but the last - is
+// fetched while the kernels before still run; only q and the last key wait for them.  With the states of the recurrences likewise, a
+// decode step of a 2048-wide design (four layers, two of each mixer, two requests of 1160 keys) 311 us before and 297 so.
+template <bool ROWS, bool AHEAD = false>
 __global__ void __launch_bounds__(AM_WARPS * 32) attn_bias_mma_kernel(AttnBiasArgs a, int req0) {
   pdl_launch_dependents();
-  pdl_wait();
+  if (!AHEAD) pdl_wait();
   typedef __nv_bfloat16 E;
   extern __shared__ __align__(16) unsigned char am_smem[];
   // CTAs of a cluster (1 or more; ROWS: 1) share the rows
@@ -190,48 +193,80 @@ __global__ void __launch_bounds__(AM_WARPS * 32) attn_bias_mma_kernel(AttnBiasAr
   const float scale2 = a.scale * log2e;
   const float cap2 = a.softcap * log2e, cap_in = a.softcap > 0.f ? a.scale / a.softcap : 0.f;   // capped scores, in units of log 2
   uint32_t qf[AM_MAXD / 16][4];
+  auto load_q = [&]() {
 #pragma unroll
-  for (int ks = 0; ks < AM_MAXD / 16; ++ks) {
-    if (ks < ksteps) {
-      const E* q0 = (const E*)a.q + (int64_t)tok[0] * a.ldq + head[0] * dim + ks * 16 + qc;
-      const E* q1 = (const E*)a.q + (int64_t)tok[1] * a.ldq + head[1] * dim + ks * 16 + qc;
-      qf[ks][0] = pos[0] >= 0 ? *reinterpret_cast<const uint32_t*>(q0) : 0u;
-      qf[ks][1] = pos[1] >= 0 ? *reinterpret_cast<const uint32_t*>(q1) : 0u;
-      qf[ks][2] = pos[0] >= 0 ? *reinterpret_cast<const uint32_t*>(q0 + 8) : 0u;
-      qf[ks][3] = pos[1] >= 0 ? *reinterpret_cast<const uint32_t*>(q1 + 8) : 0u;
-    } else {
-      qf[ks][0] = qf[ks][1] = qf[ks][2] = qf[ks][3] = 0u;
+    for (int ks = 0; ks < AM_MAXD / 16; ++ks) {
+      if (ks < ksteps) {
+        const E* q0 = (const E*)a.q + (int64_t)tok[0] * a.ldq + head[0] * dim + ks * 16 + qc;
+        const E* q1 = (const E*)a.q + (int64_t)tok[1] * a.ldq + head[1] * dim + ks * 16 + qc;
+        qf[ks][0] = pos[0] >= 0 ? *reinterpret_cast<const uint32_t*>(q0) : 0u;
+        qf[ks][1] = pos[1] >= 0 ? *reinterpret_cast<const uint32_t*>(q1) : 0u;
+        qf[ks][2] = pos[0] >= 0 ? *reinterpret_cast<const uint32_t*>(q0 + 8) : 0u;
+        qf[ks][3] = pos[1] >= 0 ? *reinterpret_cast<const uint32_t*>(q1 + 8) : 0u;
+      } else {
+        qf[ks][0] = qf[ks][1] = qf[ks][2] = qf[ks][3] = 0u;
+      }
     }
-  }
+  };
+  if (!AHEAD) load_q();
   float o[AM_MAXD / 8][4];
 #pragma unroll
   for (int v = 0; v < AM_MAXD / 8; ++v) o[v][0] = o[v][1] = o[v][2] = o[v][3] = 0.f;
   float m[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f};
   const int32_t* bt = a.block_table + (int64_t)b * a.max_blocks;
   const int kseg = dim >> 3, vseg = vdim >> 3, vld = a.v_ld > 0 ? a.v_ld : vdim;
-  for (int kt = ROWS ? 0 : crank * AM_WARPS + warp; kt < ntiles; kt += ROWS ? 1 : AM_WARPS * S) {
+  const int kt_first = ROWS ? 0 : crank * AM_WARPS + warp;
+  // where key j0 + lane of a tile lives (-1: nowhere)
+  auto row_at = [&](bool ptile, int j0) -> int64_t {
+    const int jl = j0 + lane;
+    if (ptile) return jl < pre_cta ? prefix_row(a, bt, g, jl) : -1;
+    return jl <= pos_last ? ((int64_t)bt[jl / a.block_size] * a.G + g) * a.block_size + jl % a.block_size : -1;
+  };
+  // a tile's keys and values for one warp: the 16-byte pieces of a row are fetched by consecutive lanes (whole warps run the loops: the
+  // shuffle needs every lane); key `skip` is left out
+  auto stage = [&](E* dst, const E* src, int segs, int st, int64_t ld, int64_t myrow, int skip) {
+    for (int idx = lane; idx < AM_KT * segs; idx += 32) {
+      const int key = idx / segs, seg = idx % segs;
+      const int64_t row = __shfl_sync(0xffffffffu, myrow, key);
+      asm volatile("{\n.reg .pred p;\nsetp.eq.u32 p, %3, 0;\n@p cp.async.cg.shared.global [%0], [%1], 16, %2;\n}" ::"r"((uint32_t)__cvta_generic_to_shared(dst + key * st + seg * 8)),
+                   "l"(src + (row >= 0 ? row * ld + seg * 8 : 0)), "r"(row >= 0 ? 16 : 0), "r"((uint32_t)(AHEAD && key == skip)) : "memory");
+    }
+  };
+  if constexpr (AHEAD) {
+    const int j0 = lo_min + kt_first * AM_KT, own = pos_last - j0;      // (no prefix keys here)
+    const E* kc = (const E*)a.k_cache;
+    const E* vc = (const E*)a.v_cache;
+    int64_t myrow = -1;
+    if (kt_first < ntiles) {
+      myrow = row_at(false, j0);
+      stage(Ks, kc, kseg, kst, dim, myrow, own);
+      stage(Vs, vc, vseg, vst, vld, myrow, own);
+    }
+    pdl_wait();
+    load_q();
+    if (kt_first < ntiles && own < AM_KT) {
+      const int64_t row = __shfl_sync(0xffffffffu, myrow, own);
+      for (int i = lane; i < kseg + vseg; i += 32) {
+        const bool key = i < kseg;
+        const int seg = key ? i : i - kseg;
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared((key ? Ks + own * kst : Vs + own * vst) + seg * 8)),
+                     "l"((key ? kc + row * dim : vc + row * vld) + seg * 8) : "memory");
+      }
+    }
+  }
+  for (int kt = kt_first; kt < ntiles; kt += ROWS ? 1 : AM_WARPS * S) {
     const bool ptile = kt < ptiles;                         // a tile of prefix keys: j0 counts them from 0
     const int j0 = ptile ? kt * AM_KT : lo_min + (kt - ptiles) * AM_KT;
     const E* kc = (const E*)(ptile && a.pool > 0 ? a.pk_cache : a.k_cache);
     const E* vc = (const E*)(ptile && a.pool > 0 ? a.pv_cache : a.v_cache);
     if (ROWS) __syncthreads();                              // the previous tile has been read by every warp
-    // stage the tile: lane i knows where key j0 + i lives; the 16-byte pieces of a row are fetched by consecutive lanes
-    const int jl = j0 + lane;
     int64_t myrow = -1;
-    if (ptile) { if (jl < pre_cta) myrow = prefix_row(a, bt, g, jl); }
-    else if (jl <= pos_last) myrow = ((int64_t)bt[jl / a.block_size] * a.G + g) * a.block_size + jl % a.block_size;
-    // (whole warps run the loops: the shuffle needs every lane)
+    if (!AHEAD || kt != kt_first) myrow = row_at(ptile, j0);
     if constexpr (!ROWS) {
-      auto stage = [&](E* dst, const E* src, int segs, int st, int64_t ld) {
-        for (int idx = lane; idx < AM_KT * segs; idx += 32) {
-          const int key = idx / segs, seg = idx % segs;
-          const int64_t row = __shfl_sync(0xffffffffu, myrow, key);
-          asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst + key * st + seg * 8)),
-                       "l"(src + (row >= 0 ? row * ld + seg * 8 : 0)), "r"(row >= 0 ? 16 : 0) : "memory");
-        }
-      };
-      stage(Ks, kc, kseg, kst, dim);
-      stage(Vs, vc, vseg, vst, vld);
+      if (!AHEAD || kt != kt_first) {
+        stage(Ks, kc, kseg, kst, dim, myrow, -1);
+        stage(Vs, vc, vseg, vst, vld, myrow, -1);
+      }
       asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;" ::: "memory");
     } else {
       // four 16-byte pieces are requested before the first is stored, so a tile costs a few memory round trips, not one per piece
@@ -464,8 +499,10 @@ static int bias_cluster(int64_t ctas, int tiles) {
 }
 static cudaError_t launch_bias_split(dim3 grid, int S, size_t smem, cudaStream_t st, const AttnBiasArgs& a, int req0) {
   grid.x *= S;
-  if (S == 1) return launch_pdl(attn_bias_mma_kernel<false>, grid, dim3(AM_WARPS * 32), smem, st, a, req0);
-  prefer_max_shared(attn_bias_mma_kernel<false>);
+  // pooled blocks may be written in the step, and the first tokens of a window are tiles of their own
+  auto kern = req0 == 0 && a.max_q == 1 && a.keys_before && a.pool == 0 && a.keep_first == 0 ? attn_bias_mma_kernel<false, true> : attn_bias_mma_kernel<false>;
+  if (S == 1) return launch_pdl(kern, grid, dim3(AM_WARPS * 32), smem, st, a, req0);
+  prefer_max_shared(kern);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid; cfg.blockDim = dim3(AM_WARPS * 32); cfg.dynamicSmemBytes = smem; cfg.stream = st;
   cudaLaunchAttribute attr[2];
@@ -474,7 +511,7 @@ static cudaError_t launch_bias_split(dim3 grid, int S, size_t smem, cudaStream_t
   attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr; cfg.numAttrs = pdl_for_this_launch() ? 2 : 1;
-  return cudaLaunchKernelEx(&cfg, attn_bias_mma_kernel<false>, a, req0);
+  return cudaLaunchKernelEx(&cfg, kern, a, req0);
 }
 
 inline namespace KGE_ELT_NS {
@@ -505,7 +542,8 @@ int attn_bias_chunk(const AttnBiasArgs& a, cudaStream_t st) {
     const size_t tile = tile_of(a.dim, a.vdim), split = split_of(a.dim, a.vdim), sums = sums_of(a.vdim);
     // the function's limit on this device, for every size
     if (split + sums > 48 * 1024)
-      KGE_CUDA_OK(cudaFuncSetAttribute(attn_bias_mma_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(split_of(AM_MAXD, AM_MAXD) + sums_of(AM_MAXD))));
+      for (auto kern : {attn_bias_mma_kernel<false>, attn_bias_mma_kernel<false, true>})
+        KGE_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(split_of(AM_MAXD, AM_MAXD) + sums_of(AM_MAXD))));
     // the leading one-token requests, then the rest; 64-row CTAs where a request has that many rows and its output
     // pairs can be stored as 32-bit words
     const int D = std::min(std::max(a.num_decode, 0), a.B);

@@ -977,6 +977,7 @@ int hybrid_forward(kge_engine* e, int T, int B, int R, int max_blocks, const Ste
       ro.k_cache = L.kc; ro.v_cache = L.vc; ro.T = T; ro.H = h.heads; ro.G = h.kv_heads; ro.dim = h.dim; ro.vdim = h.vdim; ro.block_size = bs; ro.elt = elt;
       HFWD(C_KVW, (double)T * (2.0 * nq + 3.0 * h.kv_heads * h.dim) * es, 0, rotary_norm_kvwrite(ro, st));
       AttnBiasArgs aa;
+      aa.keys_before = e->step_keys_before;
       aa.q = e->pbuf; aa.ldq = ldp; aa.out = e->mixbuf; aa.ldo = ko; aa.k_cache = L.kc; aa.v_cache = L.vc;
       aa.block_table = m.btab; aa.max_blocks = max_blocks; aa.seq_lens = m.seq_lens; aa.qsl = m.qsl; aa.positions = m.pos; aa.token_req = m.treq;
       aa.B = B; aa.T = T; aa.H = h.heads; aa.G = h.kv_heads; aa.dim = h.dim; aa.vdim = h.vdim; aa.block_size = bs; aa.chunk = 0;
@@ -1028,6 +1029,7 @@ int hybrid_forward(kge_engine* e, int T, int B, int R, int max_blocks, const Ste
         HFWD(C_KVW, (double)T * (nk + nv) * es * (1.0 + 1.0 / h.pool), 0, pool_kv_write(pk, st));
       }
       AttnBiasArgs aa;
+      aa.keys_before = e->step_keys_before;
       aa.q = qkv; aa.ldq = ldq; aa.out = e->mixbuf; aa.ldo = ka; aa.k_cache = L.kc; aa.v_cache = L.vc;
       aa.block_table = m.btab; aa.max_blocks = max_blocks; aa.seq_lens = m.seq_lens; aa.qsl = m.qsl; aa.positions = m.pos; aa.token_req = m.treq;
       aa.B = B; aa.T = T; aa.H = h.heads; aa.G = h.kv_heads; aa.dim = h.dim; aa.vdim = h.vdim; aa.block_size = bs; aa.chunk = 0;
@@ -1149,6 +1151,7 @@ int hybrid_forward(kge_engine* e, int T, int B, int R, int max_blocks, const Ste
           }
         } else {
           AttnBiasArgs aa;                                               // all heads on one key/value head whose values are the rows' first numbers
+          aa.keys_before = e->step_keys_before;
           aa.q = e->qabs; aa.ldq = H * row; aa.out = e->olat; aa.ldo = H * rank; aa.k_cache = aa.v_cache = cache; aa.v_ld = row;
           aa.block_table = m.btab; aa.max_blocks = max_blocks; aa.seq_lens = m.seq_lens; aa.qsl = m.qsl; aa.positions = m.pos; aa.token_req = m.treq;
           aa.B = B; aa.T = Ta; aa.H = H; aa.G = 1; aa.dim = row; aa.vdim = rank; aa.block_size = bs; aa.window = window; aa.scale = h.scale; aa.sinks = L.sinks; aa.elt = elt;
@@ -1248,6 +1251,7 @@ int hybrid_forward(kge_engine* e, int T, int B, int R, int max_blocks, const Ste
       ro.k_cache = L.kc; ro.v_cache = L.vc; ro.T = T; ro.H = h.heads; ro.G = h.kv_heads; ro.dim = h.dim; ro.vdim = h.vdim; ro.block_size = bs; ro.elt = elt;
       HFWD(C_KVW, (double)T * (2.0 * nq + 2.0 * nk + 2.0 * nv) * es, 0, head_norm_rotary_kvwrite(ro, st));
       AttnBiasArgs aa;
+      aa.keys_before = e->step_keys_before;
       aa.q = e->pbuf; aa.ldq = ldp; aa.out = e->mixbuf; aa.ldo = ka; aa.k_cache = L.kc; aa.v_cache = L.vc;
       aa.block_table = m.btab; aa.max_blocks = max_blocks; aa.seq_lens = m.seq_lens; aa.qsl = m.qsl; aa.positions = m.pos; aa.token_req = m.treq;
       aa.B = B; aa.T = T; aa.H = h.heads; aa.G = h.kv_heads; aa.dim = h.dim; aa.vdim = h.vdim; aa.block_size = bs; aa.window = h.window; aa.scale = h.scale; aa.elt = elt;
@@ -1302,6 +1306,7 @@ int hybrid_forward(kge_engine* e, int T, int B, int R, int max_blocks, const Ste
       lk.positions = m.pos; lk.slots = m.slots; lk.k_cache = L.kc; lk.v_cache = L.vc; lk.T = T; lk.H = H; lk.dim = h.dim; lk.vdim = h.vdim; lk.block_size = bs; lk.elt = elt;
       HFWD(C_KVW, (double)T * (2.0 * H * h.rot_part + 2.0 * H * (h.dim + h.vdim)) * es, 0, latent_rotary_kvwrite(lk, st));
       AttnBiasArgs aa;
+      aa.keys_before = e->step_keys_before;
       aa.q = q; aa.ldq = ldq; aa.out = e->mixbuf; aa.ldo = nv; aa.k_cache = L.kc; aa.v_cache = L.vc;
       aa.block_table = m.btab; aa.max_blocks = max_blocks; aa.seq_lens = m.seq_lens; aa.qsl = m.qsl; aa.positions = m.pos; aa.token_req = m.treq;
       aa.B = B; aa.T = T; aa.H = H; aa.G = H; aa.dim = h.dim; aa.vdim = h.vdim; aa.block_size = bs; aa.chunk = 0;
@@ -1336,6 +1341,7 @@ int hybrid_forward(kge_engine* e, int T, int B, int R, int max_blocks, const Ste
       HFWD(C_KVW, 2.0 * T * h.kv_heads * (h.dim + h.vdim) * es, 0,
            kv_write_any(at(e->pbuf, L.off_k), ldp, at(e->pbuf, L.off_v), ldp, m.slots, L.kc, L.vc, T, h.kv_heads, h.dim, h.vdim, bs, elt, st));
       AttnBiasArgs aa;
+      aa.keys_before = e->step_keys_before;
       aa.q = e->pbuf; aa.ldq = ldp; aa.out = e->mixbuf; aa.ldo = ko; aa.k_cache = L.kc; aa.v_cache = L.vc;
       aa.block_table = m.btab; aa.max_blocks = max_blocks; aa.seq_lens = m.seq_lens; aa.qsl = m.qsl; aa.positions = m.pos; aa.token_req = m.treq;
       aa.B = B; aa.T = T; aa.H = h.heads; aa.G = h.kv_heads; aa.dim = h.dim; aa.vdim = h.vdim; aa.block_size = bs; aa.chunk = h.chunk;

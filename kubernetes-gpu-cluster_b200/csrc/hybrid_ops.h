@@ -188,6 +188,7 @@ struct AttnBiasArgs {
   int v_ld = 0;                            // elements between value rows (0: vdim); values may be the first columns of the key rows
   int elt = KGE_ELT_BF16;
   int max_seq = 0;                         // the longest request's keys in this step (0 = unknown: what its blocks hold)
+  bool keys_before = false;                // every request's keys but its last, positions and block table are from before the step
 };
 int attn_bias_chunk(const AttnBiasArgs& a, cudaStream_t st);
 inline int pool_slots_per_block(int block_size, int pool) { return (block_size + pool - 1) / pool; }

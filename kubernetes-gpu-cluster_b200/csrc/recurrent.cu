@@ -922,27 +922,28 @@ template <typename E>
 __global__ void __launch_bounds__(256) mlstm_token_kernel(MlstmArgs a) {
   cluster_arrive_relaxed();                                    // waited for before the first remote store
   pdl_launch_dependents();
-  pdl_wait();
   __shared__ __align__(16) float qs[ML_MAXD], ks[ML_MAXD], part[8][33], np_s[8], squares[8];
   const int b = blockIdx.x, h = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, c = blockIdx.z * 32 + lane;
   const int dim = a.dim, vdim = a.vdim, per = (dim + 7) / 8, d0 = warp * per, d1 = min(dim, d0 + per);
+  // slots, positions and the state are from before the step (its first kernel starts behind all of the step before)
   const bool in = c < vdim, fresh = a.positions[b] == 0;
   float* slot = a.state + (int64_t)a.slots[b] * a.slot_stride + (int64_t)h * ((int64_t)dim * vdim + dim + 1);
-  const float ip = a.gates[(int64_t)b * 2 * a.H + h], fp = a.gates[(int64_t)b * 2 * a.H + a.H + h];
-  const float vv0 = in ? ldf((const E*)a.v + (int64_t)b * a.ld + h * vdim + c) : 0.f;
   float gate = 0.f, w = 0.f;
-  if (warp == 0 && in) { gate = ldf((const E*)a.g + (int64_t)b * a.ld + h * vdim + c); w = ldf((const E*)a.norm_w + h * vdim + c); }
-  float nk = 0.f, nq = 0.f, nv = 0.f;
-  if (tid < dim) {
-    nk = ldf((const E*)a.k + (int64_t)b * a.ld + h * dim + tid);
-    nq = ldf((const E*)a.q + (int64_t)b * a.ld + h * dim + tid) * a.q_scale;
-    nv = fresh ? 0.f : slot[(int64_t)dim * vdim + tid];
-    ks[tid] = nk; qs[tid] = nq;
-  }
-  const float m0 = fresh ? 0.f : slot[(int64_t)dim * vdim + dim];
+  if (warp == 0 && in) w = ldf((const E*)a.norm_w + h * vdim + c);
+  const float nv = tid < dim && !fresh ? slot[(int64_t)dim * vdim + tid] : 0.f, m0 = fresh ? 0.f : slot[(int64_t)dim * vdim + dim];
   float S[ML_MAXD / 8];
 #pragma unroll
   for (int k = 0; k < ML_MAXD / 8; ++k) S[k] = d0 + k < d1 && in && !fresh ? slot[(int64_t)(d0 + k) * vdim + c] : 0.f;
+  pdl_wait();
+  const float ip = a.gates[(int64_t)b * 2 * a.H + h], fp = a.gates[(int64_t)b * 2 * a.H + a.H + h];
+  const float vv0 = in ? ldf((const E*)a.v + (int64_t)b * a.ld + h * vdim + c) : 0.f;
+  if (warp == 0 && in) gate = ldf((const E*)a.g + (int64_t)b * a.ld + h * vdim + c);
+  float nk = 0.f, nq = 0.f;
+  if (tid < dim) {
+    nk = ldf((const E*)a.k + (int64_t)b * a.ld + h * dim + tid);
+    nq = ldf((const E*)a.q + (int64_t)b * a.ld + h * dim + tid) * a.q_scale;
+    ks[tid] = nk; qs[tid] = nq;
+  }
   const float it = a.cap * tanhf(ip / a.cap), fc = a.cap * tanhf(fp / a.cap), ft = fminf(fc, 0.f) - log1pf(expf(-fabsf(fc)));
   const float mn = fmaxf(ft + m0, it), fa = expf(ft + m0 - mn), ia = expf(it - mn), vv = ia * vv0;
   __syncthreads();

@@ -504,7 +504,7 @@ __global__ void __launch_bounds__(320) rglru_step_kernel(RglruArgs a, int bw, in
   const int ch = z * bw + c0 + n0 + 2 * t4;
   const f2 sp = pk(rg_rate<E>(a, ch), rg_rate<E>(a, ch + 1));
   const f2 br = a.b_r ? rg_load<2>((const E*)a.b_r + ch) : pk1(0.f), bi = a.b_i ? rg_load<2>((const E*)a.b_i + ch) : pk1(0.f);
-  pdl_wait();
+  // slots, positions and the state are from before the step (its first kernel starts behind all of the step before)
   auto row_of = [&](int t) { return RgRow{0, a.positions[t], a.state + (int64_t)a.slots[t] * a.slot_stride}; };
   float* slot[2];
   f2 S[2], y[2];
@@ -513,9 +513,18 @@ __global__ void __launch_bounds__(320) rglru_step_kernel(RglruArgs a, int bw, in
     if (g + 8 * h < n) {
       const RgRow r = row_of(t0 + g + 8 * h);
       slot[h] = const_cast<float*>(r.slot);
-      y[h] = rg_load<2>((const E*)a.yx + (int64_t)(t0 + g + 8 * h) * 2 * a.width + ch);
       S[h] = r.pos > 0 ? rg_state<2>(r.slot + ch) : pk1(0.f);
     }
+  const int lines = (bw + 31) / 32;
+  for (int i = tid; i < n * lines; i += blockDim.x) {          // the inputs before, 128 bytes at a time
+    const int r = i / lines, c = z * bw + (i - r * lines) * 32;
+    const float* tail = row_of(t0 + r).slot + a.width + c;
+    for (int j = 0; j < taps - 1; ++j) asm volatile("prefetch.global.L1 [%0];" ::"l"(tail + (int64_t)j * a.width));
+  }
+  pdl_wait();
+#pragma unroll
+  for (int h = 0; h < 2; ++h)
+    if (g + 8 * h < n) y[h] = rg_load<2>((const E*)a.yx + (int64_t)(t0 + g + 8 * h) * 2 * a.width + ch);
   for (int i = tid; i < 16 * pieces; i += blockDim.x) {
     const int r = i / pieces, p = (i - r * pieces) * 8, c = z * bw + p;
     f2 acc[4];
