@@ -515,12 +515,6 @@ __global__ void __launch_bounds__(320) rglru_step_kernel(RglruArgs a, int bw, in
       slot[h] = const_cast<float*>(r.slot);
       S[h] = r.pos > 0 ? rg_state<2>(r.slot + ch) : pk1(0.f);
     }
-  const int lines = (bw + 31) / 32;
-  for (int i = tid; i < n * lines; i += blockDim.x) {          // the inputs before, 128 bytes at a time
-    const int r = i / lines, c = z * bw + (i - r * lines) * 32;
-    const float* tail = row_of(t0 + r).slot + a.width + c;
-    for (int j = 0; j < taps - 1; ++j) asm volatile("prefetch.global.L1 [%0];" ::"l"(tail + (int64_t)j * a.width));
-  }
   pdl_wait();
 #pragma unroll
   for (int h = 0; h < 2; ++h)
