@@ -518,11 +518,16 @@ __global__ void __launch_bounds__(MC_COLS * ML_NSL) mlstm_chunk_kernel(MlstmArgs
 // three bfloat16 terms that add up to its 24 bits, so every product is exact to fp32 and sums are fp32; a chunk's update is
 // summed by itself and then joined to C by one fma.  A chunk costs four barriers and ~250 MMAs per warp; the next chunk's
 // rows arrive by cp.async meanwhile.
-// What bounds it: the chain of chunks (2 requests x 4 heads x 8 column blocks = 64 blocks), not throughput: 7 us a chunk.
-// Prompts of 1150 and 1162 tokens, 4 heads of 128 x 256: 151 us (the fp32 kernel above 1101), error against 64 bits 1.0e-6 of
-// the read-out and 2.5e-7 of the state (1.5e-6 and 5.0e-7); one prompt of 1300 with a state before it: 159 us (1223), 6.6e-7
-// and 1.1e-7 (7.5e-7 and 2.3e-7).
+// What bounds it: mma.sync, 32 cycles a quarter of an SM for 16 x 8 x 16 numbers, in the chain of a request's chunks: 7.5 us each.  Where
+// that leaves SMs without work (2 requests x 4 heads x 8 column blocks), up to eight blocks share a head's columns: each goes over all
+// chunks before its own with the updates of the state alone (a third of the work, the same numbers in every block) and reads out its own,
+// whose run is the shorter the more lies before it; the last writes the state.  Nothing is exchanged.  us with one block and so: prompts of
+// 1150 and 1162 tokens, 4 heads of 128 x 256 (two blocks) 150 / 102, one of 1300 (four) 157 / 79, of 4096 471 / 229, of 129 27 / 19.  The
+// head's column blocks, which formed a cluster because of n and m, are free of each other: 4 x 1024 tokens 252 / 142.
+// Prompts of 1150 and 1162 tokens: error against 64 bits 1.0e-6 of the read-out and 2.5e-7 of the state (the fp32 kernel above, 1101 us,
+// 1.5e-6 and 5.0e-7); one prompt of 1300 with a state before it: 6.6e-7 and 1.1e-7 (7.5e-7 and 2.3e-7).
 // A request with one row of the step takes a plain path on the same block (fp32, one pass over its columns).
+constexpr float MM_SHARE = 0.65f;      // a run of chunks beside the one before it
 constexpr int MM_CH = 64, MM_COLS = 32, MM_THREADS = 256, MM_LDQ = 128 + 8, MM_LDV = MM_COLS + 8;
 struct MlstmTile {
   __nv_bfloat16 q[2][MM_CH][MM_LDQ], k[2][MM_CH][MM_LDQ], v[2][MM_CH][MM_LDV];
@@ -554,13 +559,15 @@ __device__ __forceinline__ void ml_split(float lo, float hi, uint32_t (&t)[3]) {
   }
 }
 
+template <bool SHARED>
 __global__ void __launch_bounds__(MM_THREADS) mlstm_mma_kernel(MlstmArgs a) {
   pdl_launch_dependents();
   pdl_wait();
   typedef __nv_bfloat16 E;
   extern __shared__ __align__(16) unsigned char mm_raw[];
   MlstmTile& sm = *reinterpret_cast<MlstmTile*>(mm_raw);
-  const int b = blockIdx.x, h = blockIdx.y, c0 = blockIdx.z * MM_COLS, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t4 = lane & 3;
+  // ranks of a cluster share a head's columns of a request: rank r has the read-outs of the r-th run of chunks
+  const int S = SHARED ? (int)cluster_nctarank() : 1, rank = SHARED ? (int)cluster_ctarank() : 0, b = blockIdx.x / S, h = blockIdx.y, c0 = blockIdx.z * MM_COLS, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t4 = lane & 3;
   const int dim = a.dim, vdim = a.vdim, H = a.H;
   const int rs = a.qsl[b], re = a.qsl[b + 1];
   if (re <= rs) return;
@@ -571,11 +578,11 @@ __global__ void __launch_bounds__(MM_THREADS) mlstm_mma_kernel(MlstmArgs a) {
   const int ncol = min(MM_COLS, vdim - c0);
   const float m0 = fresh ? 0.f : slot[(int64_t)dim * vdim + dim];
   for (int d = tid; d < 128; d += MM_THREADS) sm.nv[d] = d < dim && !fresh ? slot[(int64_t)dim * vdim + d] : 0.f;
-  // the blocks of a head form a cluster: the one that writes n and m back waits until all have read them
   __syncthreads();
-  cluster_arrive();
 
+  float* nm = a.nm_scratch + ((int64_t)b * H + h) * (dim + 1);
   if (re - rs == 1) {
+    if (rank + 1 < S) return;
     // one token: thread = (column, eighth of the key dimensions)
     const int col = lane, per = (dim + 7) / 8, d0 = warp * per, d1 = min(dim, d0 + per);
     const float it = a.gates[(int64_t)rs * 2 * H + h], ft = a.gates[(int64_t)rs * 2 * H + H + h];
@@ -610,10 +617,9 @@ __global__ void __launch_bounds__(MM_THREADS) mlstm_mma_kernel(MlstmArgs a) {
       for (int w = 0; w < 8; ++w) { o += part[w * 32 + col]; nq += sm.nq[w]; }
       a.o_scratch[(int64_t)rs * H * vdim + h * vdim + c0 + col] = o / (fmaxf(fabsf(nq), expf(-mn)) + a.den_eps);
     }
-    cluster_wait();
     if (blockIdx.z == 0) {
-      for (int d = tid; d < dim; d += MM_THREADS) slot[(int64_t)dim * vdim + d] = sm.nv[d];
-      if (tid == 0) slot[(int64_t)dim * vdim + dim] = mn;
+      for (int d = tid; d < dim; d += MM_THREADS) nm[d] = sm.nv[d];
+      if (tid == 0) nm[dim] = mn;
     }
     return;
   }
@@ -639,7 +645,17 @@ __global__ void __launch_bounds__(MM_THREADS) mlstm_mma_kernel(MlstmArgs a) {
       const int d = mt0 + g + 8 * (q >> 1), col = n * 8 + t4 * 2 + (q & 1);
       C[n][q] = d < dim && col < ncol && !fresh ? slot[(int64_t)d * vdim + c0 + col] : 0.f;
     }
-  write_terms();
+  if (SHARED) cluster_arrive();                                      // the last rank writes the state back when all have read it
+  // the rank's run: [own0, own1), each MM_SHARE of the one before it, since what lies before a run costs its rank the updates only
+  const int chunks = (re - rs + MM_CH - 1) / MM_CH;
+  auto border = [&](int r) {
+    float before = 0.f, all = 0.f, w = 1.f;
+    for (int i = 0; i < S; ++i, w *= MM_SHARE) { all += w; if (i < r) before += w; }
+    return r >= S ? re : min(re, rs + MM_CH * (int)(chunks * (before / all) + 0.5f));
+  };
+  const int own0 = SHARED ? border(rank) : rs, own1 = SHARED ? border(rank + 1) : re;
+  const bool last = !SHARED || rank + 1 == S;
+  if (!SHARED || own0 == rs) write_terms();
 
   // rows of 64 tokens: q and k in 16-byte pieces (dim / 8 per row), v likewise (the host checked the alignment)
   const int pieces = dim / 8;
@@ -647,10 +663,11 @@ __global__ void __launch_bounds__(MM_THREADS) mlstm_mma_kernel(MlstmArgs a) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(in ? src : qp), "r"(in ? 16u : 0u) : "memory");
   };
   auto fetch = [&](int t0, int st) {
+    const bool full = !SHARED || t0 >= own0;                   // no read-out: no q
     for (int i = tid; i < MM_CH * pieces; i += MM_THREADS) {
       const int r = i / pieces, c = (i - r * pieces) * 8;
       const bool in = t0 + r < re;
-      copy16(&sm.q[st][r][c], qp + (int64_t)(t0 + r) * a.ld + c, in);
+      if (full) copy16(&sm.q[st][r][c], qp + (int64_t)(t0 + r) * a.ld + c, in);
       copy16(&sm.k[st][r][c], kp + (int64_t)(t0 + r) * a.ld + c, in);
     }
     const int r = tid >> 2, c = (tid & 3) * 8;
@@ -660,9 +677,11 @@ __global__ void __launch_bounds__(MM_THREADS) mlstm_mma_kernel(MlstmArgs a) {
   const int rg = (warp & 3) * 16, half = warp >> 2;            // this warp's 16 tokens; its half of the keys / key dimensions
   const int ksteps = dim / 16, kh = (ksteps + 1) / 2, k_begin = half ? kh : 0, k_end = half ? ksteps : kh;
   double m = m0;                                               // (warp 0) the running maximum before the chunk
-  fetch(rs, 0);
+  const int end = last ? re : own0 < own1 ? own1 : rs;         // (a rank without a run has nothing to do)
+  if (rs < end) fetch(rs, 0);
   int st = 0;
-  for (int t0 = rs; t0 < re; t0 += MM_CH, st ^= 1) {
+  for (int t0 = rs; t0 < end; t0 += MM_CH, st ^= 1) {
+    const bool full = !SHARED || t0 >= own0;
     // the gate scalars of the chunk, two tokens per lane of the first warp: with e_s = i_s - b_s and M_t = max(m, max_{s<=t} e_s),
     // m_t = b_t + M_t, and the weights above are e^(m - M_t) and e^(e_s - M_t)
     float it[2], ft[2];
@@ -676,7 +695,7 @@ __global__ void __launch_bounds__(MM_THREADS) mlstm_mma_kernel(MlstmArgs a) {
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     __syncthreads();                                           // the chunk's rows and C's terms are there; the other stage is free
-    if (t0 + MM_CH < re) fetch(t0 + MM_CH, st ^ 1);
+    if (t0 + MM_CH < end) fetch(t0 + MM_CH, st ^ 1);
     if (warp == 0) {
       // running sums in 64 bits: b_t grows with the chunk, and what the weights need are differences
       const double pair = (double)ft[0] + (double)ft[1];
@@ -702,7 +721,7 @@ __global__ void __launch_bounds__(MM_THREADS) mlstm_mma_kernel(MlstmArgs a) {
       m = bL + ML;
     }
     // q_t . k_s for this warp's tokens and its half of the keys (none where all keys lie behind the tokens)
-    const bool keys = half * 32 <= rg + 15;
+    const bool keys = full && half * 32 <= rg + 15;
     float sc[4][4];
 #pragma unroll
     for (int n = 0; n < 4; ++n) sc[n][0] = sc[n][1] = sc[n][2] = sc[n][3] = 0.f;
@@ -711,7 +730,7 @@ __global__ void __launch_bounds__(MM_THREADS) mlstm_mma_kernel(MlstmArgs a) {
     for (int n = 0; n < MM_COLS / 8; ++n)
 #pragma unroll
       for (int q = 0; q < 4; ++q) in[n][q] = ia[n][q] = 0.f;
-    for (int k = 0; k < ksteps; ++k) {
+    for (int k = 0; k < (full ? ksteps : 0); ++k) {
       uint32_t af[4];
       const bool mine = k >= k_begin && k < k_end;
       if (!keys && !mine) continue;
@@ -740,7 +759,7 @@ __global__ void __launch_bounds__(MM_THREADS) mlstm_mma_kernel(MlstmArgs a) {
             ml_mma(in[2 * n2 + 1], af, bf[2], bf[3]);
           }
     }
-    {
+    if (full) {
       // n . q_t, four threads per token
       const int tok = tid >> 2;
       float acc = 0.f;
@@ -809,12 +828,13 @@ __global__ void __launch_bounds__(MM_THREADS) mlstm_mma_kernel(MlstmArgs a) {
           }
         }
     }
+    float num[MM_COLS / 8][4];
+    if (full) {
 #pragma unroll
     for (int r = 0; r < 2; ++r) {
       rowsum[r] += __shfl_xor_sync(0xffffffffu, rowsum[r], 1);
       rowsum[r] += __shfl_xor_sync(0xffffffffu, rowsum[r], 2);
     }
-    float num[MM_COLS / 8][4];
 #pragma unroll
     for (int n = 0; n < MM_COLS / 8; ++n)
 #pragma unroll
@@ -827,8 +847,9 @@ __global__ void __launch_bounds__(MM_THREADS) mlstm_mma_kernel(MlstmArgs a) {
           *reinterpret_cast<float2*>(&sm.out[rg + g + 8 * r][n * 8 + t4 * 2]) = make_float2(num[n][2 * r], num[n][2 * r + 1]);
       if (t4 == 0) { sm.rows[rg + g] = rowsum[0]; sm.rows[rg + g + 8] = rowsum[1]; }
     }
+    }
     __syncthreads();                                           // all have read C's terms; x, the sums and the halves are there
-    if (!half) {
+    if (full && !half) {
 #pragma unroll
       for (int r = 0; r < 2; ++r) {
         const int tok = rg + g + 8 * r, t = t0 + tok;
@@ -845,6 +866,7 @@ __global__ void __launch_bounds__(MM_THREADS) mlstm_mma_kernel(MlstmArgs a) {
         }
       }
     }
+    if (!last && t0 + MM_CH >= end) break;                     // the state is another rank's to go on with
     // C' = G C + k^T x
     const float G = sm.G;
     if (has_c) {
@@ -869,10 +891,12 @@ __global__ void __launch_bounds__(MM_THREADS) mlstm_mma_kernel(MlstmArgs a) {
       for (int n = 0; n < MM_COLS / 8; ++n)
 #pragma unroll
         for (int q = 0; q < 4; ++q) C[n][q] = fmaf(G, C[n][q], D[n][q]);
-      write_terms();
+      if (!SHARED || t0 + MM_CH >= own0) write_terms();
     }
     if (tid < 128) sm.nv[tid] = fmaf(G, sm.nv[tid], sm.nsum[0][tid] + sm.nsum[1][tid]);
   }
+  if (SHARED) cluster_wait();
+  if (!last) return;
   if (has_c) {
 #pragma unroll
     for (int n = 0; n < MM_COLS / 8; ++n)
@@ -882,10 +906,9 @@ __global__ void __launch_bounds__(MM_THREADS) mlstm_mma_kernel(MlstmArgs a) {
         if (col < ncol) slot[(int64_t)d * vdim + c0 + col] = C[n][q];
       }
   }
-  cluster_wait();
   if (blockIdx.z == 0) {
-    if (tid < dim) slot[(int64_t)dim * vdim + tid] = sm.nv[tid];           // its own entry of the last update
-    if (tid == 0) slot[(int64_t)dim * vdim + dim] = (float)m;
+    if (tid < dim) nm[tid] = sm.nv[tid];           // its own entry of the last update
+    if (tid == 0) nm[dim] = (float)m;
   }
 }
 
@@ -895,12 +918,10 @@ __global__ void mlstm_norm_gate_kernel(MlstmArgs a) {
   pdl_wait();
   __shared__ float red[33];
   const int t = blockIdx.x, h = blockIdx.y;
-  if (t >= a.T) {                                              // blocks beyond the tokens: a request's new n and m
-    const int b = t - a.T;
-    const float* nm = a.nm_scratch + ((int64_t)b * a.H + h) * (a.dim + 1);
-    float* slot = a.state + (int64_t)a.slots[b] * a.slot_stride + ((int64_t)h + 1) * ((int64_t)a.dim * a.vdim + a.dim + 1) - (a.dim + 1);
+  if (t < a.B) {                                               // a request's new n and m
+    const float* nm = a.nm_scratch + ((int64_t)t * a.H + h) * (a.dim + 1);
+    float* slot = a.state + (int64_t)a.slots[t] * a.slot_stride + ((int64_t)h + 1) * ((int64_t)a.dim * a.vdim + a.dim + 1) - (a.dim + 1);
     for (int d = threadIdx.x; d <= a.dim; d += blockDim.x) slot[d] = nm[d];
-    return;
   }
   const float* o = a.o_scratch + (int64_t)t * a.H * a.vdim + h * a.vdim;
   float ss = 0.f;
@@ -983,9 +1004,17 @@ __global__ void __launch_bounds__(256) mlstm_token_kernel(MlstmArgs a) {
   }
 }
 
+// Blocks that share a head's columns of a request (a cluster): as many as one an SM has room for, and no more than there are chunks
+static int mlstm_ranks(const MlstmArgs& a) {
+  const int64_t blocks = (int64_t)a.B * a.H * ((a.vdim + MM_COLS - 1) / MM_COLS), rows = a.max_rows > 0 ? a.max_rows : a.T - a.B + 1;
+  int S = 1;
+  while (S < 8 && blocks * (S + 1) <= 148 && rows > (int64_t)S * MM_CH) ++S;
+  return S;
+}
 // Tensor-core chunks or the fp32 ones, by estimates (us) from measurements at 8 x 32 x 32 to 4 x 128 x 256 and 1 to 256 requests: a
 // tensor-core block fills an SM and takes 9 us beside 7 per 64 tokens of the longest request, an fp32 one shares it with two others,
-// 8 us and 1.1 per token (0.6 to 1.1 by head size).  4 x 128 x 256, tensor cores and fp32: 2 x 1150 tokens 152 / 1278, 200 and 64
+// 8 us and 1.1 per token (0.6 to 1.1 by head size).  (Blocks that share a head's columns only shorten requests of several chunks, where
+// the tensor cores are ahead by far.)  4 x 128 x 256, tensor cores (one block) and fp32: 2 x 1150 tokens 152 / 1278, 200 and 64
 // single ones 134 / 290, 8 x 40 36 / 65; 30 x 16 88 / 84, 64 x 8 178 / 73, 60 and 200 single ones 429 / 174, 100 x 2 263 / 60.
 static bool mlstm_use_mma(const MlstmArgs& a) {
   const double rows = a.max_rows > 0 ? a.max_rows : a.T - a.B + 1, blocks = (double)a.B * a.H * ((a.vdim + 31) / 32);
@@ -1009,27 +1038,29 @@ int mlstm_step(const MlstmArgs& a, cudaStream_t st) {
       KGE_CUDA_OK(cudaLaunchKernelEx(&cfg, kern, a));
       return 0;
     }
-    const dim3 grid(a.B, a.H, (a.vdim + ML_COLS - 1) / ML_COLS), g2(a.T + a.B, a.H);
+    const dim3 grid(a.B, a.H, (a.vdim + ML_COLS - 1) / ML_COLS), g2(a.T, a.H);
     const int nt = std::min(256, (a.vdim + 31) / 32 * 32);
     KGE_CUDA_OK(launch_pdl(mlstm_log_gates_kernel, dim3((a.T * 2 * a.H + 255) / 256), dim3(256), 0, st, const_cast<float*>(a.gates), a.T, a.H, a.cap));
     const size_t csm_bytes = ((size_t)2 * ML_CH * a.dim + ML_CH * ML_CH + ML_MAXD + 5 * ML_CH + (1 + ML_NSL) * ML_CH * MC_COLS) * 4;
     const dim3 cgrid(a.B, a.H, (a.vdim + MC_COLS - 1) / MC_COLS);
-    // tensor-core chunks: bfloat16 rows in 16-byte pieces, key dimensions in steps of 16, a head's column blocks in one cluster
+    // tensor-core chunks: bfloat16 rows in 16-byte pieces, key dimensions in steps of 16, at most 256 columns
     const bool mma_ok = a.elt == KGE_ELT_BF16 && a.dim % 16 == 0 && a.vdim % 8 == 0 && a.vdim <= 8 * MM_COLS && a.ld % 8 == 0 &&
                         ((reinterpret_cast<uintptr_t>(a.q) | reinterpret_cast<uintptr_t>(a.k) | reinterpret_cast<uintptr_t>(a.v)) & 15) == 0;
     if (a.T > a.B && mma_ok && mlstm_use_mma(a)) {
-      KGE_CUDA_OK(cudaFuncSetAttribute(mlstm_mma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(MlstmTile)));
-      prefer_max_shared(mlstm_mma_kernel);
+      const int Z = (a.vdim + MM_COLS - 1) / MM_COLS, S = mlstm_ranks(a);
+      auto kern = S > 1 ? mlstm_mma_kernel<true> : mlstm_mma_kernel<false>;
+      KGE_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(MlstmTile)));
+      prefer_max_shared(kern);
       cudaLaunchConfig_t cfg = {};
-      cfg.gridDim = dim3(a.B, a.H, (a.vdim + MM_COLS - 1) / MM_COLS); cfg.blockDim = dim3(MM_THREADS); cfg.dynamicSmemBytes = sizeof(MlstmTile); cfg.stream = st;
+      cfg.gridDim = dim3(a.B * S, a.H, Z); cfg.blockDim = dim3(MM_THREADS); cfg.dynamicSmemBytes = sizeof(MlstmTile); cfg.stream = st;
       cudaLaunchAttribute attr[2];
       attr[0].id = cudaLaunchAttributeClusterDimension;
-      attr[0].val.clusterDim.x = 1; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = cfg.gridDim.z;
+      attr[0].val.clusterDim.x = S; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
       attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
       attr[1].val.programmaticStreamSerializationAllowed = 1;
       cfg.attrs = attr; cfg.numAttrs = pdl_for_this_launch() ? 2 : 1;
-      KGE_CUDA_OK(cudaLaunchKernelEx(&cfg, mlstm_mma_kernel, a));
-      KGE_CUDA_OK(launch_pdl(mlstm_norm_gate_kernel<__nv_bfloat16>, dim3(a.T, a.H), dim3(nt), 0, st, a));
+      KGE_CUDA_OK(cudaLaunchKernelEx(&cfg, kern, a));
+      KGE_CUDA_OK(launch_pdl(mlstm_norm_gate_kernel<__nv_bfloat16>, g2, dim3(nt), 0, st, a));
       return 0;
     }
     if (a.T > a.B) {

@@ -1,5 +1,6 @@
 """Small steps of layer-list models: grouped and strided projections of up to 8 rows (linear_few_kernel), distance-biased attention with
 its keys split over clusters and (64 and 128 wide, prompts) in the tcgen05 kernel, against the float64 oracle."""
+import numpy as np
 import pytest
 
 from oracle import hybrid as oh
@@ -144,4 +145,48 @@ def test_short_biased_pieces(kge, tmp_path, hd):
     for rid, pieces in enumerate([[32, 33, 5], [31, 1, 38], [33, 37], [20, 20, 30]]):
         check(run_pieces(llm, rid, toks, pieces), want, "bfloat16", f"pieces {pieces}")
         llm.trace_end(rid)
+    llm.close()
+
+
+@pytest.mark.parametrize("heads,dim,vdim,lens", [
+    (1, 128, 32, [64, 65, 129, 193, 257, 449, 512, 513, 700]),      # one to eight blocks for the same columns
+    (2, 48, 72, [1, 130, 1, 64, 321]),                              # requests of one token and of one chunk beside longer ones
+    (3, 16, 256, [200, 90]),
+    (5, 128, 256, [150, 70, 10, 3]),                                # no room for a second block
+])
+def test_matrix_memory_prompts_in_runs_of_chunks(kge, tmp_path, heads, dim, vdim, lens):
+    """A request's chunks shared out over the blocks of a cluster: all requests in one step, first without a state, then on from it, and the
+    decode steps behind, which read what the last block wrote; beside the same tokens in pieces of one chunk, which one block takes.
+    The two do the same fp32 arithmetic (but for the running maximum, kept in 64 bits within a step): what may differ is a 16-bit
+    rounding of a mixer output, 2^-8 of it, at most some 2^-6 of the logits' size.  Against the oracle the middle row of each chunk is held to
+    4 x 2^-8 (roundings of q, k, v and the output): a run that went wrong is wrong in all of its rows, while single rows whose normaliser
+    cancels magnify the roundings of their q and k (0.063 at one token of 1402, with one block as with eight)."""
+    cfg = oh.make_config(layers=("parallel",), mlps=(None,), left_scale=0.0, m_heads=heads, m_dim=dim, m_vdim=vdim)
+    W = oh.make_weights(cfg, seed=59)
+    n = len(lens)
+    P = [prompt(cfg, 2 * m + 2, 60 + r) for r, m in enumerate(lens)]
+    llm = make_engine(kge, tmp_path, cfg, W, "bfloat16", tokens=8192, seqs=n + 1)
+    got = [[] for _ in range(n)]
+    for part in range(4):
+        sizes = [m if part < 2 else 1 for m in lens]
+        at = [sum(len(x) for x in got[r]) for r in range(n)]
+        for r in range(n):
+            llm.trace_add(r, P[r][at[r]:at[r] + sizes[r]])
+        lg = np.split(llm.trace_step([(r, m, list(range(m))) for r, m in enumerate(sizes)]), np.cumsum(sizes)[:-1])
+        for r in range(n):
+            got[r].append(lg[r])
+    for r in range(n):
+        llm.trace_end(r)
+    for r, m in enumerate(lens):
+        mine = np.concatenate(got[r])
+        whole = [min(64, m - i) for i in range(0, m, 64)]
+        other = run_pieces(llm, n + r, P[r], whole + whole + [1, 1])
+        llm.trace_end(n + r)
+        want = oh.forward(cfg, W, P[r]).numpy()
+        size = np.sqrt((want ** 2).mean())
+        err = np.sqrt(((mine - other) ** 2).mean(-1)) / size
+        assert err.max() < 2.0 ** -6, f"request {r}: row {err.argmax()} is {err.max():.3g} of the logits' size from the pieces'"
+        err = np.sqrt(((mine - want) ** 2).mean(-1)) / size
+        mid = [np.median(err[i:i + 64]) for i in range(0, len(err), 64)]
+        assert max(mid) < 2.0 ** -6, f"request {r}: {max(mid):.3g} of the logits' size in chunk {int(np.argmax(mid))}"
     llm.close()
