@@ -144,7 +144,7 @@ norm_kernel(bf16* __restrict__ y, bf16* __restrict__ residual, const bf16* __res
 // The same for many rows: a CTA goes through rows with the next two of each thread group on their way (cp.async into pieces of shared
 // memory that the same thread reads back), weights in registers.  GT threads a row, four 16-byte pieces each; one barrier a sum.
 // The kernel above is a chain of load, sum and store per CTA and keeps 60 KB an SM in flight at best.  us above and here: RMSNorm of
-// 4098 x 8192 39 / 34, LayerNorm of 8192 x 2048 31.7 / 16.9.
+// 8192 x 4096 35.1 / 30.0 (20.5 at the rate of a copy), of 8192 x 768 10.7 / 8.3, LayerNorm of 8192 x 2048 31.7 / 16.9.
 constexpr int kNormStages = 3, kNormThreads = 256;
 template <int MODE> constexpr int norm_rows_smem() { return kNormStages * (MODE == 1 || MODE == 3 ? 2 : 1) * kMaxVecPerThread * kNormThreads * 16; }
 
@@ -253,69 +253,6 @@ norm_rows_kernel(bf16* __restrict__ y, bf16* __restrict__ residual, const bf16* 
       }
     }
   }
-}
-
-// MODE 0 and 1 of a few hundred rows on: WPR warps a row, NV 16-byte pieces a thread, all of a row asked for at once and kept as they came,
-// four warps (or a row's eight) a CTA; no loop over rows.  The kernel of a CTA per row holds numbers in fp32 and has a CTA's start for
-// each row, the one above has the start of its ring.  RMSNorm, us before and here: 297 x 2048 2.75 / 2.05, 1339 x 2048 4.3 / 3.35, 4000 x 2048
-// 9.5 / 6.0 (5.4 TB/s), 1339 x 4096 5.8 / 4.5, 4000 x 1024 6.35 / 3.6; sum and RMSNorm of 900 x 1024 3.15 / 2.75, 1600 x 2048 5.6 / 4.5, 2500 x 4096 10.8 / 10.0.
-template <int MODE, int NV, int WPR>
-__global__ void __launch_bounds__((WPR > 4 ? WPR : 4) * 32)
-norm_piece_kernel(bf16* __restrict__ y, bf16* __restrict__ residual, const bf16* __restrict__ x, const bf16* __restrict__ w, int T, int d, float eps) {
-  constexpr int TPR = WPR * 32, RPC = WPR > 4 ? 1 : 4 / WPR;
-  __shared__ float red[RPC][WPR];
-  pdl_launch_dependents();
-  const int lt = threadIdx.x % TPR, sub = threadIdx.x / TPR, nvec = d / 8;
-  uint4 ww[NV], a[NV], r[MODE == 1 ? NV : 1];
-#pragma unroll
-  for (int j = 0; j < NV; ++j) if (lt + j * TPR < nvec) ww[j] = *reinterpret_cast<const uint4*>(w + (lt + j * TPR) * 8);
-  pdl_wait();
-  const int64_t row = (int64_t)blockIdx.x * RPC + sub;
-  if (row >= T) return;                                        // (all threads of a row)
-#pragma unroll
-  for (int j = 0; j < NV; ++j) {
-    const bool in = lt + j * TPR < nvec;
-    a[j] = in ? *reinterpret_cast<const uint4*>(x + row * d + (lt + j * TPR) * 8) : make_uint4(0, 0, 0, 0);
-    if (MODE == 1) r[j] = in ? *reinterpret_cast<const uint4*>(residual + row * d + (lt + j * TPR) * 8) : make_uint4(0, 0, 0, 0);
-  }
-  auto piece = [&](int j, float (&f)[8]) {                     // its numbers, in MODE 1 the sum's, not rounded
-    f[0] = bf_lo(a[j].x); f[1] = bf_hi(a[j].x); f[2] = bf_lo(a[j].y); f[3] = bf_hi(a[j].y);
-    f[4] = bf_lo(a[j].z); f[5] = bf_hi(a[j].z); f[6] = bf_lo(a[j].w); f[7] = bf_hi(a[j].w);
-    if (MODE == 1) {
-      const uint4 q = r[MODE == 1 ? j : 0];
-      f[0] += bf_lo(q.x); f[1] += bf_hi(q.x); f[2] += bf_lo(q.y); f[3] += bf_hi(q.y);
-      f[4] += bf_lo(q.z); f[5] += bf_hi(q.z); f[6] += bf_lo(q.w); f[7] += bf_hi(q.w);
-    }
-  };
-  float acc = 0.f;
-#pragma unroll
-  for (int j = 0; j < NV; ++j) {
-    float f[8];
-    piece(j, f);
-    if (MODE == 1 && lt + j * TPR < nvec)
-      *reinterpret_cast<uint4*>(residual + row * d + (lt + j * TPR) * 8) = make_uint4(pack_bf2(f[0], f[1]), pack_bf2(f[2], f[3]), pack_bf2(f[4], f[5]), pack_bf2(f[6], f[7]));
-#pragma unroll
-    for (int k = 0; k < 8; ++k) acc = fmaf(f[k], f[k], acc);
-  }
-  acc = warp_sum(acc);
-  if (WPR > 1) {
-    if (threadIdx.x % 32 == 0) red[sub][lt / 32] = acc;
-    asm volatile("bar.sync %0, %1;" ::"r"(1 + sub), "n"(TPR) : "memory");
-    acc = 0.f;
-#pragma unroll
-    for (int i = 0; i < WPR; ++i) acc += red[sub][i];
-  }
-  const float rstd = 1.0f / sqrtf(acc / (float)d + eps);
-#pragma unroll
-  for (int j = 0; j < NV; ++j)
-    if (lt + j * TPR < nvec) {
-      const float wf[8] = {bf_lo(ww[j].x), bf_hi(ww[j].x), bf_lo(ww[j].y), bf_hi(ww[j].y), bf_lo(ww[j].z), bf_hi(ww[j].z), bf_lo(ww[j].w), bf_hi(ww[j].w)};
-      float f[8], o[8];
-      piece(j, f);
-#pragma unroll
-      for (int k = 0; k < 8; ++k) o[k] = rbf(f[k] * rstd) * wf[k];   // weight mul in bf16
-      *reinterpret_cast<uint4*>(y + row * d + (lt + j * TPR) * 8) = make_uint4(pack_bf2(o[0], o[1]), pack_bf2(o[2], o[3]), pack_bf2(o[4], o[5]), pack_bf2(o[6], o[7]));
-    }
 }
 
 // ------------------------------------------------------------------------ silu * mul
@@ -496,22 +433,12 @@ extern "C" int KGE_API(kge_embed)(void* out, const int32_t* ids, const void* tab
 
 template <int MODE>
 static int launch_norm_rows(int gt, void* y, void* residual, const void* x, const void* w, const void* b, int T, int d, float eps, cudaStream_t st) {
-  auto kern = MODE == 0 ? norm_rows_kernel<MODE, 256> : gt == 32 ? norm_rows_kernel<MODE, MODE ? 32 : 256> : gt == 64 ? norm_rows_kernel<MODE, MODE ? 64 : 256> : gt == 128 ? norm_rows_kernel<MODE, MODE ? 128 : 256> : norm_rows_kernel<MODE, 256>;      // (MODE 0: wide rows only)
+  auto kern = gt == 32 ? norm_rows_kernel<MODE, 32> : gt == 64 ? norm_rows_kernel<MODE, 64> : gt == 128 ? norm_rows_kernel<MODE, 128> : norm_rows_kernel<MODE, 256>;
   constexpr int smem = norm_rows_smem<MODE>();
   KGE_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
   const int groups = kNormThreads / gt, ctas = 148 * (smem > 64 * 1024 ? 2 : 3), want = (T + groups - 1) / groups;
   KGE_CUDA_OK(launch_pdl(kern, dim3(want < ctas ? want : ctas), dim3(kNormThreads), smem, st, (bf16*)y, (bf16*)residual, (const bf16*)x, (const bf16*)w,
                          (const bf16*)b, T, d, eps));
-  return 0;
-}
-
-// NV 16-byte pieces a thread: as many warps a row as that takes
-template <int MODE, int NV>
-static int launch_norm_piece(void* y, void* residual, const void* x, const void* w, int T, int d, float eps, cudaStream_t st) {
-  constexpr int kOne = NV * 256;                               // numbers of one warp
-  auto kern = d <= kOne ? norm_piece_kernel<MODE, NV, 1> : d <= 2 * kOne ? norm_piece_kernel<MODE, NV, 2> : d <= 4 * kOne ? norm_piece_kernel<MODE, NV, 4> : norm_piece_kernel<MODE, NV, 8>;
-  const int rows = d <= kOne ? 4 : d <= 2 * kOne ? 2 : 1;
-  KGE_CUDA_OK(launch_pdl(kern, dim3((T + rows - 1) / rows), dim3(d <= 4 * kOne ? 128 : 256), 0, st, (bf16*)y, (bf16*)residual, (const bf16*)x, (const bf16*)w, T, d, eps));
   return 0;
 }
 
@@ -525,18 +452,9 @@ static int norm_common(int mode, void* y, void* residual, const void* x, const v
   const int th = row_threads(d);
   KGE_REQUIRE((d / 8 + th - 1) / th <= kMaxVecPerThread, "kge norm: d=%d too large", d);
   cudaStream_t s = (cudaStream_t)stream;
-  // norm_piece_kernel, us there and elsewhere.  RMSNorm beyond two rows an SM: two pieces a thread, but four where a row then needs fewer
-  // warps and there are rows enough (4000 x 1024 5.9 with two, 4.7 with four; 4000 x 4096 10.1 and 9.4, both with late weights).  The sum and RMSNorm:
-  // narrow rows up to eight an SM (297 x 768 2.5 / 2.4, 450 x 768 2.55 / 2.65, 1184 x 1024 2.8 / 3.4, 1339 x 1024 3.8 / 3.6), wide ones from there on
-  // (1184 x 2048 4.6 / 4.0, 1339 x 2048 4.4 / 5.0) while both tensors stay in L2 (3000 x 4096 11.9 / 12.7, 4000 x 4096 21.3 / 18.1).
-  if (y && T > 2 * 148 && d <= 4096) {
-    if (mode == 0)
-      return (d <= 1024 ? T >= 1250 : d > 2048 && T >= 2500) ? launch_norm_piece<0, 4>(y, residual, x, w, T, d, eps, s) : launch_norm_piece<0, 2>(y, residual, x, w, T, d, eps, s);
-    if (mode == 1 && (d <= 1024 ? T >= 400 && T <= 8 * 148 : T >= 1250 && (int64_t)T * d <= 12500000)) return launch_norm_piece<1, 2>(y, residual, x, w, T, d, eps, s);
-  }
   // Rows in a loop (norm_rows_kernel) where there are enough of them to fill its pipeline, us there and with a CTA per row: plain RMSNorm
-  // (wide rows) from 4096 rows on, others from 2 M numbers on (LayerNorm of 1339 x 2048 6.0 / 7.2, of 1000 x 768 2.8 / 2.7; sum and RMSNorm of
-  // 2000 x 1024 3.8 / 4.6).
+  // from 4096 rows on (4096 x 2048 10.6 / 11.9, 8192 x 768 8.3 / 10.7; 2048 x 4096 10.6 / 10.5), others from 2 M numbers on (LayerNorm of
+  // 1339 x 2048 6.0 / 7.2, sum and RMSNorm of 2048 x 4096 11.1 / 12.3; LayerNorm of 1000 x 768 2.8 / 2.7).
   if (y && d <= 8 * kMaxVecPerThread * kNormThreads && (mode == 0 ? T >= 4096 : (int64_t)T * d >= 2000000)) {
     const int gt = d <= 1024 ? 32 : d <= 2048 ? 64 : d <= 4096 ? 128 : 256;
     return mode == 0 ? launch_norm_rows<0>(gt, y, residual, x, w, b, T, d, eps, s) : mode == 1 ? launch_norm_rows<1>(gt, y, residual, x, w, b, T, d, eps, s)

@@ -1,4 +1,4 @@
-"""Norms of many rows (csrc/elementwise.cu, norm_rows_kernel and norm_piece_kernel) against float64: each number of threads per row, rows and pieces that fill no
+"""Norms of many rows (csrc/elementwise.cu, norm_rows_kernel) against float64: each number of threads per row, rows and pieces that fill no
 round of the loop."""
 import pytest
 import torch
@@ -26,8 +26,7 @@ def close(y, ref, roundings, kind):
 
 
 @pytest.mark.parametrize("kind", ["", "_f16"])
-@pytest.mark.parametrize("T,d", [(4096, 768), (4099, 1024), (4097, 1032), (4500, 2048), (4097, 3080), (4098, 8192), (1339, 2048), (489, 4096), (250000, 8),
-                                 (296, 1024), (297, 8), (298, 512), (299, 520), (401, 1032), (1183, 1024), (1250, 1032), (1249, 776), (1251, 2056), (2501, 2056), (2503, 4096), (3053, 4096), (300, 4104)])
+@pytest.mark.parametrize("T,d", [(4096, 768), (4099, 1024), (4097, 1032), (4500, 2048), (4097, 3080), (4098, 8192), (1339, 2048), (489, 4096), (250000, 8)])
 def test_rmsnorm(kge, kind, T, d):
     x, res, w, _ = inputs(T, d, kind)
     y = torch.empty_like(x)
