@@ -405,7 +405,10 @@ static int launch_attn(bf16* out, const bf16* q, int q_stride, const bf16* kc, c
     const bool few = HD == 64 && (int64_t)ns * KV * B <= 2 * 148;
     auto pick = [&](auto plain, auto ahead) { return early ? ahead : plain; };      // (128-wide heads have one form)
     const bool tma = tunable(TUN_ATTN_TMA) && bs >= 32 && decode_tma_supported(B, KV, bs);
-    if (ns > 1 && ns <= 8 && !extras && (tunable(TUN_ATTN_CLUSTER_MERGE) || (few && !tma))) {
+    const bool asked = ns > 1 && ns <= 8 && !extras && tunable(TUN_ATTN_CLUSTER_MERGE);
+    const int64_t need = ns > 1 && !asked ? (int64_t)B * H * ns * (HD + 2) * 4 : 0;      // (the same for launches that merge in a cluster by themselves)
+    KGE_REQUIRE(need == 0 || (ws && ws_bytes >= need), "kge_paged_attn: workspace %lld < %lld bytes", (long long)ws_bytes, (long long)need);
+    if (asked || (ns > 1 && ns <= 8 && !extras && few && !tma)) {
       // split-KV CTAs of one (request, kv head) as a cluster, merged over DSMEM: no workspace and one kernel.  By itself for small
       // launches of 64-wide heads (the line of kDecodeStagesFew): 32 / 8 heads, one request of 500 keys 6.7 us with the merge kernel and
       // 6.2 so, 4 of 2000 8.9 and 8.0, 16 of 300 7.5 and 6.7, 8 of 2000 level; but 128-wide heads 8.2 and 8.5 (one of 500; 8 of 500 with
@@ -428,8 +431,6 @@ static int launch_attn(bf16* out, const bf16* q, int q_stride, const bf16* kc, c
     }
     float* po = nullptr; float* pml = nullptr;
     if (ns > 1) {
-      const int64_t need = (int64_t)B * H * ns * (HD + 2) * 4;
-      KGE_REQUIRE(ws && ws_bytes >= need, "kge_paged_attn: workspace %lld < %lld bytes", (long long)ws_bytes, (long long)need);
       po = (float*)ws;
       pml = po + (int64_t)B * H * ns * HD;
     }

@@ -641,6 +641,15 @@ def test_decode_attention_variants_give_the_same_bits(kge, L, H, KV, hd, q_lens,
         assert torch.equal(a.view(torch.int16), other.view(torch.int16))
 
 
+def test_a_split_decode_launch_asks_for_its_workspace(kge, L):
+    """Refused by the host before a launch, also where the pieces merge without it."""
+    z = torch.zeros(64 * 64 * 64, dtype=BF, device="cuda")
+    bt, sl, qsl = (torch.tensor(v, dtype=torch.int32, device="cuda") for v in ([list(range(1, 33))], [500], [0, 1]))
+    args = [p(z), p(z), 3 * 256, p(z), p(z), p(bt), 32, p(sl), p(qsl), 1, 1, 1]
+    assert L.kge_paged_attn(*args, 500, 4, 4, 64, 16, 0.125, None, 0, None) != 0
+    assert L.kge_paged_attn(*args, 500, 4, 4, 64, 16, 0.125, p(z), 4 * 2 * 66 * 4 - 1, None) != 0
+
+
 PERSISTENT_CASES = [
     # H, KV, hd, block size, seq_lens, forced split factor
     (32, 8, 128, 64, [2100 + 3 * i for i in range(48)], 0),        # 48 x 8 x 2 items > 296 resident CTAs: several items per CTA
