@@ -40,14 +40,14 @@ __device__ __forceinline__ void rg_compose2(f2& A, f2& B, f2 a, f2 b) {
   rg_compose(A1, B1, a1, b1);
   A = pk(A0, A1); B = pk(B0, B1);
 }
-// a_t and b_t = sqrt(1 - a_t^2) i_t u_t of two numbers from the pre-activations of r and i; sp = decay * softplus(lam)
-__device__ __forceinline__ void rg_coefficients(f2 r, f2 i, f2 u, f2 sp, f2& a, f2& b) {
-  const f2 x = mul2(sp, sigmoid2(r));
-  a = exp_neg2(x);
-  b = mul2(mul2(complement_root2(x, a), sigmoid2(i)), u);
+// a_t and b_t = sqrt(1 - a_t^2) i_t u_t of two numbers from the pre-activations of r and i; rate = -decay * softplus(lam)
+__device__ __forceinline__ void rg_coefficients(f2 r, f2 i, f2 u, f2 rate, f2& a, f2& b) {
+  const f2 w = mul2(rate, sigmoid2(r));
+  a = exp2_(w);
+  b = mul2(mul2(complement_root2(w), sigmoid2(i)), u);
 }
 template <typename E>
-__device__ __forceinline__ float rg_rate(const RglruArgs& a, int c) { return fminf(a.decay_c * softplusf_(ldf((const E*)a.lam + c)), 1e30f); }
+__device__ __forceinline__ float rg_rate(const RglruArgs& a, int c) { return -a.decay_c * softplusf_(ldf((const E*)a.lam + c)); }
 
 // V neighbouring channels of a row
 template <int V, typename E>
@@ -83,7 +83,7 @@ __global__ void __launch_bounds__(128) rglru_ab_kernel(RglruArgs a, float* gates
   pdl_wait();
   const int c = (blockIdx.y * 128 + threadIdx.x) * V, t0 = blockIdx.x * RG_TILE, n = min(RG_TILE, a.T - t0);
   if (c >= a.width) return;
-  const f2 sp = pk(rg_rate<E>(a, c), V == 2 ? rg_rate<E>(a, c + V - 1) : 0.f);
+  const f2 rate = pk(rg_rate<E>(a, c), V == 2 ? rg_rate<E>(a, c + V - 1) : 0.f);
   f2 A = pk1(1.f), B = pk1(0.f);
   for (int k0 = 0; k0 < n; k0 += 4) {
     f2 gr[4], gi[4], uv[4], s0[4];
@@ -101,7 +101,7 @@ __global__ void __launch_bounds__(128) rglru_ab_kernel(RglruArgs a, float* gates
     for (int k = 0; k < 4; ++k) {
       if (k0 + k >= n) break;
       f2 av, bv;
-      rg_coefficients(gr[k], gi[k], uv[k], sp, av, bv);
+      rg_coefficients(gr[k], gi[k], uv[k], rate, av, bv);
       if (first[k]) { bv = fma2(av, s0[k], bv); av = pk1(reset_mark()); }
       float* gt = gates + (int64_t)(t0 + k0 + k) * 2 * a.width + c;
       rg_store<V>(gt, av);
@@ -364,7 +364,7 @@ __global__ void __launch_bounds__(QUADS * 128) rglru_gates_kernel(RglruArgs a, f
   // this warp's unit of a tile: 32 channels, half of the tokens
   const int m = gw < QUADS / 4 * 8 ? gw / 8 : MT - 1, rest = QUADS - 4 * m;
   const int half = rest >= 4 ? gw / 4 & 1 : rest == 2 ? quad >> 1 : gw & 1, ch32 = rt_channels(QUADS, m, quad), ch = z * BW + ch32 * 32 + lane;
-  const f2 sp = pk1(rg_rate<E>(a, ch)), br = pk1(a.b_r ? ldf((const E*)a.b_r + ch) : 0.f), bi = pk1(a.b_i ? ldf((const E*)a.b_i + ch) : 0.f);
+  const f2 rate = pk1(rg_rate<E>(a, ch)), br = pk1(a.b_r ? ldf((const E*)a.b_r + ch) : 0.f), bi = pk1(a.b_i ? ldf((const E*)a.b_i + ch) : 0.f);
   pdl_wait();
   asm volatile("cp.async.wait_all;" ::: "memory");
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -453,7 +453,7 @@ __global__ void __launch_bounds__(QUADS * 128) rglru_gates_kernel(RglruArgs a, f
           const unsigned char* uk = us + k * 64 + (((lane >> 3) ^ (k >> 1 & 3)) << 4);
           const f2 u = pk(ldf(reinterpret_cast<const E*>(uk)), ldf(reinterpret_cast<const E*>(uk + 64)));
           f2 av, bv;
-          rg_coefficients(add2(pk(__uint_as_float(rr[k]), __uint_as_float(rr[k + 1])), br), add2(pk(__uint_as_float(ri[k]), __uint_as_float(ri[k + 1])), bi), u, sp, av, bv);
+          rg_coefficients(add2(pk(__uint_as_float(rr[k]), __uint_as_float(rr[k + 1])), br), add2(pk(__uint_as_float(ri[k]), __uint_as_float(ri[k + 1])), bi), u, rate, av, bv);
           float a2[2], b2[2];
           upk(av, a2[0], a2[1]);
           upk(bv, b2[0], b2[1]);
@@ -502,7 +502,7 @@ __global__ void __launch_bounds__(320) rglru_step_kernel(RglruArgs a, int bw, in
   const int z = blockIdx.y, c0 = blockIdx.z * cols, n0 = warp * 8, pieces = bw / 8, taps = TAPS ? TAPS : a.taps;
   rg_fetch_weights(W, a, z, c0, cols, bw);
   const int ch = z * bw + c0 + n0 + 2 * t4;
-  const f2 sp = pk(rg_rate<E>(a, ch), rg_rate<E>(a, ch + 1));
+  const f2 rate = pk(rg_rate<E>(a, ch), rg_rate<E>(a, ch + 1));
   const f2 br = a.b_r ? rg_load<2>((const E*)a.b_r + ch) : pk1(0.f), bi = a.b_i ? rg_load<2>((const E*)a.b_i + ch) : pk1(0.f);
   // slots, positions and the state are from before the step (its first kernel starts behind all of the step before)
   auto row_of = [&](int t) { return RgRow{0, a.positions[t], a.state + (int64_t)a.slots[t] * a.slot_stride}; };
@@ -537,7 +537,7 @@ __global__ void __launch_bounds__(320) rglru_step_kernel(RglruArgs a, int bw, in
     if (g + 8 * h < n) {
       const uint32_t uu = *reinterpret_cast<const uint32_t*>(U + (g + 8 * h) * ldw + c0 + n0 + 2 * t4);
       f2 av, bv;
-      rg_coefficients(add2(pk(acc[0][0][2 * h], acc[0][0][2 * h + 1]), br), add2(pk(acc[1][0][2 * h], acc[1][0][2 * h + 1]), bi), pk(bf_lo(uu), bf_hi(uu)), sp, av, bv);
+      rg_coefficients(add2(pk(acc[0][0][2 * h], acc[0][0][2 * h + 1]), br), add2(pk(acc[1][0][2 * h], acc[1][0][2 * h + 1]), bi), pk(bf_lo(uu), bf_hi(uu)), rate, av, bv);
       const f2 s = fma2(av, S[h], bv);
       rg_keep<2>(slot[h] + ch, s);
       rg_store<2>((E*)a.out + (int64_t)(t0 + g + 8 * h) * a.width + ch, mul2(s, gelu_tanh2(y[h])));

@@ -100,6 +100,20 @@ def test_recurrence_by_tiles(kge, tmp_path, width, blocks, taps):
 
 
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+def test_a_rate_that_is_not_a_number_spreads(kge, tmp_path, dtype):
+    """In prompt pieces and in decode steps, whichever kernels take them."""
+    cfg = oh.make_config(layers=("rglru",), mlps=(None,), r_width=64, r_blocks=2)
+    W = oh.make_weights(cfg, seed=43)
+    lam = next(k for k in W if k.endswith("mix.lam"))
+    W[lam] = W[lam].clone()
+    W[lam][37] = float("nan")
+    toks = prompt(cfg, 40)
+    llm = make_engine(kge, tmp_path, cfg, W, dtype)
+    assert np.isnan(run_pieces(llm, 0, toks, [33, 1, 4, 1, 1])).all()
+    llm.close()
+
+
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 @pytest.mark.parametrize("heads,dim,vdim,requests", [(3, 128, 256, 3), (1, 4, 8, 9), (2, 36, 40, 5), (2, 128, 33, 2), (1, 16, 264, 2)])
 def test_matrix_memory_token_by_token(kge, tmp_path, heads, dim, vdim, requests, dtype):
     """Decode steps in one launch: key dimensions that do not fill their warps, value columns that end inside a block and take one to eight
