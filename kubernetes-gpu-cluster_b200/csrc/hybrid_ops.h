@@ -276,6 +276,17 @@ int rglru_conv(const RglruArgs& a, cudaStream_t st);
 int rglru_scan(const RglruArgs& a, cudaStream_t st);
 // Both and the gate projections together.  Decode steps (one row a request; rglru_step_ok): one launch, u and gates unused.  Other steps
 // (rglru_gates_ok): rglru_gates turns x into the coefficients a, b (in `gates`), rglru_walk those into out and state.
+// Warps of a block of rglru_step, each with eight of a diagonal block's `bw` columns; the blocks of a diagonal block are a cluster.  The fewest
+// blocks that leave a block four warps or fewer, else as many as there can be: eight in a portable cluster, ten warps in a block.  0 where
+// the columns can't be shared out so (bw = 176 and 208: 22 and 26 groups), or bw is no multiple of 16 up to 256: then the general path.
+inline int rglru_step_warps(int bw) {
+  if (bw <= 0 || bw % 16 != 0 || bw > 256) return 0;
+  const int groups = bw / 8;
+  int warps = 0;
+  for (int parts = 1; parts <= 8 && (warps == 0 || warps > 4); ++parts)
+    if (groups % parts == 0 && groups / parts <= 10) warps = groups / parts;
+  return warps;
+}
 bool rglru_step_ok(const RglruArgs& a);
 bool rglru_gates_ok(const RglruArgs& a);
 int rglru_step(const RglruArgs& a, cudaStream_t st);

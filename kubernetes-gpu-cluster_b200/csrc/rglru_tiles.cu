@@ -561,26 +561,19 @@ __global__ void __launch_bounds__(320) rglru_step_kernel(RglruArgs a, int bw, in
   }
 }
 
-// Columns of a block of rglru_step_kernel: eight per warp, ten warps at most; a diagonal block is spread over up to eight blocks.
-static int rg_groups(int groups) {
-  for (int parts = 1; parts <= groups; ++parts)
-    if (groups % parts == 0 && groups / parts <= 10 && (parts >= std::min(groups, 8) || groups / parts <= 4)) return groups / parts;
-  return 1;
-}
-
 static bool rg_rows_ok(const RglruArgs& a) {
   return a.elt == KGE_ELT_BF16 && a.blocks > 0 && a.blocks <= 65535 && a.width % a.blocks == 0 && a.taps >= 1 && a.taps <= RG_MAX_TAPS &&
          ((reinterpret_cast<uintptr_t>(a.yx) | reinterpret_cast<uintptr_t>(a.w_r) | reinterpret_cast<uintptr_t>(a.w_i) | reinterpret_cast<uintptr_t>(a.conv_b) | reinterpret_cast<uintptr_t>(a.out)) & 15) == 0 &&
          ((reinterpret_cast<uintptr_t>(a.b_r) | reinterpret_cast<uintptr_t>(a.b_i)) & 3) == 0;
 }
-bool rglru_step_ok(const RglruArgs& a) { return rg_rows_ok(a) && a.width / a.blocks % 16 == 0 && a.width / a.blocks <= 256; }
+bool rglru_step_ok(const RglruArgs& a) { return rg_rows_ok(a) && rglru_step_warps(a.width / a.blocks) > 0; }
 bool rglru_gates_ok(const RglruArgs& a) { return rg_rows_ok(a) && rt_fits(a.width / a.blocks); }
 
 static bool rg_four_taps(const RglruArgs& a) { return a.taps == 4 && (reinterpret_cast<uintptr_t>(a.conv_w) & 15) == 0; }
 
 template <int TAPS>
 static int rg_step(const RglruArgs& a, cudaStream_t st) {
-  const int bw = a.width / a.blocks, groups = rg_groups(bw / 8), cols = groups * 8, parts = bw / cols;
+  const int bw = a.width / a.blocks, groups = rglru_step_warps(bw), cols = groups * 8, parts = bw / cols;
   auto kern = rglru_step_kernel<TAPS>;
   KGE_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (2 * 80 + 16) * (256 + 8) * 2));
   prefer_max_shared(kern);

@@ -67,11 +67,13 @@ def test_block_diagonal_gates_of_many_rows(kge, tmp_path, width, blocks, rows):
     llm.close()
 
 
-@pytest.mark.parametrize("width,blocks,taps", [(64, 2, 4), (192, 3, 3), (256, 2, 4), (480, 3, 4), (320, 2, 2), (512, 2, 4), (66, 2, 4)])
+@pytest.mark.parametrize("width,blocks,taps", [(64, 2, 4), (192, 3, 3), (256, 2, 4), (480, 3, 4), (320, 2, 2), (512, 2, 4), (66, 2, 4),
+                                               (352, 2, 4), (416, 2, 3), (480, 2, 4), (384, 2, 4), (448, 2, 2)])
 def test_recurrence_by_tiles(kge, tmp_path, width, blocks, taps):
-    """Convolution, gates and coefficients in one kernel (blocks of 32, 64, 128 and 160 channels; 256 and 33 take the general ones), the
+    """Convolution, gates and coefficients in one kernel (blocks of 32, 64, 128 and 160 channels; others take the general ones), the
     recurrence by tiles of 32 rows: pieces that end before, at and behind a tile's edge and span more tiles than are composed at once;
-    many requests that begin and end inside one tile, beside decode rows; then decode steps of more requests than a block has rows."""
+    many requests that begin and end inside one tile, beside decode rows; then decode steps of more requests than a block has rows, in one
+    launch where the columns of a diagonal block can be shared out over at most eight blocks (not 176, 208 and 33)."""
     cfg = oh.make_config(layers=("rglru",), mlps=(None,), r_width=width, r_blocks=blocks, r_conv=taps)
     W = oh.make_weights(cfg, seed=43)
     toks = prompt(cfg, 420)
