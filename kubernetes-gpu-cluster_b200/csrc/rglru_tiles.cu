@@ -335,7 +335,6 @@ __host__ __device__ constexpr bool rt_fits(int bw) { return bw == 32 || bw == 64
 
 template <int QUADS, int TAPS>
 __global__ void __launch_bounds__(QUADS * 128) rglru_gates_kernel(RglruArgs a, float* gates, int units) {
-  pdl_launch_dependents();
   typedef __nv_bfloat16 E;
   constexpr int BW = QUADS * 32, MT = rt_row_tiles(QUADS), PIECES = BW / 8, GROUP = QUADS * 64, ROWS_A = QUADS * 128 * 64, ROWS_U = RT_N * 64;
   constexpr uint32_t COLS = 2 * MT * RT_N;                     // of a group: [gate][row tile][token]
@@ -371,6 +370,8 @@ __global__ void __launch_bounds__(QUADS * 128) rglru_gates_kernel(RglruArgs a, f
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  // the columns are held: blocks of a later kernel that took them first would wait for this one
+  pdl_launch_dependents();
   const uint32_t tmem = tmem_slot + grp * COLS, bar = (uint32_t)__cvta_generic_to_shared(&bars[grp]);
   // the block's share of the units of 32 tokens, and what of it ends at the last token
   const int u0 = (int)((int64_t)units * blockIdx.x / gridDim.x), u1 = (int)((int64_t)units * (blockIdx.x + 1) / gridDim.x), end = min(u1 * RG_TILE, a.T);

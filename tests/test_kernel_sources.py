@@ -56,3 +56,18 @@ def test_waits_for_tensor_memory_hold_back_what_reads_it():
             assert call, path
             waits += 1
     assert waits >= 8
+
+
+TENSOR_MEMORY = [(f, k, b) for f, k, b in kernels() if "tcgen05.alloc" in b and "pdl_launch_dependents" in b]
+
+
+def test_the_kernels_with_tensor_memory_are_found():
+    assert {k for _, k, _ in TENSOR_MEMORY} >= {"gemm_tc_kernel", "gemm_wide_kernel", "attn_tc_kernel", "attn_pair_kernel", "rglru_gates_kernel"}
+
+
+@pytest.mark.parametrize("file,kernel,body", TENSOR_MEMORY, ids=[k for _, k, _ in TENSOR_MEMORY])
+def test_tensor_memory_is_allocated_before_the_next_kernel_may_start(file, kernel, body):
+    """An allocation waits until columns are free.  Blocks of a later kernel that had taken them would wait for this kernel to end."""
+    alloc, start = body.index("tcgen05.alloc"), body.index("pdl_launch_dependents")
+    assert alloc < start, (file, kernel)
+    assert "__syncthreads()" in body[alloc:start], (file, kernel)      # by one warp: the others may not announce it earlier
