@@ -512,6 +512,10 @@ int paged_attn_step(void* out, const void* q, int q_stride, const void* k_cache,
   return paged_attn_extras(out, q, q_stride, k_cache, v_cache, block_table, max_blocks_per_seq, seq_lens, query_start_loc, B, T, max_q_len,
                            max_seq_len, H, KV, hd, block_size, scale, 0.f, nullptr, workspace, workspace_bytes, stream, max_q_len == 1);
 }
+// whether paged_attn_step does with these sizes what kge_paged_attn does not
+bool paged_attn_reads_ahead(int B, int H, int KV, int hd, int block_size) {
+  return hd == 64 && H % KV == 0 && H / KV <= 16 && !(tunable(TUN_ATTN_TMA) && block_size >= 32 && decode_tma_supported(B, KV, block_size));
+}
 // whether a pure decode step with these sizes reaches a kernel that has the cap and the sinks
 bool paged_attn_extras_decode_ok(int B, int H, int KV, int hd, int block_size) {
   return (hd == 64 || hd == 128) && H % KV == 0 && H / KV <= 16 && tunable(TUN_ATTN_TMA) && block_size >= 32 &&

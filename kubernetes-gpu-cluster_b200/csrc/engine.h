@@ -206,6 +206,7 @@ struct kge_engine {
 
   // a decode step in which no request's keys before its last are written: they can be read while the kernel that writes the last still runs
   bool step_keys_before = false;
+  bool hyb_reads_ahead = false;              // layer lists: some mixer's attention reads such keys early
   std::vector<int32_t> block_writer;         // [num_blocks] request of the step that writes to the block + 1 (all zero between steps)
   bool step_rows_all = false;                // the step's logits rows are its tokens, in order: nothing to gather
   kge::bf16* res_next = nullptr;             // [8, d]: the residual stream's other buffer in small steps (norm_gemm.h)

@@ -62,6 +62,7 @@ static int linear_rc(kge_engine* e, bf16* y, const bf16* x, const Linear& l, int
 __global__ void mask_logits_kernel(bf16* logits, const int32_t* pairs, int n, int ld, int vocab, bool f16);
 int tp_all_reduce(kge_engine* e, bf16* buf, int64_t n);   // tp.cu
 int tp_all_gather_logits(kge_engine* e, int R);           // tp.cu (NCCL path)
+inline namespace b16 { bool paged_attn_reads_ahead(int B, int H, int KV, int hd, int block_size); }      // attn.cu (of both element types)
 
 // The row-parallel projection before this point left its output (under TP: this rank's partial sum) in e->h:
 // all-reduce it, add it to the residual stream and normalise into e->xn.  Single GPU: the fused add + norm kernel.
@@ -211,6 +212,10 @@ int engine_forward(kge_engine* e, int T, int B, int R, int max_blocks, int max_q
   return 0;
 }
 
+// Whether any launch of a decode step of B requests has a use for keys that were there before it (layer lists: by their mixers)
+static bool step_reads_ahead(const kge_engine* e, int B) {
+  return e->spec.is_hybrid() ? e->hyb_reads_ahead : paged_attn_reads_ahead(B, e->H_loc, e->KV_loc, e->spec.hd, e->cfg.block_size);
+}
 int engine_decode_step(kge_engine* e, int B, int stride, int max_seq_len, const StepMeta& dm, bool any_random, double sum_seq) {
   const double attn_flops = 4.0 * sum_seq;
   const bool hybrid = e->spec.is_hybrid();
@@ -225,13 +230,14 @@ int engine_decode_step(kge_engine* e, int B, int stride, int max_seq_len, const 
   if (!e->use_graphs || e->timing || e->step_num_masks > 0 || e->layer_dump_host)      // a masked step is rare and its mask list is not part of a graph
     return forward();
   const bool logits = hybrid && e->want_logits32;      // only layer-list models launch anything for logits that are read back
+  const bool before = e->step_keys_before && step_reads_ahead(e, B);
   for (auto& g : e->graphs)
-    if (g.B == B && g.ns == ns && g.stride == stride && g.rnd == any_random && g.logits == logits && g.before == e->step_keys_before) {
+    if (g.B == B && g.ns == ns && g.stride == stride && g.rnd == any_random && g.logits == logits && g.before == before) {
       KGE_CUDA_OK(cudaGraphLaunch(g.exec, e->stream));
       e->launches += g.launches;
       return 0;
     }
-  const int64_t key = ((int64_t)B << 40) ^ ((int64_t)ns << 32) ^ ((int64_t)stride << 2) ^ (logits ? 2 : 0) ^ (any_random ? 1 : 0) ^ (e->step_keys_before ? (int64_t)1 << 62 : 0);
+  const int64_t key = ((int64_t)B << 40) ^ ((int64_t)ns << 32) ^ ((int64_t)stride << 2) ^ (logits ? 2 : 0) ^ (any_random ? 1 : 0) ^ (before ? (int64_t)1 << 62 : 0);
   int* seen = nullptr;
   for (auto& kv : e->graph_seen) if (kv.first == key) seen = &kv.second;
   if (!seen) { e->graph_seen.push_back({key, 0}); seen = &e->graph_seen.back().second; }
@@ -246,7 +252,7 @@ int engine_decode_step(kge_engine* e, int B, int stride, int max_seq_len, const 
   cudaError_t ce = cudaStreamEndCapture(e->stream, &graph);
   if (rc) { if (graph) cudaGraphDestroy(graph); return rc; }
   KGE_REQUIRE(ce == cudaSuccess && graph, "decode graph capture failed: %s", cudaGetErrorString(ce));
-  kge_engine::DecodeGraph g{B, ns, stride, any_random, logits, e->step_keys_before, nullptr, e->launches - l0};
+  kge_engine::DecodeGraph g{B, ns, stride, any_random, logits, before, nullptr, e->launches - l0};
   ce = cudaGraphInstantiate(&g.exec, graph, 0);
   cudaGraphDestroy(graph);
   KGE_REQUIRE(ce == cudaSuccess, "cudaGraphInstantiate failed: %s", cudaGetErrorString(ce));
@@ -367,7 +373,7 @@ static int run_step(kge_engine* e, const kge_step_batch* b, const float* temp, c
     max_seq = std::max(max_seq, b->seq_lens[i]);
   }
   KGE_REQUIRE(b->query_start_loc[B] == T, "kge_step: query_start_loc[B]=%d != T=%d", b->query_start_loc[B], T);
-  e->step_keys_before = decode_only && max_q == 1 && keys_before_step(e, b);
+  e->step_keys_before = decode_only && max_q == 1 && step_reads_ahead(e, B) && keys_before_step(e, b);
   if (e->recording) {
     kge_engine::RecordedStep rs{};
     rs.T = T; rs.B = B; rs.R = R; rs.stride = stride; rs.max_q = max_q; rs.max_seq = max_seq;

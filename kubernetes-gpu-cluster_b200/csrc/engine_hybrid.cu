@@ -732,6 +732,7 @@ int hybrid_engine_build(kge_engine* e, const ModelDir& md, int64_t dummy_seed, s
     const HybridLayerSpec& h = s.hybrid[i];
     if (!h.has_cache()) continue;
     const int64_t nk = (int64_t)nb * e->cfg.block_size * h.cache_k_row(), nv = (int64_t)nb * e->cfg.block_size * h.cache_v_row();
+    e->hyb_reads_ahead |= !e->f32 && h.pool == 0 && h.keep_first == 0;      // (as attn_bias_chunk has it)
     e->hyb[i].kc = aalloc(nk, es);
     if (nv > 0) e->hyb[i].vc = aalloc(nv, es);      // cached latents: one row per token is key and value
     if (!e->hyb[i].kc || (nv > 0 && !e->hyb[i].vc)) return fail("KV pool allocation failed");

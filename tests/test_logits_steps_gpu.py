@@ -124,3 +124,22 @@ def test_keys_before_the_step_read_ahead(kge, tmp_path, name, lengths):
     both = step([(long, n - 1, prompts[long][n - 1:]), (long, n, [ids[long][0]])])[1]
     close(both, np.stack([ref[0][long], ref[1][long]]), "two rows of one sequence")
     llm.close()
+
+
+@pytest.mark.parametrize("block_size,graphs", [(16, 2), (32, 1)])
+def test_steps_whose_launches_are_alike_share_a_graph(kge, tmp_path, block_size, graphs):
+    """Steps of two requests with blocks of their own, and steps in which one row writes a block that the other reads: attention over blocks of
+    16 tokens reads ahead in the first kind only, over blocks of 32 in neither."""
+    cfg = om.CONFIGS["tiny-llama"]
+    om.save_model_dir(tmp_path, cfg, om.make_weights(cfg, seed=0))
+    llm = kge.LLM(str(tmp_path), max_model_len=128, max_num_seqs=2, max_num_batched_tokens=128, block_size=block_size, num_gpu_blocks_override=2 * 128 // block_size + 1,
+                  enable_prefix_caching=False)
+    per = 128 // block_size
+    table = 1 + np.arange(2 * per, dtype=np.int32).reshape(2, per)
+    for rows in ([(0, 40), (1, 40)], [(0, 40), (0, 41)]):
+        for _ in range(12):
+            pos = np.asarray([n for _, n in rows], dtype=np.int32)
+            slots = np.asarray([table[r, n // block_size] * block_size + n % block_size for r, n in rows], dtype=np.int64)
+            llm.raw_step(np.asarray([5, 6], dtype=np.int32), pos, np.arange(3, dtype=np.int32), pos + 1, table[[r for r, _ in rows]], per, slots, np.arange(2, dtype=np.int32))
+    assert llm.decode_graphs == graphs
+    llm.close()
