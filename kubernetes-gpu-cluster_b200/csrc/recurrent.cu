@@ -918,10 +918,12 @@ __global__ void mlstm_norm_gate_kernel(MlstmArgs a) {
   pdl_wait();
   __shared__ float red[33];
   const int t = blockIdx.x, h = blockIdx.y;
-  if (t < a.B) {                                               // a request's new n and m
-    const float* nm = a.nm_scratch + ((int64_t)t * a.H + h) * (a.dim + 1);
-    float* slot = a.state + (int64_t)a.slots[t] * a.slot_stride + ((int64_t)h + 1) * ((int64_t)a.dim * a.vdim + a.dim + 1) - (a.dim + 1);
+  if (t >= a.T) {                                              // blocks beyond the tokens: a request's new n and m
+    const int b = t - a.T;
+    const float* nm = a.nm_scratch + ((int64_t)b * a.H + h) * (a.dim + 1);
+    float* slot = a.state + (int64_t)a.slots[b] * a.slot_stride + ((int64_t)h + 1) * ((int64_t)a.dim * a.vdim + a.dim + 1) - (a.dim + 1);
     for (int d = threadIdx.x; d <= a.dim; d += blockDim.x) slot[d] = nm[d];
+    return;
   }
   const float* o = a.o_scratch + (int64_t)t * a.H * a.vdim + h * a.vdim;
   float ss = 0.f;
@@ -1102,7 +1104,7 @@ int mlstm_step(const MlstmArgs& a, cudaStream_t st) {
       KGE_CUDA_OK(cudaLaunchKernelEx(&cfg, kern, a));
       return 0;
     }
-    const dim3 grid(a.B, a.H, (a.vdim + ML_COLS - 1) / ML_COLS), g2(a.T, a.H);
+    const dim3 grid(a.B, a.H, (a.vdim + ML_COLS - 1) / ML_COLS), g2(a.T + a.B, a.H);
     const int nt = std::min(256, (a.vdim + 31) / 32 * 32);
     KGE_CUDA_OK(launch_pdl(mlstm_log_gates_kernel, dim3((a.T * 2 * a.H + 255) / 256), dim3(256), 0, st, const_cast<float*>(a.gates), a.T, a.H, a.cap));
     const size_t csm_bytes = ((size_t)2 * ML_CH * a.dim + ML_CH * ML_CH + ML_MAXD + 5 * ML_CH + (1 + ML_NSL) * ML_CH * MC_COLS) * 4;
