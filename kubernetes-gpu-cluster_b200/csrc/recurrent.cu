@@ -989,10 +989,11 @@ __global__ void __launch_bounds__(256) mlstm_norm_gate_wide_kernel(MlstmArgs a) 
     *reinterpret_cast<uint4*>((E*)a.out + (int64_t)t * a.ldo + h * vdim + c) = make_uint4(r[0], r[1], r[2], r[3]);
   }
 }
-// bfloat16 rows: the kernel above where pieces of 16 bytes are aligned and rows are more than the SMs hold blocks of 256 threads at once (one
-// prompt of 100 tokens and 4 heads, the whole chunkwise form: 16.7 us with a block a row, 17.2 with a warp; 4096 x 4 145 and 124)
+// bfloat16 rows: the kernel above where pieces of 16 bytes are aligned and there is more than the SMs hold in blocks of 256 threads at once (one
+// prompt of 100 tokens and 4 heads of 256, the whole chunkwise form: 16.7 us with a block a row, 17.2 with a warp; 4096 tokens 145 and 124;
+// 200 single tokens, 8 heads of 64, the whole step 27.3 and 28.5)
 static int mlstm_norm_gate(const MlstmArgs& a, dim3 grid, int threads, cudaStream_t st) {
-  const bool wide = (int64_t)a.T * a.H > 8 * 148 && a.vdim % 8 == 0 && a.vdim <= 1024 && a.ld % 8 == 0 && a.ldo % 8 == 0 &&
+  const bool wide = (int64_t)a.T * a.H * a.vdim > 8 * 148 * 256 && a.vdim % 8 == 0 && a.vdim <= 1024 && a.ld % 8 == 0 && a.ldo % 8 == 0 &&
                     ((reinterpret_cast<uintptr_t>(a.o_scratch) | reinterpret_cast<uintptr_t>(a.g) | reinterpret_cast<uintptr_t>(a.norm_w) | reinterpret_cast<uintptr_t>(a.out)) & 15) == 0;
   const dim3 wgrid((unsigned)(((int64_t)(a.T + a.B) * a.H + 7) / 8));
   if (!wide) KGE_CUDA_OK(launch_pdl(mlstm_norm_gate_kernel<__nv_bfloat16>, grid, dim3(threads), 0, st, a));
@@ -1070,6 +1071,13 @@ __global__ void __launch_bounds__(256) mlstm_token_kernel(MlstmArgs a) {
   }
 }
 
+// Decode steps in one launch: at most eight blocks of 32 columns; where heads of few key dimensions fill the SMs many times over, what a
+// block costs beside its state weighs more than the launches.  Three launches and one, us, 8 heads of 256 columns: 16 keys 64 requests (4096
+// blocks) 31.5 / 33.5, 250 94.7 / 113.6; 32 keys 250 99.8 / 115.3; 64 keys 128 requests 62.3 / 68.1; from 96 keys on ahead everywhere (128
+// requests 3 %, of 128 keys 7 %), up to 2048 blocks for all sizes (2 to 60 %).
+static bool mlstm_one_launch(const MlstmArgs& a) {
+  return a.vdim <= 8 * 32 && (a.dim >= 96 || (int64_t)a.B * a.H * ((a.vdim + 31) / 32) <= 2048);
+}
 // Blocks that share a head's columns of a request (a cluster): as many as one an SM has room for, and no more than there are chunks
 static int mlstm_ranks(const MlstmArgs& a) {
   const int64_t blocks = (int64_t)a.B * a.H * ((a.vdim + MM_COLS - 1) / MM_COLS), rows = a.max_rows > 0 ? a.max_rows : a.T - a.B + 1;
@@ -1090,7 +1098,7 @@ static bool mlstm_use_mma(const MlstmArgs& a) {
 int mlstm_step(const MlstmArgs& a, cudaStream_t st) {
   if (a.T <= 0 || a.B <= 0) return 0;
   if (a.o_scratch && a.nm_scratch && a.dim <= ML_MAXD && a.dim % 4 == 0 && a.H <= 65535) {
-    if (a.T == a.B && a.vdim <= 8 * 32) {
+    if (a.T == a.B && mlstm_one_launch(a)) {
       auto kern = a.elt == KGE_ELT_F32 ? mlstm_token_kernel<float> : mlstm_token_kernel<__nv_bfloat16>;
       prefer_max_shared(kern);
       cudaLaunchConfig_t cfg = {};
