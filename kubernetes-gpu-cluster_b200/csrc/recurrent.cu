@@ -6,6 +6,7 @@
 // A request whose first row of the step is position 0 starts from zero; otherwise from what its slot holds.  Rows of a
 // request are processed in order, so cutting a prompt into steps anywhere gives the same arithmetic.
 #include <algorithm>
+#include <atomic>
 
 #include "common.cuh"
 #include "elt_access.cuh"
@@ -1078,12 +1079,33 @@ __global__ void __launch_bounds__(256) mlstm_token_kernel(MlstmArgs a) {
 static bool mlstm_one_launch(const MlstmArgs& a) {
   return a.vdim <= 8 * 32 && (a.dim >= 96 || (int64_t)a.B * a.H * ((a.vdim + 31) / 32) <= 2048);
 }
-// Blocks that share a head's columns of a request (a cluster): as many as one an SM has room for, and no more than there are chunks
+// Clusters of S blocks that run at once on this device: one block an SM, and what is left of a GPC beyond a multiple of S stays empty
+// (148, 74, 45, 33, 26, 22, 15 and 15 on a B200).  0: not known.
+static int mlstm_clusters(int S) {
+  static std::atomic<int> known[16][9];      // [device][S], plus one
+  int dev = 0, n = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) { cudaGetLastError(); return 0; }
+  std::atomic<int>* const at = dev < 16 ? &known[dev][S] : nullptr;
+  if (at && at->load(std::memory_order_relaxed)) return at->load(std::memory_order_relaxed) - 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(S); cfg.blockDim = dim3(MM_THREADS); cfg.dynamicSmemBytes = sizeof(MlstmTile);
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = S; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr; cfg.numAttrs = 1;
+  if (cudaFuncSetAttribute(mlstm_mma_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(MlstmTile)) != cudaSuccess ||
+      cudaOccupancyMaxActiveClusters(&n, mlstm_mma_kernel<true>, &cfg) != cudaSuccess) { cudaGetLastError(); return 0; }
+  if (at) at->store(n + 1, std::memory_order_relaxed);
+  return n;
+}
+// Blocks that share a head's columns of a request (a cluster): as many as leave all clusters running at once, and no more than there are
+// chunks.  (48 clusters of three are three more than fit: three prompts of 200 tokens, 4 heads of 16 x 128, 29.4 us with one block,
+// 31.8 with three, 24.3 with two.)
 static int mlstm_ranks(const MlstmArgs& a) {
   const int64_t blocks = (int64_t)a.B * a.H * ((a.vdim + MM_COLS - 1) / MM_COLS), rows = a.max_rows > 0 ? a.max_rows : a.T - a.B + 1;
-  int S = 1;
-  while (S < 8 && blocks * (S + 1) <= 148 && rows > (int64_t)S * MM_CH) ++S;
-  return S;
+  for (int S = (int)std::min<int64_t>(8, (rows + MM_CH - 1) / MM_CH); S > 1; --S)
+    if (blocks <= mlstm_clusters(S)) return S;
+  return 1;
 }
 // Tensor-core chunks or the fp32 ones, by estimates (us) from measurements at 8 x 32 x 32 to 4 x 128 x 256 and 1 to 256 requests: a
 // tensor-core block fills an SM and takes 9 us beside 7 per 64 tokens of the longest request, an fp32 one shares it with two others,
