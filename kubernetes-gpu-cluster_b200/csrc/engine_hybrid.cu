@@ -846,9 +846,16 @@ int hybrid_forward(kge_engine* e, int T, int B, int R, int max_blocks, const Ste
   // Behind the last layer's mixer a row depends on no other, and of a prompt step only the rows that logits were asked of are read
   // again: the output projection and the feed-forward run over those, brought to the front of their buffers in one launch.  A 2048-wide
   // design of four layers with 16 experts in the last, prompts of 1150 and 1162 tokens: 1723 us a step with every row, 1511
-  // so.  The line: below four rows a logits row the products stay in the same row tiles, and 256 rows are
-  // sixteen turns of the copying kernel; places out of order (scripted steps only) can't move within one buffer.  Layer dumps hold every row.
-  bool front = !decode_only && R <= 256 && 4 * R <= T && !e->layer_dump_host;
+  // so.  The lines: below four rows a logits row the products stay in the same row tiles; places out of order (scripted steps only) can't move
+  // within one buffer; layer dumps hold every row.  And the launch has to pay.  A dense feed-forward's products take up to 16 rows as fast as one
+  // (512 wide, 5 tokens 110 us a step without and 117 with it, 40 tokens 11 less), many narrow rows are level (128 wide, 40 of 160 tokens 4 more);
+  // experts are as many as rows choose (2048 wide, 5 tokens 30 us less); without a feed-forward there is the output projection only (512 wide, 600
+  // tokens level, 3000 9 us less; 2048 wide, 600 tokens 18 less).
+  const HybridLayerSpec& last = s.hybrid[s.L - 1];
+  const int64_t numbers = (int64_t)T * d;
+  const bool pays = R == 0 || (last.mlp == HybridLayerSpec::NONE ? numbers >= 1 << 20 : last.mlp == HybridLayerSpec::MOE ? T > (d >= 512 ? 4 : 16)
+                                                                                      : T > 16 && (R <= 16 || numbers >= 1 << 18));
+  bool front = !decode_only && pays && R <= 256 && 4 * R <= T && !e->layer_dump_host;
   for (int r = 0; r + 1 < R && front; ++r) front = hm.rows[r] < hm.rows[r + 1];
   const int32_t* out_rows = m.rows;                  // of the residual stream, for the head
   const int n_out = R;

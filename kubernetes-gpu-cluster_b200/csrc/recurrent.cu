@@ -913,6 +913,16 @@ __global__ void __launch_bounds__(MM_THREADS) mlstm_mma_kernel(MlstmArgs a) {
   }
 }
 
+// n and m, dim + 1 numbers, by n threads: five at a time, since loads do not pass stores by themselves
+__device__ __forceinline__ void ml_copy_nm(float* slot, const float* nm, int dim, int i, int n) {
+  for (; i <= dim; i += 5 * n) {
+    float v[5];
+#pragma unroll
+    for (int k = 0; k < 5; ++k) if (i + k * n <= dim) v[k] = nm[i + k * n];
+#pragma unroll
+    for (int k = 0; k < 5; ++k) if (i + k * n <= dim) slot[i + k * n] = v[k];
+  }
+}
 template <typename E>
 __global__ void mlstm_norm_gate_kernel(MlstmArgs a) {
   pdl_launch_dependents();
@@ -923,7 +933,7 @@ __global__ void mlstm_norm_gate_kernel(MlstmArgs a) {
     const int b = t - a.T;
     const float* nm = a.nm_scratch + ((int64_t)b * a.H + h) * (a.dim + 1);
     float* slot = a.state + (int64_t)a.slots[b] * a.slot_stride + ((int64_t)h + 1) * ((int64_t)a.dim * a.vdim + a.dim + 1) - (a.dim + 1);
-    for (int d = threadIdx.x; d <= a.dim; d += blockDim.x) slot[d] = nm[d];
+    ml_copy_nm(slot, nm, a.dim, threadIdx.x, blockDim.x);
     return;
   }
   const float* o = a.o_scratch + (int64_t)t * a.H * a.vdim + h * a.vdim;
@@ -952,8 +962,7 @@ __global__ void __launch_bounds__(256) mlstm_norm_gate_wide_kernel(MlstmArgs a) 
     if (b >= a.B) return;
     const float* nm = a.nm_scratch + ((int64_t)b * a.H + h) * (a.dim + 1);
     float* slot = a.state + (int64_t)a.slots[b] * a.slot_stride + ((int64_t)h + 1) * ((int64_t)a.dim * vdim + a.dim + 1) - (a.dim + 1);
-#pragma unroll 5
-    for (int d = lane; d <= a.dim; d += 32) slot[d] = nm[d];
+    ml_copy_nm(slot, nm, a.dim, lane, 32);
     return;
   }
   const float* o = a.o_scratch + ((int64_t)t * a.H + h) * vdim;
