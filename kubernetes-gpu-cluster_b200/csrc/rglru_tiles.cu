@@ -22,7 +22,7 @@
 
 namespace kge {
 
-constexpr int RG_TILE = 32, RG_PART = 8;       // tokens of a tile; rows of the walk in flight
+constexpr int RG_TILE = 32;                    // tokens of a tile
 constexpr int RG_MAX_TAPS = 16;
 
 __device__ __forceinline__ bool is_reset(float a) { return __float_as_uint(a) == 0x80000000u; }     // -0: no exponential is
@@ -140,10 +140,12 @@ __global__ void __launch_bounds__(RB_WARPS * 32) rglru_ab_kernel(RglruArgs a, fl
   rg_store<V>(to + a.width, B);
 }
 
-// The walk: half a tile's rows are asked for at once, the first half's before anything else.  Blocks behind the tiles, one a request, bring the
-//  convolution's inputs up to date (in the walk it cost steps with many requests a trip to memory a row).
-template <typename E, int V>
-__global__ void __launch_bounds__(64, 12) rglru_walk_kernel(RglruArgs a, const float* __restrict__ gates, int tiles) {
+// The walk: PART of a tile's rows are in flight at a time, the first ones before anything else.  Eight leave room for twelve blocks an SM; sixteen
+// halve the trips to memory of launches that leave SMs idle (40 tokens of 1536 channels 9.5 us and 7.6, 600 12.0 and
+// 11.3).  Blocks behind the tiles, one a request, bring the
+// convolution's inputs up to date (in the walk it cost steps with many requests a trip to memory a row).
+template <typename E, int V, int PART>
+__global__ void __launch_bounds__(64, PART == 8 ? 12 : 6) rglru_walk_kernel(RglruArgs a, const float* __restrict__ gates, int tiles) {
   pdl_launch_dependents();
   pdl_wait();
   __shared__ int slot_s[RG_TILE], starts_s;                    // of each row; the row at which the first row's request begins
@@ -175,10 +177,10 @@ __global__ void __launch_bounds__(64, 12) rglru_walk_kernel(RglruArgs a, const f
   // addresses as a row's, the same for all threads, and a 32-bit column
   const int tile = blockIdx.x, t0 = tile * RG_TILE, n = min(RG_TILE, a.T - t0);
   const uint32_t cu = (uint32_t)c;
-  f2 av[RG_PART], bv[RG_PART], yv[RG_PART];
+  f2 av[PART], bv[PART], yv[PART];
   auto fetch = [&](int k0) {
 #pragma unroll
-    for (int k = 0; k < RG_PART; ++k) {
+    for (int k = 0; k < PART; ++k) {
       const int64_t r = (int64_t)(t0 + min(k0 + k, n - 1)) * ld;
       av[k] = rg_load<V>(gates + r + cu);
       bv[k] = rg_load<V>(gates + r + a.width + cu);
@@ -217,25 +219,25 @@ __global__ void __launch_bounds__(64, 12) rglru_walk_kernel(RglruArgs a, const f
   }
   const bool whole = n == RG_TILE && starts_s < t0 && (ends & 0x7fffffffu) == 0;      // no request begins in the tile
 #pragma unroll 1
-  for (int k0 = 0; k0 < n; k0 += RG_PART) {
+  for (int k0 = 0; k0 < n; k0 += PART) {
     E* out = (E*)a.out + (int64_t)(t0 + k0) * a.width;
     if (whole) {
 #pragma unroll
-      for (int k = 0; k < RG_PART; ++k) {
+      for (int k = 0; k < PART; ++k) {
         S = fma2(av[k], S, bv[k]);
         rg_store<V>(out + (int64_t)k * a.width + cu, mul2(S, gelu_tanh2(yv[k])));
       }
-      if (k0 + RG_PART == RG_TILE && ends) rg_keep<V>(a.state + (int64_t)slot_s[RG_TILE - 1] * a.slot_stride + c, S);
+      if (k0 + PART == RG_TILE && ends) rg_keep<V>(a.state + (int64_t)slot_s[RG_TILE - 1] * a.slot_stride + c, S);
     } else {
 #pragma unroll
-      for (int k = 0; k < RG_PART; ++k) {
+      for (int k = 0; k < PART; ++k) {
         f2 none = pk1(0.f);
         rg_compose2(none, S, av[k], bv[k]);
         if (k0 + k < n) rg_store<V>(out + (int64_t)k * a.width + cu, mul2(S, gelu_tanh2(yv[k])));
         if (ends >> (k0 + k) & 1) rg_keep<V>(a.state + (int64_t)slot_s[k0 + k] * a.slot_stride + c, S);
       }
     }
-    if (k0 + RG_PART < n) fetch(k0 + RG_PART);
+    if (k0 + PART < n) fetch(k0 + PART);
   }
 }
 
@@ -653,7 +655,9 @@ template <typename E, int V>
 static int rg_by_channel(const RglruArgs& a, bool walk, cudaStream_t st) {
   const dim3 grid((a.T + RG_TILE - 1) / RG_TILE, (a.width + 32 * V - 1) / (32 * V));
   KGE_REQUIRE(grid.y <= 65535 && a.tiles, "rglru: width %d", a.width);
-  if (walk) KGE_CUDA_OK(launch_pdl(rglru_walk_kernel<E, V>, dim3(grid.x + a.B, (a.width + 64 * V - 1) / (64 * V)), dim3(64), 0, st, a, a.gates, (int)grid.x));
+  const dim3 wgrid(grid.x + a.B, (a.width + 64 * V - 1) / (64 * V));
+  auto walker = V == 2 && (int64_t)wgrid.x * wgrid.y <= 6 * 148 ? rglru_walk_kernel<E, V, V == 2 ? 16 : 8> : rglru_walk_kernel<E, V, 8>;
+  if (walk) KGE_CUDA_OK(launch_pdl(walker, wgrid, dim3(64), 0, st, a, a.gates, (int)grid.x));
   else KGE_CUDA_OK(launch_pdl(rglru_ab_kernel<E, V>, grid, dim3(RB_WARPS * 32), 0, st, a, const_cast<float*>(a.gates)));
   return 0;
 }
