@@ -8,8 +8,9 @@
 //           A threshold below the counted keys is looked for in the next 8192 (wide spreads in float16; never seen otherwise);
 //   draw    the Gumbel-max form the reference uses, argmax(p_i / q_i) with q ~ Exp(1), over the kept set: each warp lists its kept
 //           elements first and shares them out; q = -log u >= 1 - u tells without the logarithm that most cannot win.
-// What bounds it: instruction issue of Philox (ten rounds per kept element) for flat rows, the chain of five cluster exchanges (1 to
-// 2 us each) for the others; the one read of V * 2 bytes is about 2 us.
+// What bounds it: instruction issue of Philox (ten rounds per kept element) for flat rows, the chain of cluster barriers for the others (about
+// 1 us each: the start's and the last exchange's for greedy rows, a third for the maximum where a token is drawn, three more for a threshold,
+// two for a second one that finds its keys counted); the one read of V * 2 bytes is about 2 us.
 // 32 rows x 128256 normal logits (spread 2.5) on a B200, us, before (intervals of keys cut in eight or four by a pass over the elements
 // and a cluster exchange each, 6 to 12 of them; every kept element's logarithm) and now: greedy 6.8 / 5.9, top-k 20 with top-p 0.8
 // 42.1 / 22.4, top-p 0.95 59.3 / 25.4, unfiltered 36.4 / 32.2, those in turn 51.2 / 23.9; one row of 32000, top-p 19.3 / 11.8; 150
@@ -178,9 +179,73 @@ sample_kernel(int32_t* __restrict__ out, const bf16* __restrict__ logits, int V,
   const bool aligned = (reinterpret_cast<uintptr_t>(row) & 15) == 0;
   const float temp = temperature ? temperature[b] : 0.f;
   const bool greedy = temp < 1e-5f;
-  const float inv_t = greedy ? 1.f : 1.f / temp;
+  const float inv_t = 1.f / temp;
   const int pieces = (V + 7) / 8, stride = nc * kSampleThreads, first = rank * kSampleThreads + tid;
   int phase = 0;
+
+  // Greedy rows, by themselves: the first element of the largest key, NaN left out, the two zeros equal.  What counts for few logits is the
+  // instructions, and that they lie together (in one path with the draw a row of 1000 took 2.98 us, of 4695 3.45; 2.35 and 2.75 so).
+  if (greedy) {
+    int key = 0, piece = 0x7fffffff, n = tid;
+#pragma unroll 1
+    for (int v8 = first; v8 < pieces; v8 += 4 * stride, n += 4 * kSampleThreads) {
+      uint4 a[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) if (v8 + j * stride < pieces) a[j] = load_keys(row, v8 + j * stride, V, aligned);
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (v8 + j * stride < pieces) {
+          const uint32_t two = __vmaxu2(__vmaxu2(a[j].x, a[j].y), __vmaxu2(a[j].z, a[j].w));
+          int k = (int)max(two & 0xffffu, two >> 16);
+          if (k > (int)kTop) {                                 // a NaN among the eight
+            const uint32_t w[4] = {a[j].x, a[j].y, a[j].z, a[j].w};
+            k = 0;
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+              const int x = (int)((e & 1) ? w[e / 2] >> 16 : w[e / 2] & 0xffffu);
+              if (x <= (int)kTop) k = max(k, x);
+            }
+          }
+          if (k == 0x7fff) k = 0x8000;
+          if (k > key) { key = k; piece = v8 + j * stride; }
+          if constexpr (STAGED) held[n + j * kSampleThreads] = a[j];
+        }
+    }
+    auto first_of_largest = [&](int& k, int& at) {
+      const int best = __reduce_max_sync(0xffffffffu, k);
+      at = __reduce_min_sync(0xffffffffu, k == best ? at : 0x7fffffff);
+      k = best;
+    };
+    first_of_largest(key, piece);
+    if (lane == 0) { sh.warp[0][wid] = (uint32_t)key; sh.warp[1][wid] = (uint32_t)piece; }
+    cluster_wait();                                            // the peers run: their shared memory may be written
+    __syncthreads();
+    if (wid == 0) {
+      key = (int)sh.warp[0][lane % kSampleWarps];
+      piece = (int)sh.warp[1][lane % kSampleWarps];
+      first_of_largest(key, piece);
+      int at = 0x7fffffff;
+      if (key > 0) {                                           // which of the piece's eight
+        uint32_t x = 0;
+        const int i = piece * 8 + (lane & 7);
+        if constexpr (STAGED) x = reinterpret_cast<const unsigned short*>(held + (piece & (kSampleThreads - 1)) + piece / stride * kSampleThreads)[lane & 7];
+        else if (i < V) x = pack_keys(*reinterpret_cast<const unsigned short*>(row + i)) & 0xffffu;
+        at = __reduce_min_sync(0xffffffffu, (int)x == key || (x == 0x7fffu && key == 0x8000) ? i : 0x7fffffff);
+      }
+      if (lane == 0) {
+        st_cluster(&sh.all[0][rank][0], 0, (uint32_t)key);
+        st_cluster(&sh.all[0][rank][1], 0, (uint32_t)at);
+      }
+    }
+    cluster_arrive(); cluster_wait();
+    if (rank == 0 && wid == 0) {
+      key = lane < nc ? (int)sh.all[0][lane & (kMaxCluster - 1)][0] : 0;
+      int at = lane < nc ? (int)sh.all[0][lane & (kMaxCluster - 1)][1] : 0x7fffffff;
+      first_of_largest(key, at);
+      if (lane == 0) out[b] = at == 0x7fffffff ? 0 : at;
+    }
+    return;
+  }
 
   // this thread's largest key, with NaN: of even and odd elements side by side
   uint32_t both = 0;
@@ -232,213 +297,190 @@ sample_kernel(int32_t* __restrict__ out, const bf16* __restrict__ logits, int V,
   uint32_t low = 0, from = 0;                                  // the kept keys, and those of them that are drawn from
   auto weight = [&](uint32_t key) { return expf(__fmul_rn(key_value(key), inv_t) - m); };
   cluster_wait();                                              // the peers run: their shared memory may be written
-  if (greedy) {
-    if (top[0] == 0x7fff) top[0] = 0x8000;                     // the two zeros are equal values
-    // only warps that hold the block's largest look for its first element
-    const int widest = __reduce_max_sync(0xffffffffu, top[0]);
-    if (lane == 0) sh.warp[0][wid] = (uint32_t)widest;
-    __syncthreads();
-    const int largest = __reduce_max_sync(0xffffffffu, (int)sh.warp[0][lane % kSampleWarps]);
-    __syncthreads();
-    if (widest == largest && top[0] == largest && top[0]) {
-      int at = 0x7fffffff;
-      each8([&](uint4 a, int i) {
-        const uint32_t w[4] = {a.x, a.y, a.z, a.w};
-#pragma unroll
-        for (int e = 0; e < 8; ++e) {
-          int key = (int)((e & 1) ? w[e / 2] >> 16 : w[e / 2] & 0xffffu);
-          if (key == 0x7fff) key = 0x8000;
-          if (key == top[0]) at = min(at, i + e);
-        }
-      });
-      offer(key_value(top[0]), at);
-    }
-  } else {
-    cluster_reduce(top, sh, phase, MaxOp());
-    const uint32_t mk = (uint32_t)top[0];
-    m = mk ? key_value(mk) * inv_t : -INFINITY;    // max of x = logit / T: x grows with the key
-    uint32_t cut = 1;                                          // keys from here on are kept
-    auto lower_equal = [&]() {                                 // logits whose quotients are equal stay together
-      const uint32_t t = fkey(key_value(cut) * inv_t);
-      while (cut > 1 && fkey(key_value(cut - 1) * inv_t) >= t) --cut;
-    };
-    const int k = top_k ? top_k[b] : 0;
-    const float p = top_p ? top_p[b] : 1.f;
+  cluster_reduce(top, sh, phase, MaxOp());
+  const uint32_t mk = (uint32_t)top[0];
+  m = mk ? key_value(mk) * inv_t : -INFINITY;    // max of x = logit / T: x grows with the key
+  uint32_t cut = 1;                                          // keys from here on are kept
+  auto lower_equal = [&]() {                                 // logits whose quotients are equal stay together
+    const uint32_t t = fkey(key_value(cut) * inv_t);
+    while (cut > 1 && fkey(key_value(cut - 1) * inv_t) >= t) --cut;
+  };
+  const int k = top_k ? top_k[b] : 0;
+  const float p = top_p ? top_p[b] : 1.f;
 
-    // Counts of the bins [base, base + width) into `hist`; `tiny` is the weight of the shared bin and `rest` that of the bins below
-    // base, over the cluster, of keys from `low` on.  `raw`: bins are keys, inside the shared bin.
-    float rest = 0.f, tiny = 0.f;
-    auto count = [&](uint32_t base, uint32_t width, bool raw, uint32_t low, bool weights) {
-      for (int i = tid; i < kBins / 4; i += kSampleThreads) dyn[i] = make_uint4(0, 0, 0, 0);
+  // Counts of the bins [base, base + width) into `hist`; `tiny` is the weight of the shared bin and `rest` that of the bins below
+  // base, over the cluster, of keys from `low` on.  `raw`: bins are keys, inside the shared bin.
+  float rest = 0.f, tiny = 0.f;
+  auto count = [&](uint32_t base, uint32_t width, bool raw, uint32_t low, bool weights) {
+    for (int i = tid; i < kBins / 4; i += kSampleThreads) dyn[i] = make_uint4(0, 0, 0, 0);
+    __syncthreads();
+    float s[2] = {0.f, 0.f};
+    uint32_t small = 0;                                      // elements of the shared bin: counted here, there may be many
+    each8([&](uint4 a, int) {
+      const uint32_t w[4] = {a.x, a.y, a.z, a.w};
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        const uint32_t key = (e & 1) ? w[e / 2] >> 16 : w[e / 2] & 0xffffu, c = raw ? key : bin_of(key);
+        const bool shared = !raw && c == kTiny;
+        if (c - base < width && !shared) atomicAdd(hist + slot_of(c - base), 1u);
+        if (shared || c < base) {
+          small += shared;
+          if (weights && key >= low) {
+            const float x = weight(key);
+            s[0] += c < base ? x : 0.f;
+            s[1] += shared ? x : 0.f;
+          }
+        }
+      }
+    });
+    if (!raw && kTiny - base < width && small) atomicAdd(hist + slot_of(kTiny - base), small);
+    cluster_reduce(s, sh, phase, AddOp());                   // the counters are complete behind it
+    rest = s[0];
+    tiny = s[1];
+    // Each CTA adds up a slice, a thread `per` bins in a row.  Nobody else reads that slice of this CTA's counters.
+    const int per = kBins / stride;
+    const uint32_t mine = (uint32_t)__cvta_generic_to_shared(hist);
+    for (int j = 0; j < per && nc > 1; j += 2) {
+      const uint32_t at = slot_of((uint32_t)(first * per + j));
+      uint32_t x = 0, y = 0;
+#pragma unroll
+      for (int r = 0; r < kMaxCluster; ++r)
+        if (r < nc) {
+          const uint2 v = ld_cluster_v2(mapa_u32(mine + at * 4, (uint32_t)r));
+          x += v.x;
+          y += v.y;
+        }
+      hist[at] = x;
+      hist[at + 1] = y;
+    }
+  };
+  // The first bin whose sum from below exceeds want(sum of all slices), by value(bin, count): the same everywhere.  kBins: it lies
+  // below the counted ones; kBins + 1: there is none.  `upto` is the sum up to and with the bin.
+  auto find = [&](auto value, auto want_of, auto& upto) -> uint32_t {
+    using T = typename std::remove_reference<decltype(upto)>::type;
+    const int per = kBins / stride;
+    T sum = 0;
+    for (int j = 0; j < per; ++j) sum += value((uint32_t)(first * per + j), hist[slot_of((uint32_t)(first * per + j))]);
+    T incl = sum;                                            // over the threads of the warp
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const T v = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += v;
+    }
+    T start = __shfl_up_sync(0xffffffffu, incl, 1);
+    if (lane == 0) start = 0;
+    T* warp = reinterpret_cast<T*>(sh.warp[0]);
+    if (lane == 31) warp[wid] = incl;
+    if (tid == 0) sh.last = 0;
+    __syncthreads();
+    T before = 0, all = 0;
+    for (int w = 0; w < kSampleWarps; ++w) {
+      if (w == wid) before = all;
+      all += warp[w];
+    }
+    if (tid < nc) st_cluster(&sh.all[phase & 1][rank][0], (uint32_t)tid, *reinterpret_cast<uint32_t*>(&all));
+    cluster_arrive(); cluster_wait();
+    T total = 0, below = 0;
+    for (int r = 0; r < nc; ++r) total += *reinterpret_cast<T*>(&sh.all[phase & 1][r][0]);
+    const T want = want_of(total);
+    total = 0;
+    int owner = -1;
+    for (int r = 0; r < nc; ++r) {
+      const T next = total + *reinterpret_cast<T*>(&sh.all[phase & 1][r][0]);
+      if (owner < 0 && next > want) { owner = r; below = total; }
+      total = next;
+    }
+    ++phase;
+    if (want < 0) return kBins;
+    if (owner < 0) return kBins + 1;
+    if (owner == rank) {
+      // the last thread that starts at or below `want` and adds something: sums of fp32 differ by their order, so no thread's
+      // end is compared with the next one's start
+      start = below + (before + start);
+      if (sum > 0 && start <= want) atomicMax(&sh.last, (uint32_t)tid);
       __syncthreads();
-      float s[2] = {0.f, 0.f};
-      uint32_t small = 0;                                      // elements of the shared bin: counted here, there may be many
-      each8([&](uint4 a, int) {
-        const uint32_t w[4] = {a.x, a.y, a.z, a.w};
-#pragma unroll
-        for (int e = 0; e < 8; ++e) {
-          const uint32_t key = (e & 1) ? w[e / 2] >> 16 : w[e / 2] & 0xffffu, c = raw ? key : bin_of(key);
-          const bool shared = !raw && c == kTiny;
-          if (c - base < width && !shared) atomicAdd(hist + slot_of(c - base), 1u);
-          if (shared || c < base) {
-            small += shared;
-            if (weights && key >= low) {
-              const float x = weight(key);
-              s[0] += c < base ? x : 0.f;
-              s[1] += shared ? x : 0.f;
-            }
+      if (tid == (int)sh.last) {
+        T run = start;
+        uint32_t at = kBins + 1;
+        for (int j = 0; j < per && !(run > want); ++j)
+          if (const uint32_t n = hist[slot_of((uint32_t)(first * per + j))]) {
+            at = (uint32_t)(first * per + j);
+            run += value(at, n);
           }
-        }
-      });
-      if (!raw && kTiny - base < width && small) atomicAdd(hist + slot_of(kTiny - base), small);
-      cluster_reduce(s, sh, phase, AddOp());                   // the counters are complete behind it
-      rest = s[0];
-      tiny = s[1];
-      // Each CTA adds up a slice, a thread `per` bins in a row.  Nobody else reads that slice of this CTA's counters.
-      const int per = kBins / stride;
-      const uint32_t mine = (uint32_t)__cvta_generic_to_shared(hist);
-      for (int j = 0; j < per && nc > 1; j += 2) {
-        const uint32_t at = slot_of((uint32_t)(first * per + j));
-        uint32_t x = 0, y = 0;
-#pragma unroll
-        for (int r = 0; r < kMaxCluster; ++r)
-          if (r < nc) {
-            const uint2 v = ld_cluster_v2(mapa_u32(mine + at * 4, (uint32_t)r));
-            x += v.x;
-            y += v.y;
-          }
-        hist[at] = x;
-        hist[at + 1] = y;
-      }
-    };
-    // The first bin whose sum from below exceeds want(sum of all slices), by value(bin, count): the same everywhere.  kBins: it lies
-    // below the counted ones; kBins + 1: there is none.  `upto` is the sum up to and with the bin.
-    auto find = [&](auto value, auto want_of, auto& upto) -> uint32_t {
-      using T = typename std::remove_reference<decltype(upto)>::type;
-      const int per = kBins / stride;
-      T sum = 0;
-      for (int j = 0; j < per; ++j) sum += value((uint32_t)(first * per + j), hist[slot_of((uint32_t)(first * per + j))]);
-      T incl = sum;                                            // over the threads of the warp
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const T v = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += v;
-      }
-      T start = __shfl_up_sync(0xffffffffu, incl, 1);
-      if (lane == 0) start = 0;
-      T* warp = reinterpret_cast<T*>(sh.warp[0]);
-      if (lane == 31) warp[wid] = incl;
-      if (tid == 0) sh.last = 0;
-      __syncthreads();
-      T before = 0, all = 0;
-      for (int w = 0; w < kSampleWarps; ++w) {
-        if (w == wid) before = all;
-        all += warp[w];
-      }
-      if (tid < nc) st_cluster(&sh.all[phase & 1][rank][0], (uint32_t)tid, *reinterpret_cast<uint32_t*>(&all));
-      cluster_arrive(); cluster_wait();
-      T total = 0, below = 0;
-      for (int r = 0; r < nc; ++r) total += *reinterpret_cast<T*>(&sh.all[phase & 1][r][0]);
-      const T want = want_of(total);
-      total = 0;
-      int owner = -1;
-      for (int r = 0; r < nc; ++r) {
-        const T next = total + *reinterpret_cast<T*>(&sh.all[phase & 1][r][0]);
-        if (owner < 0 && next > want) { owner = r; below = total; }
-        total = next;
-      }
-      ++phase;
-      if (want < 0) return kBins;
-      if (owner < 0) return kBins + 1;
-      if (owner == rank) {
-        // the last thread that starts at or below `want` and adds something: sums of fp32 differ by their order, so no thread's
-        // end is compared with the next one's start
-        start = below + (before + start);
-        if (sum > 0 && start <= want) atomicMax(&sh.last, (uint32_t)tid);
-        __syncthreads();
-        if (tid == (int)sh.last) {
-          T run = start;
-          uint32_t at = kBins + 1;
-          for (int j = 0; j < per && !(run > want); ++j)
-            if (const uint32_t n = hist[slot_of((uint32_t)(first * per + j))]) {
-              at = (uint32_t)(first * per + j);
-              run += value(at, n);
-            }
-          for (int r = 0; r < nc; ++r) {
-            st_cluster(&sh.found[0], (uint32_t)r, at);
-            st_cluster(&sh.found[1], (uint32_t)r, *reinterpret_cast<uint32_t*>(&run));
-          }
+        for (int r = 0; r < nc; ++r) {
+          st_cluster(&sh.found[0], (uint32_t)r, at);
+          st_cluster(&sh.found[1], (uint32_t)r, *reinterpret_cast<uint32_t*>(&run));
         }
       }
-      cluster_arrive(); cluster_wait();
-      upto = *reinterpret_cast<T*>(&sh.found[1]);
-      return sh.found[0];
-    };
-    // mass: the smallest key whose weight from below exceeds (1 - p) of all, of the keys from `low` on; else the k-th largest key.
-    // counted: the counters hold the first bins already, and `low` lies among them, above the shared one.
-    auto search = [&](int mass, uint32_t largest, uint32_t low, bool counted) -> uint32_t {
-      uint32_t hi = bin_of(largest) + 1, lowest = 1;
-      bool raw = false;
-      int above = 0, ends = 0;
-      float goal = -1.f;
-      for (;;) {
-        const uint32_t base = hi - lowest > kBins ? hi - kBins : lowest;
-        if (!counted) count(base, hi - base, raw, low, mass); else rest = tiny = 0.f;
-        counted = false;
-        uint32_t at;
-        int all = 0;
-        if (mass) {
-          float upto;
-          at = find([&](uint32_t i, uint32_t n) -> float {
-            const uint32_t c = base + i, key = raw || c <= kNeg ? c : c + kGap;
-            if (n == 0) return 0.f;
-            if (!raw && c == kTiny) return tiny;
-            return key >= low ? (float)n * weight(key) : 0.f;
-          }, [&](float total) {
-            if (goal == -1.f) goal = (1.f - p) * (rest + total);
-            return goal - rest;
-          }, upto);
-        } else {
-          at = find([](uint32_t, uint32_t n) { return (int)n; }, [&](int total) { all = total; return above + total - k; }, ends);
-        }
-        if (at == kBins + 1) return largest;
-        if (at == kBins) {
-          if (base == lowest) return lowest;                   // by rounding only
-          above += all;
-          hi = base;
-          continue;
-        }
-        at += base;
-        if (raw || at != kTiny) return raw || at <= kNeg ? at : at + kGap;
-        above += all - ends;
-        raw = true;
-        hi = kPos;
-        lowest = kTiny;
+    }
+    cluster_arrive(); cluster_wait();
+    upto = *reinterpret_cast<T*>(&sh.found[1]);
+    return sh.found[0];
+  };
+  // mass: the smallest key whose weight from below exceeds (1 - p) of all, of the keys from `low` on; else the k-th largest key.
+  // counted: the counters hold the first bins already, and `low` lies among them, above the shared one.
+  auto search = [&](int mass, uint32_t largest, uint32_t low, bool counted) -> uint32_t {
+    uint32_t hi = bin_of(largest) + 1, lowest = 1;
+    bool raw = false;
+    int above = 0, ends = 0;
+    float goal = -1.f;
+    for (;;) {
+      const uint32_t base = hi - lowest > kBins ? hi - kBins : lowest;
+      if (!counted) count(base, hi - base, raw, low, mass); else rest = tiny = 0.f;
+      counted = false;
+      uint32_t at;
+      int all = 0;
+      if (mass) {
+        float upto;
+        at = find([&](uint32_t i, uint32_t n) -> float {
+          const uint32_t c = base + i, key = raw || c <= kNeg ? c : c + kGap;
+          if (n == 0) return 0.f;
+          if (!raw && c == kTiny) return tiny;
+          return key >= low ? (float)n * weight(key) : 0.f;
+        }, [&](float total) {
+          if (goal == -1.f) goal = (1.f - p) * (rest + total);
+          return goal - rest;
+        }, upto);
+      } else {
+        at = find([](uint32_t, uint32_t n) { return (int)n; }, [&](int total) { all = total; return above + total - k; }, ends);
       }
-    };
-    bool counted = false;
+      if (at == kBins + 1) return largest;
+      if (at == kBins) {
+        if (base == lowest) return lowest;                   // by rounding only
+        above += all;
+        hi = base;
+        continue;
+      }
+      at += base;
+      if (raw || at != kTiny) return raw || at <= kNeg ? at : at + kGap;
+      above += all - ends;
+      raw = true;
+      hi = kPos;
+      lowest = kTiny;
+    }
+  };
+  bool counted = false;
 #pragma unroll 1
-    for (int mass = 0; mass < 2; ++mass) {
-      if (mass ? !(p < 1.f) : !(k > 0 && k < V)) continue;
-      if (mass && top[1] > (int)kTop) { cut = max(cut, mk); continue; }       // a NaN leaves the largest logit alone
-      const uint32_t key = search(mass, (uint32_t)(mass ? mk : top[1]), cut, counted);
-      const uint32_t hi = bin_of((uint32_t)top[1]) + 1, at = bin_of(key);
-      cut = max(cut, key);
-      lower_equal();
-      // whether the counters are the first ones still, and what the threshold of the mass needs is in them
-      counted = at > kTiny && at + kBins >= hi && bin_of(cut) > kTiny && bin_of(cut) + kBins >= hi;
-    }
-    // argmax of exp(x - max) / q over the kept set; the maximum is always kept
-    cut = min(cut, max(mk, 1u));
-    // The largest score is W / Exp(1), W >= 1 the kept weights' sum: below `floor` with a probability of e^-16.7, and then the draw
-    // is repeated without it.  What cannot reach it, or the best score of the warp so far, is left out before its logarithm.
-    floor = 0.06f;
-    low = from = cut;
-    if (exp_noise) floor = 0.f;
-    else {
-      const float v = (m - 19.6f) * temp;                      // q >= 2^-24.1: a weight below e^-19.45 cannot reach 0.06
-      if (fabsf(v) < 3e4f && fabsf(m) < 1e5f) from = min(max(cut, value_key(v) - 1), max(mk, 1u));
-    }
+  for (int mass = 0; mass < 2; ++mass) {
+    if (mass ? !(p < 1.f) : !(k > 0 && k < V)) continue;
+    if (mass && top[1] > (int)kTop) { cut = max(cut, mk); continue; }       // a NaN leaves the largest logit alone
+    const uint32_t key = search(mass, (uint32_t)(mass ? mk : top[1]), cut, counted);
+    const uint32_t hi = bin_of((uint32_t)top[1]) + 1, at = bin_of(key);
+    cut = max(cut, key);
+    lower_equal();
+    // whether the counters are the first ones still, and what the threshold of the mass needs is in them
+    counted = at > kTiny && at + kBins >= hi && bin_of(cut) > kTiny && bin_of(cut) + kBins >= hi;
+  }
+  // argmax of exp(x - max) / q over the kept set; the maximum is always kept
+  cut = min(cut, max(mk, 1u));
+  // The largest score is W / Exp(1), W >= 1 the kept weights' sum: below `floor` with a probability of e^-16.7, and then the draw
+  // is repeated without it.  What cannot reach it, or the best score of the warp so far, is left out before its logarithm.
+  floor = 0.06f;
+  low = from = cut;
+  if (exp_noise) floor = 0.f;
+  else {
+    const float v = (m - 19.6f) * temp;                      // q >= 2^-24.1: a weight below e^-19.45 cannot reach 0.06
+    if (fabsf(v) < 3e4f && fabsf(m) < 1e5f) from = min(max(cut, value_key(v) - 1), max(mk, 1u));
   }
   const uint64_t seed = seeds ? seeds[b] : 0;
   uint16_t* list = reinterpret_cast<uint16_t*>(hist) + wid * 1024;
@@ -525,7 +567,7 @@ sample_kernel(int32_t* __restrict__ out, const bf16* __restrict__ logits, int V,
   };
 #pragma unroll 1
   for (;;) {
-    if (!greedy) draw();
+    draw();
     // the best of the cluster, of equal ones the first: known to every CTA
     warp_best();
     if (lane == 0) { sh.warp[0][wid] = __float_as_uint(best); sh.warp[1][wid] = (uint32_t)bi; }
@@ -540,7 +582,6 @@ sample_kernel(int32_t* __restrict__ out, const bf16* __restrict__ logits, int V,
       }
     }
     cluster_arrive(); cluster_wait();
-    if (greedy && wid != 0) break;
     best = lane < nc ? __uint_as_float(sh.all[phase & 1][lane & (kMaxCluster - 1)][0]) : -INFINITY;
     bi = lane < nc ? (int)sh.all[phase & 1][lane & (kMaxCluster - 1)][1] : 0x7fffffff;
     warp_best();
