@@ -214,9 +214,13 @@ __global__ void __launch_bounds__(1024) moe_group_kernel(MoeRouteArgs a) {
 }
 
 // Decode steps of a few tokens: scores, choice and grouping in one launch of one block.  A warp has a row of the router at a time, the
-// first one asked for before the kernel before has ended: what this costs is latency.  Same order of summation as dot_part.  16 experts of
-// 2048, top 2, us back to back (with cold caches), in two launches and here: 1 token 7.2 (18.5) and 4.2 (10.3), 2 tokens 7.3 (16.4) and
-// 5.1 (12.3), 4 tokens 7.4 (16.4) and 6.8 (12.3); 8 tokens 7.5 and 10.4: one block's arithmetic, so they stay with a block a token.
+// first one asked for before the kernel before has ended: what this costs is latency.  Same order of summation as dot_part.  Top 2 of 16 experts
+// of 2048 (bfloat16), us back to back (with cold caches), in two launches and here: 1 token 7.2 (18.5) and 4.2 (10.3), 2 tokens 7.3 (16.4) and
+// 5.1 (12.3), 4 tokens 7.4 (16.4) and 6.8 (12.3); 8 tokens 7.5 and 10.4: one block's arithmetic, so they stay with a block a token.  Top 8 of
+// 128 experts, 4 tokens: 1024 wide 26.6 (43.3) and 30.2 (31.7), 2048 wide 34.7 (64.5) and 36.1 (39.4): behind with warm weights, but a decode
+// step's are cold (six such layers 1024 wide, 1 to 4 tokens: 474, 571, 578, 590 us a step and 319, 445, 483, 531; 8 experts level to 7 us
+// less).  Rows of less than 2 KB have no such trip to save: 256 wide, 128 experts, 4 tokens 17.5 (20.7) and 25.7 (26.5), 2 tokens 17.3 (22.0) and
+// 18.5 (20.1), 32 experts, 4 tokens 7.5 (8.0) and 9.0 (9.0), so they come here one at a time, or two with up to 32 experts.
 constexpr int MF_WARPS = 16, MF_TOKENS = 4, MF_AHEAD = 8;
 template <typename E>
 __global__ void __launch_bounds__(MF_WARPS * 32) moe_few_kernel(MoeRouteArgs a, int per) {
@@ -336,7 +340,8 @@ int moe_route(const MoeRouteArgs& a, cudaStream_t st) {
   cudaError_t ce;
   const int row = 16 / (a.elt == KGE_ELT_F32 ? 4 : 2);
   const size_t few = (size_t)a.T * a.d * (16 / row) + smem * a.T + (size_t)2 * a.E * 4;
-  if (!a.logits && a.T <= MF_TOKENS && a.E <= 128 && few <= 48 * 1024 && a.d % row == 0 && a.ldh % row == 0 &&
+  const bool by_one_block = a.T == 1 || (a.T == 2 && a.E <= 32) || (a.T <= MF_TOKENS && a.d * (16 / row) >= 2048);
+  if (!a.logits && by_one_block && a.E <= 128 && few <= 48 * 1024 && a.d % row == 0 && a.ldh % row == 0 &&
       ((reinterpret_cast<uintptr_t>(a.h) | reinterpret_cast<uintptr_t>(a.w_router) | reinterpret_cast<uintptr_t>(a.w_extra)) & 15) == 0) {
     if (a.elt == KGE_ELT_F32) KGE_CUDA_OK(launch_pdl(moe_few_kernel<float>, dim3(1), dim3(MF_WARPS * 32), few, st, a, per));
     else KGE_CUDA_OK(launch_pdl(moe_few_kernel<__nv_bfloat16>, dim3(1), dim3(MF_WARPS * 32), few, st, a, per));
