@@ -138,6 +138,22 @@ def test_matrix_memory_token_by_token(kge, tmp_path, heads, dim, vdim, requests,
 
 
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+@pytest.mark.parametrize("heads,dim,vdim,requests", [(8, 16, 256, 32), (8, 16, 256, 33), (4, 48, 136, 110), (8, 96, 256, 33)])
+def test_matrix_memory_of_many_requests(kge, tmp_path, heads, dim, vdim, requests, dtype):
+    """Decode steps on either side of the line between one launch and three (2048 blocks of less than 96 key dimensions)."""
+    cfg = oh.make_config(layers=("parallel",), mlps=(None,), left_scale=0.0, m_heads=heads, m_dim=dim, m_vdim=vdim)
+    W = oh.make_weights(cfg, seed=47)
+    toks = prompt(cfg, 6)
+    want = oh.forward(cfg, W, toks)
+    llm = make_engine(kge, tmp_path, cfg, W, dtype, tokens=16 * requests, seqs=requests)
+    for t in range(6):
+        for r in range(requests):
+            llm.trace_add(r, [toks[t]])
+        check(llm.trace_step([(r, 1, [0]) for r in range(requests)]), want[[t] * requests], dtype, f"step {t}")
+    llm.close()
+
+
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 @pytest.mark.parametrize("experts,top,width", [(16, 2, 512), (17, 4, 2056), (33, 3, 40), (128, 5, 136), (129, 2, 136)])
 def test_routing_of_a_few_tokens(kge, tmp_path, experts, top, width, dtype):
     """Scores, choice and grouping in one launch: one row a warp, several, the last count of experts it takes and the first it does not, rows
@@ -169,6 +185,8 @@ def test_short_biased_pieces(kge, tmp_path, hd):
     (2, 48, 72, [1, 130, 1, 64, 321]),                              # requests of one token and of one chunk beside longer ones
     (3, 16, 256, [200, 90]),
     (5, 128, 256, [150, 70, 10, 3]),                                # no room for a second block
+    (4, 128, 256, [300, 20]),                                       # norm and gate by a warp a row, a piece a lane
+    (4, 16, 128, [200, 200, 200]),                                  # 48 clusters: of two, since 45 of three fit
     (2, 128, 264, [700, 2]), (2, 4, 520, [650]), (9, 32, 40, [135]),      # (other sums; norm and gate by a warp a row: two and four pieces a lane, less than one)
 ])
 def test_matrix_memory_prompts_in_runs_of_chunks(kge, tmp_path, heads, dim, vdim, lens):

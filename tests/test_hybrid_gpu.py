@@ -493,3 +493,20 @@ def test_last_layer_of_the_asked_rows(kge, tmp_path, design):
     llm.trace_add(1, toks[:40]); llm.trace_add(2, toks[:33]); llm.trace_add(3, toks[:1])
     check(llm.trace_step([(3, 1, [0]), (1, 40, []), (2, 33, [5, 32])]), want[[0, 5, 32]], "float32", "three requests")
     llm.close()
+
+
+@pytest.mark.parametrize("dtype,mlp,width,n,places", [
+    ("float32", None, 2048, 511, [0, 510]), ("bfloat16", None, 2048, 512, [0, 511]),      # without a feed-forward: the last step before 2^20 numbers, and the first
+    ("bfloat16", "dense", 64, 16, [15]), ("bfloat16", "dense", 64, 17, [0, 16]),          # the first step that is worth the copy
+    ("float32", "dense", 640, 409, range(0, 408, 4)), ("bfloat16", "dense", 640, 412, range(1, 412, 4)),      # many rows: from 2^18 numbers on; more than 48 KB of shared memory
+    ("float32", "moe", 98, 400, range(3, 400, 4)), ("float32", "moe", 96, 1024, range(0, 1024, 4)),           # rows that are no multiple of 16 bytes; the most rows there are
+    ("bfloat16", "moe", 512, 5, [4]), ("bfloat16", "moe", 512, 4, [1])])
+def test_last_layer_of_asked_rows_where_it_pays(kge, tmp_path, dtype, mlp, width, n, places):
+    """Steps on either side of the lines for the copy of the asked rows, and the copy's own edges."""
+    cfg = oh.make_config(width=width, layers=("rglru",), mlps=(mlp,), ff=48, expert_ff=16, shared_ff=16)
+    W = oh.make_weights(cfg, seed=37)
+    toks = prompt(cfg, n, 38)
+    llm = make_engine(kge, tmp_path, cfg, W, dtype, tokens=1024, seqs=2)
+    llm.trace_add(0, toks)
+    check(llm.trace_step([(0, n, list(places))]), oh.forward(cfg, W, toks)[list(places)], dtype)
+    llm.close()
