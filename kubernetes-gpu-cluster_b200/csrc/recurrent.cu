@@ -10,6 +10,7 @@
 
 #include "common.cuh"
 #include "elt_access.cuh"
+#include "gate_math.cuh"
 #include "hybrid_ops.h"
 
 namespace kge {
@@ -128,7 +129,6 @@ int rglru_conv(const RglruArgs& a, cudaStream_t st) {
 }
 
 __device__ __forceinline__ float sigmoidf_(float v) { return 1.f / (1.f + expf(-v)); }
-__device__ __forceinline__ float softplusf_(float v) { return v > 20.f ? v : log1pf(expf(v)); }
 __device__ __forceinline__ float gelu_tanhf_(float v) { return 0.5f * v * (1.f + tanhf(0.79788456080286536f * (v + 0.044715f * v * v * v))); }
 
 template <typename E>

@@ -3,14 +3,15 @@
 // composition (A, B); a second one applies the compositions of the tiles before its own (a fma each) and walks its 32 tokens.
 // A request's first row starts from the slot's state: its b takes a S_slot in, and its a becomes RESET, which drops what comes from
 // the rows before it (another request's, which may be infinite, so no product with zero).
-//   rglru_gates_kernel  bfloat16, block-diagonal gates in steps of 16: convolution, both gate projections on mma.sync and the coefficients
-//                       from one read of x; u never leaves shared memory.  STEP: decode steps, one row a request, to the outputs.
-//   rglru_ab_kernel     any sizes, and float32: coefficients from gate pre-activations
-//   rglru_walk_kernel   the walk, times gelu(y); leaves the new state
+//   rglru_gates_kernel  prompt steps, bfloat16, diagonal blocks of 32, 64, 128 or 160 channels: convolution, both gate projections on tcgen05 and
+//                       the coefficients from one read of x; u never leaves shared memory
+//   rglru_ab_kernel     prompt steps of any other sizes, and float32: coefficients from gate pre-activations
+//   rglru_walk_kernel   the walk behind either, times gelu(y); leaves the new state
+//   rglru_step_kernel   decode steps, bfloat16, one row a request: from x to the outputs, products on mma.sync (a block has 16 rows)
 // Two prompts of 1156 tokens, width 2560 in 16 blocks, us back to back: convolution 14, gates 2 x 22, coefficients 31, a chain of one
-// warp per 32 channels 37 and outputs 15 before, 142 in all; 33 + 15 now, 54 in all (4 x 2048: 383 and 173; 200 tokens beside 64 single ones: 70 and 25).
-// Decode steps of 2, 64 and 200 requests: 11.6, 29.9 and 37.4 in four launches, 5.1, 15.9 and 32.5 in one.
-// What bounds them: the first, issue of exponentials and reciprocals and the latency of its stages; the walk, reading a and b (12 bytes a
+// warp per 32 channels 37 and outputs 15 before, 142 in all; 39 + 17 now, 60 in all (4 x 2048: 383 and 185).  Decode steps of 2, 64 and 200
+// requests: 11.6, 29.9 and 37.4 in four launches, 5.3, 16.0 and 32.7 in one.
+// What bounds them: the first, issue of the activations and the latency of its stages; the walk, reading a and b (12 bytes a
 // number with y) with half of the warps that would fit.
 #include <algorithm>
 
@@ -241,8 +242,8 @@ __global__ void __launch_bounds__(64, PART == 8 ? 12 : 6) rglru_walk_kernel(Rglr
   }
 }
 
-// Convolution, gates and coefficients.  A block has `cols` columns of one diagonal block and walks over its rows, the weights of both
-// gates in shared memory; a warp has eight columns of both gates, so r and i of a number meet in one thread.
+// The gate products of decode steps, on mma.sync: a block has 16 rows and `cols` columns of one diagonal block, the weights of both gates in
+// shared memory; a warp has eight columns of both gates, so r and i of a number meet in one thread.
 __device__ __forceinline__ void rg_mma(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
   asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
                : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
@@ -250,27 +251,20 @@ __device__ __forceinline__ void rg_mma(float (&c)[4], const uint32_t (&a)[4], ui
 __device__ __forceinline__ void rg_ldsm(uint32_t (&r)[4], const void* p) {
   asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"((uint32_t)__cvta_generic_to_shared(p)) : "memory");
 }
-// acc[gate][m] = 16 m.. rows of U x the warp's eight columns of W [gate][cols][bw]
-template <int MT>
-__device__ __forceinline__ void rg_products(float (&acc)[2][MT][4], const __nv_bfloat16* W, const __nv_bfloat16* U, int cols, int n0, int bw, int lane) {
+// acc[gate] = 16 rows of U x the warp's eight columns of W [gate][cols][bw]
+__device__ __forceinline__ void rg_products(float (&acc)[2][4], const __nv_bfloat16* W, const __nv_bfloat16* U, int cols, int n0, int bw, int lane) {
   const int ldw = bw + 8;                                      // rows 16 bytes apart in their banks
 #pragma unroll
-  for (int q = 0; q < 2; ++q)
-#pragma unroll
-    for (int m = 0; m < MT; ++m) acc[q][m][0] = acc[q][m][1] = acc[q][m][2] = acc[q][m][3] = 0.f;
+  for (int q = 0; q < 2; ++q) acc[q][0] = acc[q][1] = acc[q][2] = acc[q][3] = 0.f;
   const __nv_bfloat16* w = W + (int64_t)((lane >> 4) * cols + n0 + (lane & 7)) * ldw + ((lane >> 3) & 1) * 8;
   const __nv_bfloat16* u = U + (lane & 15) * ldw + (lane >> 4) * 8;
 #pragma unroll 2
   for (int k = 0; k < bw; k += 16) {
-    uint32_t bf[4];                                            // r's two halves of 16 keys, i's
+    uint32_t bf[4], af[4];                                     // r's two halves of 16 keys, i's
     rg_ldsm(bf, w + k);
-#pragma unroll
-    for (int m = 0; m < MT; ++m) {
-      uint32_t af[4];
-      rg_ldsm(af, u + m * 16 * ldw + k);
-      rg_mma(acc[0][m], af, bf[0], bf[1]);
-      rg_mma(acc[1][m], af, bf[2], bf[3]);
-    }
+    rg_ldsm(af, u + k);
+    rg_mma(acc[0], af, bf[0], bf[1]);
+    rg_mma(acc[1], af, bf[2], bf[3]);
   }
 }
 __device__ __forceinline__ void rg_fetch_weights(__nv_bfloat16* W, const RglruArgs& a, int z, int c0, int cols, int bw) {
@@ -559,14 +553,14 @@ __global__ void __launch_bounds__(320) rglru_step_kernel(RglruArgs a, int bw, in
   asm volatile("cp.async.wait_all;" ::: "memory");
   __syncthreads();
   cluster_arrive();                                            // the old inputs have been read
-  float acc[2][1][4];
-  rg_products<1>(acc, W, U, cols, n0, bw, lane);
+  float acc[2][4];
+  rg_products(acc, W, U, cols, n0, bw, lane);
 #pragma unroll
   for (int h = 0; h < 2; ++h)
     if (g + 8 * h < n) {
       const uint32_t uu = *reinterpret_cast<const uint32_t*>(U + (g + 8 * h) * ldw + c0 + n0 + 2 * t4);
       f2 av, bv;
-      rg_coefficients(add2(pk(acc[0][0][2 * h], acc[0][0][2 * h + 1]), br), add2(pk(acc[1][0][2 * h], acc[1][0][2 * h + 1]), bi), pk(bf_lo(uu), bf_hi(uu)), rate, av, bv);
+      rg_coefficients(add2(pk(acc[0][2 * h], acc[0][2 * h + 1]), br), add2(pk(acc[1][2 * h], acc[1][2 * h + 1]), bi), pk(bf_lo(uu), bf_hi(uu)), rate, av, bv);
       const f2 s = fma2(av, S[h], bv);
       rg_keep<2>(slot[h] + ch, s);
       rg_store<2>((E*)a.out + (int64_t)(t0 + g + 8 * h) * a.width + ch, mul2(s, gelu_tanh2(y[h])));

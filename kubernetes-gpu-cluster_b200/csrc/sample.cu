@@ -12,7 +12,7 @@
 // 1 us each: the start's and the last exchange's for greedy rows, a third for the maximum where a token is drawn, three more for a threshold,
 // two for a second one that finds its keys counted); the one read of V * 2 bytes is about 2 us.
 // 32 rows x 128256 normal logits (spread 2.5) on a B200, us, before (intervals of keys cut in eight or four by a pass over the elements
-// and a cluster exchange each, 6 to 12 of them; every kept element's logarithm) and now: greedy 6.8 / 5.9, top-k 20 with top-p 0.8
+// and a cluster exchange each, 6 to 12 of them; every kept element's logarithm) and now: greedy 6.8 / 4.8, top-k 20 with top-p 0.8
 // 42.1 / 22.4, top-p 0.95 59.3 / 25.4, unfiltered 36.4 / 32.2, those in turn 51.2 / 23.9; one row of 32000, top-p 19.3 / 11.8; 150
 // rows of 2049, top-k and top-p 31.5 / 17.5.
 #include <type_traits>
