@@ -187,7 +187,7 @@ def test_short_biased_pieces(kge, tmp_path, hd):
     (5, 128, 256, [150, 70, 10, 3]),                                # no room for a second block
     (4, 128, 256, [300, 20]),                                       # norm and gate by a warp a row, a piece a lane
     (4, 16, 128, [200, 200, 200]),                                  # 48 clusters: of two, since 45 of three fit
-    (2, 128, 264, [700, 2]), (2, 4, 520, [650]), (9, 32, 40, [135]),      # (other sums; norm and gate by a warp a row: two and four pieces a lane, less than one)
+    (2, 128, 264, [700, 2]), (2, 4, 520, [650]), (9, 32, 40, [135]), (9, 32, 40, [860]),      # (other sums; norm and gate by a warp a row: two and four pieces a lane, less than one)
 ])
 def test_matrix_memory_prompts_in_runs_of_chunks(kge, tmp_path, heads, dim, vdim, lens):
     """A request's chunks shared out over the blocks of a cluster: all requests in one step, first without a state, then on from it, and the

@@ -912,6 +912,43 @@ def test_sample_thresholds_wherever_they_lie(kge, L, shape, V, dtype):
             check_draws(got, lg.float(), V, temp, k, pp, noise)
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("V,ld", [(1, 1), (9, 16), (4096, 4096), (4099, 4101), (50272, 50272), (128256, 128264), (800003, 800003)])
+def test_sample_greedy_rows(kge, L, V, ld, dtype):
+    """The first of the largest, NaN left out, the two zeros equal: ties inside a piece of eight, between threads, warps and CTAs, at the ends of the
+    row, rows of infinities and of NaN alone; one to eight CTAs a row, staged and read again, aligned and not; beside drawn rows in the same launch."""
+    g = torch.Generator().manual_seed(V)
+    nan, inf = float("nan"), float("inf")
+    x = (torch.randn(12, ld, generator=g) * 3 - 40).to(dtype)
+    x[:, V:] = 100                                                                   # behind the row
+    at = sorted({0, V // 3, V // 3 + 1, V // 3 + 8, V // 2, V - 1} & set(range(V)))
+    x[1, at] = 5.0
+    x[2, at[1:]] = 5.0
+    x[3, V - 1] = 5.0
+    x[4, at] = 0.0; x[4, at[0]] = -0.0                                               # zeros are the largest: the first, whatever its sign
+    x[5, at] = -0.0; x[5, at[-1]] = 0.0
+    x[6, at] = inf
+    x[7] = -inf; x[7, V:] = 100
+    x[8, at] = nan; x[8, V // 4] = 7.0 if V // 4 not in at else nan
+    x[9, :V] = nan
+    x[10, :V] = nan; x[10, V // 2] = -inf
+    temp = torch.zeros(12); temp[11] = 0.9                                           # (row 11 is drawn)
+    td, kd, ppd, sd = dev(temp), dev(torch.zeros(12, dtype=torch.int32)), dev(torch.ones(12)), dev(torch.arange(12))
+    fn = L.kge_sample_f16 if dtype == torch.float16 else L.kge_sample
+    out, xd = torch.full((12,), -1, dtype=torch.int32, device="cuda"), dev(x)
+    sync()
+    check_ok(kge, fn(p(out), p(xd), 12, V, ld, p(td), p(kd), p(ppd), None, p(sd), 0, None, 0, None), "sample")
+    sync()
+    got = out.cpu().tolist()
+    row = torch.where(torch.isnan(x[:, :V]), torch.full((), -inf, dtype=torch.float64), x[:, :V].double()) + 0.0
+    for b in range(11):
+        number = ~torch.isnan(x[b, :V])
+        best = row[b][number].max() if number.any() else None
+        want = 0 if best is None else int(((row[b] == best) & number).nonzero()[0])
+        assert got[b] == want, (b, got[b], want)
+    assert 0 <= got[11] < V
+
+
 def test_sample_a_draw_whose_noise_is_none(kge, L):
     """A seed whose uniform number at index 2 is 1 exactly: its noise is -0 and its score the lowest there is, below the bound under
     which elements are left out, so the draw is repeated without that bound."""
